@@ -28,6 +28,7 @@
 #include <mutex>
 #include <sstream>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/oeq_b200.h"
@@ -220,6 +221,9 @@ struct Mapping {
     int epi = 1;                              // edges per staged item (uvu_kernels.cuh, EPI)
     int stage_cap = 4;                        // most stages a group takes
     int chunk_floor = 32;                     // smallest chunk of consecutive edges a launch may deal out
+    int slice_warps = 0, n_slice = 1;         // slice kernels (uvu_slice_kernels.cuh): warps per CTA (0: not one of them)
+    bool slice_full = false;
+    int slice_stages = 2, slice_smem = 0, slice_regs = 0;
     int threads() const { return ng * mulg * ps + 32 * ng * producer + 32 * helper_warps; }
     int fixed_bytes(int stages) const { return ng * stages * (16 + 8 * (epi > 1 ? 4 + 2 * epi : 4)) + ng * 128 + sw_bytes; }
     int smem(int stages) const { return fixed_bytes(stages) + ng * (stages * stage_bytes + extra_bytes); }
@@ -660,6 +664,65 @@ bool uvu_tc_geometry(const Problem& p, UvuTcGeometry& g, int npad = 0) {
     return true;
 }
 
+// Tables of the slice kernels: the paths grouped by their two input irreps (first-input major), and the
+// Clebsch-Gordan entries of a group ordered by (i, j), so that a product x_i y_j is formed once for all its paths.
+void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m) {
+    struct Entry { int i, j, path, k; double v; };
+    std::vector<int> ga, gb, ge = {0}, gp = {0}, plist, toff(p.instr.size(), 0), ei, ej, et, enew, efirst;
+    std::vector<double> ev;
+    int tmax = 1;
+    for (size_t a = 0; a < p.in1.size(); ++a)
+        for (size_t b = 0; b < p.in2.size(); ++b) {
+            std::vector<Entry> es;
+            int t = 0;
+            for (size_t q = 0; q < p.instr.size(); ++q) {
+                const Instr& ins = p.instr[q];
+                if (ins.i1 != (int)a || ins.i2 != (int)b) continue;
+                plist.push_back((int)q);
+                toff[q] = t;
+                t += p.out[ins.io].dim;
+                for (size_t z = 0; z < ins.cv.size(); ++z) es.push_back({ins.ci[z], ins.cj[z], (int)q, ins.ck[z], ins.cv[z]});
+            }
+            if (t == 0) continue;
+            tmax = std::max(tmax, t);
+            std::stable_sort(es.begin(), es.end(), [](const Entry& x, const Entry& y) {
+                return std::make_tuple(x.i, x.j, x.path, x.k) < std::make_tuple(y.i, y.j, y.path, y.k);
+            });
+            std::vector<int> seen(t, 0);
+            for (size_t n = 0; n < es.size(); ++n) {
+                const int tt = toff[es[n].path] + es[n].k;
+                ei.push_back(es[n].i); ej.push_back(es[n].j); et.push_back(tt); ev.push_back(es[n].v);
+                enew.push_back(n == 0 || es[n].i != es[n - 1].i || es[n].j != es[n - 1].j);
+                efirst.push_back(!seen[tt]);
+                seen[tt] = 1;
+            }
+            ga.push_back((int)a); gb.push_back((int)b);
+            ge.push_back((int)ei.size()); gp.push_back((int)plist.size());
+        }
+    auto put_int = [](std::ostringstream& o, int v) { o << v; };
+    s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages
+      << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ";\n";
+    s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ";\n";
+    emit_array(s, "int", "GRP_A", ga, put_int);
+    emit_array(s, "int", "GRP_B", gb, put_int);
+    emit_array(s, "int", "GRP_E", ge, put_int);
+    emit_array(s, "int", "GRP_P", gp, put_int);
+    emit_array(s, "int", "P_LIST", plist, put_int);
+    emit_array(s, "int", "T_OFF", toff, put_int);
+    emit_array(s, "int", "E_I", ei, put_int);
+    emit_array(s, "int", "E_J", ej, put_int);
+    emit_array(s, "int", "E_T", et, put_int);
+    emit_array(s, "bool", "E_NEW", enew, put_int);
+    emit_array(s, "bool", "E_FIRST", efirst, put_int);
+    const bool f64 = p.dtype == OEQ_F64;
+    emit_array(s, "T", "E_V", ev, [f64](std::ostringstream& o, double v) {
+        char buf[64];
+        if (f64) snprintf(buf, sizeof buf, "%a", v);
+        else snprintf(buf, sizeof buf, "%af", (double)(float)v);
+        o << buf;
+    });
+}
+
 std::string descriptor_text(const Problem& p, const Mapping& m, const UvwConfig* uvw = nullptr) {
     std::ostringstream s;
     s.precision(17);
@@ -764,6 +827,7 @@ std::string descriptor_text(const Problem& p, const Mapping& m, const UvwConfig*
         }
         s << "};\n";
     }
+    if (m.slice_warps) emit_slice_tables(s, p, m);
     if (uvw)
         s << "constexpr int TILE_R = " << uvw->tile_r << ", UVC = " << uvw->uvc << ", DMAX = " << uvw->dmax
           << ", MWMAX = " << uvw->mwmax << ", UVW_THREADS = " << uvw->threads << ";\n";
@@ -872,7 +936,7 @@ struct Kernel {
     int stages = 0, smem = 0, regs = 0, ctas_per_sm = 1, sm_count = 0;
     bool is_uvu_tc = false;       // tensor-core forward of the convolution: one CTA per SM
     UvuTcGeometry tc_geo;
-    int threads() const { return is_uvu_tc ? 128 * map.ps + 64 : map.threads(); }
+    int threads() const { return map.slice_warps ? 32 * map.slice_warps : (is_uvu_tc ? 128 * map.ps + 64 : map.threads()); }
 };
 
 int build_uvu(const Problem& p, int kind, Kernel& k) {
@@ -1016,6 +1080,110 @@ int build_uvu_dblc(const Problem& p, bool deterministic, bool grads, Kernel& k) 
     k.compiled = true;
     return OEQ_OK;
 }
+
+// ---- slice kernels (uvu_slice_kernels.cuh): one warp per (edges, slice of 32 channels)
+constexpr int K_SLICE_FWD_DET = 50, K_SLICE_FWD_ATOMIC = 51, K_SLICE_BWD_DET = 52, K_SLICE_BWD_ATOMIC = 53;
+
+// A row is one slice of up to 32 channels, or every multiplicity is the same multiple of 32.
+bool slice_shape(const Problem& p, Mapping& m) {
+    if (p.mode != OEQ_MODE_UVU || p.shared || p.y_dim > 32) return false;
+    for (const Irrep& r : p.in2)
+        if (r.mul != 1) return false;
+    int lo = 1 << 30, hi = 0;
+    for (const Irrep& r : p.in1) { lo = std::min(lo, r.mul); hi = std::max(hi, r.mul); }
+    for (const Irrep& r : p.out) { lo = std::min(lo, r.mul); hi = std::max(hi, r.mul); }
+    if (hi > 256 || hi < 1) return false;
+    m.slice_full = lo == hi && hi % 32 == 0;
+    if (hi > 32 && !m.slice_full) return false;
+    m.n_slice = m.slice_full ? hi / 32 : 1;
+    return env_int("OEQ_B200_SLICE", 1) != 0;
+}
+
+// Warps per SM by the registers a thread needs (65 536 over the warps, in steps of the warps that share a
+// scheduler), stages by shared memory.
+bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_bytes) {
+    const int e = p.elem();
+    int xch = 0;
+    for (const Irrep& r : p.in1) xch += r.dim;
+    const int xs = pad16((m.slice_full ? 32 * xch : p.x_dim) * e);
+    const int ws = p.unit ? 0 : pad16((m.slice_full ? 32 * (int)p.instr.size() : p.w_numel) * e);
+    const int stage = 16 + pad16(2 * p.y_dim * e) + 2 * xs + 2 * ws;
+    if (regs > 256) return false;
+    m.slice_regs = regs;
+    const int target = env_int("OEQ_B200_SLICE_WARPS_SM", regs <= 124 ? 16 : (regs <= 164 ? 12 : 8));
+    m.slice_warps = m.n_slice * std::max(1, 4 / m.n_slice);
+    if (m.slice_warps > 8) m.slice_warps = m.n_slice;
+    for (int ctas = std::max(1, target / m.slice_warps); ctas >= 1; --ctas)
+        for (int st = env_int("OEQ_B200_SLICE_STAGES", 3); st >= 2; --st) {
+            const int smem = m.slice_warps * (st * stage + warp_bytes) + cta_bytes;
+            if (smem <= SMEM_LIMIT && ctas * (smem + 1024) <= SMEM_LIMIT + 1024) {
+                m.min_ctas = ctas;
+                m.slice_stages = st;
+                m.slice_smem = smem;
+                return true;
+            }
+        }
+    return false;
+}
+
+int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
+    Mapping& m = k.map;
+    if (!slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
+    int zpc = 0, d1 = 1, tmax = 1, d3 = 1;
+    for (const Irrep& r : p.out) { zpc += r.dim; d3 = std::max(d3, r.dim); }
+    for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
+    for (size_t a = 0; a < p.in1.size(); ++a)
+        for (size_t b = 0; b < p.in2.size(); ++b) {
+            int t = 0;
+            for (const Instr& i : p.instr)
+                if (i.i1 == (int)a && i.i2 == (int)b) t += p.out[i.io].dim;
+            tmax = std::max(tmax, t);
+        }
+    const int w = p.elem() / 4;
+    const int regs = zpc * w + 2 * (p.y_dim + d1 + tmax) + 24;
+    if (!slice_fit(p, m, regs, pad16(32 * d3 * p.elem()), 0)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+    m.mulg = 32;
+    m.z_ph_begin = {0, p.z_dim};
+    m.w_ph_begin = {0, p.w_numel};
+    m.phase_of_instr.assign(p.instr.size(), 0);
+    assign_partitions(p, false, m);
+    int rc = compile_kernel(descriptor_text(p, m), "uvu_slice_kernels.cuh", deterministic ? K_SLICE_FWD_DET : K_SLICE_FWD_ATOMIC, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
+int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
+    Mapping& m = k.map;
+    if (!env_int("OEQ_B200_BWD_RECV", 1) || !slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
+    int zpc = 0, d1 = 1, d2 = 1;
+    for (const Irrep& r : p.out) zpc += r.dim;
+    for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
+    for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
+    const int e = p.elem(), w = e / 4, per = 3 - w;         // registers of a value, edges computed together
+    const int regs = w * (zpc + per * (2 * p.y_dim + 3 * d1 + d2)) + 12;
+    int pitch = 8;
+    while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
+    if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;
+    const int groups = m.n_slice >= 4 ? 1 : 4 / m.n_slice;
+    const int dyg = m.n_slice > 1 ? 2 * m.n_slice * pitch * e : 0;
+    if (!slice_fit(p, m, regs, 32 * pitch * e, groups * dyg)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+    m.mulg = 32;
+    m.z_ph_begin = {0, p.z_dim};
+    m.w_ph_begin = {0, p.w_numel};
+    m.phase_of_instr.assign(p.instr.size(), 0);
+    assign_partitions(p, true, m);
+    int rc = compile_kernel(descriptor_text(p, m), "uvu_slice_kernels.cuh", deterministic ? K_SLICE_BWD_DET : K_SLICE_BWD_ATOMIC, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
+// Where a thread of the backward slice kernel needs more than 200 registers (two warps per scheduler) and the edges
+// fill the machine, the receiver-order group kernel with its staging warps is the faster one: MACE-large, 600 k edges
+// 5.1 against 5.6 ms atomic, but at 15 k edges 178 against 152 us.
+bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || slice.map.slice_regs > 200; }
+constexpr long long RECV_MIN_EDGES = 65536;
 
 constexpr int K_FWD_DET_TC = 30, K_FWD_ATOMIC_TC = 31;
 
@@ -1224,9 +1392,10 @@ int load_kernel(Kernel& k, const char* entry, bool want_reduce) {
     OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
     int stages = std::min(k.map.max_stages(), env_int("OEQ_B200_STAGES", 4));
     if (k.is_uvu_tc) stages = k.tc_geo.stages;
+    if (k.map.slice_warps) stages = k.map.slice_stages;
     if (stages < 2) return fail(OEQ_ERR_UNSUPPORTED, "not enough shared memory for two stages");
     k.stages = stages;
-    k.smem = k.is_uvu_tc ? k.tc_geo.smem : k.map.smem(stages);
+    k.smem = k.map.slice_warps ? k.map.slice_smem : (k.is_uvu_tc ? k.tc_geo.smem : k.map.smem(stages));
     OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
     cudaFuncAttributes attr;
     if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
@@ -1301,6 +1470,38 @@ int launch_uvu(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream,
     return OEQ_OK;
 }
 
+// Edges per chunk and CTAs of a slice kernel.  Node rows that fit in L2 are gathered from there whatever the order:
+// each walker then takes one run of the edge list (at least 8 edges), which needs its ends aligned once.  Larger graphs
+// are dealt in chunks of 128 edges, so that the walkers stay in one neighbourhood of the list.
+void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes, long long& grid, int& chunk) {
+    const int per_cta = k.map.slice_warps / k.map.n_slice;
+    const long long most = (long long)k.sm_count * k.ctas_per_sm;
+    const long long walkers = most * per_cta;
+    chunk = env_int("OEQ_B200_CHUNK", 0);
+    if (chunk <= 0) {
+        chunk = 128;
+        if (gathered_bytes <= (48u << 20) || edges < walkers * 512) chunk = (int)std::max<long long>(8, (edges + walkers - 1) / walkers);
+    }
+    const long long chunks = (edges + chunk - 1) / chunk;
+    grid = std::max<long long>(1, std::min(most, (chunks + per_cta - 1) / per_cta));
+}
+
+int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream) {
+    const int e = p.elem();
+    const bool full = k.map.slice_full;
+    int flags = 0;
+    if ((full || (p.x_dim * e) % 16 == 0) && aligned16(prm.X)) flags |= 1;
+    if ((full || (p.w_numel * e) % 16 == 0) && aligned16(prm.W)) flags |= 4;
+    // rows out: Z by output irrep; dX, or the scratch rows (16-byte aligned with the same pitch)
+    if (prm.dX ? ((full || (p.x_dim * e) % 16 == 0) && aligned16(prm.ws ? prm.ws : prm.dX)) : aligned16(prm.Z)) flags |= 8;
+    prm.flags = flags;
+    long long grid = 1;
+    slice_launch_shape(k, prm.n_items, (size_t)prm.n_nodes * p.x_dim * e, grid, prm.chunk);
+    void* args[] = {&prm};
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)k.threads()), args, (size_t)k.smem, stream));
+    return OEQ_OK;
+}
+
 long long uvu_grid(const Kernel& k, long long n_items) {
     long long want = (n_items + k.map.ng - 1) / k.map.ng;
     return std::max<long long>(1, std::min<long long>((long long)k.sm_count * k.ctas_per_sm, want));
@@ -1335,6 +1536,8 @@ struct oeq_conv {
     Kernel fwd, bwd;
     Kernel fwd_tc;              // tensor-core forward pass, when the problem qualifies
     bool has_fwd_tc = false;
+    Kernel fwd_slice, bwd_slice;    // slice kernels, for the problems that have their shape
+    bool has_fwd_slice = false, has_bwd_slice = false;
     Kernel bwd_recv;            // receiver-order backward pass (needs scratch in the deterministic variant)
     bool has_bwd_recv = false;
     cudaKernel_t sum_rows_fn = nullptr, clear_fn = nullptr;
@@ -1407,17 +1610,16 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
     UvuTcGeometry geo;
     const bool tc = (kinds & 6) && uvu_tc_geometry(p, geo);
     const bool recv = (kinds & 6) && recv_backward_supported(p);
-    if (kinds & 2) {
-        if ((rc = one(K_FWD_DET)) || (rc = one(K_BWD_DET))) return rc;
-        Kernel k, kr;
-        if (tc && (rc = build_uvu_tc(p, true, k))) return rc;
-        if (recv && (rc = build_uvu_recv(p, true, kr))) return rc;
-    }
-    if (kinds & 4) {
-        if ((rc = one(K_FWD_ATOMIC)) || (rc = one(K_BWD_ATOMIC))) return rc;
-        Kernel k, kr;
-        if (tc && (rc = build_uvu_tc(p, false, k))) return rc;
-        if (recv && (rc = build_uvu_recv(p, false, kr))) return rc;
+    for (int det = 1; det >= 0; --det) {
+        if (!(kinds & (det ? 2 : 4))) continue;
+        Kernel f, b, k, kr;
+        const int rf = build_slice_fwd(p, det != 0, f), rb = build_slice_bwd(p, det != 0, b);
+        if (rf && rf != OEQ_ERR_UNSUPPORTED) return rf;
+        if (rb && rb != OEQ_ERR_UNSUPPORTED) return rb;
+        if (rf && (rc = one(det ? K_FWD_DET : K_FWD_ATOMIC))) return rc;
+        if ((rc = one(det ? K_BWD_DET : K_BWD_ATOMIC))) return rc;
+        if (tc && (rc = build_uvu_tc(p, det != 0, k))) return rc;
+        if (recv && recv_beside_slice(!rb, b) && (rc = build_uvu_recv(p, det != 0, kr))) return rc;
     }
     if ((kinds & 8) && (kinds & 6) && conv_double_backward_supported(p)) {
         for (int det = 0; det < 2; ++det) {
@@ -1850,14 +2052,22 @@ int oeq_conv_create(const oeq_problem_desc* desc, int deterministic, oeq_conv** 
     h->deterministic = deterministic != 0;
     int rc = ingest(desc, h->prob);
     if (!rc) rc = check_conv_problem(h->prob);
-    if (!rc) rc = build_uvu(h->prob, deterministic ? K_FWD_DET : K_FWD_ATOMIC, h->fwd);
+    // what the problem's launches use: slice kernels where it has their shape (the group kernels behind them are then
+    // only for lists beyond 32-bit counts, specialised on demand, and the receiver-order group kernel for wide rows)
+    auto optional = [&](int rc2, bool& has) {
+        has = rc2 == OEQ_OK;
+        if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
+    };
+    if (!rc) optional(build_slice_fwd(h->prob, h->deterministic, h->fwd_slice), h->has_fwd_slice);
+    if (!rc && !h->has_fwd_slice) rc = build_uvu(h->prob, deterministic ? K_FWD_DET : K_FWD_ATOMIC, h->fwd);
     if (!rc) rc = build_uvu(h->prob, deterministic ? K_BWD_DET : K_BWD_ATOMIC, h->bwd);
     UvuTcGeometry geo;
     if (!rc && uvu_tc_geometry(h->prob, geo)) {
         rc = build_uvu_tc(h->prob, h->deterministic, h->fwd_tc);
         h->has_fwd_tc = !rc;
     }
-    if (!rc && recv_backward_supported(h->prob)) {
+    if (!rc) optional(build_slice_bwd(h->prob, h->deterministic, h->bwd_slice), h->has_bwd_slice);
+    if (!rc && recv_beside_slice(h->has_bwd_slice, h->bwd_slice) && recv_backward_supported(h->prob)) {
         rc = build_uvu_recv(h->prob, h->deterministic, h->bwd_recv);
         h->has_bwd_recv = !rc;
     }
@@ -1875,6 +2085,8 @@ int oeq_conv_destroy(oeq_conv* h) {
     if (h->fwd.lib) cudaLibraryUnload(h->fwd.lib);
     if (h->bwd.lib) cudaLibraryUnload(h->bwd.lib);
     if (h->fwd_tc.lib) cudaLibraryUnload(h->fwd_tc.lib);
+    if (h->fwd_slice.lib) cudaLibraryUnload(h->fwd_slice.lib);
+    if (h->bwd_slice.lib) cudaLibraryUnload(h->bwd_slice.lib);
     if (h->bwd_recv.lib) cudaLibraryUnload(h->bwd_recv.lib);
     if (h->dbl_z.lib) cudaLibraryUnload(h->dbl_z.lib);
     if (h->dbl_g.lib) cudaLibraryUnload(h->dbl_g.lib);
@@ -1892,7 +2104,7 @@ size_t oeq_conv_workspace_bytes(const oeq_conv* h, int64_t nodes, int64_t edges)
     // Forward: none (the segmented reduction is node-aligned: no scratch, no fix-up pass).  Deterministic
     // backward: one dX row per edge, capped (the pass then runs over blocks of edges); optional -- without
     // it the sender-order kernel runs.
-    if (!h || !h->deterministic || !h->has_bwd_recv || edges <= 0) return 0;
+    if (!h || !h->deterministic || !(h->has_bwd_recv || h->has_bwd_slice) || edges <= 0) return 0;
     const size_t cap = (size_t)std::max(1, env_int("OEQ_B200_BWD_SCRATCH_MB", 8192)) << 20;
     return std::min((size_t)edges * recv_row_bytes(h->prob), cap);
 }
@@ -1914,6 +2126,17 @@ int oeq_conv_forward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, c
     // the tensor-core kernel stages rows with bulk copies only: it needs 16-byte aligned X and W
     const bool tc = h->has_fwd_tc && aligned16(X) && aligned16(W) && !env_int("OEQ_B200_NO_BULK", 0);
     int rc = ensure_status(&h->d_status);
+    // (the slice kernels count nodes and edges in 32 bits)
+    if (!rc && !tc && h->has_fwd_slice && edges < (1ll << 31) - 4096 && nodes < (1ll << 31) - 4096) {
+        if ((rc = load_kernel(h->fwd_slice, "oeq_uvu_kernel", false))) return rc;
+        UvuParams prm{};
+        prm.X = X; prm.Y = Y; prm.W = W; prm.Z = Z;
+        prm.rows = (const long long*)rows; prm.cols = (const long long*)cols;
+        prm.n_items = edges; prm.n_nodes = nodes; prm.status = h->d_status;
+        h->last_stream = st;
+        return launch_slice(h->fwd_slice, p, prm, st);
+    }
+    if (!rc && !tc && !h->fwd.compiled) rc = build_uvu(p, h->deterministic ? K_FWD_DET : K_FWD_ATOMIC, h->fwd);
     if (!rc) rc = tc ? load_kernel(h->fwd_tc, "oeq_uvu_tc_kernel", false) : load_kernel(h->fwd, "oeq_uvu_kernel", false);
     if (rc) return rc;
     UvuParams prm{};
@@ -1968,7 +2191,10 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
     // caller's scratch holds the rows of a useful block of edges
     const size_t row = recv_row_bytes(p);
     long long block_edges = 0;
-    if (h->has_bwd_recv) {
+    // (slice kernels count edges and nodes in 32 bits)
+    const bool sliced = h->has_bwd_slice && edges < (1ll << 31) - 4096 && nodes < (1ll << 31) - 4096 &&
+                        !(h->has_bwd_recv && edges >= RECV_MIN_EDGES);
+    if (h->has_bwd_recv || sliced) {
         if (!h->deterministic) block_edges = edges;
         else if (workspace && aligned16(workspace)) {
             block_edges = (long long)std::min<size_t>(workspace_bytes / row, (size_t)edges);
@@ -1976,7 +2202,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         }
     }
     if (block_edges > 0) {
-        Kernel& k = h->bwd_recv;
+        Kernel& k = sliced ? h->bwd_slice : h->bwd_recv;
         if (!k.loaded) {
             if ((rc = load_kernel(k, "oeq_uvu_kernel", false))) return rc;
             if (h->deterministic) {
@@ -1988,7 +2214,13 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         char* dYb = (char*)dY; char* dWb = (char*)dW;
         h->last_bwd_launches = 0;
         const int dx_bulk = ((p.x_dim * e) % 16 == 0 && aligned16(dX)) ? 32 : 0;
-        const int sum_chunk = std::max(1, env_int("OEQ_B200_SUM_CHUNK", 64));
+        auto launch = [&](UvuParams& prm) { return sliced ? launch_slice(k, p, prm, st) : launch_uvu(k, p, prm, st, dx_bulk); };
+        // sender runs per warp of the row sum: 64 edges, fewer when the edges would leave warps idle
+        int sum_chunk = env_int("OEQ_B200_SUM_CHUNK", 0);
+        if (sum_chunk <= 0) {
+            sum_chunk = 64;
+            while (sum_chunk > 8 && edges < (long long)sum_chunk * k.sm_count * 48) sum_chunk /= 2;
+        }
         auto pass1 = [&](long long e0, long long n, void* scratch, UvuParams& prm) {
             prm.X = X; prm.dZ = dZ; prm.dX = dX;
             prm.Y = Yb + (size_t)e0 * p.y_dim * e; prm.W = Wb + (size_t)e0 * p.w_numel * e;
@@ -2000,7 +2232,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         if (!h->deterministic) {
             UvuParams prm{};
             pass1(0, edges, nullptr, prm);
-            if ((rc = launch_uvu(k, p, prm, st, dx_bulk))) return rc;
+            if ((rc = launch(prm))) return rc;
             h->last_bwd_launches = 1;
             return OEQ_OK;
         }
@@ -2056,7 +2288,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
                         prm.sum_items = edges; prm.sum_e_lo = prev_e0; prm.sum_e_hi = prev_e0 + prev_n;
                         prm.sum_first = b == 1; prm.sum_chunk = sum_chunk;
                     }
-                    if ((rc = launch_uvu(k, p, prm, st, dx_bulk))) return rc;
+                    if ((rc = launch(prm))) return rc;
                     ++h->last_bwd_launches;
                     prev_e0 = e0; prev_n = n;
                 }
@@ -2068,7 +2300,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
             const long long n = std::min(block_edges, edges - e0);
             UvuParams prm{};
             pass1(e0, n, workspace, prm);
-            if ((rc = launch_uvu(k, p, prm, st, dx_bulk))) return rc;
+            if ((rc = launch(prm))) return rc;
             ++h->last_bwd_launches;
             if ((rc = sum_launch(e0, n, workspace, first))) return rc;
             first = false;
@@ -2240,8 +2472,9 @@ int oeq_conv_check(oeq_conv* h) { return h ? check_status(h->d_status, h->last_s
 
 int oeq_conv_launch_info(const oeq_conv* h, int which, int* threads, int* ng, int* ps, int* stages, int* smem, int* regs) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
-    if (which) return launch_info(h->has_bwd_recv && h->bwd_recv.loaded ? h->bwd_recv : h->bwd, threads, ng, ps, stages, smem, regs);
-    return launch_info(h->has_fwd_tc && h->fwd_tc.loaded ? h->fwd_tc : h->fwd, threads, ng, ps, stages, smem, regs);
+    const Kernel& k = which ? (h->bwd_slice.loaded ? h->bwd_slice : h->bwd_recv.loaded ? h->bwd_recv : h->bwd)
+                            : (h->fwd_tc.loaded ? h->fwd_tc : h->has_fwd_slice ? h->fwd_slice : h->fwd);
+    return launch_info(k, threads, ng, ps, stages, smem, regs);
 }
 
 }  // extern "C"

@@ -2121,7 +2121,10 @@ extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, 
     out[i] = s;
 }
 
-#if OEQ_KERNEL == OEQ_K_BWD_RECV_DET || OEQ_KERNEL == OEQ_K_DBLC_G_DET || OEQ_KERNEL == OEQ_K_DBLC_G_ATOMIC
+#endif  // OEQ_UVU_NO_ENTRY
+
+#define OEQ_K_SLICE_BWD_DET 52      // (uvu_slice_kernels.cuh)
+#if OEQ_KERNEL == OEQ_K_BWD_RECV_DET || OEQ_KERNEL == OEQ_K_DBLC_G_DET || OEQ_KERNEL == OEQ_K_DBLC_G_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_BWD_DET
 // Clears `bytes` bytes (a multiple of 4) at a 4-byte aligned address.  A kernel rather than a memset call: a
 // memset may be served by a copy engine, where it would queue behind host transfers that other streams have
 // in flight and stall the stream that runs the backward pass.
@@ -2147,4 +2150,3 @@ extern "C" __global__ void __launch_bounds__(256) oeq_sum_sender_rows(const oeq:
                          (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31);
 }
 #endif
-#endif  // OEQ_UVU_NO_ENTRY
