@@ -105,6 +105,47 @@ def lib():
     return _lib
 
 
+_torch_lib = None
+_registered = []    # handles of the registered ops: an op can be called as long as the process lives
+
+
+def register_ops(forward, gradient, handle, *, deterministic=False, shared=False, has_weights=True, f64=False, dims=(),
+                 second=None):
+    """Register the torch ops ``openequivariance_b200::<forward>`` and ``::<gradient>`` of one operator (native kernels
+    and autograd, ``csrc/oeq_torch.cpp``) and return their overloads.  ``dims``: x, y, z row lengths and the number of
+    weights; ``second``: an op already registered for the second derivatives."""
+    global _torch_lib
+    import torch
+    lib()
+    with _lock:
+        if _torch_lib is None:
+            from .build import build_torch_library
+            t = C.CDLL(build_torch_library())
+            t.oeq_torch_error.restype = C.c_char_p
+            t.oeq_torch_register.argtypes = [C.c_char_p] * 3 + [_P, _P] + [_INT] * 4 + [_I64] * 4
+            _torch_lib = t
+    is_conv = isinstance(handle, ConvHandle)
+    code = _torch_lib.oeq_torch_register(forward.encode(), gradient.encode(), second.encode() if second else None,
+                                         None if is_conv else handle.ptr, handle.ptr if is_conv else None,
+                                         int(deterministic), int(shared), int(has_weights), int(f64), *dims)
+    if code:
+        raise RuntimeError("registering torch ops failed: " + _torch_lib.oeq_torch_error().decode(errors="replace"))
+    _registered.append(handle)
+    ns = torch.ops.openequivariance_b200
+    ops = getattr(ns, forward).default, getattr(ns, gradient).default
+    z_dim = dims[2]
+
+    @torch.library.register_fake(f"openequivariance_b200::{forward}")
+    def _(L1_in, *args):
+        return L1_in.new_empty(L1_in.shape[0], z_dim)
+
+    @torch.library.register_fake(f"openequivariance_b200::{gradient}")
+    def _(*args):
+        return [t.new_empty(*t.shape) for t in args[:3 if has_weights else 2]]
+
+    return ops
+
+
 def check(code: int):
     if code != OEQ_OK:
         raise OeqError(code, lib().oeq_last_error().decode(errors="replace"))

@@ -28,7 +28,6 @@ for edge lists that are not structurally symmetric.
 """
 
 import itertools
-import typing
 
 import numpy as np
 import torch
@@ -285,87 +284,23 @@ class TensorProductConv(TensorProductBase):
     # ------------------------------------------------------------------ torch ops
 
     def setup_torch_module(self):
-        conv = self
-        T = torch.Tensor
+        conv, cfg = self, self.config
+        index = "Tensor rows, Tensor cols" + (", Tensor transpose_perm" if self.deterministic else "")
+        second = f"conv_second{self.conv_id}"
+        torch.library.define(f"openequivariance_b200::{second}",
+                             "(Tensor x, Tensor y, Tensor w, Tensor dz, Tensor ex, Tensor ey, Tensor ew, "
+                             f"{index}) -> Tensor[]")
 
-        if not self.deterministic:
-            @torch.library.custom_op(f"openequivariance_b200::conv_forward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def forward(L1_in: T, L2_in: T, weights: T, rows: T, cols: T) -> T:
-                return conv._forward_impl(L1_in, L2_in, weights, rows, cols)
+        @torch.library.impl(f"openequivariance_b200::{second}", "CUDA")
+        def _(*args):
+            # empty where the library has no fused second derivatives here: the caller composes them
+            fused = conv._double_backward_impl(*args) if conv._has_fused_double_backward() else None
+            return [] if fused is None else list(fused)
 
-            @forward.register_fake
-            def _(L1_in, L2_in, weights, rows, cols):
-                return L1_in.new_empty(L1_in.shape[0], conv.L3.dim)
-
-            @torch.library.custom_op(f"openequivariance_b200::conv_backward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def backward_helper(L1_in: T, L2_in: T, weights: T, L3_grad: T, rows: T,
-                                cols: T) -> typing.List[T]:
-                return list(conv._backward_impl(L1_in, L2_in, weights, L3_grad, rows, cols))
-
-            @backward_helper.register_fake
-            def _(L1_in, L2_in, weights, L3_grad, rows, cols):
-                return [L1_in.new_empty(*L1_in.shape), L2_in.new_empty(*L2_in.shape),
-                        weights.new_empty(*weights.shape)]
-            n_index = 2
-        else:
-            @torch.library.custom_op(f"openequivariance_b200::conv_forward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def forward(L1_in: T, L2_in: T, weights: T, rows: T, cols: T, transpose_perm: T) -> T:
-                return conv._forward_impl(L1_in, L2_in, weights, rows, cols, transpose_perm)
-
-            @forward.register_fake
-            def _(L1_in, L2_in, weights, rows, cols, transpose_perm):
-                return L1_in.new_empty(L1_in.shape[0], conv.L3.dim)
-
-            @torch.library.custom_op(f"openequivariance_b200::conv_backward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def backward_helper(L1_in: T, L2_in: T, weights: T, L3_grad: T, rows: T, cols: T,
-                                transpose_perm: T) -> typing.List[T]:
-                return list(conv._backward_impl(L1_in, L2_in, weights, L3_grad, rows, cols, transpose_perm))
-
-            @backward_helper.register_fake
-            def _(L1_in, L2_in, weights, L3_grad, rows, cols, transpose_perm):
-                return [L1_in.new_empty(*L1_in.shape), L2_in.new_empty(*L2_in.shape),
-                        weights.new_empty(*weights.shape)]
-            n_index = 3
-
-        nones = (None,) * n_index
-
-        def setup_context(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in, ctx.weights = inputs[:3]
-            ctx.index = inputs[3:]
-
-        def backward(ctx, grad_output):
-            gx, gy, gw = backward_helper(ctx.L1_in, ctx.L2_in, ctx.weights, grad_output, *ctx.index)
-            return (gx, gy, gw) + nones
-
-        forward.register_autograd(backward, setup_context=setup_context)
-
-        def setup_context_double_backward(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in, ctx.weights, ctx.L3_grad = inputs[:4]
-            ctx.index = inputs[4:]
-
-        def double_backward(ctx, grad_output):
-            # same trilinear identity as the batch product, with the graph held fixed
-            x, y, w, dz, idx = ctx.L1_in, ctx.L2_in, ctx.weights, ctx.L3_grad, ctx.index
-            ex, ey, ew = grad_output[0], grad_output[1], grad_output[2]
-            if not torch.is_grad_enabled() and conv._has_fused_double_backward():
-                # nothing differentiates through this result: two launches that stage an edge's rows once each
-                fused = conv._double_backward_impl(x, y, w, dz, ex, ey, ew, *idx)
-                if fused is not None:
-                    return tuple(fused) + nones
-            a = backward_helper(ex, ey, w, dz, *idx)
-            b = backward_helper(x, y, ew, dz, *idx)
-            c = backward_helper(ex, y, w, dz, *idx)
-            d = backward_helper(x, ey, w, dz, *idx)
-            gz = forward(ex, y, w, *idx) + forward(x, ey, w, *idx) + forward(x, y, ew, *idx)
-            return (a[0] + b[0], a[1] + b[1], c[2] + d[2], gz) + nones
-
-        backward_helper.register_autograd(double_backward, setup_context=setup_context_double_backward)
-        self.forward = forward
-        self.backward_helper = backward_helper
+        self.forward, self.backward_helper = _native.register_ops(
+            f"conv_forward{self.conv_id}", f"conv_backward{self.conv_id}", self.internal,
+            deterministic=self.deterministic, f64=self.irrep_dtype == np.float64,
+            dims=(self.L1.dim, self.L2.dim, self.L3.dim, cfg.weight_numel), second=second)
 
     # ------------------------------------------------------------------ host-array entry points
 
@@ -399,99 +334,10 @@ class _UnitWeightConv:
         self.L1, self.L2, self.L3 = problem.irreps_in1, problem.irreps_in2, problem.irreps_out
         self.conv_id = next(_conv_ids)
         self.internal = _native.ConvHandle(problem, deterministic, unit_weights=True)
-        self._scratch = None
-        self._setup_ops()
-
-    def _forward_impl(self, x, y, rows, cols, perm=None):
-        _require_cuda(x, y, rows, cols)
-        x, y, rows, cols = x.contiguous(), y.contiguous(), rows.contiguous(), cols.contiguous()
-        z = torch.empty((x.shape[0], self.L3.dim), dtype=x.dtype, device=x.device)
-        with torch.cuda.device(x.device):
-            self.internal.forward(x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), 0, rows.data_ptr(),
-                                  cols.data_ptr(), z.data_ptr(), 0, 0, torch.cuda.current_stream().cuda_stream)
-        return z
-
-    def _backward_impl(self, x, y, dz, rows, cols, perm=None):
-        _require_cuda(x, y, dz, rows, cols)
-        if self.deterministic and perm is None:
-            raise ValueError("the deterministic convolution needs sender_perm")
-        x, y, dz, rows, cols = x.contiguous(), y.contiguous(), dz.contiguous(), rows.contiguous(), cols.contiguous()
-        perm_ptr = perm.contiguous().data_ptr() if (perm is not None and self.deterministic) else 0
-        dx, dy = torch.empty_like(x), torch.empty_like(y)
-        with torch.cuda.device(x.device):
-            ws_ptr = ws_bytes = 0
-            want = self.internal.workspace_bytes(x.shape[0], rows.shape[0]) if self.deterministic else 0
-            if want:
-                if self._scratch is None or self._scratch.numel() < want or self._scratch.device != x.device:
-                    self._scratch = torch.empty(want, dtype=torch.uint8, device=x.device)
-                ws_ptr, ws_bytes = self._scratch.data_ptr(), self._scratch.numel()
-            self.internal.backward(x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), 0, dz.data_ptr(),
-                                   rows.data_ptr(), cols.data_ptr(), perm_ptr, dx.data_ptr(), dy.data_ptr(), 0,
-                                   ws_ptr, ws_bytes, torch.cuda.current_stream().cuda_stream)
-        return dx, dy
-
-    def _setup_ops(self):
-        conv = self
-        T = torch.Tensor
-        if self.deterministic:
-            @torch.library.custom_op(f"openequivariance_b200::conv_edge_sum{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def forward(L1_in: T, L2_in: T, rows: T, cols: T, transpose_perm: T) -> T:
-                return conv._forward_impl(L1_in, L2_in, rows, cols, transpose_perm)
-
-            @torch.library.custom_op(f"openequivariance_b200::conv_edge_sum_backward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def backward_helper(L1_in: T, L2_in: T, L3_grad: T, rows: T, cols: T,
-                                transpose_perm: T) -> typing.List[T]:
-                return list(conv._backward_impl(L1_in, L2_in, L3_grad, rows, cols, transpose_perm))
-            n_index = 3
-        else:
-            @torch.library.custom_op(f"openequivariance_b200::conv_edge_sum{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def forward(L1_in: T, L2_in: T, rows: T, cols: T) -> T:
-                return conv._forward_impl(L1_in, L2_in, rows, cols)
-
-            @torch.library.custom_op(f"openequivariance_b200::conv_edge_sum_backward{self.conv_id}", mutates_args=(),
-                                     device_types="cuda")
-            def backward_helper(L1_in: T, L2_in: T, L3_grad: T, rows: T, cols: T) -> typing.List[T]:
-                return list(conv._backward_impl(L1_in, L2_in, L3_grad, rows, cols))
-            n_index = 2
-
-        @forward.register_fake
-        def _(L1_in, L2_in, *index):
-            return L1_in.new_empty(L1_in.shape[0], conv.L3.dim)
-
-        @backward_helper.register_fake
-        def _(L1_in, L2_in, L3_grad, *index):
-            return [L1_in.new_empty(*L1_in.shape), L2_in.new_empty(*L2_in.shape)]
-
-        nones = (None,) * n_index
-
-        def setup_context(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in = inputs[:2]
-            ctx.index = inputs[2:]
-
-        def backward(ctx, grad_output):
-            gx, gy = backward_helper(ctx.L1_in, ctx.L2_in, grad_output, *ctx.index)
-            return (gx, gy) + nones
-
-        forward.register_autograd(backward, setup_context=setup_context)
-
-        def setup_context_double_backward(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in, ctx.L3_grad = inputs[:3]
-            ctx.index = inputs[3:]
-
-        def double_backward(ctx, grad_output):
-            # S is bilinear in (X, Y): d<ex,dX>+<ey,dY> / dX = dX(ey, dS), / dY = dY(ex, dS), / dS = S(ex, y) + S(x, ey)
-            x, y, ds, idx = ctx.L1_in, ctx.L2_in, ctx.L3_grad, ctx.index
-            ex, ey = grad_output[0], grad_output[1]
-            a = backward_helper(ex, ey, ds, *idx)
-            gs = forward(ex, y, *idx) + forward(x, ey, *idx)
-            return (a[0], a[1], gs) + nones
-
-        backward_helper.register_autograd(double_backward, setup_context=setup_context_double_backward)
-        self.forward = forward
-        self.backward_helper = backward_helper
+        self.forward, self.backward_helper = _native.register_ops(
+            f"conv_edge_sum{self.conv_id}", f"conv_edge_sum_backward{self.conv_id}", self.internal,
+            deterministic=deterministic, has_weights=False, f64=problem.irrep_dtype == np.float64,
+            dims=(self.L1.dim, self.L2.dim, self.L3.dim, 0))
 
 
 LoopUnrollConv = TensorProductConv

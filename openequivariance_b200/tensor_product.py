@@ -24,7 +24,6 @@ reference).
 """
 
 import itertools
-import typing
 
 import numpy as np
 import torch
@@ -168,59 +167,10 @@ class TensorProduct(TensorProductBase):
     # ------------------------------------------------------------------ torch ops
 
     def setup_torch_custom_op(self):
-        tp = self
-
-        @torch.library.custom_op(f"openequivariance_b200::tp_forward{self.tp_id}", mutates_args=(),
-                                 device_types="cuda")
-        def forward(L1_in: torch.Tensor, L2_in: torch.Tensor, weights: torch.Tensor) -> torch.Tensor:
-            return tp._forward_impl(L1_in, L2_in, weights)
-
-        @forward.register_fake
-        def _(L1_in, L2_in, weights):
-            return L1_in.new_empty(L1_in.shape[0], tp.L3.dim)
-
-        @torch.library.custom_op(f"openequivariance_b200::tp_grad_helper{self.tp_id}", mutates_args=(),
-                                 device_types="cuda")
-        def backward_helper(L1_in: torch.Tensor, L2_in: torch.Tensor, weights: torch.Tensor,
-                            L3_grad: torch.Tensor) -> typing.List[torch.Tensor]:
-            return list(tp._backward_impl(L1_in, L2_in, weights, L3_grad))
-
-        @backward_helper.register_fake
-        def _(L1_in, L2_in, weights, L3_grad):
-            return [L1_in.new_empty(*L1_in.shape), L2_in.new_empty(*L2_in.shape),
-                    weights.new_empty(*weights.shape)]
-
-        def setup_context(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in, ctx.weights = inputs
-
-        def backward(ctx, grad_output):
-            gx, gy, gw = backward_helper(ctx.L1_in, ctx.L2_in, ctx.weights, grad_output)
-            return gx, gy, gw
-
-        forward.register_autograd(backward, setup_context=setup_context)
-
-        def setup_context_double_backward(ctx, inputs, output):
-            ctx.L1_in, ctx.L2_in, ctx.weights, ctx.L3_grad = inputs
-
-        def double_backward(ctx, grad_output):
-            # The product is trilinear in (x, y, w).  With cotangents (ex, ey, ew) of (dX, dY, dW):
-            #   d/d(dz) = f(ex, y, w) + f(x, ey, w) + f(x, y, ew)
-            #   d/dx    = dX(ey, w, dz) + dX(y, ew, dz)     and likewise for y and w.
-            x, y, w, dz = ctx.L1_in, ctx.L2_in, ctx.weights, ctx.L3_grad
-            ex, ey, ew = grad_output[0], grad_output[1], grad_output[2]
-            if tp._has_fused_double_backward and not torch.is_grad_enabled():
-                # nothing differentiates through this result: one launch that reads the row's arrays once
-                return tp._double_backward_impl(x, y, w, dz, ex, ey, ew)
-            a = backward_helper(ex, ey, w, dz)   # dX(ey, w), dY(ex, w)
-            b = backward_helper(x, y, ew, dz)    # dX(y, ew), dY(x, ew)
-            c = backward_helper(ex, y, w, dz)    # dW(ex, y)
-            d = backward_helper(x, ey, w, dz)    # dW(x, ey)
-            gz = forward(ex, y, w) + forward(x, ey, w) + forward(x, y, ew)
-            return a[0] + b[0], a[1] + b[1], c[2] + d[2], gz
-
-        backward_helper.register_autograd(double_backward, setup_context=setup_context_double_backward)
-        self.forward = forward
-        self.backward_helper = backward_helper
+        cfg = self.config
+        self.forward, self.backward_helper = _native.register_ops(
+            f"tp_forward{self.tp_id}", f"tp_grad_helper{self.tp_id}", self.internal, shared=cfg.shared_weights,
+            f64=self.irrep_dtype == np.float64, dims=(self.L1.dim, self.L2.dim, self.L3.dim, cfg.weight_numel))
 
     # ------------------------------------------------------------------ host-array entry points
 
