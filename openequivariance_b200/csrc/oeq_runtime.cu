@@ -865,7 +865,7 @@ int compile_kernel(const std::string& descriptor, const std::string& main_header
     std::string common, body;
     if (!read_file(dir + "/oeq_common.cuh", common) || !read_file(dir + "/" + main_header, body))
         return fail(OEQ_ERR_COMPILE, "kernel headers not found in " + dir);
-    for (const char* inc : {"tc_common.cuh", "uvu_kernels.cuh"}) {   // headers that the kernel files include
+    for (const char* inc : {"tc_common.cuh", "uvu_kernels.cuh", "uvw_kernels.cuh"}) {   // headers that the kernel files include
         std::string text;
         if (main_header != inc && read_file(dir + "/" + inc, text)) common += text;
     }
@@ -928,7 +928,7 @@ int compile_kernel(const std::string& descriptor, const std::string& main_header
 struct Kernel {
     Mapping map;
     UvwConfig uvw;
-    bool is_uvw = false;
+    bool is_uvw = false, is_uvw_row = false;
     Compiled code;
     bool compiled = false, loaded = false;
     cudaLibrary_t lib = nullptr;
@@ -1101,13 +1101,13 @@ bool slice_shape(const Problem& p, Mapping& m) {
 
 // Warps per SM by the registers a thread needs (65 536 over the warps, in steps of the warps that share a
 // scheduler), stages by shared memory.
-bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_bytes) {
+bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_bytes, bool second = false) {
     const int e = p.elem();
     int xch = 0;
     for (const Irrep& r : p.in1) xch += r.dim;
     const int xs = pad16((m.slice_full ? 32 * xch : p.x_dim) * e);
     const int ws = p.unit ? 0 : pad16((m.slice_full ? 32 * (int)p.instr.size() : p.w_numel) * e);
-    const int stage = 16 + pad16(2 * p.y_dim * e) + 2 * xs + 2 * ws;
+    const int stage = 16 + (second ? 2 : 1) * (pad16(2 * p.y_dim * e) + 2 * xs + 2 * ws);     // (rows and cotangent rows)
     if (regs > 256) return false;
     m.slice_regs = regs;
     const int target = env_int("OEQ_B200_SLICE_WARPS_SM", regs <= 124 ? 16 : (regs <= 164 ? 12 : 8));
@@ -1179,11 +1179,61 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     return OEQ_OK;
 }
 
+// Second derivatives of the convolution in slices: the gradient with respect to dZ (forward walk), or those with
+// respect to X, Y, W (backward walk).
+constexpr int K_SLICE_DBL_Z_DET = 54, K_SLICE_DBL_Z_ATOMIC = 55, K_SLICE_DBL_G_DET = 56, K_SLICE_DBL_G_ATOMIC = 57;
+
+int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k) {
+    Mapping& m = k.map;
+    if (p.unit || !slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
+    int zpc = 0, d1 = 1, d2 = 1, d3 = 1;
+    for (const Irrep& r : p.out) { zpc += r.dim; d3 = std::max(d3, r.dim); }
+    for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
+    for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
+    const int e = p.elem(), w = e / 4, per = 3 - w;
+    const int regs = w * (zpc + per * (grads ? 2 * p.y_dim + 6 * d1 + d2 : 2 * p.y_dim + 4 * d1 + 2)) + 12;
+    int pitch = 8;
+    while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
+    if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;
+    const int groups = m.n_slice >= 4 ? 1 : 4 / m.n_slice;
+    const int dyg = m.n_slice > 1 ? 2 * m.n_slice * pitch * e : 0;
+    if (!slice_fit(p, m, regs, grads ? 32 * pitch * e : pad16(32 * d3 * e), grads ? groups * dyg : 0, true))
+        return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+    m.mulg = 32;
+    m.z_ph_begin = {0, p.z_dim};
+    m.w_ph_begin = {0, p.w_numel};
+    m.phase_of_instr.assign(p.instr.size(), 0);
+    assign_partitions(p, grads, m);
+    const int kind = grads ? (deterministic ? K_SLICE_DBL_G_DET : K_SLICE_DBL_G_ATOMIC) : (deterministic ? K_SLICE_DBL_Z_DET : K_SLICE_DBL_Z_ATOMIC);
+    int rc = compile_kernel(descriptor_text(p, m), "uvu_slice_kernels.cuh", kind, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
 // Where a thread of the backward slice kernel needs more than 200 registers (two warps per scheduler) and the edges
 // fill the machine, the receiver-order group kernel with its staging warps is the faster one: MACE-large, 600 k edges
 // 5.1 against 5.6 ms atomic, but at 15 k edges 178 against 152 us.
 bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || slice.map.slice_regs > 200; }
 constexpr long long RECV_MIN_EDGES = 65536;
+
+// Problems for which fused second derivatives may exist (whether they fit is known once they are built).
+bool conv_second_possible(const Problem& p) {
+    Mapping m;
+    return !p.unit && env_int("OEQ_B200_FUSED_DOUBLE_BACKWARD", 1) != 0 && (conv_double_backward_supported(p) || slice_shape(p, m));
+}
+
+// Both second-derivative kernels of a convolution: slice kernels, or the group kernels where a row does not fit them.
+int build_conv_dbl(const Problem& p, bool deterministic, Kernel& z, Kernel& g) {
+    int rc = build_slice_dbl(p, deterministic, false, z);
+    if (!rc) rc = build_slice_dbl(p, deterministic, true, g);
+    if (rc != OEQ_ERR_UNSUPPORTED) return rc;
+    z = Kernel();
+    g = Kernel();
+    if (!conv_double_backward_supported(p)) return rc;
+    rc = build_uvu_dblc(p, deterministic, false, z);
+    return rc ? rc : build_uvu_dblc(p, deterministic, true, g);
+}
 
 constexpr int K_FWD_DET_TC = 30, K_FWD_ATOMIC_TC = 31;
 
@@ -1338,7 +1388,42 @@ int build_uvw_tc_bwd(const Problem& p, int kernel_id, Kernel& k) {
     return OEQ_OK;
 }
 
+// One row per CTA for 'uvw' with per-row weights (uvw_row_kernels.cuh): T of a row (and dT) in shared memory, eight
+// input channels of a path in registers.  Rows that take more keep the tiled kernel.
+constexpr int K_UVW_ROW_FWD = 12, K_UVW_ROW_BWD = 13, UVW_ROW_WARPS = 8;
+
+int uvw_row_smem(const Problem& p, bool bwd) {
+    auto r4 = [](long long n) { return (n + 3) / 4 * 4; };
+    long long t = 0;
+    for (const Instr& i : p.instr) t += (long long)p.in1[i.i1].mul * p.in2[i.i2].mul * p.out[i.io].dim;
+    const long long e = r4(p.x_dim) + r4(p.y_dim) + r4(p.z_dim) + r4(t) * (bwd ? 2 : 1) + (bwd ? UVW_ROW_WARPS * p.y_dim : 0);
+    return (int)std::min<long long>(e * p.elem(), 1ll << 30);
+}
+
+bool uvw_row_supported(const Problem& p) {
+    if (p.mode != OEQ_MODE_UVW || p.shared) return false;
+    for (const Irrep& r : p.out)
+        if (r.dim * 8 * (p.elem() / 4) > 128) return false;
+    return uvw_row_smem(p, true) <= 100 * 1024;
+}
+
+int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
+    k.is_uvw = k.is_uvw_row = true;
+    k.uvw.tile_r = 1;       // (the tiled kernel's bodies are not compiled)
+    k.uvw.threads = 32 * UVW_ROW_WARPS;
+    k.map.part_of_out.assign(p.out.size(), 0);
+    k.map.part_of_instr.assign(p.instr.size(), 0);
+    k.map.zr_off.assign(p.out.size(), 0);
+    k.map.xr_off.assign(p.in1.size(), 0);
+    const std::string rows = "namespace oeqd { constexpr int ROW_WARPS = " + std::to_string(UVW_ROW_WARPS) + "; }\n";
+    int rc = compile_kernel(descriptor_text(p, k.map, &k.uvw) + rows, "uvw_row_kernels.cuh", bwd ? K_UVW_ROW_BWD : K_UVW_ROW_FWD, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
 int build_tp(const Problem& p, bool bwd, Kernel& k) {
+    if (uvw_row_supported(p)) return build_uvw_row(p, bwd, k);
     if (p.mode == OEQ_MODE_UVW) return build_uvw(p, bwd ? K_UVW_BWD : K_UVW_FWD, k);
     return build_uvu(p, bwd ? K_BWD_BATCH : K_FWD_BATCH, k);
 }
@@ -1346,12 +1431,12 @@ int build_tp(const Problem& p, bool bwd, Kernel& k) {
 int load_uvw(Kernel& k, const Problem& p, bool bwd) {
     if (k.loaded) return OEQ_OK;
     OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_kernel"));
-    OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, "oeq_reduce_partials"));
+    OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, k.is_uvw_row ? "oeq_uvw_row_kernel" : "oeq_uvw_kernel"));
+    if (!k.is_uvw_row) OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, "oeq_reduce_partials"));
     int dev = 0;
     OEQ_CUDA(cudaGetDevice(&dev));
     OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
-    k.smem = k.uvw.smem(p, bwd);
+    k.smem = k.is_uvw_row ? uvw_row_smem(p, bwd) : k.uvw.smem(p, bwd);
     OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
     cudaFuncAttributes attr;
     if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
@@ -1361,7 +1446,7 @@ int load_uvw(Kernel& k, const Problem& p, bool bwd) {
         (void)cudaGetLastError();
         occ = 1;
     }
-    k.ctas_per_sm = std::max(1, std::min(occ, 2));
+    k.ctas_per_sm = std::max(1, k.is_uvw_row ? occ : std::min(occ, 2));
     k.map.ng = 1;
     k.loaded = true;
     return OEQ_OK;
@@ -1462,6 +1547,8 @@ int launch_uvu(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream,
         chunk = 128;
         const long long groups = grid * k.map.ng;
         while (chunk > k.map.chunk_floor && prm.n_items / (groups * chunk) < 8) chunk /= 2;
+        // a short list: smaller chunks while groups would be left without one
+        while (chunk > 8 && prm.n_items < groups * chunk) chunk /= 2;
     }
     prm.chunk = std::max(1, chunk);
     void* args[] = {&prm};
@@ -1486,7 +1573,16 @@ void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes,
     grid = std::max<long long>(1, std::min(most, (chunks + per_cta - 1) / per_cta));
 }
 
-int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream) {
+// Edges per chunk of the row sum: 64, fewer when that would leave warps idle.
+int row_sum_chunk(const Kernel& k, long long edges) {
+    int chunk = env_int("OEQ_B200_SUM_CHUNK", 0);
+    if (chunk > 0) return chunk;
+    chunk = 64;
+    while (chunk > 8 && edges < (long long)chunk * k.sm_count * 48) chunk /= 2;
+    return chunk;
+}
+
+int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream, int clear_flags = 0) {
     const int e = p.elem();
     const bool full = k.map.slice_full;
     int flags = 0;
@@ -1494,7 +1590,7 @@ int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t strea
     if ((full || (p.w_numel * e) % 16 == 0) && aligned16(prm.W)) flags |= 4;
     // rows out: Z by output irrep; dX, or the scratch rows (16-byte aligned with the same pitch)
     if (prm.dX ? ((full || (p.x_dim * e) % 16 == 0) && aligned16(prm.ws ? prm.ws : prm.dX)) : aligned16(prm.Z)) flags |= 8;
-    prm.flags = flags;
+    prm.flags = flags & ~clear_flags;
     long long grid = 1;
     slice_launch_shape(k, prm.n_items, (size_t)prm.n_nodes * p.x_dim * e, grid, prm.chunk);
     void* args[] = {&prm};
@@ -1621,14 +1717,12 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if (tc && (rc = build_uvu_tc(p, det != 0, k))) return rc;
         if (recv && recv_beside_slice(!rb, b) && (rc = build_uvu_recv(p, det != 0, kr))) return rc;
     }
-    if ((kinds & 8) && (kinds & 6) && conv_double_backward_supported(p)) {
+    if ((kinds & 8) && (kinds & 6) && conv_second_possible(p)) {
         for (int det = 0; det < 2; ++det) {
             if (!(kinds & (det ? 2 : 4))) continue;
-            for (int grads = 0; grads < 2; ++grads) {
-                Kernel k;
-                rc = build_uvu_dblc(p, det != 0, grads != 0, k);
-                if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
-            }
+            Kernel z, g;
+            rc = build_conv_dbl(p, det != 0, z, g);
+            if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
         }
     }
     return OEQ_OK;
@@ -2215,12 +2309,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         h->last_bwd_launches = 0;
         const int dx_bulk = ((p.x_dim * e) % 16 == 0 && aligned16(dX)) ? 32 : 0;
         auto launch = [&](UvuParams& prm) { return sliced ? launch_slice(k, p, prm, st) : launch_uvu(k, p, prm, st, dx_bulk); };
-        // sender runs per warp of the row sum: 64 edges, fewer when the edges would leave warps idle
-        int sum_chunk = env_int("OEQ_B200_SUM_CHUNK", 0);
-        if (sum_chunk <= 0) {
-            sum_chunk = 64;
-            while (sum_chunk > 8 && edges < (long long)sum_chunk * k.sm_count * 48) sum_chunk /= 2;
-        }
+        const int sum_chunk = row_sum_chunk(k, edges);
         auto pass1 = [&](long long e0, long long n, void* scratch, UvuParams& prm) {
             prm.X = X; prm.dZ = dZ; prm.dX = dX;
             prm.Y = Yb + (size_t)e0 * p.y_dim * e; prm.W = Wb + (size_t)e0 * p.w_numel * e;
@@ -2236,22 +2325,12 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
             h->last_bwd_launches = 1;
             return OEQ_OK;
         }
-        // rows of nodes that send nothing are never written by the row sum (cleared by a kernel: a memset call
-        // may land on a copy engine behind the caller's host transfers)
-        {
-            unsigned long long words = (unsigned long long)nodes * p.x_dim * e / 4;
-            void* ptr = dX;
-            void* args[] = {&ptr, &words};
-            const unsigned grid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((unsigned long long)k.sm_count * 8, (words / 4 + 255) / 256));
-            OEQ_CUDA(cudaLaunchKernel((const void*)h->clear_fn, dim3(grid), dim3(256), args, 0, st));
-            ++h->last_bwd_launches;
-        }
         auto sum_launch = [&](long long e0, long long n, void* scratch, bool first) -> int {
             UvuParams sp{};
             sp.dX = dX; sp.ws = scratch;
             sp.rows = (const long long*)rows; sp.cols = (const long long*)cols; sp.perm = (const long long*)perm;
             sp.n_items = edges; sp.n_nodes = nodes; sp.status = h->d_status;
-            sp.flags = first ? 64 : 0;
+            sp.flags = (first ? 64 : 0) | (n == edges ? 128 : 0);
             sp.chunk = sum_chunk;
             sp.e_lo = e0; sp.e_hi = e0 + n;
             const long long chunks = (edges + sp.chunk - 1) / sp.chunk;
@@ -2270,6 +2349,16 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         const size_t min_block_bytes = (size_t)std::max(1, env_int("OEQ_B200_PIPELINE_BLOCK_MB", 1024)) << 20;
         const long long min_block = std::max<long long>(recv_min_block_edges(), (long long)(min_block_bytes / row));
         const bool pipelined = k.map.helper_warps > 0 && edges >= 4 * min_block;
+        // several blocks: rows of nodes that send nothing are never written by the row sum (cleared by a kernel: a
+        // memset call may land on a copy engine behind the caller's host transfers)
+        if (pipelined || block_edges < edges) {
+            unsigned long long words = (unsigned long long)nodes * p.x_dim * e / 4;
+            void* ptr = dX;
+            void* args[] = {&ptr, &words};
+            const unsigned grid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((unsigned long long)k.sm_count * 8, (words / 4 + 255) / 256));
+            OEQ_CUDA(cudaLaunchKernel((const void*)h->clear_fn, dim3(grid), dim3(256), args, 0, st));
+            ++h->last_bwd_launches;
+        }
         if (pipelined) {
             const long long half = (long long)(workspace_bytes / row / 2);
             long long be = std::min<long long>(half, (edges + 3) / 4);
@@ -2336,7 +2425,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
 // ---------------------------------------------------------------- second derivatives of the convolution
 
 int oeq_conv_has_double_backward(const oeq_conv* h) {
-    return h && h->dbl_state >= 0 && conv_double_backward_supported(h->prob) ? 1 : 0;
+    return h && h->dbl_state >= 0 && conv_second_possible(h->prob) ? 1 : 0;
 }
 
 int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, const void* Y, const void* W,
@@ -2369,8 +2458,7 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
     int rc = ensure_status(&h->d_status);
     if (rc) return rc;
     if (h->dbl_state == 0) {
-        rc = build_uvu_dblc(p, h->deterministic, false, h->dbl_z);
-        if (!rc) rc = build_uvu_dblc(p, h->deterministic, true, h->dbl_g);
+        rc = build_conv_dbl(p, h->deterministic, h->dbl_z, h->dbl_g);
         if (!rc) rc = load_kernel(h->dbl_z, "oeq_uvu_kernel", false);
         if (!rc) rc = load_kernel(h->dbl_g, "oeq_uvu_kernel", false);
         if (!rc) {
@@ -2380,6 +2468,9 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
         h->dbl_state = rc ? -1 : 1;
         if (rc) return rc;
     }
+    const bool sliced = h->dbl_g.map.slice_warps > 0;
+    if (sliced && (edges >= (1ll << 31) - 4096 || nodes >= (1ll << 31) - 4096))
+        return fail(OEQ_ERR_UNSUPPORTED, "fused second derivatives count nodes and edges in 32 bits");
     h->last_stream = st;
     // bulk copies of a kind of row only when the row and its cotangent row both qualify
     int clear = 0;
@@ -2393,11 +2484,12 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
         prm.X = X; prm.Y = Y; prm.W = W; prm.Z = GdZ; prm.EX = EX; prm.EY = EY; prm.EW = EW;
         prm.rows = (const long long*)rows; prm.cols = (const long long*)cols;
         prm.n_items = edges; prm.n_nodes = nodes; prm.status = h->d_status;
-        if ((rc = launch_uvu(h->dbl_z, p, prm, st, 0, 0, nullptr, clear))) return rc;
+        rc = sliced ? launch_slice(h->dbl_z, p, prm, st, clear) : launch_uvu(h->dbl_z, p, prm, st, 0, 0, nullptr, clear);
+        if (rc) return rc;
     }
     // gradients with respect to X, Y, W: the receiver-order walk, GX through scratch rows or bulk reductions
     Kernel& k = h->dbl_g;
-    {
+    if (!h->deterministic || block_edges < edges) {     // (one row sum over the whole list writes every row itself)
         unsigned long long words = (unsigned long long)nodes * p.x_dim * e / 4;
         void* ptr = GX;
         void* args[] = {&ptr, &words};
@@ -2405,7 +2497,7 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
         OEQ_CUDA(cudaLaunchKernel((const void*)h->dbl_clear_fn, dim3(grid), dim3(256), args, 0, st));
     }
     const int dx_bulk = ((p.x_dim * e) % 16 == 0 && aligned16(GX)) ? 32 : 0;
-    const int sum_chunk = std::max(1, env_int("OEQ_B200_SUM_CHUNK", 64));
+    const int sum_chunk = row_sum_chunk(k, edges);
     bool first = true;
     for (long long e0 = 0; e0 < edges; e0 += block_edges) {
         const long long n = std::min(block_edges, edges - e0);
@@ -2418,13 +2510,14 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
         prm.rows = (const long long*)rows + e0; prm.cols = (const long long*)cols + e0;
         prm.n_items = n; prm.n_nodes = nodes; prm.status = h->d_status;
         prm.ws = h->deterministic ? workspace : nullptr;
-        if ((rc = launch_uvu(k, p, prm, st, dx_bulk, 0, nullptr, clear))) return rc;
+        rc = sliced ? launch_slice(k, p, prm, st, clear) : launch_uvu(k, p, prm, st, dx_bulk, 0, nullptr, clear);
+        if (rc) return rc;
         if (h->deterministic) {
             UvuParams sp{};
             sp.dX = GX; sp.ws = workspace;
             sp.rows = (const long long*)rows; sp.cols = (const long long*)cols; sp.perm = (const long long*)perm;
             sp.n_items = edges; sp.n_nodes = nodes; sp.status = h->d_status;
-            sp.flags = first ? 64 : 0;
+            sp.flags = (first ? 64 : 0) | (n == edges ? 128 : 0);
             sp.chunk = sum_chunk;
             sp.e_lo = e0; sp.e_hi = e0 + n;
             const long long chunks = (edges + sp.chunk - 1) / sp.chunk;

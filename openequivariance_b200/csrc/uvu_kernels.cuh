@@ -55,7 +55,7 @@
 namespace oeq {
 using namespace oeqd;
 
-#if defined(OEQ_KERNEL) && OEQ_KERNEL >= 40 && OEQ_KERNEL <= 43
+#if defined(OEQ_KERNEL) && ((OEQ_KERNEL >= 40 && OEQ_KERNEL <= 43) || (OEQ_KERNEL >= 54 && OEQ_KERNEL <= 57))
 constexpr bool DBLC = true;     // stages also carry the cotangents EX (at the sender), EY, EW
 #else
 constexpr bool DBLC = false;
@@ -1656,8 +1656,9 @@ __device__ void run_backward_recv(const UvuParams& p, const Smem<true, MODE, tru
 // the sender-ordered edge list; chunk ends are moved forward to the next sender boundary, so a sender's
 // edges are never split between two warps: every row of dX has one writer and a fixed summation order.
 // 32 positions are examined at a time; positions whose edge lies outside the range cost one coalesced
-// load and a ballot.  `first`: store the rows of the senders met (the host has cleared dX, so nodes that
-// send nothing stay zero); otherwise add.
+// load and a ballot.  `first`: store the rows of the senders met; otherwise add.  `gap_nodes` > 0 (the number of
+// nodes, when the range is the whole list): rows of nodes that send nothing are written as zeros; otherwise the host
+// has cleared dX.
 __device__ __forceinline__ long long align_sender(const long long* cols, const long long* perm, long long n, long long t,
                                                   int lane) {
     if (t <= 0) return 0;
@@ -1674,7 +1675,7 @@ __device__ __forceinline__ long long align_sender(const long long* cols, const l
 
 __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, const long long* __restrict__ cols,
                                 const long long* __restrict__ perm, long long n_items, long long e_lo, long long e_hi,
-                                bool first, int chunk, long long warps, long long wid, int lane) {
+                                bool first, int chunk, long long gap_nodes, long long warps, long long wid, int lane) {
     constexpr int VEC = 16 / ELEM;                                  // elements per 16-byte load
     constexpr int XS = XB / ELEM;
     constexpr int NV = (XS / VEC + 31) / 32;                        // 16-byte pieces per lane
@@ -1697,6 +1698,10 @@ __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, 
         }
 #pragma unroll
         for (int i = 0; i < NV * VEC; ++i) acc[i] = (T)0;
+    };
+    auto zero_nodes = [&](long long lo, long long hi) {
+        for (long long node = lo; node < hi; ++node)
+            for (int i = lane; i < X_DIM; i += 32) dX[node * (long long)X_DIM + i] = (T)0;
     };
     const long long n_chunks = (n_items + chunk - 1) / chunk;
     for (long long c = wid; c < n_chunks; c += warps) {
@@ -1754,15 +1759,22 @@ __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, 
 #pragma unroll
                 for (int q = 0; q < U; ++q) {
                     if (q < n) {
-                        if (prev >= 0 && sj[q] != prev) flush(prev);
-                        prev = sj[q];
+                        if (sj[q] != prev) {
+                            if (prev >= 0) flush(prev);
+                            // (the nodes before a later chunk's first sender belong to the chunk before it)
+                            if (gap_nodes > 0 && (prev >= 0 || c == 0)) zero_nodes(prev + 1, sj[q]);
+                            prev = sj[q];
+                        }
 #pragma unroll
                         for (int i = 0; i < NV * VEC; ++i) acc[i] += val[q][i];
                     }
                 }
             }
         }
-        if (prev >= 0) flush(prev);
+        if (prev >= 0) {
+            flush(prev);
+            if (gap_nodes > 0) zero_nodes(prev + 1, end >= n_items ? gap_nodes : cols[perm[end]]);
+        }
     }
 }
 
@@ -1787,7 +1799,7 @@ __device__ __forceinline__ void uvu_body_recv(const UvuParams& p) {
         if constexpr (HELPER_WARPS > 0) {
             if (p.sum_items > 0)
                 sum_sender_rows(p.sum_ws, p.dX, p.sum_cols, p.sum_perm, p.sum_items, p.sum_e_lo, p.sum_e_hi, p.sum_first != 0,
-                                p.sum_chunk, (long long)gridDim.x * HELPER_WARPS,
+                                p.sum_chunk, 0, (long long)gridDim.x * HELPER_WARPS,
                                 (long long)blockIdx.x * HELPER_WARPS + ((tid - NCONSUMERS - NSTAGING) >> 5), tid & 31);
         }
         return;
@@ -2124,7 +2136,10 @@ extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, 
 #endif  // OEQ_UVU_NO_ENTRY
 
 #define OEQ_K_SLICE_BWD_DET 52      // (uvu_slice_kernels.cuh)
-#if OEQ_KERNEL == OEQ_K_BWD_RECV_DET || OEQ_KERNEL == OEQ_K_DBLC_G_DET || OEQ_KERNEL == OEQ_K_DBLC_G_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_BWD_DET
+#define OEQ_K_SLICE_DBL_G_DET 56
+#define OEQ_K_SLICE_DBL_G_ATOMIC 57
+#if OEQ_KERNEL == OEQ_K_BWD_RECV_DET || OEQ_KERNEL == OEQ_K_DBLC_G_DET || OEQ_KERNEL == OEQ_K_DBLC_G_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_BWD_DET || \
+    OEQ_KERNEL == OEQ_K_SLICE_DBL_G_DET || OEQ_KERNEL == OEQ_K_SLICE_DBL_G_ATOMIC
 // Clears `bytes` bytes (a multiple of 4) at a 4-byte aligned address.  A kernel rather than a memset call: a
 // memset may be served by a copy engine, where it would queue behind host transfers that other streams have
 // in flight and stall the stream that runs the backward pass.
@@ -2146,7 +2161,7 @@ extern "C" __global__ void oeq_clear(unsigned int* ptr, unsigned long long words
 // edges, or every block when the launches carry no helper warps): see sum_sender_rows.
 extern "C" __global__ void __launch_bounds__(256) oeq_sum_sender_rows(const oeq::UvuParams p) {
     oeq::sum_sender_rows(reinterpret_cast<const oeqd::T*>(p.ws), p.dX, p.cols, p.perm, p.n_items, p.e_lo, p.e_hi,
-                         (p.flags & 64) != 0, p.chunk, (long long)gridDim.x * (blockDim.x >> 5),
+                         (p.flags & 64) != 0, p.chunk, (p.flags & 128) ? p.n_nodes : 0, (long long)gridDim.x * (blockDim.x >> 5),
                          (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31);
 }
 #endif

@@ -18,6 +18,8 @@
 #define OEQ_K_SLICE_FWD_DET 50
 #define OEQ_K_SLICE_FWD_ATOMIC 51
 #define OEQ_K_SLICE_BWD_ATOMIC 53
+#define OEQ_K_SLICE_DBL_Z_DET 54
+#define OEQ_K_SLICE_DBL_Z_ATOMIC 55
 
 namespace oeq {
 
@@ -68,9 +70,12 @@ template <int P> __host__ __device__ constexpr int ws_off() { return FULL ? 32 *
 struct SliceStage {
     static constexpr int OFF_HDR = 0;           // first edge, receiver, sender of edge 0, sender of edge 1 (-1: one edge)
     static constexpr int OFF_Y = 16;
-    static constexpr int OFF_X = OFF_Y + YSB;   // two rows
-    static constexpr int OFF_W = OFF_X + 2 * XSB;
-    static constexpr int BYTES = OFF_W + 2 * WSB;
+    static constexpr int OFF_EY = OFF_Y + YSB;  // (second derivatives: the cotangent rows beside the rows)
+    static constexpr int OFF_X = OFF_EY + (DBLC ? YSB : 0);     // two rows
+    static constexpr int OFF_EX = OFF_X + 2 * XSB;
+    static constexpr int OFF_W = OFF_EX + (DBLC ? 2 * XSB : 0);
+    static constexpr int OFF_EW = OFF_W + 2 * WSB;
+    static constexpr int BYTES = OFF_EW + (DBLC ? 2 * WSB : 0);
 };
 constexpr int MAX_OUT_D = []() { int m = 1; for (int o = 0; o < N_OUT; ++o) m = OUT_D[o] > m ? OUT_D[o] : m; return m; }();
 constexpr int SL_FLUSH = pad16(32 * MAX_OUT_D * ELEM);              // transposition buffer of one output irrep
@@ -305,18 +310,27 @@ struct SliceCopies {
         using L = SliceStage;
         const bool two = s1 >= 0;
         if (lane == 0) *reinterpret_cast<int4*>(st + L::OFF_HDR) = make_int4(e0, row, s0, s1);
-        const T* y = p.Y + (long long)e0 * Y_DIM;
-        T* dy = reinterpret_cast<T*>(st + L::OFF_Y);
+        auto y_rows = [&](const T* y, unsigned char* dst) {
+            T* dy = reinterpret_cast<T*>(dst);
 #pragma unroll
-        for (int i = 0; i < (2 * Y_DIM + 31) / 32; ++i) {
-            const int q = lane + 32 * i, h = q >= Y_DIM ? 1 : 0, j = q - h * Y_DIM;
-            if (q < (two ? 2 : 1) * Y_DIM) cp_async_elem<ELEM>(dy + (PK::N == 2 ? 2 * j + h : q), y + q);
-        }
-        x_row(st + L::OFF_X, p.X + (long long)s0 * X_DIM);
-        w_row(st + L::OFF_W, p.W + (long long)e0 * W_NUMEL);
-        if (two) {
-            x_row(st + L::OFF_X + XSB, p.X + (long long)s1 * X_DIM);
-            w_row(st + L::OFF_W + WSB, p.W + (long long)(e0 + 1) * W_NUMEL);
+            for (int i = 0; i < (2 * Y_DIM + 31) / 32; ++i) {
+                const int q = lane + 32 * i, h = q >= Y_DIM ? 1 : 0, j = q - h * Y_DIM;
+                if (q < (two ? 2 : 1) * Y_DIM) cp_async_elem<ELEM>(dy + (PK::N == 2 ? 2 * j + h : q), y + q);
+            }
+        };
+        y_rows(p.Y + (long long)e0 * Y_DIM, st + L::OFF_Y);
+        if constexpr (DBLC) y_rows(p.EY + (long long)e0 * Y_DIM, st + L::OFF_EY);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (q == 0 || two) {
+                const long long s = q ? s1 : s0, e = e0 + q;
+                x_row(st + L::OFF_X + q * XSB, p.X + s * X_DIM);
+                w_row(st + L::OFF_W + q * WSB, p.W + e * W_NUMEL);
+                if constexpr (DBLC) {
+                    x_row(st + L::OFF_EX + q * XSB, p.EX + s * X_DIM);
+                    w_row(st + L::OFF_EW + q * WSB, p.EW + e * W_NUMEL);
+                }
+            }
         }
     }
 };
@@ -354,6 +368,52 @@ template <int O> __host__ __device__ constexpr bool out_vec_ok() {
 //
 // Bound by register reads: an FMA with an immediate reads two registers, one with three register operands three,
 // and a scheduler's two banks deliver two a cycle.
+
+// Second derivatives, gradient with respect to dZ: T(ex, y, w) + T(x, ey, w) + T(x, y, ew) of a pair, as one
+// contraction: with r = w ex + ew x, t_ij = r_i y_j + (w x_i) ey_j and z_k += C_ijk t_ij.
+template <class YA, class ZA>
+__device__ __forceinline__ void slice_second_z(const unsigned char* st, int e, bool two, int lane, const YA& y, ZA& z) {
+    using L = SliceStage;
+    V2 ey[Y_DIM];
+    load_y(st + L::OFF_EY, e, ey);
+    sfor<0, N_IN1>([&](auto a_) {
+        constexpr int a = a_;
+        if constexpr (any_part_uses_in1(a)) {
+            constexpr int D1 = IN1_D[a];
+            const bool live = FULL || lane < IN1_MUL[a];
+            V2 x[D1], ex[D1];
+#pragma unroll
+            for (int i = 0; i < D1; ++i) {
+                x[i] = live ? load_pair(st + L::OFF_X, XSB, xs_off<a>() + lane * D1 + i, e) : PK::all((T)0);
+                ex[i] = live ? load_pair(st + L::OFF_EX, XSB, xs_off<a>() + lane * D1 + i, e) : PK::all((T)0);
+            }
+            sfor<0, N_INSTR>([&](auto p_) {
+                constexpr int P = p_;
+                if constexpr (I_IN1[P] == a) {
+                    constexpr int b = I_IN2[P], R = out_reg_off(I_OUT[P]);
+                    const V2 w = live ? load_pair(st + L::OFF_W, WSB, ws_off<P>() + lane, e) : PK::all((T)0);
+                    const V2 ew = live ? load_pair(st + L::OFF_EW, WSB, ws_off<P>() + lane, e) : PK::all((T)0);
+                    V2 r[D1], wx[D1], t;
+#pragma unroll
+                    for (int i = 0; i < D1; ++i) {
+                        r[i] = PK::fma(w, ex[i], PK::mul(ew, x[i]));
+                        wx[i] = PK::mul(w, x[i]);
+                    }
+                    sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
+                        constexpr int n = n_;
+                        constexpr int J = IN2_OFF[b] + CG_J[n];
+                        if constexpr (cg_pair_first<P, n>()) t = PK::fma(r[CG_I[n]], y[J], PK::mul(wx[CG_I[n]], ey[J]));
+                        T& zk = z[R + CG_K[n]];
+                        zk = fma((T)CG_V[n], PK::get(t, 0), zk);
+                        if constexpr (PK::N == 2) {
+                            if (two) zk = fma((T)CG_V[n], PK::get(t, 1), zk);
+                        }
+                    });
+                }
+            });
+        }
+    });
+}
 
 template <int MODE>
 __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp, int lane) {
@@ -444,9 +504,10 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
         for (int e = 0; e < (PK::N == 2 || !two ? 1 : 2); ++e) {
             V2 y[Y_DIM];
             load_y(st + L::OFF_Y, e, y);
+            if constexpr (DBLC) slice_second_z(st, e, two, lane, y, z);
             sfor<0, N_IN1>([&](auto a_) {
                 constexpr int a = a_;
-                if constexpr (any_part_uses_in1(a)) {
+                if constexpr (any_part_uses_in1(a) && !DBLC) {
                     constexpr int D1 = IN1_D[a];
                     const bool live = FULL || lane < IN1_MUL[a];
                     V2 x[D1];
@@ -597,17 +658,62 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                 constexpr int a = a_;
                 constexpr int D1 = IN1_D[a];
                 const bool live = FULL || lane < IN1_MUL[a];
-                T x[NE][D1], dx[NE][D1];
+                T x[NE][D1], dx[NE][D1], ex[DBLC ? NE : 1][D1];
 #pragma unroll
                 for (int q = 0; q < NE; ++q)
 #pragma unroll
                     for (int i = 0; i < D1; ++i) {
                         x[q][i] = live ? sx[q][xs_off<a>() + lane * D1 + i] : (T)0;
                         dx[q][i] = (T)0;
+                        if constexpr (DBLC) ex[q][i] = live ? sx[q][(L::OFF_EX - L::OFF_X) / ELEM + xs_off<a>() + lane * D1 + i] : (T)0;
                     }
                 sfor<0, N_INSTR>([&](auto p_) {
                     constexpr int P = p_;
-                    if constexpr (I_IN1[P] == a) {
+                    if constexpr (I_IN1[P] == a && DBLC) {
+                        // gx = w A(ey) + ew A(y), gw = <ex, A(y)> + <x, A(ey)>, gy = B(w ex + ew x) with
+                        // A_i(v) = sum_j v_j P_ij, B_j(v) = sum_i v_i P_ij
+                        constexpr int b = I_IN2[P], D2 = IN2_D[b], R = out_reg_off(I_OUT[P]);
+                        T w[NE], ew[NE], r[NE][D1], ay[NE][D1], ae[NE][D1], ey[NE][D2], pij = (T)0;
+#pragma unroll
+                        for (int q = 0; q < NE; ++q) {
+                            w[q] = live ? sw[q][ws_off<P>() + lane] : (T)0;
+                            ew[q] = live ? sw[q][(L::OFF_EW - L::OFF_W) / ELEM + ws_off<P>() + lane] : (T)0;
+                            const T* sey = reinterpret_cast<const T*>(st + L::OFF_EY) + (NE == 2 ? q : e * Y_DIM);
+#pragma unroll
+                            for (int j = 0; j < D2; ++j) ey[q][j] = sey[(IN2_OFF[b] + j) * NE];
+#pragma unroll
+                            for (int i = 0; i < D1; ++i) {
+                                r[q][i] = fma(w[q], ex[q][i], ew[q] * x[q][i]);
+                                ay[q][i] = ae[q][i] = (T)0;
+                            }
+                        }
+                        sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
+                            constexpr int n = n_;
+                            if constexpr (cg_pair_first<P, n>()) pij = (T)CG_V[n] * gz[R + CG_K[n]];
+                            else pij = fma((T)CG_V[n], gz[R + CG_K[n]], pij);
+                            if constexpr (cg_pair_last<P, n>()) {
+#pragma unroll
+                                for (int q = 0; q < NE; ++q) {
+                                    ay[q][CG_I[n]] = fma(y[q][IN2_OFF[b] + CG_J[n]], pij, ay[q][CG_I[n]]);
+                                    ae[q][CG_I[n]] = fma(ey[q][CG_J[n]], pij, ae[q][CG_I[n]]);
+                                    T& d = dy[q][IN2_OFF[b] + CG_J[n]];
+                                    d = fma(r[q][CG_I[n]], pij, d);
+                                }
+                            }
+                        });
+#pragma unroll
+                        for (int q = 0; q < NE; ++q) {
+                            T gw = (T)0;
+#pragma unroll
+                            for (int i = 0; i < D1; ++i) {
+                                gw = fma(ex[q][i], ay[q][i], gw);
+                                gw = fma(x[q][i], ae[q][i], gw);
+                                dx[q][i] = fma(w[q], ae[q][i], dx[q][i]);
+                                dx[q][i] = fma(ew[q], ay[q][i], dx[q][i]);
+                            }
+                            if (live && (q == 0 || two)) __stcs(dw[q] + W_OFF[P] + slice * 32 + lane, gw);
+                        }
+                    } else if constexpr (I_IN1[P] == a) {
                         constexpr int b = I_IN2[P], D2 = IN2_D[b], R = out_reg_off(I_OUT[P]);
                         T av[NE][D1], bv[NE][D2], pij = (T)0;
 #pragma unroll
@@ -624,26 +730,28 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                             if constexpr (cg_pair_last<P, n>()) {
 #pragma unroll
                                 for (int q = 0; q < NE; ++q) {
-                                    av[q][CG_I[n]] = fma(y[q][IN2_OFF[b] + CG_J[n]], pij, av[q][CG_I[n]]);
-                                    bv[q][CG_J[n]] = fma(x[q][CG_I[n]], pij, bv[q][CG_J[n]]);
+                                    T& ai = UNIT_W ? dx[q][CG_I[n]] : av[q][CG_I[n]];
+                                    T& bj = UNIT_W ? dy[q][IN2_OFF[b] + CG_J[n]] : bv[q][CG_J[n]];
+                                    ai = fma(y[q][IN2_OFF[b] + CG_J[n]], pij, ai);
+                                    bj = fma(x[q][CG_I[n]], pij, bj);
                                 }
                             }
                         });
+                        if constexpr (!UNIT_W) {
 #pragma unroll
-                        for (int q = 0; q < NE; ++q) {
-                            const T w = UNIT_W ? (T)1 : (live ? sw[q][ws_off<P>() + lane] : (T)0);
-                            T tw = (T)0;
+                            for (int q = 0; q < NE; ++q) {
+                                const T w = live ? sw[q][ws_off<P>() + lane] : (T)0;
+                                T tw = (T)0;
 #pragma unroll
-                            for (int i = 0; i < D1; ++i) {
-                                if constexpr (!UNIT_W) tw = fma(x[q][i], av[q][i], tw);
-                                dx[q][i] = UNIT_W ? dx[q][i] + av[q][i] : fma(w, av[q][i], dx[q][i]);
-                            }
+                                for (int i = 0; i < D1; ++i) {
+                                    tw = fma(x[q][i], av[q][i], tw);
+                                    dx[q][i] = fma(w, av[q][i], dx[q][i]);
+                                }
 #pragma unroll
-                            for (int j = 0; j < D2; ++j) {
-                                T& d = dy[q][IN2_OFF[b] + j];
-                                d = UNIT_W ? d + bv[q][j] : fma(w, bv[q][j], d);
-                            }
-                            if constexpr (!UNIT_W) {
+                                for (int j = 0; j < D2; ++j) {
+                                    T& d = dy[q][IN2_OFF[b] + j];
+                                    d = fma(w, bv[q][j], d);
+                                }
                                 if (live && (q == 0 || two)) __stcs(dw[q] + W_OFF[P] + slice * 32 + lane, tw);
                             }
                         }
@@ -730,9 +838,13 @@ extern "C" __global__ void __launch_bounds__(32 * oeq::SL_WARPS, oeqd::MIN_CTAS)
     oeq::slice_forward<oeq::MODE_DET>(p, smem_raw, warp, lane);
 #elif OEQ_KERNEL == OEQ_K_SLICE_FWD_ATOMIC
     oeq::slice_forward<oeq::MODE_ATOMIC>(p, smem_raw, warp, lane);
-#elif OEQ_KERNEL == OEQ_K_SLICE_BWD_DET
+#elif OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_DET
+    oeq::slice_forward<oeq::MODE_DET>(p, smem_raw, warp, lane);
+#elif OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_ATOMIC
+    oeq::slice_forward<oeq::MODE_ATOMIC>(p, smem_raw, warp, lane);
+#elif OEQ_KERNEL == OEQ_K_SLICE_BWD_DET || OEQ_KERNEL == OEQ_K_SLICE_DBL_G_DET
     oeq::slice_backward<oeq::MODE_DET>(p, smem_raw, warp, lane);
-#elif OEQ_KERNEL == OEQ_K_SLICE_BWD_ATOMIC
+#elif OEQ_KERNEL == OEQ_K_SLICE_BWD_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_DBL_G_ATOMIC
     oeq::slice_backward<oeq::MODE_ATOMIC>(p, smem_raw, warp, lane);
 #else
 #error "OEQ_KERNEL must select one of the slice kernels"

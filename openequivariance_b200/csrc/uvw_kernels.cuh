@@ -16,6 +16,9 @@
 #pragma once
 #include "oeq_common.cuh"
 
+#define OEQ_K_UVW_FWD 10
+#define OEQ_K_UVW_BWD 11
+
 namespace oeq {
 using namespace oeqd;
 
@@ -62,6 +65,7 @@ __device__ __forceinline__ void uvw_cg_forward(const XA& x, const YA& y, TA& t) 
     });
 }
 
+#if OEQ_KERNEL == OEQ_K_UVW_FWD || OEQ_KERNEL == OEQ_K_UVW_BWD
 // Shared memory layout (element counts come from the descriptor).
 struct UvwSmem {
     T* xs;   // [TILE_R][X_DIM]
@@ -369,16 +373,11 @@ __device__ void uvw_backward(const UvwParams& p) {
 
 }  // namespace oeq
 
-#define OEQ_K_UVW_FWD 10
-#define OEQ_K_UVW_BWD 11
-
 extern "C" __global__ void __launch_bounds__(oeq::NT, 1) oeq_uvw_kernel(const oeq::UvwParams p) {
 #if OEQ_KERNEL == OEQ_K_UVW_FWD
     oeq::uvw_forward(p);
 #elif OEQ_KERNEL == OEQ_K_UVW_BWD
     oeq::uvw_backward(p);
-#else
-#error "OEQ_KERNEL must select one of the uvw kernels"
 #endif
 }
 
@@ -390,3 +389,6 @@ extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, 
     for (long long g = 0; g < groups; ++g) s += ws[g * n + i];
     out[i] = s;
 }
+#else
+}  // namespace oeq
+#endif

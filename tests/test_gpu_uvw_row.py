@@ -1,0 +1,32 @@
+"""'uvw' with per-row weights: the one-row-per-CTA kernels at chunk remainders of every multiplicity, second inputs of
+multiplicity above one, one row, and more rows than CTAs; a problem whose row does not fit them (tiled kernel)."""
+import numpy as np
+import pytest
+import torch
+
+import openequivariance_b200 as oeq
+from oracle import tp_oracle as orc
+from helpers import REL_TOL, rel_err, tp_inputs, to_e3nn, to_oeq
+
+pytestmark = pytest.mark.gpu
+
+ODD = ("40x0e+9x1o+1x2e", "2x0e+3x1o", "36x0e+33x1o+5x1e+1x0o")
+WIDE = ("128x2e+128x3o", "4x1o+4x2e", "16x2e+16x3o")
+
+
+@pytest.mark.parametrize("irreps,batch", [(ODD, 1), (ODD, 7), (ODD, 2500), (WIDE, 3)], ids=["one", "few", "many", "tiled"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
+def test_row_weights(irreps, batch, dtype):
+    p = oeq.FullyConnectedTPProblem(*irreps, shared_weights=False, irrep_dtype=dtype, weight_dtype=dtype)
+    arrays = tp_inputs(p, batch, 3)
+    x, y, w, dz = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (*arrays[:2], to_oeq(p, arrays[2]), arrays[3]))
+    tp = oeq.TensorProduct(p, torch_op=True)
+    z = tp(x, y, w)
+    dx, dy, dw = tp.backward_helper(x, y, w, dz)
+    tp.check_device_status()
+    some = slice(0, batch) if batch < 100 else np.r_[0:3, batch // 2, batch - 3:batch]     # (the oracle is slow)
+    sub = [a[some] for a in arrays]
+    want = [orc.tp_forward(p, *sub[:3]), *orc.tp_backward(p, *sub)]
+    for got, ref in zip((z, dx, dy), want):
+        assert rel_err(got.cpu().numpy()[some], ref) < REL_TOL[dtype]
+    assert rel_err(to_e3nn(p, dw.cpu().numpy()[some]), want[3]) < REL_TOL[dtype]
