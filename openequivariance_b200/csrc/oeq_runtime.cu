@@ -1573,13 +1573,20 @@ void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes,
     grid = std::max<long long>(1, std::min(most, (chunks + per_cta - 1) / per_cta));
 }
 
-// Edges per chunk of the row sum: 64, fewer when that would leave warps idle.
-int row_sum_chunk(const Kernel& k, long long edges) {
+// Row sum: a warp takes a chunk of the sender-ordered edge list and 512 bytes of the rows.  64 edges per chunk, fewer
+// when that would leave warps idle.
+constexpr int SUM_WARPS_PER_SM = 48;
+long long row_sum_blocks(const Problem& p) { return (pad16(p.x_dim * p.elem()) + 511) / 512; }
+int row_sum_chunk(const Kernel& k, const Problem& p, long long edges) {
     int chunk = env_int("OEQ_B200_SUM_CHUNK", 0);
     if (chunk > 0) return chunk;
     chunk = 64;
-    while (chunk > 8 && edges < (long long)chunk * k.sm_count * 48) chunk /= 2;
+    while (chunk > 8 && edges * row_sum_blocks(p) < (long long)chunk * k.sm_count * SUM_WARPS_PER_SM) chunk /= 2;
     return chunk;
+}
+long long row_sum_grid(const Kernel& k, const Problem& p, long long edges, int chunk) {
+    const long long warps = (edges + chunk - 1) / chunk * row_sum_blocks(p);
+    return std::max<long long>(1, std::min<long long>((long long)k.sm_count * (SUM_WARPS_PER_SM / 8), (warps + 7) / 8));
 }
 
 int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream, int clear_flags = 0) {
@@ -2309,7 +2316,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
         h->last_bwd_launches = 0;
         const int dx_bulk = ((p.x_dim * e) % 16 == 0 && aligned16(dX)) ? 32 : 0;
         auto launch = [&](UvuParams& prm) { return sliced ? launch_slice(k, p, prm, st) : launch_uvu(k, p, prm, st, dx_bulk); };
-        const int sum_chunk = row_sum_chunk(k, edges);
+        const int sum_chunk = row_sum_chunk(k, p, edges);
         auto pass1 = [&](long long e0, long long n, void* scratch, UvuParams& prm) {
             prm.X = X; prm.dZ = dZ; prm.dX = dX;
             prm.Y = Yb + (size_t)e0 * p.y_dim * e; prm.W = Wb + (size_t)e0 * p.w_numel * e;
@@ -2333,8 +2340,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
             sp.flags = (first ? 64 : 0) | (n == edges ? 128 : 0);
             sp.chunk = sum_chunk;
             sp.e_lo = e0; sp.e_hi = e0 + n;
-            const long long chunks = (edges + sp.chunk - 1) / sp.chunk;
-            const long long grid = std::max<long long>(1, std::min<long long>((long long)k.sm_count * 6, (chunks + 7) / 8));
+            const long long grid = row_sum_grid(k, p, edges, sp.chunk);
             void* args[] = {&sp};
             OEQ_CUDA(cudaLaunchKernel((const void*)h->sum_rows_fn, dim3((unsigned)grid), dim3(256), args, 0, st));
             ++h->last_bwd_launches;
@@ -2497,7 +2503,7 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
         OEQ_CUDA(cudaLaunchKernel((const void*)h->dbl_clear_fn, dim3(grid), dim3(256), args, 0, st));
     }
     const int dx_bulk = ((p.x_dim * e) % 16 == 0 && aligned16(GX)) ? 32 : 0;
-    const int sum_chunk = row_sum_chunk(k, edges);
+    const int sum_chunk = row_sum_chunk(k, p, edges);
     bool first = true;
     for (long long e0 = 0; e0 < edges; e0 += block_edges) {
         const long long n = std::min(block_edges, edges - e0);
@@ -2520,8 +2526,7 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
             sp.flags = (first ? 64 : 0) | (n == edges ? 128 : 0);
             sp.chunk = sum_chunk;
             sp.e_lo = e0; sp.e_hi = e0 + n;
-            const long long chunks = (edges + sp.chunk - 1) / sp.chunk;
-            const long long grid = std::max<long long>(1, std::min<long long>((long long)k.sm_count * 6, (chunks + 7) / 8));
+            const long long grid = row_sum_grid(k, p, edges, sp.chunk);
             void* args[] = {&sp};
             OEQ_CUDA(cudaLaunchKernel((const void*)h->dbl_sum_fn, dim3((unsigned)grid), dim3(256), args, 0, st));
             first = false;

@@ -1659,6 +1659,10 @@ __device__ void run_backward_recv(const UvuParams& p, const Smem<true, MODE, tru
 // load and a ballot.  `first`: store the rows of the senders met; otherwise add.  `gap_nodes` > 0 (the number of
 // nodes, when the range is the whole list): rows of nodes that send nothing are written as zeros; otherwise the host
 // has cleared dX.
+template <class U> struct VecOf;
+template <> struct VecOf<float> { typedef float4 type; };
+template <> struct VecOf<double> { typedef double2 type; };
+
 __device__ __forceinline__ long long align_sender(const long long* cols, const long long* perm, long long n, long long t,
                                                   int lane) {
     if (t <= 0) return 0;
@@ -1673,38 +1677,57 @@ __device__ __forceinline__ long long align_sender(const long long* cols, const l
     return n;
 }
 
+// A warp takes NV 16-byte pieces per lane of every row: one 512-byte block of columns with eight rows in flight where a
+// launch has warps to spare (with whole rows a warp has one 4.6 KB row in flight: 56 k rows took 80 us, now 58), whole
+// rows for the few helper warps of a receiver-order launch.
+template <int NV, int U>
 __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, const long long* __restrict__ cols,
                                 const long long* __restrict__ perm, long long n_items, long long e_lo, long long e_hi,
                                 bool first, int chunk, long long gap_nodes, long long warps, long long wid, int lane) {
+    typedef typename VecOf<T>::type V;
     constexpr int VEC = 16 / ELEM;                                  // elements per 16-byte load
     constexpr int XS = XB / ELEM;
-    constexpr int NV = (XS / VEC + 31) / 32;                        // 16-byte pieces per lane
-    T acc[NV * VEC];
-#pragma unroll
-    for (int i = 0; i < NV * VEC; ++i) acc[i] = (T)0;
-    auto flush = [&](long long node) {
-        T* xrow = dX + node * (long long)X_DIM;
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const int base = (lane + 32 * v) * VEC;
-            if (base < X_DIM) {
-#pragma unroll
-                for (int q = 0; q < VEC; ++q)
-                    if (base + q < X_DIM) {
-                        if (first) xrow[base + q] = acc[v * VEC + q];
-                        else xrow[base + q] += acc[v * VEC + q];
-                    }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < NV * VEC; ++i) acc[i] = (T)0;
-    };
-    auto zero_nodes = [&](long long lo, long long hi) {
-        for (long long node = lo; node < hi; ++node)
-            for (int i = lane; i < X_DIM; i += 32) dX[node * (long long)X_DIM + i] = (T)0;
-    };
+    constexpr int BLOCKS = (XS + 32 * VEC * NV - 1) / (32 * VEC * NV);
+    const bool vec_out = X_DIM % VEC == 0 && (reinterpret_cast<unsigned long long>(dX) & 15) == 0;
     const long long n_chunks = (n_items + chunk - 1) / chunk;
-    for (long long c = wid; c < n_chunks; c += warps) {
+    for (long long item = wid; item < n_chunks * BLOCKS; item += warps) {
+        const long long c = item / BLOCKS;
+        const int col0 = ((int)(item - c * BLOCKS) * 32 * NV + lane) * VEC;     // piece v: col0 + v * 32 * VEC
+        __align__(16) T acc[NV][VEC];
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) acc[v][i] = (T)0;
+        auto flush = [&](long long node) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int col = col0 + v * 32 * VEC;
+                T* out = dX + node * (long long)X_DIM + col;
+                if (col < X_DIM) {
+                    if (vec_out) {
+                        V t = *reinterpret_cast<V*>(acc[v]);
+                        if (!first) {
+                            const V o = *reinterpret_cast<const V*>(out);
+#pragma unroll
+                            for (int i = 0; i < VEC; ++i) reinterpret_cast<T*>(&t)[i] += reinterpret_cast<const T*>(&o)[i];
+                        }
+                        *reinterpret_cast<V*>(out) = t;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < VEC; ++i)
+                            if (col + i < X_DIM) out[i] = first ? acc[v][i] : out[i] + acc[v][i];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) acc[v][i] = (T)0;
+            }
+        };
+        auto zero_nodes = [&](long long lo, long long hi) {
+            for (long long node = lo; node < hi; ++node)
+                for (int v = 0; v < NV; ++v)
+                    for (int i = 0; i < VEC; ++i)
+                        if (col0 + v * 32 * VEC + i < X_DIM) dX[node * (long long)X_DIM + col0 + v * 32 * VEC + i] = (T)0;
+        };
         const long long pos = align_sender(cols, perm, n_items, c * chunk, lane);
         const long long end = c + 1 >= n_chunks ? n_items : align_sender(cols, perm, n_items, (c + 1) * chunk, lane);
         long long prev = -1;
@@ -1716,49 +1739,28 @@ __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, 
             unsigned mask = __ballot_sync(0xffffffffu, in_block);
             if (mask == 0) continue;
             if (in_block) s = cols[e];
-            // Short rows: the loads of up to U rows go out together (a row at a time would pay the DRAM latency
-            // per row); the rows are still added one after the other, in order.
-            constexpr int U = (NV * VEC <= 16) ? 4 : (NV * VEC <= 32 ? 2 : 1);
+            const int row_of = (int)(e - e_lo);                     // (the scratch holds fewer than 2^31 rows)
             while (mask) {
-                long long ej[U], sj[U];
-                T val[U][NV * VEC];
-                int n = 0;
+                long long sj[U];
+                __align__(16) T val[U][NV][VEC];
 #pragma unroll
                 for (int q = 0; q < U; ++q) {
-                    ej[q] = 0; sj[q] = -1;
+                    sj[q] = -1;
                     if (mask) {
                         const int src = __ffs(mask) - 1;
                         mask &= mask - 1;
-                        ej[q] = __shfl_sync(0xffffffffu, e, src);
+                        const long long row = __shfl_sync(0xffffffffu, row_of, src);
                         sj[q] = __shfl_sync(0xffffffffu, s, src);
-                        n = q + 1;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < U; ++q) {
-                    if (q < n) {
-                        const T* row = temp + (ej[q] - e_lo) * (long long)XS;
 #pragma unroll
                         for (int v = 0; v < NV; ++v) {
-                            const int b4 = (lane + 32 * v) * VEC;
-                            if (b4 < XS) {
-                                if constexpr (ELEM == 4) {
-                                    const float4 t = __ldcs(reinterpret_cast<const float4*>(row + b4));
-                                    val[q][v * VEC + 0] = t.x; val[q][v * VEC + 1] = t.y; val[q][v * VEC + 2] = t.z; val[q][v * VEC + 3] = t.w;
-                                } else {
-                                    const double2 t = __ldcs(reinterpret_cast<const double2*>(row + b4));
-                                    val[q][v * VEC + 0] = t.x; val[q][v * VEC + 1] = t.y;
-                                }
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < VEC; ++c) val[q][v * VEC + c] = (T)0;
-                            }
+                            const int col = col0 + v * 32 * VEC;
+                            if (col < X_DIM) *reinterpret_cast<V*>(val[q][v]) = __ldcs(reinterpret_cast<const V*>(temp + row * XS + col));
                         }
                     }
                 }
 #pragma unroll
                 for (int q = 0; q < U; ++q) {
-                    if (q < n) {
+                    if (sj[q] >= 0) {
                         if (sj[q] != prev) {
                             if (prev >= 0) flush(prev);
                             // (the nodes before a later chunk's first sender belong to the chunk before it)
@@ -1766,7 +1768,9 @@ __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, 
                             prev = sj[q];
                         }
 #pragma unroll
-                        for (int i = 0; i < NV * VEC; ++i) acc[i] += val[q][i];
+                        for (int v = 0; v < NV; ++v)
+#pragma unroll
+                            for (int i = 0; i < VEC; ++i) acc[v][i] += val[q][v][i];
                     }
                 }
             }
@@ -1777,6 +1781,7 @@ __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, 
         }
     }
 }
+constexpr int ROW_PIECES = (XB / 16 + 31) / 32;      // 16-byte pieces per lane of a whole row
 
 template <int MODE>
 __device__ __forceinline__ void uvu_body_recv(const UvuParams& p) {
@@ -1798,7 +1803,7 @@ __device__ __forceinline__ void uvu_body_recv(const UvuParams& p) {
     if (tid >= NCONSUMERS + NSTAGING) {
         if constexpr (HELPER_WARPS > 0) {
             if (p.sum_items > 0)
-                sum_sender_rows(p.sum_ws, p.dX, p.sum_cols, p.sum_perm, p.sum_items, p.sum_e_lo, p.sum_e_hi, p.sum_first != 0,
+                sum_sender_rows<ROW_PIECES, (ROW_PIECES <= 4 ? 4 : ROW_PIECES <= 8 ? 2 : 1)>(p.sum_ws, p.dX, p.sum_cols, p.sum_perm, p.sum_items, p.sum_e_lo, p.sum_e_hi, p.sum_first != 0,
                                 p.sum_chunk, 0, (long long)gridDim.x * HELPER_WARPS,
                                 (long long)blockIdx.x * HELPER_WARPS + ((tid - NCONSUMERS - NSTAGING) >> 5), tid & 31);
         }
@@ -2160,7 +2165,7 @@ extern "C" __global__ void oeq_clear(unsigned int* ptr, unsigned long long words
 // The row sum of the deterministic receiver-order backward pass as a launch of its own (the last block of
 // edges, or every block when the launches carry no helper warps): see sum_sender_rows.
 extern "C" __global__ void __launch_bounds__(256) oeq_sum_sender_rows(const oeq::UvuParams p) {
-    oeq::sum_sender_rows(reinterpret_cast<const oeqd::T*>(p.ws), p.dX, p.cols, p.perm, p.n_items, p.e_lo, p.e_hi,
+    oeq::sum_sender_rows<1, 8>(reinterpret_cast<const oeqd::T*>(p.ws), p.dX, p.cols, p.perm, p.n_items, p.e_lo, p.e_hi,
                          (p.flags & 64) != 0, p.chunk, (p.flags & 128) ? p.n_nodes : 0, (long long)gridDim.x * (blockDim.x >> 5),
                          (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31);
 }
