@@ -133,6 +133,8 @@ struct Problem {
     std::vector<Irrep> in1, in2, out;
     std::vector<Instr> instr;
     int dtype = 0, shared = 0, mode = 0;
+    bool unit_y = false;        // the second input is the number 1 for every row (no array)
+    bool transposed_w = false;  // the weight array is that of the problem with first input and output exchanged
     int unit = 0;               // no weight array: every weight is 1 (shared_weights == 2 in the descriptor)
     int x_dim = 0, y_dim = 0, z_dim = 0, w_numel = 0;
     int elem() const { return dtype == OEQ_F64 ? 8 : 4; }
@@ -732,6 +734,7 @@ std::string descriptor_text(const Problem& p, const Mapping& m, const UvwConfig*
     s << "constexpr int X_DIM = " << p.x_dim << ", Y_DIM = " << p.y_dim << ", Z_DIM = " << p.z_dim
       << ", W_NUMEL = " << p.w_numel << ";\n";
     s << "constexpr bool SHARED_W = " << (p.shared ? "true" : "false") << ";\n";
+    s << "constexpr bool UNIT_Y = " << (p.unit_y ? "true" : "false") << ", TRANSPOSED_W = " << (p.transposed_w ? "true" : "false") << ";\n";
     s << "constexpr bool UNIT_W = " << (p.unit ? "true" : "false") << ";\n";
     s << "constexpr int N_IN1 = " << p.in1.size() << ", N_IN2 = " << p.in2.size() << ", N_OUT = " << p.out.size()
       << ", N_INSTR = " << p.instr.size() << ";\n";
@@ -1282,7 +1285,8 @@ struct TcGeometry {
     int smem = 0;
 };
 
-bool uvw_tc_geometry(const Problem& p, TcGeometry& g) {
+// `pad`: output multiplicities may be rounded up to 16 (the products W dZ of the backward pass).
+bool uvw_tc_geometry(const Problem& p, TcGeometry& g, bool pad = false) {
     if (p.mode != OEQ_MODE_UVW || !p.shared || p.dtype != OEQ_F32) return false;
     if (!env_int("OEQ_B200_UVW_TC", 1)) return false;
     int w_max = 0, mw_max = 16;
@@ -1295,8 +1299,8 @@ bool uvw_tc_geometry(const Problem& p, TcGeometry& g) {
                 blocks += (p.in1[t.i1].mul + 31) / 32;
             }
         if (blocks == 0) continue;
-        const int mw = p.out[o].mul;
-        if (mw % 16 != 0 || mw > 256 || p.out[o].dim > 64) return false;
+        const int mw = (p.out[o].mul + 15) / 16 * 16;
+        if ((!pad && mw != p.out[o].mul) || mw > 256 || p.out[o].dim > 64) return false;
         const int bytes = blocks * 2 * mw * 128;
         w_max = std::max(w_max, bytes);
         mw_max = std::max(mw_max, mw);
@@ -1325,54 +1329,68 @@ int build_uvw_tc(const Problem& p, Kernel& k) {
     return OEQ_OK;
 }
 
-// ---- tensor-core backward for 'uvw' (mirrors the constexpr geometry of uvw_tc_bwd_kernels.cuh)
-constexpr int K_UVW_TC_DW = 21, K_UVW_TC_DXY = 22;
+// ---- tensor-core backward for 'uvw': the weight gradient (mirrors the constexpr geometry of uvw_tc_bwd_kernels.cuh)
+constexpr int K_UVW_TC_DW = 21;
 
-struct TcBwdGeometry {
-    int dw_smem = 0;
-    int dxy_smem = 0;           // 0: the dX/dY kernel does not take this problem
-    size_t wt_bytes = 0;        // transposed packed weights
-};
-
-bool uvw_tc_bwd_geometry(const Problem& p, TcBwdGeometry& g) {
+bool uvw_tc_dw_geometry(const Problem& p, int& smem) {
     TcGeometry fwd;
     if (!uvw_tc_geometry(p, fwd)) return false;          // same class of problems as the forward pass
     if (!env_int("OEQ_B200_UVW_TC_BWD", 1)) return false;
     int mw_max = 16;
-    for (const Irrep& r : p.out) mw_max = std::max(mw_max, r.mul);
+    for (const Irrep& r : p.out) {
+        mw_max = std::max(mw_max, r.mul);
+        if (r.dim > 32) return false;                    // a stage holds at least one batch row
+    }
     for (const Instr& t : p.instr)
         if (p.in1[t.i1].mul > 128) return false;
     if (mw_max > 128) return false;
     const int stage = 2 * 128 * 128 + 2 * mw_max * 128;
     const int stages = std::min(4, (200 * 1024) / stage);
     if (stages < 2) return false;
-    g.dw_smem = stages * stage + (2 * stages + 4) * 8 + 16 + 1024;
-    if (g.dw_smem > SMEM_LIMIT) return false;
-    // dX/dY kernel: one set of A tiles, two buffers of one path's transposed weights, the epilogue staging
-    // buffer, two sets of an X row and a dX row per epilogue warp
-    int kb_max = 1, mup_max = 16, wt_max = 0, row_max = 0;
-    size_t wt_total = 0;
-    for (const Irrep& r : p.out) kb_max = std::max(kb_max, (r.mul + 31) / 32);
-    for (const Instr& t : p.instr) {
-        const int mup = (p.in1[t.i1].mul + 15) / 16 * 16;
-        const int bytes = ((p.out[t.io].mul + 31) / 32) * 2 * mup * 128;
-        mup_max = std::max(mup_max, mup);
-        wt_max = std::max(wt_max, bytes);
-        wt_total += bytes;
-        row_max = std::max(row_max, p.in1[t.i1].mul * p.in1[t.i1].dim);
-    }
-    const int nacc = std::min(4, 512 / (2 * mup_max));
-    const int off_w = kb_max * 2 * 128 * 128;
-    const int off_stg = off_w + 2 * ((wt_max + 1023) / 1024 * 1024);
-    const int off_row = off_stg + (128 * (mup_max + 1) * 4 + 15) / 16 * 16;
-    const int off_bar = off_row + 12 * 4 * ((row_max * 4 + 15) / 16 * 16);
-    const int dxy = off_bar + (2 * 1 + 2 * nacc + 4) * 8 + 16 + 1024;
-    if (nacc >= 1 && dxy <= SMEM_LIMIT) {
-        g.dxy_smem = dxy;
-        g.wt_bytes = wt_total;
-    }
-    return true;
+    smem = stages * stage + (2 * stages + 4) * 8 + 16 + 1024;
+    return smem <= SMEM_LIMIT;
 }
+
+// ---- dX and dY of the same class of problems in two steps over a scratch array dT [row][path][u][k]:
+//   dT_p[b,u,k] = sum_w W_p[u,w] dZ[b,w,k]: a 'uvw' forward pass from the output irreps, with the second input the
+//   number 1 and the weights transposed, one output block per path (`product`);
+//   dX, dY from dT: the channel-wise backward pass with every weight 1 (`channels`).
+void uvw_gradient_problems(const Problem& p, Problem& product, Problem& channels) {
+    product = Problem();
+    product.mode = OEQ_MODE_UVW;
+    product.shared = 1;
+    product.unit_y = product.transposed_w = true;
+    product.in1 = p.out;
+    product.x_dim = p.z_dim;
+    product.in2 = {Irrep{1, 0, 1, 1, 0}};
+    product.y_dim = 1;
+    product.w_numel = p.w_numel;
+    channels = p;
+    channels.mode = OEQ_MODE_UVU;
+    channels.shared = 0;
+    channels.unit = 1;
+    channels.out.clear();
+    int off = 0;
+    for (size_t n = 0; n < p.instr.size(); ++n) {
+        const Instr& t = p.instr[n];
+        Irrep block = p.out[t.io];
+        block.mul = p.in1[t.i1].mul;
+        block.off = off;
+        off += block.mul * block.dim;
+        product.out.push_back(block);
+        channels.out.push_back(block);
+        Instr q = t;
+        q.i1 = t.io; q.i2 = 0; q.io = (int)n; q.pw = 1.0;
+        q.ci.clear(); q.cj.clear(); q.ck.clear(); q.cv.clear();
+        for (int k = 0; k < block.dim; ++k) { q.ci.push_back(k); q.cj.push_back(0); q.ck.push_back(k); q.cv.push_back(1.0); }
+        product.instr.push_back(q);
+        channels.instr[n].io = (int)n;
+        channels.instr[n].mode = OEQ_MODE_UVU;
+    }
+    product.z_dim = channels.z_dim = off;
+}
+// Scratch rows: all of them up to 1 GiB, then blocks.
+constexpr size_t UVW_DT_BYTES = 1u << 30;
 
 int build_uvw_tc_bwd(const Problem& p, int kernel_id, Kernel& k) {
     k.is_uvw = true;
@@ -1420,6 +1438,15 @@ int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
     if (rc) return rc;
     k.compiled = true;
     return OEQ_OK;
+}
+
+// Both kernels of the two-step dX / dY (OEQ_ERR_UNSUPPORTED where a row does not fit them).
+int build_uvw_gradients(const Problem& p, Problem& product, Problem& channels, TcGeometry& g, Kernel& kp, Kernel& kc) {
+    uvw_gradient_problems(p, product, channels);
+    if (!uvw_tc_geometry(product, g, true)) return fail(OEQ_ERR_UNSUPPORTED, "rows do not fit the tensor-core product");
+    int rc = build_uvw_tc(product, kp);
+    if (!rc) rc = build_uvu(channels, K_BWD_BATCH, kc);
+    return rc;
 }
 
 int build_tp(const Problem& p, bool bwd, Kernel& k) {
@@ -1620,13 +1647,17 @@ struct oeq_tp {
     Kernel fwd_tc;              // tensor-core forward ('uvw', shared FP32 weights), when the problem qualifies
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
-    Kernel bwd_dxy_tc;          // tensor-core dX / dY of the same class of problems (when its tiles fit)
-    bool has_bwd_tc = false, has_dxy_tc = false;
+    bool has_bwd_tc = false;
+    int dw_smem = 0;
+    // dX and dY of the same class of problems: dT = W dZ on the tensor cores, then the channel-wise backward pass
+    Problem grad_product, grad_channels;
+    Kernel grad_product_k, grad_channels_k;
+    TcGeometry grad_tc;
+    bool has_grad_tc = false;
+    void* d_packed_t = nullptr; // the transposed weights, split and swizzled
+    cudaKernel_t pack_t_fn = nullptr;
     Kernel dbl;                 // one-pass second derivatives ('uvu', per-row weights)
     bool has_dbl = false;
-    TcBwdGeometry tc_bwd;
-    void* d_packed_t = nullptr; // weights transposed, split and swizzled for the dX/dY kernel
-    cudaKernel_t pack_t_fn = nullptr;
     TcGeometry tc;
     void* d_packed = nullptr;   // weights split and swizzled for the tensor cores (owned by the handle)
     cudaKernel_t pack_fn = nullptr;
@@ -1687,11 +1718,13 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if ((rc = build_tp(p, false, f)) || (rc = build_tp(p, true, b))) return rc;
         TcGeometry g;
         if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, tc))) return rc;
-        TcBwdGeometry gb;
-        Kernel dw, dxy;
-        if (uvw_tc_bwd_geometry(p, gb)) {
+        int smem = 0;
+        Kernel dw, product, channels;
+        if (uvw_tc_dw_geometry(p, smem)) {
             if ((rc = build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
-            if (gb.dxy_smem > 0 && (rc = build_uvw_tc_bwd(p, K_UVW_TC_DXY, dxy))) return rc;
+            Problem pp, pc;
+            rc = build_uvw_gradients(p, pp, pc, g, product, channels);
+            if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
         }
         return OEQ_OK;
     }
@@ -1748,12 +1781,13 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
         rc = build_uvw_tc(h->prob, h->fwd_tc);
         h->has_tc = rc == OEQ_OK;
     }
-    if (!rc && uvw_tc_bwd_geometry(h->prob, h->tc_bwd)) {
+    if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem)) {
         rc = build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
         h->has_bwd_tc = rc == OEQ_OK;
-        if (!rc && h->tc_bwd.dxy_smem > 0 && env_int("OEQ_B200_UVW_TC_DXY", 1)) {
-            rc = build_uvw_tc_bwd(h->prob, K_UVW_TC_DXY, h->bwd_dxy_tc);
-            h->has_dxy_tc = rc == OEQ_OK;
+        if (!rc) {
+            const int rc2 = build_uvw_gradients(h->prob, h->grad_product, h->grad_channels, h->grad_tc, h->grad_product_k, h->grad_channels_k);
+            h->has_grad_tc = rc2 == OEQ_OK;
+            if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
         }
     }
     if (!rc && double_backward_supported(h->prob)) {
@@ -1774,7 +1808,7 @@ int oeq_tp_destroy(oeq_tp* h) {
     if (h->d_status) cudaFree(h->d_status);
     if (h->d_packed) cudaFree(h->d_packed);
     if (h->d_packed_t) cudaFree(h->d_packed_t);
-    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_tc, &h->bwd_dw_tc, &h->bwd_dxy_tc, &h->dbl})
+    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->dbl})
         if (k->lib) cudaLibraryUnload(k->lib);
     delete h;
     return OEQ_OK;
@@ -1789,6 +1823,54 @@ static int ensure_status(int** d_status) {
     return OEQ_OK;
 }
 
+static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack, void*& packed) {
+    if (k.loaded) return OEQ_OK;
+    OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+    OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_tc_kernel"));
+    OEQ_CUDA(cudaLibraryGetKernel(&pack, k.lib, "oeq_uvw_pack_weights"));
+    int dev = 0;
+    OEQ_CUDA(cudaGetDevice(&dev));
+    OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
+    k.smem = geo.smem;
+    OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
+    else (void)cudaGetLastError();
+    OEQ_CUDA(cudaMalloc(&packed, geo.packed_bytes));
+    k.loaded = true;
+    return OEQ_OK;
+}
+
+// `pack`: the weights have to be brought into the operand layout first (once per call).
+static int launch_uvw_tc(Kernel& k, cudaKernel_t pack_fn, void* packed, bool pack, long long batch, const void* X, const void* Y,
+                         const void* W, void* Z, int* status, cudaStream_t st) {
+    if (pack) {
+        void* args[] = {(void*)&W, &packed};
+        OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(64), dim3(256), args, 0, st));
+    }
+    struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; unsigned long long* prof; }
+        tp{X, Y, packed, Z, batch, status, nullptr};
+    void* args[] = {&tp};
+    const long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
+#ifdef OEQ_DEV_PROFILE
+    if (env_int("OEQ_B200_TC_PROFILE", 0)) {
+        // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr
+        OEQ_CUDA(cudaMalloc(&tp.prof, 32 * 8));
+        OEQ_CUDA(cudaMemsetAsync(tp.prof, 0, 32 * 8, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
+        unsigned long long hb[32];
+        OEQ_CUDA(cudaMemcpyAsync(hb, tp.prof, sizeof hb, cudaMemcpyDeviceToHost, st));
+        OEQ_CUDA(cudaStreamSynchronize(st));
+        cudaFree(tp.prof);
+        fprintf(stderr, "[oeq_b200 uvw tc profile] mma: wait %llu issue %llu | epilogue: tiles %llu wait %llu drain %llu\n", hb[8], hb[9],
+                hb[18], hb[16], hb[17]);
+        return OEQ_OK;
+    }
+#endif
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
+    return OEQ_OK;
+}
+
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
@@ -1798,49 +1880,8 @@ int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const
     if (rc) return rc;
     h->last_stream = (cudaStream_t)stream;
     if (h->has_tc) {
-        Kernel& k = h->fwd_tc;
-        cudaStream_t st = (cudaStream_t)stream;
-        if (!k.loaded) {
-            OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-            OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_tc_kernel"));
-            OEQ_CUDA(cudaLibraryGetKernel(&h->pack_fn, k.lib, "oeq_uvw_pack_weights"));
-            int dev = 0;
-            OEQ_CUDA(cudaGetDevice(&dev));
-            OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
-            k.smem = h->tc.smem;
-            OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
-            cudaFuncAttributes attr;
-            if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
-            else (void)cudaGetLastError();
-            OEQ_CUDA(cudaMalloc(&h->d_packed, h->tc.packed_bytes));
-            k.loaded = true;
-        }
-        {
-            void* packed = h->d_packed;
-            void* args[] = {(void*)&W, &packed};
-            OEQ_CUDA(cudaLaunchKernel((const void*)h->pack_fn, dim3(64), dim3(256), args, 0, st));
-        }
-        struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; unsigned long long* prof; }
-            tp{X, Y, h->d_packed, Z, batch, h->d_status, nullptr};
-        void* args[] = {&tp};
-        const long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
-#ifdef OEQ_DEV_PROFILE
-        if (env_int("OEQ_B200_TC_PROFILE", 0)) {
-            // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr
-            OEQ_CUDA(cudaMalloc(&tp.prof, 32 * 8));
-            OEQ_CUDA(cudaMemsetAsync(tp.prof, 0, 32 * 8, st));
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
-            unsigned long long hb[32];
-            OEQ_CUDA(cudaMemcpyAsync(hb, tp.prof, sizeof hb, cudaMemcpyDeviceToHost, st));
-            OEQ_CUDA(cudaStreamSynchronize(st));
-            cudaFree(tp.prof);
-            fprintf(stderr, "[oeq_b200 uvw tc profile] producer: stages %llu wait %llu fill %llu | mma: wait %llu issue %llu | "
-                            "epilogue: tiles %llu wait %llu drain %llu\n", hb[2], hb[0], hb[1], hb[8], hb[9], hb[18], hb[16], hb[17]);
-            return OEQ_OK;
-        }
-#endif
-        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
-        return OEQ_OK;
+        if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed))) return rc;
+        return launch_uvw_tc(h->fwd_tc, h->pack_fn, h->d_packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     }
     if (h->prob.mode == OEQ_MODE_UVW) {
         if ((rc = load_uvw(h->fwd, h->prob, false))) return rc;
@@ -1869,7 +1910,9 @@ size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch) {
     } else {
         groups = 256ll * 4 * h->bwd.map.ng;
     }
-    return (size_t)groups * h->prob.w_numel * h->prob.elem();
+    size_t bytes = (size_t)groups * h->prob.w_numel * h->prob.elem();
+    if (h->has_grad_tc) bytes = std::max(bytes, std::min((size_t)batch * h->grad_product.z_dim * 4, UVW_DT_BYTES));
+    return bytes;
 }
 
 int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, const void* dZ, void* dX,
@@ -1908,15 +1951,15 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
                 int dev = 0;
                 OEQ_CUDA(cudaGetDevice(&dev));
                 OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
-                k.smem = h->tc_bwd.dw_smem;
+                k.smem = h->dw_smem;
                 OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
                 k.loaded = true;
             }
             long long dw_ctas = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 31) / 32));
             if ((size_t)dw_ctas * p.w_numel * p.elem() > workspace_bytes)
                 return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
-            struct { const void* X; const void* Y; const void* Wt; const void* dZ; void* dX; void* dY; void* ws; long long batch;
-                     int* status; unsigned long long* prof; } tp{X, Y, nullptr, dZ, dX, dY, workspace, batch, h->d_status, nullptr};
+            struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; }
+                tp{X, Y, dZ, workspace, batch, h->d_status};
             void* targs[] = {&tp};
             OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas), dim3(21 * 32), targs, (size_t)k.smem, st));
             int n = p.w_numel;
@@ -1925,43 +1968,25 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
             up.skip_dw = 1;
             up.ws = nullptr;
-            if (h->has_dxy_tc) {
-                // dX and dY on the tensor cores too: the FMA kernel is not launched at all
-                Kernel& kx = h->bwd_dxy_tc;
-                if (!kx.loaded) {
-                    OEQ_CUDA(cudaLibraryLoadData(&kx.lib, kx.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-                    OEQ_CUDA(cudaLibraryGetKernel(&kx.fn, kx.lib, "oeq_uvw_tc_dxy_kernel"));
-                    OEQ_CUDA(cudaLibraryGetKernel(&h->pack_t_fn, kx.lib, "oeq_uvw_pack_weights_t"));
-                    kx.sm_count = k.sm_count;
-                    kx.smem = h->tc_bwd.dxy_smem;
-                    OEQ_CUDA(cudaFuncSetAttribute((const void*)kx.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kx.smem));
-                    OEQ_CUDA(cudaMalloc(&h->d_packed_t, h->tc_bwd.wt_bytes));
-                    kx.loaded = true;
+            // dX and dY in two steps over dT rows, which take the partial gradients' place in the workspace
+            const size_t row = (size_t)h->grad_product.z_dim * 4;
+            const long long block = h->has_grad_tc && aligned16(workspace) ? (long long)std::min<size_t>((size_t)batch, workspace_bytes / row) : 0;
+            if (block > 0 && (block == batch || block >= 4096)) {
+                if ((rc = load_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t))) return rc;
+                if ((rc = load_kernel(h->grad_channels_k, "oeq_uvu_kernel", false))) return rc;
+                for (long long b0 = 0; b0 < batch; b0 += block) {
+                    const long long rows = std::min<long long>(block, batch - b0);
+                    if ((rc = launch_uvw_tc(h->grad_product_k, h->pack_t_fn, h->d_packed_t, b0 == 0, rows,
+                                            (const char*)dZ + (size_t)b0 * p.z_dim * 4, nullptr, W, workspace, h->d_status, st))) return rc;
+                    UvuParams prm{};
+                    prm.X = (const char*)X + (size_t)b0 * p.x_dim * 4;
+                    prm.Y = (const char*)Y + (size_t)b0 * p.y_dim * 4;
+                    prm.dZ = workspace;
+                    prm.dX = (char*)dX + (size_t)b0 * p.x_dim * 4;
+                    prm.dY = (char*)dY + (size_t)b0 * p.y_dim * 4;
+                    prm.n_items = rows; prm.n_nodes = rows; prm.status = h->d_status;
+                    if ((rc = launch_uvu(h->grad_channels_k, h->grad_channels, prm, st))) return rc;
                 }
-                void* packed = h->d_packed_t;
-                void* pargs[] = {(void*)&W, &packed};
-                OEQ_CUDA(cudaLaunchKernel((const void*)h->pack_t_fn, dim3(64), dim3(256), pargs, 0, st));
-                OEQ_CUDA(cudaMemsetAsync(dX, 0, (size_t)batch * p.x_dim * p.elem(), st));
-                OEQ_CUDA(cudaMemsetAsync(dY, 0, (size_t)batch * p.y_dim * p.elem(), st));
-                tp.Wt = h->d_packed_t;
-                const long long ctas_x = std::max<long long>(1, std::min<long long>(kx.sm_count, (batch + 23) / 24));
-#ifdef OEQ_DEV_PROFILE
-                if (env_int("OEQ_B200_TC_PROFILE", 0)) {
-                    // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr
-                    OEQ_CUDA(cudaMalloc(&tp.prof, 32 * 8));
-                    OEQ_CUDA(cudaMemsetAsync(tp.prof, 0, 32 * 8, st));
-                    OEQ_CUDA(cudaLaunchKernel((const void*)kx.fn, dim3((unsigned)ctas_x), dim3(16 * 32), targs, (size_t)kx.smem, st));
-                    unsigned long long hb[32];
-                    OEQ_CUDA(cudaMemcpyAsync(hb, tp.prof, sizeof hb, cudaMemcpyDeviceToHost, st));
-                    OEQ_CUDA(cudaStreamSynchronize(st));
-                    cudaFree(tp.prof);
-                    fprintf(stderr, "[oeq_b200 uvw dxy profile] producer: stages %llu wait %llu fill %llu | mma: wait-acc %llu wait-full %llu "
-                                    "issue %llu | epilogue: wait %llu drain %llu rows %llu sync %llu | per row: n %llu compute %llu dy %llu\n", hb[2], hb[0], hb[1], hb[8], hb[9],
-                            hb[10], hb[16], hb[17], hb[18], hb[19], hb[26], hb[24], hb[25]);
-                    return OEQ_OK;
-                }
-#endif
-                OEQ_CUDA(cudaLaunchKernel((const void*)kx.fn, dim3((unsigned)ctas_x), dim3(16 * 32), targs, (size_t)kx.smem, st));
                 return OEQ_OK;
             }
         }

@@ -52,7 +52,8 @@ constexpr int tc_blocks_before(int o, int p_end) {   // [MW x 32] weight blocks 
         if (I_OUT[p] == o) n += tc_khalves(p);
     return n;
 }
-constexpr int tc_block_bytes(int o) { return OUT_MUL[o] * 128; }                 // one hi (or lo) block
+constexpr int tc_mwp(int o) { return (OUT_MUL[o] + 15) / 16 * 16; }              // N of the MMA: a multiple of 16
+constexpr int tc_block_bytes(int o) { return tc_mwp(o) * 128; }                  // one hi (or lo) block
 constexpr int tc_w_bytes(int o) { return tc_blocks_before(o, N_INSTR) * 2 * tc_block_bytes(o); }
 constexpr int tc_w_offset(int o) {   // byte offset of output o inside the packed weight buffer
     int b = 0;
@@ -66,11 +67,11 @@ constexpr int tc_w_max() {
 }
 constexpr int tc_mw_max() {
     int m = 16;
-    for (int o = 0; o < N_OUT; ++o) m = OUT_MUL[o] > m ? OUT_MUL[o] : m;
+    for (int o = 0; o < N_OUT; ++o) m = tc_mwp(o) > m ? tc_mwp(o) : m;
     return m;
 }
-constexpr bool tc_wide(int o) { return 2 * OUT_MUL[o] <= 256; }
-constexpr int tc_acc_cols(int o) { return tc_wide(o) ? 2 * OUT_MUL[o] : OUT_MUL[o]; }
+constexpr bool tc_wide(int o) { return 2 * tc_mwp(o) <= 256; }
+constexpr int tc_acc_cols(int o) { return tc_wide(o) ? 2 * tc_mwp(o) : tc_mwp(o); }
 // One ring of accumulator tiles serves all output irreps: equal tile width and count for all of them, so that
 // tile index and barrier phase follow from one running counter.
 constexpr int tc_acc_cols_max() {
@@ -109,19 +110,46 @@ struct TcBars {
     }
 };
 
+// Offset of W_p[u, w] (MU x MW, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks,
+// u-chunk major, each chunk [u][w].
+template <int P, int MU, int MW>
+__device__ __forceinline__ int tc_weight_offset(int u, int w) {
+    const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
+    const int ulen = (MU - (uc << 5)) < 32 ? (MU - (uc << 5)) : 32;
+    const int wlen = (MW - (wc << 5)) < 32 ? (MW - (wc << 5)) : 32;
+    return W_OFF[P] + (uc << 5) * MW + ulen * (wc << 5) + ul * wlen + wl;
+}
+
 // rows of the batch owned by this CTA
 __device__ __forceinline__ void tc_row_range(long long batch, long long& lo, long long& hi) {
     lo = batch * blockIdx.x / gridDim.x;
     hi = batch * (blockIdx.x + 1) / gridDim.x;
 }
 
+// Batch rows of a chunk and the accumulator row of (batch row r, component k): k-major, with the rows rounded down to
+// a multiple of eight where that costs at most an eighth of the tile.  A producer warp then keeps its row of the
+// swizzle pattern (r mod 8) and every store of a stage has a compile-time offset.
+constexpr int tc_rpc(int o) {
+    const int full = 128 / OUT_D[o], r8 = full / 8 * 8;
+    return r8 * OUT_D[o] >= 112 ? r8 : full;
+}
+
 // ---------------------------------------------------------------------------- producers
+//
+// Bound by issue: 39 instructions per element of T when every store computed its swizzled address and every row its
+// predicates.  Warp w takes the rows r = w mod 8 (mod 8); the two sets of eight warps take alternate groups of eight
+// rows, swapped from stage to stage so that an odd number of groups does not leave one set waiting.
 template <int O>
 __device__ __forceinline__ bool tc_produce_output(const UvwTcParams& p, unsigned char* smem, const TcBars& bars,
                                                   long long row_lo, long long row_hi, long long& stage_it, int warp,
                                                   int lane) {
     constexpr int D3 = OUT_D[O];
-    constexpr int RPC = 128 / D3;
+    constexpr int RPC = tc_rpc(O);
+    static_assert(TC_PRODUCER_WARPS == 16, "two sets of eight warps");
+    constexpr bool FAST = RPC % 8 == 0;
+    constexpr int Q = (RPC + 7) / 8;            // groups of eight rows
+    const int w8 = warp & 7, set = warp >> 3;
+    const int base = w8 * 128 + (((lane >> 2) ^ w8) << 4) + ((lane & 3) << 2);
     bool ok = true;
     for (long long b0 = row_lo; b0 < row_hi && ok; b0 += RPC) {
         const int rows = (int)(row_hi - b0 < RPC ? row_hi - b0 : RPC);
@@ -130,35 +158,39 @@ __device__ __forceinline__ bool tc_produce_output(const UvwTcParams& p, unsigned
             if constexpr (I_OUT[P] == O) {
                 constexpr int a = I_IN1[P], b = I_IN2[P];
                 constexpr int D1 = IN1_D[a], D2 = IN2_D[b], MU = IN1_MUL[a];
+                constexpr int QB = D1 + D2 + D3 <= 6 ? 8 : (D1 + D2 + D3 <= 14 ? 2 : 1);    // groups whose loads go out together
                 for (int h = 0; h < tc_khalves(P) && ok; ++h) {
                     const int s = (int)(stage_it % TC_NA);
                     const long long use = stage_it / TC_NA;
-                    // all global loads of this warp's rows go out first, so their latency is paid once per
-                    // stage and overlaps the wait for the stage to be handed back
-                    constexpr int RW = (RPC + TC_PRODUCER_WARPS - 1) / TC_PRODUCER_WARPS;
+                    const int q0 = (set + (int)stage_it) & 1;
                     const int u = h * 32 + lane;
-                    float xs[RW][D1], ys[RW][D2];
+                    const bool u_live = MU % 32 == 0 || u < MU;
+                    const float* xb = p.X + (b0 + w8) * (long long)X_DIM + IN1_OFF[a] + u * D1;
+                    const float* yb = p.Y + (b0 + w8) * (long long)Y_DIM + IN2_OFF[b];
+                    unsigned char* hi = smem + TC_OFF_A + s * TC_STAGE_BYTES + base;
+                    bool waited = use == 0;
+#pragma unroll 1
+                    for (int qq = q0; qq < Q && ok; qq += 2 * QB) {
+                        float xs[QB][D1], ys[QB][D2];
 #pragma unroll
-                    for (int q = 0; q < RW; ++q) {
-                        const int r = warp + q * TC_PRODUCER_WARPS;
-                        const bool live = r < rows;
-                        const float* xrow = p.X + (b0 + (live ? r : 0)) * (long long)X_DIM + IN1_OFF[a];
-                        const float* yrow = p.Y + (b0 + (live ? r : 0)) * (long long)Y_DIM + IN2_OFF[b];
+                        for (int i = 0; i < QB; ++i) {
+                            const int q = qq + 2 * i, r = 8 * q + w8;
+                            const bool live = r < rows;
+                            const float* xr = xb + (long long)q * (8 * X_DIM);
+                            const float* yr = yb + (long long)q * (8 * Y_DIM);
 #pragma unroll
-                        for (int i = 0; i < D1; ++i) xs[q][i] = (live && u < MU) ? __ldg(xrow + u * D1 + i) : 0.f;
+                            for (int c = 0; c < D1; ++c) xs[i][c] = live && u_live ? __ldg(xr + c) : 0.f;
 #pragma unroll
-                        for (int j = 0; j < D2; ++j) ys[q][j] = live ? __ldg(yrow + j) : 0.f;
-                    }
-                    const bool prof = p.prof && blockIdx.x == 0 && warp == 0 && lane == 0;
-                    const long long t0 = prof ? clock64() : 0;
-                    if (use > 0) ok = mbar_wait(bars.a_empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TC_A_EMPTY);
-                    const long long t1 = prof ? clock64() : 0;
-                    if (ok) {
-                        unsigned char* hi = smem + TC_OFF_A + s * TC_STAGE_BYTES;
-                        unsigned char* lo = hi + TC_STAGE_HALF;
+                            for (int c = 0; c < D2; ++c) ys[i][c] = UNIT_Y ? 1.f : (live ? __ldg(yr + c) : 0.f);
+                        }
+                        if (!waited) {          // (the first loads overlap the wait for the stage to be handed back)
+                            ok = mbar_wait(bars.a_empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TC_A_EMPTY);
+                            waited = true;
+                            if (!ok) break;
+                        }
 #pragma unroll
-                        for (int q = 0; q < RW; ++q) {
-                            const int r = warp + q * TC_PRODUCER_WARPS;
+                        for (int i = 0; i < QB; ++i) {
+                            const int q = qq + 2 * i, r = 8 * q + w8;
                             if (r < rows) {
                                 float t[D3];
 #pragma unroll
@@ -167,27 +199,27 @@ __device__ __forceinline__ bool tc_produce_output(const UvwTcParams& p, unsigned
                                 sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
                                     constexpr int N = n_;
                                     if constexpr (N == CG_BEGIN[P] || CG_I[N] != CG_I[N - 1] || CG_J[N] != CG_J[N - 1])
-                                        xy = xs[q][CG_I[N]] * ys[q][CG_J[N]];
+                                        xy = UNIT_Y ? xs[i][CG_I[N]] : xs[i][CG_I[N]] * ys[i][CG_J[N]];
                                     t[CG_K[N]] = fmaf(xy, (float)CG_V[N], t[CG_K[N]]);
                                 });
+                                unsigned char* hq = hi + q * 1024;
 #pragma unroll
                                 for (int k = 0; k < D3; ++k) {
-                                    const int off = tc_swizzle(r * D3 + k, lane);
+                                    unsigned char* dst = FAST ? hq + k * (RPC / 8) * 1024
+                                                              : smem + TC_OFF_A + s * TC_STAGE_BYTES + tc_swizzle(k * RPC + r, lane);
                                     const float th = tf32_hi(t[k]);
-                                    *reinterpret_cast<float*>(hi + off) = th;
-                                    *reinterpret_cast<float*>(lo + off) = t[k] - th;   // exact; read as TF32 by the MMA
+                                    *reinterpret_cast<float*>(dst) = th;
+                                    *reinterpret_cast<float*>(dst + TC_STAGE_HALF) = t[k] - th;     // exact; read as TF32 by the MMA
                                 }
                             }
                         }
+                    }
+                    // (a warp without rows in this stage still waits: the stage may not be announced early)
+                    if (ok && !waited) ok = mbar_wait(bars.a_empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TC_A_EMPTY);
+                    if (ok) {
                         fence_async_smem();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bars.a_full + s);
-                        if (prof) {
-                            const long long t2 = clock64();
-                            atomicAdd(p.prof + 0, (unsigned long long)(t1 - t0));   // wait for the stage
-                            atomicAdd(p.prof + 1, (unsigned long long)(t2 - t1));   // loads landing, T, stores
-                            atomicAdd(p.prof + 2, 1ull);
-                        }
                     }
                     ++stage_it;
                 }
@@ -203,8 +235,8 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
                                               long long row_lo, long long row_hi, long long& stage_it, long long& acc_it,
                                               int& w_use, unsigned tmem_base) {
     constexpr int D3 = OUT_D[O];
-    constexpr int RPC = 128 / D3;
-    constexpr int MW = OUT_MUL[O];
+    constexpr int RPC = tc_rpc(O);
+    constexpr int MW = tc_mwp(O);
     // Issuing a tcgen05.mma costs about 90 cycles whatever its size, so hi.hi and hi.lo go out as one MMA: the
     // lo tile of the weights follows the hi tile in shared memory, and a B descriptor over 2 MW rows covers
     // both.  The accumulator tile is then [hi.hi + lo.hi | hi.lo], summed by the epilogue.
@@ -304,8 +336,8 @@ __device__ __forceinline__ bool tc_epilogue_output(const UvwTcParams& p, unsigne
                                                    long long row_lo, long long row_hi, long long& acc_it,
                                                    unsigned tmem_base, int ewarp, int lane) {
     constexpr int D3 = OUT_D[O];
-    constexpr int RPC = 128 / D3;
-    constexpr int MW = OUT_MUL[O];
+    constexpr int RPC = tc_rpc(O);
+    constexpr int MW = OUT_MUL[O], MWP = tc_mwp(O);
     constexpr bool WIDE = tc_wide(O);
     constexpr int ACC_COLS = TC_ACC_COLS;
     constexpr int NACC = TC_NACC;
@@ -325,13 +357,13 @@ __device__ __forceinline__ bool tc_epilogue_output(const UvwTcParams& p, unsigne
         ok = tc_epilogue_all(ok);
         if (!ok) break;
         tc_fence_after();
-        // (ewarp is the warp's TMEM lane quarter) accumulator row m = 32 * ewarp + lane holds (row m / D3, component m % D3) for all w
+        // (ewarp is the warp's TMEM lane quarter) accumulator row m = 32 * ewarp + lane holds (row m % RPC, component m / RPC) for all w
         const unsigned taddr = tmem_base + ((unsigned)(ewarp * 32) << 16) + (unsigned)(t * ACC_COLS);
 #pragma unroll
-        for (int c0 = 0; c0 < MW; c0 += 16) {
+        for (int c0 = 0; c0 < MWP; c0 += 16) {
             unsigned v[16], v2[16];
             tc_load16(taddr + (unsigned)c0, v);
-            if constexpr (WIDE) tc_load16(taddr + (unsigned)(MW + c0), v2);   // the hi.lo half of the tile
+            if constexpr (WIDE) tc_load16(taddr + (unsigned)(MWP + c0), v2);   // the hi.lo half of the tile
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
@@ -343,12 +375,12 @@ __device__ __forceinline__ bool tc_epilogue_output(const UvwTcParams& p, unsigne
         tc_fence_before();
         asm volatile("bar.sync 1, %0;" ::"n"(TC_EPILOGUE_WARPS * 32) : "memory");
         if (et == 0) mbar_arrive(bars.acc_empty + t);   // the accumulator tile may be overwritten
-        // staged rows (row * D3 + k) x w  ->  Z[row][OUT_OFF + w * D3 + k], contiguous per batch row
+        // staged rows (k * RPC + row) x w  ->  Z[row][OUT_OFF + w * D3 + k], contiguous per batch row
         constexpr int ROWLEN = MW * D3;
         for (int e = et; e < rows * ROWLEN; e += TC_EPILOGUE_WARPS * 32) {
             const int r = e / ROWLEN, j = e - r * ROWLEN;
             const int w = j / D3, k = j - w * D3;
-            p.Z[(b0 + r) * (long long)Z_DIM + OUT_OFF[O] + j] = stg[(r * D3 + k) * TC_STG_PITCH + w];
+            p.Z[(b0 + r) * (long long)Z_DIM + OUT_OFF[O] + j] = stg[(k * RPC + r) * TC_STG_PITCH + w];
         }
         asm volatile("bar.sync 1, %0;" ::"n"(TC_EPILOGUE_WARPS * 32) : "memory");
         if (prof) {
@@ -459,21 +491,15 @@ extern "C" __global__ void oeq_uvw_pack_weights(const float* __restrict__ W, flo
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     oeq::sfor<0, N_INSTR>([&](auto p_) {
         constexpr int P = p_;
-        constexpr int O = I_OUT[P], MU = IN1_MUL[I_IN1[P]], MW = OUT_MUL[O];
+        constexpr int O = I_OUT[P], MU = IN1_MUL[I_IN1[P]], MW = OUT_MUL[O], MWP = oeq::tc_mwp(O);
         constexpr int KH = oeq::tc_khalves(P), BLOCK = oeq::tc_block_bytes(O);
         unsigned char* base = reinterpret_cast<unsigned char*>(packed) + oeq::tc_w_offset(O) +
                               oeq::tc_blocks_before(O, P) * 2 * BLOCK;
-        for (int e = tid; e < KH * MW * 32; e += nthreads) {
-            const int col = e & 31, w = (e >> 5) % MW, h = e / (32 * MW);
+        for (int e = tid; e < KH * MWP * 32; e += nthreads) {
+            const int col = e & 31, w = (e >> 5) % MWP, h = e / (32 * MWP);
             const int u = h * 32 + col;
             float v = 0.f;
-            if (u < MU) {
-                // kernel weight order: 32-wide (u, w) chunks, u-chunk major, each chunk [u][w] (v == 1)
-                const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
-                const int ulen = (MU - (uc << 5)) < 32 ? (MU - (uc << 5)) : 32;
-                const int wlen = (MW - (wc << 5)) < 32 ? (MW - (wc << 5)) : 32;
-                v = W[W_OFF[P] + (uc << 5) * MW + ulen * (wc << 5) + ul * wlen + wl];
-            }
+            if (u < MU && w < MW) v = W[TRANSPOSED_W ? oeq::tc_weight_offset<P, MW, MU>(w, u) : oeq::tc_weight_offset<P, MU, MW>(u, w)];
             const float hi = oeq::tf32_round(v), lo = oeq::tf32_round(v - hi);
             unsigned char* blk = base + h * 2 * BLOCK;
             *reinterpret_cast<float*>(blk + oeq::tc_swizzle(w, col)) = hi;
