@@ -134,7 +134,10 @@ struct Problem {
     std::vector<Instr> instr;
     int dtype = 0, shared = 0, mode = 0;
     bool unit_y = false;        // the second input is the number 1 for every row (no array)
-    bool transposed_w = false;  // the weight array is that of the problem with first input and output exchanged
+    bool transposed_w = false;  // the weight array is that of the problem with first input and output exchanged, and an
+                                // output block joins several of its paths (subs, per instruction)
+    struct Sub { int start, mul, w_off; };
+    std::vector<std::vector<Sub>> subs;
     int unit = 0;               // no weight array: every weight is 1 (shared_weights == 2 in the descriptor)
     int x_dim = 0, y_dim = 0, z_dim = 0, w_numel = 0;
     int elem() const { return dtype == OEQ_F64 ? 8 : 4; }
@@ -734,6 +737,19 @@ std::string descriptor_text(const Problem& p, const Mapping& m, const UvwConfig*
     s << "constexpr int X_DIM = " << p.x_dim << ", Y_DIM = " << p.y_dim << ", Z_DIM = " << p.z_dim
       << ", W_NUMEL = " << p.w_numel << ";\n";
     s << "constexpr bool SHARED_W = " << (p.shared ? "true" : "false") << ";\n";
+    if (p.mode == OEQ_MODE_UVW) {
+        auto put = [](std::ostringstream& o, int v) { o << v; };
+        std::vector<int> begin = {0}, start, mul, off;
+        for (size_t n = 0; n < p.instr.size(); ++n) {
+            if (n < p.subs.size())
+                for (const Problem::Sub& q : p.subs[n]) { start.push_back(q.start); mul.push_back(q.mul); off.push_back(q.w_off); }
+            begin.push_back((int)start.size());
+        }
+        emit_array(s, "int", "SUB_BEGIN", begin, put);
+        emit_array(s, "int", "SUB_START", start, put);
+        emit_array(s, "int", "SUB_MUL", mul, put);
+        emit_array(s, "int", "SUB_WOFF", off, put);
+    }
     s << "constexpr bool UNIT_Y = " << (p.unit_y ? "true" : "false") << ", TRANSPOSED_W = " << (p.transposed_w ? "true" : "false") << ";\n";
     s << "constexpr bool UNIT_W = " << (p.unit ? "true" : "false") << ";\n";
     s << "constexpr int N_IN1 = " << p.in1.size() << ", N_IN2 = " << p.in2.size() << ", N_OUT = " << p.out.size()
@@ -1283,6 +1299,8 @@ constexpr int K_UVW_TC_FWD = 20;
 struct TcGeometry {
     size_t packed_bytes = 0;
     int smem = 0;
+    int producers = 16, epilogues = 1;      // producer warps, groups of four epilogue warps
+    int threads() const { return 32 * (producers + 1 + 4 * epilogues); }
 };
 
 // `pad`: output multiplicities may be rounded up to 16 (the products W dZ of the backward pass).
@@ -1307,15 +1325,18 @@ bool uvw_tc_geometry(const Problem& p, TcGeometry& g, bool pad = false) {
         total += bytes;
     }
     if (total == 0) return false;
+    g.producers = p.unit_y ? 8 : 16;
+    g.epilogues = p.unit_y ? 2 : 1;
     const int off_w = 2 * 2 * 128 * 128;
     const int off_stg = off_w + (w_max + 1023) / 1024 * 1024;
-    const int off_bar = off_stg + (128 * (mw_max + 1) * 4 + 15) / 16 * 16;
+    const int pitch = (g.epilogues > 1 ? 32 : std::min(mw_max, 64)) + 1;
+    const int off_bar = off_stg + g.epilogues * ((128 * pitch * 4 + 15) / 16 * 16);
     g.smem = off_bar + (2 * 2 + 2 * 32 + 2) * 8 + 16 + 1024;
     g.packed_bytes = total;
     return g.smem <= SMEM_LIMIT;
 }
 
-int build_uvw_tc(const Problem& p, Kernel& k) {
+int build_uvw_tc(const Problem& p, const TcGeometry& g, Kernel& k) {
     k.is_uvw = true;
     int rc = choose_uvw(p, false, k.uvw);
     if (rc) return rc;
@@ -1323,7 +1344,8 @@ int build_uvw_tc(const Problem& p, Kernel& k) {
     k.map.part_of_instr.assign(p.instr.size(), 0);
     k.map.zr_off.assign(p.out.size(), 0);
     k.map.xr_off.assign(p.in1.size(), 0);
-    rc = compile_kernel(descriptor_text(p, k.map, &k.uvw), "uvw_tc_kernels.cuh", K_UVW_TC_FWD, k.code);
+    const std::string roles = "#define TC_PW " + std::to_string(g.producers) + "\n#define TC_EPI " + std::to_string(g.epilogues) + "\n";
+    rc = compile_kernel(descriptor_text(p, k.map, &k.uvw) + roles, "uvw_tc_kernels.cuh", K_UVW_TC_FWD, k.code);
     if (rc) return rc;
     k.compiled = true;
     return OEQ_OK;
@@ -1369,23 +1391,40 @@ void uvw_gradient_problems(const Problem& p, Problem& product, Problem& channels
     channels.mode = OEQ_MODE_UVU;
     channels.shared = 0;
     channels.unit = 1;
-    channels.out.clear();
+    channels.out.assign(p.instr.size(), Irrep());
     int off = 0;
-    for (size_t n = 0; n < p.instr.size(); ++n) {
-        const Instr& t = p.instr[n];
-        Irrep block = p.out[t.io];
-        block.mul = p.in1[t.i1].mul;
-        block.off = off;
-        off += block.mul * block.dim;
-        product.out.push_back(block);
-        channels.out.push_back(block);
-        Instr q = t;
-        q.i1 = t.io; q.i2 = 0; q.io = (int)n; q.pw = 1.0;
-        q.ci.clear(); q.cj.clear(); q.ck.clear(); q.cv.clear();
-        for (int k = 0; k < block.dim; ++k) { q.ci.push_back(k); q.cj.push_back(0); q.ck.push_back(k); q.cv.push_back(1.0); }
-        product.instr.push_back(q);
-        channels.instr[n].io = (int)n;
-        channels.instr[n].mode = OEQ_MODE_UVU;
+    for (size_t o = 0; o < p.out.size(); ++o) {
+        // the paths into o read the same dZ tiles: joined in one output block of up to 256 channels, as far as the
+        // weights of a block fit 128 KB of shared memory
+        const int slices = (p.out[o].mul + 31) / 32, cap = std::min(256, 131072 / (slices * 256) / 16 * 16);
+        bool open = false;
+        for (size_t n = 0; n < p.instr.size(); ++n) {
+            const Instr& t = p.instr[n];
+            if (t.io != (int)o) continue;
+            const int mul = p.in1[t.i1].mul, dim = p.out[o].dim;
+            if (!open || product.out.back().mul + mul > cap) {
+                Irrep block = p.out[o];
+                block.mul = 0;
+                block.off = off;
+                product.out.push_back(block);
+                Instr q = t;
+                q.i1 = (int)o; q.i2 = 0; q.io = (int)product.out.size() - 1; q.pw = 1.0;
+                q.ci.clear(); q.cj.clear(); q.ck.clear(); q.cv.clear();
+                for (int k = 0; k < dim; ++k) { q.ci.push_back(k); q.cj.push_back(0); q.ck.push_back(k); q.cv.push_back(1.0); }
+                product.instr.push_back(q);
+                product.subs.emplace_back();
+                open = true;
+            }
+            Irrep& block = product.out.back();
+            product.subs.back().push_back({block.mul, mul, t.w_off});
+            channels.out[n] = p.out[o];
+            channels.out[n].mul = mul;
+            channels.out[n].off = off;
+            channels.instr[n].io = (int)n;
+            channels.instr[n].mode = OEQ_MODE_UVU;
+            block.mul += mul;
+            off += mul * dim;
+        }
     }
     product.z_dim = channels.z_dim = off;
 }
@@ -1444,7 +1483,7 @@ int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
 int build_uvw_gradients(const Problem& p, Problem& product, Problem& channels, TcGeometry& g, Kernel& kp, Kernel& kc) {
     uvw_gradient_problems(p, product, channels);
     if (!uvw_tc_geometry(product, g, true)) return fail(OEQ_ERR_UNSUPPORTED, "rows do not fit the tensor-core product");
-    int rc = build_uvw_tc(product, kp);
+    int rc = build_uvw_tc(product, g, kp);
     if (!rc) rc = build_uvu(channels, K_BWD_BATCH, kc);
     return rc;
 }
@@ -1717,7 +1756,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         Kernel f, b, tc;
         if ((rc = build_tp(p, false, f)) || (rc = build_tp(p, true, b))) return rc;
         TcGeometry g;
-        if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, tc))) return rc;
+        if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, g, tc))) return rc;
         int smem = 0;
         Kernel dw, product, channels;
         if (uvw_tc_dw_geometry(p, smem)) {
@@ -1778,7 +1817,7 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
     if (!rc) rc = build_tp(h->prob, false, h->fwd);
     if (!rc) rc = build_tp(h->prob, true, h->bwd);
     if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
-        rc = build_uvw_tc(h->prob, h->fwd_tc);
+        rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
         h->has_tc = rc == OEQ_OK;
     }
     if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem)) {
@@ -1842,11 +1881,11 @@ static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack, voi
 }
 
 // `pack`: the weights have to be brought into the operand layout first (once per call).
-static int launch_uvw_tc(Kernel& k, cudaKernel_t pack_fn, void* packed, bool pack, long long batch, const void* X, const void* Y,
+static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn, void* packed, bool pack, long long batch, const void* X, const void* Y,
                          const void* W, void* Z, int* status, cudaStream_t st) {
     if (pack) {
         void* args[] = {(void*)&W, &packed};
-        OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(64), dim3(256), args, 0, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(264), dim3(256), args, 0, st));
     }
     struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; unsigned long long* prof; }
         tp{X, Y, packed, Z, batch, status, nullptr};
@@ -1857,7 +1896,7 @@ static int launch_uvw_tc(Kernel& k, cudaKernel_t pack_fn, void* packed, bool pac
         // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr
         OEQ_CUDA(cudaMalloc(&tp.prof, 32 * 8));
         OEQ_CUDA(cudaMemsetAsync(tp.prof, 0, 32 * 8, st));
-        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
         unsigned long long hb[32];
         OEQ_CUDA(cudaMemcpyAsync(hb, tp.prof, sizeof hb, cudaMemcpyDeviceToHost, st));
         OEQ_CUDA(cudaStreamSynchronize(st));
@@ -1867,7 +1906,7 @@ static int launch_uvw_tc(Kernel& k, cudaKernel_t pack_fn, void* packed, bool pac
         return OEQ_OK;
     }
 #endif
-    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3(21 * 32), args, (size_t)k.smem, st));
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
     return OEQ_OK;
 }
 
@@ -1881,7 +1920,7 @@ int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const
     h->last_stream = (cudaStream_t)stream;
     if (h->has_tc) {
         if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed))) return rc;
-        return launch_uvw_tc(h->fwd_tc, h->pack_fn, h->d_packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
+        return launch_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     }
     if (h->prob.mode == OEQ_MODE_UVW) {
         if ((rc = load_uvw(h->fwd, h->prob, false))) return rc;
@@ -1976,7 +2015,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
                 if ((rc = load_kernel(h->grad_channels_k, "oeq_uvu_kernel", false))) return rc;
                 for (long long b0 = 0; b0 < batch; b0 += block) {
                     const long long rows = std::min<long long>(block, batch - b0);
-                    if ((rc = launch_uvw_tc(h->grad_product_k, h->pack_t_fn, h->d_packed_t, b0 == 0, rows,
+                    if ((rc = launch_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t, b0 == 0, rows,
                                             (const char*)dZ + (size_t)b0 * p.z_dim * 4, nullptr, W, workspace, h->d_status, st))) return rc;
                     UvuParams prm{};
                     prm.X = (const char*)X + (size_t)b0 * p.x_dim * 4;
@@ -2081,7 +2120,7 @@ static int launch_info(const Kernel& k, int* threads, int* ng, int* ps, int* sta
 int oeq_tp_launch_info(const oeq_tp* h, int which, int* threads, int* ng, int* ps, int* stages, int* smem, int* regs) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
     if (!which && h->has_tc) {
-        if (threads) *threads = 21 * 32;
+        if (threads) *threads = h->tc.threads();
         if (ng) *ng = 1;
         if (ps) *ps = 1;
         if (stages) *stages = 2;

@@ -36,9 +36,13 @@ struct UvwTcParams {
     unsigned long long* prof;   // optional cycle accounting of CTA 0 (development aid), else null
 };
 
-constexpr int TC_PRODUCER_WARPS = 16;
-constexpr int TC_EPILOGUE_WARPS = 4;
-constexpr int TC_THREADS = (TC_PRODUCER_WARPS + 1 + TC_EPILOGUE_WARPS) * 32;
+// Roles (macros from the host): TC_PW producer warps (8 or 16) and TC_EPI groups of four epilogue warps.  Forward pass:
+// 16 and 1, since forming T bounds it.  The product W dZ of the backward pass (UNIT_Y): 8 and 2; its operand tiles are
+// dZ itself and serve up to 256 columns, and writing dT bounds it.
+constexpr int TC_PRODUCER_WARPS = TC_PW;
+constexpr int TC_EPI_GROUPS = TC_EPI;
+constexpr int TC_EPILOGUE_WARPS = 4;            // of one group
+constexpr int TC_THREADS = (TC_PRODUCER_WARPS + 1 + TC_EPI_GROUPS * TC_EPILOGUE_WARPS) * 32;
 constexpr int TC_NA = 2;                       // A-operand stages
 constexpr int TC_STAGE_HALF = 128 * 128;       // one [128 rows x 32 tf32] swizzled tile
 constexpr int TC_STAGE_BYTES = 2 * TC_STAGE_HALF;   // hi + lo
@@ -82,14 +86,17 @@ constexpr int tc_acc_cols_max() {
 constexpr int TC_ACC_COLS = tc_acc_cols_max();
 constexpr int TC_W_MAX = tc_w_max();
 constexpr int TC_MW_MAX = tc_mw_max();
-constexpr int TC_STG_PITCH = TC_MW_MAX + 1;    // floats per staged accumulator row (odd: conflict free)
+// An accumulator tile is drained in blocks of columns, dealt to the epilogue groups.
+constexpr int TC_BLOCK_COLS = TC_EPI_GROUPS > 1 ? 32 : (TC_MW_MAX < 64 ? TC_MW_MAX : 64);
+constexpr int TC_STG_PITCH = TC_BLOCK_COLS + 1;     // floats per staged accumulator row (odd: conflict free)
+constexpr int TC_STG_BYTES = (128 * TC_STG_PITCH * 4 + 15) / 16 * 16;
 constexpr int TC_TMEM_COLS = 512;
 
 // shared memory map (1024-byte aligned base): [A stages][W of one output][epilogue staging][barriers]
 constexpr int TC_OFF_A = 0;
 constexpr int TC_OFF_W = TC_OFF_A + TC_NA * TC_STAGE_BYTES;
 constexpr int TC_OFF_STG = TC_OFF_W + (TC_W_MAX + 1023) / 1024 * 1024;
-constexpr int TC_OFF_BAR = TC_OFF_STG + (128 * TC_STG_PITCH * 4 + 15) / 16 * 16;
+constexpr int TC_OFF_BAR = TC_OFF_STG + TC_EPI_GROUPS * TC_STG_BYTES;
 constexpr int TC_MAX_ACC = 32;
 constexpr int TC_NACC = TC_TMEM_COLS / TC_ACC_COLS < TC_MAX_ACC ? TC_TMEM_COLS / TC_ACC_COLS : TC_MAX_ACC;
 constexpr int TC_SMEM_BYTES = TC_OFF_BAR + (2 * TC_NA + 2 * TC_MAX_ACC + 2) * 8 + 16 + 1024;   // + alignment slack
@@ -110,14 +117,13 @@ struct TcBars {
     }
 };
 
-// Offset of W_p[u, w] (MU x MW, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks,
-// u-chunk major, each chunk [u][w].
-template <int P, int MU, int MW>
-__device__ __forceinline__ int tc_weight_offset(int u, int w) {
+// Offset of W[u, w] (mu x mw, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks, u-chunk
+// major, each chunk [u][w].
+__device__ __forceinline__ int tc_weight_offset(int mu, int mw, int u, int w) {
     const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
-    const int ulen = (MU - (uc << 5)) < 32 ? (MU - (uc << 5)) : 32;
-    const int wlen = (MW - (wc << 5)) < 32 ? (MW - (wc << 5)) : 32;
-    return W_OFF[P] + (uc << 5) * MW + ulen * (wc << 5) + ul * wlen + wl;
+    const int ulen = (mu - (uc << 5)) < 32 ? (mu - (uc << 5)) : 32;
+    const int wlen = (mw - (wc << 5)) < 32 ? (mw - (wc << 5)) : 32;
+    return (uc << 5) * mw + ulen * (wc << 5) + ul * wlen + wl;
 }
 
 // rows of the batch owned by this CTA
@@ -134,97 +140,149 @@ constexpr int tc_rpc(int o) {
     return r8 * OUT_D[o] >= 112 ? r8 : full;
 }
 
+constexpr int tc_first_path(int o) {
+    for (int p = 0; p < N_INSTR; ++p)
+        if (I_OUT[p] == o) return p;
+    return 0;
+}
+constexpr int tc_d1_max(int o) {
+    int m = 1;
+    for (int p = 0; p < N_INSTR; ++p)
+        if (I_OUT[p] == o && IN1_D[I_IN1[p]] > m) m = IN1_D[I_IN1[p]];
+    return m;
+}
+constexpr int tc_d2_max(int o) {
+    int m = 1;
+    for (int p = 0; p < N_INSTR; ++p)
+        if (I_OUT[p] == o && IN2_D[I_IN2[p]] > m) m = IN2_D[I_IN2[p]];
+    return m;
+}
+// Rows of a producer step: a warp's rows of a stage (at most one of every two groups of eight) are taken in steps whose
+// inputs fit 24 registers, twice (the step at work and the one on its way).
+constexpr int TC_SETS = TC_PRODUCER_WARPS / 8;
+constexpr int tc_rows_of_warp(int o) { return ((tc_rpc(o) + 7) / 8 + TC_SETS - 1) / TC_SETS; }
+constexpr int tc_steps(int o) {
+    const int per = tc_d1_max(o) + (UNIT_Y ? 0 : tc_d2_max(o)), fit = 24 / per > 0 ? 24 / per : 1;
+    return (tc_rows_of_warp(o) + fit - 1) / fit;
+}
+// Steps of the paths into o that come before path p_end, and the path of step n.
+constexpr int tc_sequence(int o, int p_end) {
+    int n = 0;
+    for (int p = 0; p < p_end; ++p)
+        if (I_OUT[p] == o) n += tc_khalves(p) * tc_steps(o);
+    return n;
+}
+constexpr int tc_seq_path(int o, int n) {
+    for (int p = 0; p < N_INSTR; ++p)
+        if (I_OUT[p] == o && n < tc_sequence(o, p + 1)) return p;
+    return 0;
+}
+constexpr int tc_step_rows(int o) { return (tc_rows_of_warp(o) + tc_steps(o) - 1) / tc_steps(o); }
+
 // ---------------------------------------------------------------------------- producers
 //
-// Bound by issue: 39 instructions per element of T when every store computed its swizzled address and every row its
-// predicates.  Warp w takes the rows r = w mod 8 (mod 8); the two sets of eight warps take alternate groups of eight
-// rows, swapped from stage to stage so that an odd number of groups does not leave one set waiting.
+// Bound by issue once the inputs' latency is hidden.  Warp w takes the rows r = w mod 8 (mod 8); the two sets of eight
+// warps take alternate groups of eight rows, swapped from stage to stage so that an odd number of groups does not leave
+// one set waiting.  The inputs of a step are fetched while the step before it is formed (a warp has one to three rows
+// of a stage: fetched at their use they paid the L2 latency once per stage).
 template <int O>
 __device__ __forceinline__ bool tc_produce_output(const UvwTcParams& p, unsigned char* smem, const TcBars& bars,
                                                   long long row_lo, long long row_hi, long long& stage_it, int warp,
                                                   int lane) {
     constexpr int D3 = OUT_D[O];
     constexpr int RPC = tc_rpc(O);
-    static_assert(TC_PRODUCER_WARPS == 16, "two sets of eight warps");
+    static_assert(TC_PRODUCER_WARPS % 8 == 0, "sets of eight warps");
     constexpr bool FAST = RPC % 8 == 0;
-    constexpr int Q = (RPC + 7) / 8;            // groups of eight rows
+    constexpr int STEPS = tc_steps(O), R = tc_step_rows(O);
     const int w8 = warp & 7, set = warp >> 3;
     const int base = w8 * 128 + (((lane >> 2) ^ w8) << 4) + ((lane & 3) << 2);
+    constexpr int SEQ = tc_sequence(O, N_INSTR);       // steps of a chunk; step n uses buffer n mod 2
+    float x[2][R][tc_d1_max(O)], y[2][R][tc_d2_max(O)];
+    auto first = [&](int st) { return TC_SETS == 2 ? (set + st) & 1 : set; };      // first group of eight rows in stage st
+    // inputs of path P for step j of the stage with index st: half h of the chunk at b0
+    auto fetch = [&](auto p_, long long b0, int h, int st, int j, auto& xv, auto& yv) {
+        constexpr int P = p_;
+        constexpr int a = I_IN1[P], b = I_IN2[P], D1 = IN1_D[a], D2 = IN2_D[b], MU = IN1_MUL[a];
+        const int r0 = 8 * (first(st) + TC_SETS * j * R) + w8;
+        const int rows = (int)(row_hi - b0 < RPC ? row_hi - b0 : RPC);
+        const bool u_live = MU % 32 == 0 || h * 32 + lane < MU;
+        const float* xr = p.X + (b0 + r0) * (long long)X_DIM + IN1_OFF[a] + (h * 32 + lane) * D1;
+        const float* yr = p.Y + (b0 + r0) * (long long)Y_DIM + IN2_OFF[b];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const bool live = r0 + 8 * TC_SETS * i < rows;
+#pragma unroll
+            for (int c = 0; c < D1; ++c) xv[i][c] = live && u_live ? __ldg(xr + i * (8 * TC_SETS * X_DIM) + c) : 0.f;
+            if constexpr (!UNIT_Y) {
+#pragma unroll
+                for (int c = 0; c < D2; ++c) yv[i][c] = live ? __ldg(yr + i * (8 * TC_SETS * Y_DIM) + c) : 0.f;
+            }
+        }
+    };
     bool ok = true;
+    if (row_lo < row_hi) fetch(IC<tc_first_path(O)>{}, row_lo, 0, (int)(stage_it & 1), 0, x[0], y[0]);
     for (long long b0 = row_lo; b0 < row_hi && ok; b0 += RPC) {
         const int rows = (int)(row_hi - b0 < RPC ? row_hi - b0 : RPC);
-        sfor<0, N_INSTR>([&](auto p_) {
-            constexpr int P = p_;
-            if constexpr (I_OUT[P] == O) {
-                constexpr int a = I_IN1[P], b = I_IN2[P];
-                constexpr int D1 = IN1_D[a], D2 = IN2_D[b], MU = IN1_MUL[a];
-                constexpr int QB = D1 + D2 + D3 <= 6 ? 8 : (D1 + D2 + D3 <= 14 ? 2 : 1);    // groups whose loads go out together
-                for (int h = 0; h < tc_khalves(P) && ok; ++h) {
-                    const int s = (int)(stage_it % TC_NA);
-                    const long long use = stage_it / TC_NA;
-                    const int q0 = (set + (int)stage_it) & 1;
-                    const int u = h * 32 + lane;
-                    const bool u_live = MU % 32 == 0 || u < MU;
-                    const float* xb = p.X + (b0 + w8) * (long long)X_DIM + IN1_OFF[a] + u * D1;
-                    const float* yb = p.Y + (b0 + w8) * (long long)Y_DIM + IN2_OFF[b];
-                    unsigned char* hi = smem + TC_OFF_A + s * TC_STAGE_BYTES + base;
-                    bool waited = use == 0;
-#pragma unroll 1
-                    for (int qq = q0; qq < Q && ok; qq += 2 * QB) {
-                        float xs[QB][D1], ys[QB][D2];
+        sfor<0, SEQ>([&](auto n_) {
+            constexpr int NN = n_, P = tc_seq_path(O, NN), KH = tc_khalves(P), W = NN - tc_sequence(O, P);
+            constexpr int h = W / STEPS, j = W % STEPS;
+            if (ok) {
+                auto& xc = x[NN & 1];
+                auto& yc = y[NN & 1];
+                auto& xn = x[(NN + 1) & 1];
+                auto& yn = y[(NN + 1) & 1];
+                const int s = (int)(stage_it % TC_NA), odd = (int)(stage_it & 1);
+                if constexpr (j + 1 < STEPS) fetch(IC<P>{}, b0, h, odd, j + 1, xn, yn);
+                else if constexpr (h + 1 < KH) fetch(IC<P>{}, b0, h + 1, odd ^ 1, 0, xn, yn);
+                else if constexpr (NN + 1 < SEQ) fetch(IC<tc_seq_path(O, NN + 1)>{}, b0, 0, odd ^ 1, 0, xn, yn);
+                else if (b0 + RPC < row_hi) fetch(IC<tc_first_path(O)>{}, b0 + RPC, 0, odd ^ 1, 0, xn, yn);
+                if (j == 0 && stage_it >= TC_NA)
+                    ok = mbar_wait(bars.a_empty + s, (unsigned)((stage_it / TC_NA - 1) & 1), p.status, ERR_TC_A_EMPTY);
+                if (ok) {
+                    unsigned char* tile = smem + TC_OFF_A + s * TC_STAGE_BYTES;
+                    const int q0 = first(odd);
 #pragma unroll
-                        for (int i = 0; i < QB; ++i) {
-                            const int q = qq + 2 * i, r = 8 * q + w8;
-                            const bool live = r < rows;
-                            const float* xr = xb + (long long)q * (8 * X_DIM);
-                            const float* yr = yb + (long long)q * (8 * Y_DIM);
+                    for (int i = 0; i < R; ++i) {
+                        const int q = q0 + TC_SETS * (j * R + i), r = 8 * q + w8;
+                        if (r < rows) {
+                            float t[D3];
 #pragma unroll
-                            for (int c = 0; c < D1; ++c) xs[i][c] = live && u_live ? __ldg(xr + c) : 0.f;
+                            for (int k = 0; k < D3; ++k) t[k] = 0.f;
+                            float xy = 0.f;
+                            sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto c_) {
+                                constexpr int N = c_;
+                                if constexpr (N == CG_BEGIN[P] || CG_I[N] != CG_I[N - 1] || CG_J[N] != CG_J[N - 1])
+                                    xy = UNIT_Y ? xc[i][CG_I[N]] : xc[i][CG_I[N]] * yc[i][CG_J[N]];
+                                t[CG_K[N]] = fmaf(xy, (float)CG_V[N], t[CG_K[N]]);
+                            });
+                            unsigned char* hq = tile + base + q * 1024;
 #pragma unroll
-                            for (int c = 0; c < D2; ++c) ys[i][c] = UNIT_Y ? 1.f : (live ? __ldg(yr + c) : 0.f);
-                        }
-                        if (!waited) {          // (the first loads overlap the wait for the stage to be handed back)
-                            ok = mbar_wait(bars.a_empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TC_A_EMPTY);
-                            waited = true;
-                            if (!ok) break;
-                        }
-#pragma unroll
-                        for (int i = 0; i < QB; ++i) {
-                            const int q = qq + 2 * i, r = 8 * q + w8;
-                            if (r < rows) {
-                                float t[D3];
-#pragma unroll
-                                for (int k = 0; k < D3; ++k) t[k] = 0.f;
-                                float xy = 0.f;
-                                sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
-                                    constexpr int N = n_;
-                                    if constexpr (N == CG_BEGIN[P] || CG_I[N] != CG_I[N - 1] || CG_J[N] != CG_J[N - 1])
-                                        xy = UNIT_Y ? xs[i][CG_I[N]] : xs[i][CG_I[N]] * ys[i][CG_J[N]];
-                                    t[CG_K[N]] = fmaf(xy, (float)CG_V[N], t[CG_K[N]]);
-                                });
-                                unsigned char* hq = hi + q * 1024;
-#pragma unroll
-                                for (int k = 0; k < D3; ++k) {
-                                    unsigned char* dst = FAST ? hq + k * (RPC / 8) * 1024
-                                                              : smem + TC_OFF_A + s * TC_STAGE_BYTES + tc_swizzle(k * RPC + r, lane);
-                                    const float th = tf32_hi(t[k]);
-                                    *reinterpret_cast<float*>(dst) = th;
-                                    *reinterpret_cast<float*>(dst + TC_STAGE_HALF) = t[k] - th;     // exact; read as TF32 by the MMA
-                                }
+                            for (int k = 0; k < D3; ++k) {
+                                unsigned char* dst = FAST ? hq + k * (RPC / 8) * 1024 : tile + tc_swizzle(k * RPC + r, lane);
+                                const float th = tf32_hi(t[k]);
+                                *reinterpret_cast<float*>(dst) = th;
+                                *reinterpret_cast<float*>(dst + TC_STAGE_HALF) = t[k] - th;     // exact; read as TF32 by the MMA
                             }
                         }
                     }
-                    // (a warp without rows in this stage still waits: the stage may not be announced early)
-                    if (ok && !waited) ok = mbar_wait(bars.a_empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TC_A_EMPTY);
-                    if (ok) {
+                    if constexpr (j + 1 == STEPS) {
                         fence_async_smem();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bars.a_full + s);
+                        ++stage_it;
                     }
-                    ++stage_it;
                 }
             }
         });
+        if constexpr (SEQ % 2 == 1) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+#pragma unroll
+                for (int c = 0; c < tc_d1_max(O); ++c) x[0][i][c] = x[1][i][c];
+#pragma unroll
+                for (int c = 0; c < tc_d2_max(O); ++c) y[0][i][c] = y[1][i][c];
+            }
+        }
     }
     return ok;
 }
@@ -319,14 +377,14 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
 }
 
 // ---------------------------------------------------------------------------- epilogue warps
-// AND-reduction of a flag over the epilogue warps (hardware barrier 1).
-__device__ __forceinline__ bool tc_epilogue_all(bool ok) {
+// AND-reduction of a flag over the warps of an epilogue group (hardware barrier 1 + group).
+__device__ __forceinline__ bool tc_epilogue_all(bool ok, int group) {
     unsigned r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-        "bar.red.and.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        "bar.red.and.pred p, %3, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(r)
-        : "r"((unsigned)ok), "n"(TC_EPILOGUE_WARPS * 32)
+        : "r"((unsigned)ok), "n"(TC_EPILOGUE_WARPS * 32), "r"(1 + group)
         : "memory");
     return r != 0;
 }
@@ -334,15 +392,16 @@ __device__ __forceinline__ bool tc_epilogue_all(bool ok) {
 template <int O>
 __device__ __forceinline__ bool tc_epilogue_output(const UvwTcParams& p, unsigned char* smem, const TcBars& bars,
                                                    long long row_lo, long long row_hi, long long& acc_it,
-                                                   unsigned tmem_base, int ewarp, int lane) {
+                                                   unsigned tmem_base, int ewarp, int lane, int group) {
     constexpr int D3 = OUT_D[O];
     constexpr int RPC = tc_rpc(O);
     constexpr int MW = OUT_MUL[O], MWP = tc_mwp(O);
     constexpr bool WIDE = tc_wide(O);
     constexpr int ACC_COLS = TC_ACC_COLS;
     constexpr int NACC = TC_NACC;
-    float* stg = reinterpret_cast<float*>(smem + TC_OFF_STG);
+    float* stg = reinterpret_cast<float*>(smem + TC_OFF_STG + group * TC_STG_BYTES);
     const int et = ewarp * 32 + lane;
+    const bool z_aligned = (reinterpret_cast<unsigned long long>(p.Z) & 15) == 0;
     bool ok = true;
     for (long long b0 = row_lo; b0 < row_hi && ok; b0 += RPC) {
         const int rows = (int)(row_hi - b0 < RPC ? row_hi - b0 : RPC);
@@ -354,35 +413,65 @@ __device__ __forceinline__ bool tc_epilogue_output(const UvwTcParams& p, unsigne
         if (prof) atomicAdd(p.prof + 16, (unsigned long long)(clock64() - t0));
         const long long t1 = prof ? clock64() : 0;
         // the four warps must agree before anyone touches the staging buffer or skips a barrier
-        ok = tc_epilogue_all(ok);
+        ok = tc_epilogue_all(ok, group);
         if (!ok) break;
         tc_fence_after();
         // (ewarp is the warp's TMEM lane quarter) accumulator row m = 32 * ewarp + lane holds (row m % RPC, component m / RPC) for all w
         const unsigned taddr = tmem_base + ((unsigned)(ewarp * 32) << 16) + (unsigned)(t * ACC_COLS);
+        constexpr int BLOCKS = (MWP + TC_BLOCK_COLS - 1) / TC_BLOCK_COLS, NT = TC_EPILOGUE_WARPS * 32;
+        const int first = (group + (int)(acc_it % TC_EPI_GROUPS)) % TC_EPI_GROUPS;
+        bool drained = BLOCKS <= first;             // the group has no block of this tile
+        if (drained && et == 0) mbar_arrive(bars.acc_empty + t);
+        sfor<0, BLOCKS>([&](auto b_) {
+            constexpr int B = b_, C0 = B * TC_BLOCK_COLS;
+            constexpr int COLS = MWP - C0 < TC_BLOCK_COLS ? MWP - C0 : TC_BLOCK_COLS, LIVE = MW - C0 < COLS ? MW - C0 : COLS;
+            if (B % TC_EPI_GROUPS == first) {
 #pragma unroll
-        for (int c0 = 0; c0 < MWP; c0 += 16) {
-            unsigned v[16], v2[16];
-            tc_load16(taddr + (unsigned)c0, v);
-            if constexpr (WIDE) tc_load16(taddr + (unsigned)(MWP + c0), v2);   // the hi.lo half of the tile
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c0 = 0; c0 < COLS; c0 += 16) {
+                    unsigned v[16], v2[16];
+                    tc_load16(taddr + (unsigned)(C0 + c0), v);
+                    if constexpr (WIDE) tc_load16(taddr + (unsigned)(MWP + C0 + c0), v2);   // the hi.lo half of the tile
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                float val = __uint_as_float(v[c]);
-                if constexpr (WIDE) val += __uint_as_float(v2[c]);
-                stg[(ewarp * 32 + lane) * TC_STG_PITCH + c0 + c] = val;
+                    for (int c = 0; c < 16; ++c) {
+                        float val = __uint_as_float(v[c]);
+                        if constexpr (WIDE) val += __uint_as_float(v2[c]);
+                        stg[(ewarp * 32 + lane) * TC_STG_PITCH + c0 + c] = val;
+                    }
+                }
+                tc_fence_before();
+                asm volatile("bar.sync %1, %0;" ::"n"(NT), "r"(1 + group) : "memory");
+                if (B + TC_EPI_GROUPS >= BLOCKS && et == 0) mbar_arrive(bars.acc_empty + t);    // the group is done with the tile
+                // staged rows (k * RPC + row) x w  ->  Z[row][OUT_OFF + w * D3 + k], contiguous per batch row.  A thread keeps
+                // four consecutive values of a row and walks the rows: no index division and a quarter of the stores.
+                constexpr int ROWLEN = LIVE * D3, OFF = OUT_OFF[O] + C0 * D3;
+                constexpr bool VEC = ROWLEN % 4 == 0 && OFF % 4 == 0 && Z_DIM % 4 == 0;
+                if (VEC && z_aligned) {
+                    constexpr int TPR = (ROWLEN + 3) / 4, SIDE = TPR < NT ? NT / TPR : 1;      // threads per row, rows side by side
+                    if (TPR >= NT || et < SIDE * TPR) {
+#pragma unroll 1
+                        for (int j4 = TPR < NT ? et % TPR : et; j4 < TPR; j4 += TPR < NT ? TPR : NT) {
+                            int off[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) off[i] = ((4 * j4 + i) % D3 * RPC) * TC_STG_PITCH + (4 * j4 + i) / D3;
+                            float* zrow = p.Z + b0 * (long long)Z_DIM + OFF + 4 * j4;
+#pragma unroll 4
+                            for (int r = TPR < NT ? et / TPR : 0; r < rows; r += SIDE) {
+                                const float* src = stg + r * TC_STG_PITCH;
+                                *reinterpret_cast<float4*>(zrow + r * (long long)Z_DIM) = make_float4(src[off[0]], src[off[1]], src[off[2]], src[off[3]]);
+                            }
+                        }
+                    }
+                } else {
+                    for (int e = et; e < rows * ROWLEN; e += NT) {
+                        const int r = e / ROWLEN, j = e - r * ROWLEN;
+                        const int w = j / D3, k = j - w * D3;
+                        p.Z[(b0 + r) * (long long)Z_DIM + OFF + j] = stg[(k * RPC + r) * TC_STG_PITCH + w];
+                    }
+                }
+                asm volatile("bar.sync %1, %0;" ::"n"(NT), "r"(1 + group) : "memory");
             }
-        }
-        tc_fence_before();
-        asm volatile("bar.sync 1, %0;" ::"n"(TC_EPILOGUE_WARPS * 32) : "memory");
-        if (et == 0) mbar_arrive(bars.acc_empty + t);   // the accumulator tile may be overwritten
-        // staged rows (k * RPC + row) x w  ->  Z[row][OUT_OFF + w * D3 + k], contiguous per batch row
-        constexpr int ROWLEN = MW * D3;
-        for (int e = et; e < rows * ROWLEN; e += TC_EPILOGUE_WARPS * 32) {
-            const int r = e / ROWLEN, j = e - r * ROWLEN;
-            const int w = j / D3, k = j - w * D3;
-            p.Z[(b0 + r) * (long long)Z_DIM + OUT_OFF[O] + j] = stg[(k * RPC + r) * TC_STG_PITCH + w];
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(TC_EPILOGUE_WARPS * 32) : "memory");
+        });
         if (prof) {
             atomicAdd(p.prof + 17, (unsigned long long)(clock64() - t1));
             atomicAdd(p.prof + 18, 1ull);
@@ -414,7 +503,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
         }
         for (int i = 0; i < TC_MAX_ACC; ++i) {
             mbar_init(bars.acc_full + i, 1);
-            mbar_init(bars.acc_empty + i, 1);
+            mbar_init(bars.acc_empty + i, TC_EPI_GROUPS);
         }
         mbar_init(bars.w_full, 1);
         mbar_init(bars.w_free, 1);
@@ -464,7 +553,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
             constexpr int O = o_;
             if constexpr (tc_output_has_paths(O)) {
                 // a warp may only read the TMEM lanes of its own quarter: 32 * (warp index mod 4)
-                if (ok) ok = tc_epilogue_output<O>(p, smem, bars, row_lo, row_hi, acc_it, tmem_base, warp & 3, lane);
+                if (ok) ok = tc_epilogue_output<O>(p, smem, bars, row_lo, row_hi, acc_it, tmem_base, warp & 3, lane, (warp - TC_PRODUCER_WARPS - 1) / TC_EPILOGUE_WARPS);
             }
         });
     }
@@ -499,7 +588,18 @@ extern "C" __global__ void oeq_uvw_pack_weights(const float* __restrict__ W, flo
             const int col = e & 31, w = (e >> 5) % MWP, h = e / (32 * MWP);
             const int u = h * 32 + col;
             float v = 0.f;
-            if (u < MU && w < MW) v = W[TRANSPOSED_W ? oeq::tc_weight_offset<P, MW, MU>(w, u) : oeq::tc_weight_offset<P, MU, MW>(u, w)];
+            if (u < MU && w < MW) {
+                if constexpr (TRANSPOSED_W) {
+                    // output channels are those of several paths: the weights of path q, [its channels][MU], from row SUB_START[q] on
+                    oeq::sfor<SUB_BEGIN[P], SUB_BEGIN[P + 1]>([&](auto q_) {
+                        constexpr int q = q_;
+                        if (w >= SUB_START[q] && w < SUB_START[q] + SUB_MUL[q])
+                            v = W[SUB_WOFF[q] + oeq::tc_weight_offset(SUB_MUL[q], MU, w - SUB_START[q], u)];
+                    });
+                } else {
+                    v = W[W_OFF[P] + oeq::tc_weight_offset(MU, MW, u, w)];
+                }
+            }
             const float hi = oeq::tf32_round(v), lo = oeq::tf32_round(v - hi);
             unsigned char* blk = base + h * 2 * BLOCK;
             *reinterpret_cast<float*>(blk + oeq::tc_swizzle(w, col)) = hi;
