@@ -113,7 +113,7 @@ def register_ops(forward, gradient, handle, *, deterministic=False, shared=False
                  second=None):
     """Register the torch ops ``openequivariance_b200::<forward>`` and ``::<gradient>`` of one operator (native kernels
     and autograd, ``csrc/oeq_torch.cpp``) and return their overloads.  ``dims``: x, y, z row lengths and the number of
-    weights; ``second``: an op already registered for the second derivatives."""
+    weights; ``second``: an op already registered that may replace the second derivatives (``call_second``)."""
     global _torch_lib
     import torch
     lib()
@@ -123,6 +123,7 @@ def register_ops(forward, gradient, handle, *, deterministic=False, shared=False
             t = C.CDLL(build_torch_library())
             t.oeq_torch_error.restype = C.c_char_p
             t.oeq_torch_register.argtypes = [C.c_char_p] * 3 + [_P, _P] + [_INT] * 4 + [_I64] * 4
+            t.oeq_torch_call_second.argtypes = [C.c_char_p, _INT]
             _torch_lib = t
     is_conv = isinstance(handle, ConvHandle)
     code = _torch_lib.oeq_torch_register(forward.encode(), gradient.encode(), second.encode() if second else None,
@@ -144,6 +145,11 @@ def register_ops(forward, gradient, handle, *, deterministic=False, shared=False
         return [t.new_empty(*t.shape) for t in args[:3 if has_weights else 2]]
 
     return ops
+
+
+def call_second(forward, call: bool):
+    """Let the second backward pass of the operator with this forward op call its registered ``second`` op."""
+    _torch_lib.oeq_torch_call_second(forward.encode(), int(call))
 
 
 def check(code: int):

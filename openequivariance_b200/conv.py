@@ -108,6 +108,7 @@ class TensorProductConv(TensorProductBase):
         self.deterministic = deterministic
         self.conv_id = next(_conv_ids)
         self._scratch = {}
+        self._second_replacement = None
         self.workspace_size = 0
         self.workspace_ptr = 0
         self.unit_weights = False
@@ -244,7 +245,18 @@ class TensorProductConv(TensorProductBase):
     def _has_fused_double_backward(self):
         return self.internal.has_double_backward()
 
-    def _double_backward_impl(self, x, y, w, dz, ex, ey, ew, rows, cols, perm=None):
+    @property
+    def _double_backward_impl(self):
+        """``(x, y, w, dz, ex, ey, ew, rows, cols[, perm]) -> (gx, gy, gw, gdz)`` or ``None``.  Autograd runs the same
+        launches natively; a replacement that is assigned here is what autograd calls."""
+        return self._second_replacement or self._fused_second
+
+    @_double_backward_impl.setter
+    def _double_backward_impl(self, replacement):
+        self._second_replacement = replacement
+        _native.call_second(f"conv_forward{self.conv_id}", True)
+
+    def _fused_second(self, x, y, w, dz, ex, ey, ew, rows, cols, perm=None):
         """Gradients of ``<ex, dX> + <ey, dY> + <ew, dW>`` with respect to (x, y, w, dz) in two fused launches, or
         ``None`` when the library cannot run them here (no scratch memory for the deterministic variant)."""
         self._check(x, y, w, rows, cols, perm)

@@ -184,4 +184,13 @@ __device__ __forceinline__ void red_add(T* addr, T v) {
     atomicAdd(addr, v);
 }
 
+// Offset of W[u, w] (mu x mw, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks, u-chunk
+// major, each chunk [u][w].
+__device__ __forceinline__ int weight_offset_v1(int mu, int mw, int u, int w) {
+    const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
+    const int ulen = (mu - (uc << 5)) < 32 ? (mu - (uc << 5)) : 32;
+    const int wlen = (mw - (wc << 5)) < 32 ? (mw - (wc << 5)) : 32;
+    return (uc << 5) * mw + ulen * (wc << 5) + ul * wlen + wl;
+}
+
 }  // namespace oeq

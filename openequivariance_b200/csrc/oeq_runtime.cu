@@ -1299,6 +1299,7 @@ constexpr int K_UVW_TC_FWD = 20;
 struct TcGeometry {
     size_t packed_bytes = 0;
     int smem = 0;
+    unsigned paths = 1;                     // instructions (the weights of each are packed by blocks of their own)
     int producers = 16, epilogues = 1;      // producer warps, groups of four epilogue warps
     int threads() const { return 32 * (producers + 1 + 4 * epilogues); }
 };
@@ -1333,6 +1334,7 @@ bool uvw_tc_geometry(const Problem& p, TcGeometry& g, bool pad = false) {
     const int off_bar = off_stg + g.epilogues * ((128 * pitch * 4 + 15) / 16 * 16);
     g.smem = off_bar + (2 * 2 + 2 * 32 + 2) * 8 + 16 + 1024;
     g.packed_bytes = total;
+    g.paths = (unsigned)p.instr.size();
     return g.smem <= SMEM_LIMIT;
 }
 
@@ -1486,6 +1488,51 @@ int build_uvw_gradients(const Problem& p, Problem& product, Problem& channels, T
     int rc = build_uvw_tc(product, g, kp);
     if (!rc) rc = build_uvu(channels, K_BWD_BATCH, kc);
     return rc;
+}
+
+// ---- FP64 with shared weights as register-tiled GEMMs (uvw_gemm_kernels.cuh).  Multiplicities below 16 would fill less
+// than a quarter of a tile's edge and keep the tiled kernel.
+constexpr int K_UVW_GEMM = 14, K_UVW_GEMM_DW = 15, GEMM_TILE = 64, GEMM_SMEM = 4 * 32 * 66 * 8;
+
+bool uvw_gemm_supported(const Problem& p) {
+    if (p.mode != OEQ_MODE_UVW || !p.shared || p.dtype != OEQ_F64) return false;
+    for (const Irrep& r : p.in2)
+        if (r.mul != 1) return false;
+    for (const std::vector<Irrep>* v : {&p.in1, &p.out})
+        for (const Irrep& r : *v)
+            if (r.mul < 16 || r.dim > 32) return false;
+    return true;
+}
+
+int build_uvw_gemm(const Problem& p, int kernel_id, Kernel& k) {
+    k.is_uvw = true;
+    k.map.part_of_out.assign(p.out.size(), 0);
+    k.map.part_of_instr.assign(p.instr.size(), 0);
+    k.map.zr_off.assign(p.out.size(), 0);
+    k.map.xr_off.assign(p.in1.size(), 0);
+    k.uvw.threads = 256;
+    int rc = compile_kernel(descriptor_text(p, k.map), "uvw_gemm_kernels.cuh", kernel_id, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
+// The three kernels of the backward pass: weight gradient, dT = W dZ, and dX, dY from dT.
+int build_uvw_gemm_backward(const Problem& p, Problem& product, Problem& channels, Kernel& dw, Kernel& kp, Kernel& kc) {
+    uvw_gradient_problems(p, product, channels);
+    product.dtype = p.dtype;
+    int rc = build_uvu(channels, K_BWD_BATCH, kc);
+    if (!rc) rc = build_uvw_gemm(p, K_UVW_GEMM_DW, dw);
+    if (!rc) rc = build_uvw_gemm(product, K_UVW_GEMM, kp);
+    return rc;
+}
+
+// Shares of the rows in the weight gradient: about six CTAs per SM, 64 rows or more each.
+long long gemm_shares(const Problem& p, long long batch, long long sm_count) {
+    long long tiles = 0;
+    for (const Instr& t : p.instr)
+        tiles += (long long)((p.in1[t.i1].mul + GEMM_TILE - 1) / GEMM_TILE) * ((p.out[t.io].mul + GEMM_TILE - 1) / GEMM_TILE);
+    return std::max<long long>(1, std::min((6 * sm_count + tiles - 1) / std::max<long long>(1, tiles), batch / 64));
 }
 
 int build_tp(const Problem& p, bool bwd, Kernel& k) {
@@ -1695,6 +1742,8 @@ struct oeq_tp {
     bool has_grad_tc = false;
     void* d_packed_t = nullptr; // the transposed weights, split and swizzled
     cudaKernel_t pack_t_fn = nullptr;
+    Kernel gemm, gemm_dw;       // FP64 with shared weights: the product and the weight gradient as GEMMs
+    bool has_gemm = false, has_gemm_bwd = false;
     Kernel dbl;                 // one-pass second derivatives ('uvu', per-row weights)
     bool has_dbl = false;
     TcGeometry tc;
@@ -1754,7 +1803,16 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
     if (p.mode == OEQ_MODE_UVW) {
         if (kinds & 6) return fail(OEQ_ERR_UNSUPPORTED, "fused convolution supports 'uvu' problems only");
         Kernel f, b, tc;
-        if ((rc = build_tp(p, false, f)) || (rc = build_tp(p, true, b))) return rc;
+        if (uvw_gemm_supported(p)) {
+            Problem pp, pc;
+            Kernel dw, kp, kc;
+            if ((rc = build_uvw_gemm(p, K_UVW_GEMM, f))) return rc;
+            rc = build_uvw_gemm_backward(p, pp, pc, dw, kp, kc);
+            if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
+        } else if ((rc = build_tp(p, false, f))) {
+            return rc;
+        }
+        if ((rc = build_tp(p, true, b))) return rc;
         TcGeometry g;
         if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, g, tc))) return rc;
         int smem = 0;
@@ -1814,7 +1872,16 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
     *out = nullptr;
     oeq_tp* h = new oeq_tp();
     int rc = ingest(desc, h->prob);
-    if (!rc) rc = build_tp(h->prob, false, h->fwd);
+    if (!rc && uvw_gemm_supported(h->prob)) {
+        rc = build_uvw_gemm(h->prob, K_UVW_GEMM, h->gemm);
+        h->has_gemm = rc == OEQ_OK;
+        if (!rc) {
+            const int rc2 = build_uvw_gemm_backward(h->prob, h->grad_product, h->grad_channels, h->gemm_dw, h->grad_product_k, h->grad_channels_k);
+            h->has_gemm_bwd = rc2 == OEQ_OK;
+            if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
+        }
+    }
+    if (!rc && !h->has_gemm) rc = build_tp(h->prob, false, h->fwd);
     if (!rc) rc = build_tp(h->prob, true, h->bwd);
     if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
         rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
@@ -1847,7 +1914,7 @@ int oeq_tp_destroy(oeq_tp* h) {
     if (h->d_status) cudaFree(h->d_status);
     if (h->d_packed) cudaFree(h->d_packed);
     if (h->d_packed_t) cudaFree(h->d_packed_t);
-    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->dbl})
+    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
         if (k->lib) cudaLibraryUnload(k->lib);
     delete h;
     return OEQ_OK;
@@ -1885,7 +1952,7 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
                          const void* W, void* Z, int* status, cudaStream_t st) {
     if (pack) {
         void* args[] = {(void*)&W, &packed};
-        OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(264), dim3(256), args, 0, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(16, geo.paths), dim3(256), args, 0, st));
     }
     struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; unsigned long long* prof; }
         tp{X, Y, packed, Z, batch, status, nullptr};
@@ -1910,6 +1977,43 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
     return OEQ_OK;
 }
 
+// Mirror of oeq::UvwGemmParams (uvw_gemm_kernels.cuh).
+struct UvwGemmParams {
+    const void* X; const void* Y; const void* W; const void* dZ;
+    void* Z; void* ws;
+    long long batch;
+    int shares;
+};
+
+static int load_gemm(Kernel& k) {
+    if (k.loaded) return OEQ_OK;
+    OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+    OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_gemm_kernel"));
+    OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, "oeq_reduce_partials"));
+    int dev = 0;
+    OEQ_CUDA(cudaGetDevice(&dev));
+    OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
+    k.smem = GEMM_SMEM;
+    OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+    k.loaded = true;
+    return OEQ_OK;
+}
+
+// Z (or dT) = the product of problem `p` over `batch` rows.
+static int launch_gemm(Kernel& k, const Problem& p, long long batch, const void* X, const void* Y, const void* W, void* Z, cudaStream_t st) {
+    int rc = load_gemm(k);
+    if (rc) return rc;
+    UvwGemmParams prm{X, Y, W, nullptr, Z, nullptr, batch, 1};
+    int y = 0, rows = GEMM_TILE;
+    for (const Irrep& r : p.out) {
+        y += (r.mul + GEMM_TILE - 1) / GEMM_TILE;
+        rows = std::min(rows, GEMM_TILE / r.dim);
+    }
+    void* args[] = {&prm};
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)((batch + rows - 1) / rows), (unsigned)y), dim3(256), args, (size_t)k.smem, st));
+    return OEQ_OK;
+}
+
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
@@ -1922,6 +2026,7 @@ int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const
         if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed))) return rc;
         return launch_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     }
+    if (h->has_gemm) return launch_gemm(h->gemm, h->prob, batch, X, Y, W, Z, (cudaStream_t)stream);
     if (h->prob.mode == OEQ_MODE_UVW) {
         if ((rc = load_uvw(h->fwd, h->prob, false))) return rc;
         UvwParams up{};
@@ -1949,6 +2054,8 @@ size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch) {
     } else {
         groups = 256ll * 4 * h->bwd.map.ng;
     }
+    if (h->has_gemm_bwd)
+        return std::max((size_t)gemm_shares(h->prob, batch, 256) * h->prob.w_numel * 8, std::min((size_t)batch * h->grad_product.z_dim * 8, UVW_DT_BYTES));
     size_t bytes = (size_t)groups * h->prob.w_numel * h->prob.elem();
     if (h->has_grad_tc) bytes = std::max(bytes, std::min((size_t)batch * h->grad_product.z_dim * 4, UVW_DT_BYTES));
     return bytes;
@@ -1967,6 +2074,48 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
     if (!X || !Y || !W || !dZ || !dX || !dY || !dW) return fail(OEQ_ERR_INVALID, "null buffer");
     int rc = ensure_status(&h->d_status);
     if (rc) return rc;
+    // dX and dY of a shared-weight problem from dT rows in the workspace (blocks of the batch when they do not all fit)
+    auto gradients_from_dt = [&](long long block, auto&& product) -> int {
+        const size_t e = p.elem();
+        int r = load_kernel(h->grad_channels_k, "oeq_uvu_kernel", false);
+        for (long long b0 = 0; b0 < batch && !r; b0 += block) {
+            const long long rows = std::min<long long>(block, batch - b0);
+            if ((r = product(b0, rows, (const char*)dZ + (size_t)b0 * p.z_dim * e))) break;
+            UvuParams prm{};
+            prm.X = (const char*)X + (size_t)b0 * p.x_dim * e;
+            prm.Y = (const char*)Y + (size_t)b0 * p.y_dim * e;
+            prm.dZ = workspace;
+            prm.dX = (char*)dX + (size_t)b0 * p.x_dim * e;
+            prm.dY = (char*)dY + (size_t)b0 * p.y_dim * e;
+            prm.n_items = rows; prm.n_nodes = rows; prm.status = h->d_status;
+            r = launch_uvu(h->grad_channels_k, h->grad_channels, prm, st);
+        }
+        return r;
+    };
+    if (h->has_gemm_bwd) {
+        const size_t wbytes = (size_t)p.w_numel * 8;
+        const long long block = workspace ? (long long)std::min<size_t>((size_t)batch, workspace_bytes / ((size_t)h->grad_product.z_dim * 8)) : 0;
+        if (workspace_bytes < wbytes || block < 1 || !aligned16(workspace))
+            return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
+        if ((rc = load_gemm(h->gemm_dw))) return rc;
+        h->last_stream = st;
+        Kernel& k = h->gemm_dw;
+        long long shares = std::min<long long>(gemm_shares(p, batch, k.sm_count), (long long)(workspace_bytes / wbytes));
+        int tiles = 0, n = p.w_numel;
+        for (const Instr& t : p.instr)
+            tiles += ((p.in1[t.i1].mul + GEMM_TILE - 1) / GEMM_TILE) * ((p.out[t.io].mul + GEMM_TILE - 1) / GEMM_TILE);
+        UvwGemmParams prm{X, Y, nullptr, dZ, nullptr, shares == 1 ? dW : workspace, batch, (int)shares};
+        void* args[] = {&prm};
+        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)shares, (unsigned)tiles), dim3(256), args, (size_t)k.smem, st));
+        if (shares > 1) {
+            const void* ws = workspace;
+            void* rargs[] = {&ws, &dW, &n, &shares};
+            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+        }
+        return gradients_from_dt(block, [&](long long, long long rows, const void* dz) {
+            return launch_gemm(h->grad_product_k, h->grad_product, rows, dz, nullptr, W, workspace, st);
+        });
+    }
     if (p.mode == OEQ_MODE_UVW) {
         if ((rc = load_uvw(h->bwd, p, true))) return rc;
         long long ctas = uvw_grid(h->bwd, batch);
@@ -2012,21 +2161,10 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             const long long block = h->has_grad_tc && aligned16(workspace) ? (long long)std::min<size_t>((size_t)batch, workspace_bytes / row) : 0;
             if (block > 0 && (block == batch || block >= 4096)) {
                 if ((rc = load_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t))) return rc;
-                if ((rc = load_kernel(h->grad_channels_k, "oeq_uvu_kernel", false))) return rc;
-                for (long long b0 = 0; b0 < batch; b0 += block) {
-                    const long long rows = std::min<long long>(block, batch - b0);
-                    if ((rc = launch_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t, b0 == 0, rows,
-                                            (const char*)dZ + (size_t)b0 * p.z_dim * 4, nullptr, W, workspace, h->d_status, st))) return rc;
-                    UvuParams prm{};
-                    prm.X = (const char*)X + (size_t)b0 * p.x_dim * 4;
-                    prm.Y = (const char*)Y + (size_t)b0 * p.y_dim * 4;
-                    prm.dZ = workspace;
-                    prm.dX = (char*)dX + (size_t)b0 * p.x_dim * 4;
-                    prm.dY = (char*)dY + (size_t)b0 * p.y_dim * 4;
-                    prm.n_items = rows; prm.n_nodes = rows; prm.status = h->d_status;
-                    if ((rc = launch_uvu(h->grad_channels_k, h->grad_channels, prm, st))) return rc;
-                }
-                return OEQ_OK;
+                return gradients_from_dt(block, [&](long long b0, long long rows, const void* dz) {
+                    return launch_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t, b0 == 0, rows, dz, nullptr, W, workspace,
+                                         h->d_status, st);
+                });
             }
         }
         void* args[] = {&up};

@@ -12,7 +12,9 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
+#include <atomic>
 #include <deque>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -37,6 +39,7 @@ struct Op {
     int64_t x_dim = 0, y_dim = 0, z_dim = 0, w_numel = 0;
     at::ScalarType dtype = at::kFloat;
     std::optional<OperatorHandle> forward, gradient, second;
+    std::atomic<bool> call_second{false};   // the caller replaced the fused second derivatives by the op `second`
     std::mutex mutex;
     std::vector<Tensor> scratch;    // large backward scratch, per device
 };
@@ -179,6 +182,28 @@ variable_list tp_second(const Op& op, at::ArrayRef<Tensor> in) {
     return out;
 }
 
+// Second derivatives of the convolution in its fused launches; empty where the library has none here (the caller composes
+// them).
+variable_list conv_second(Op& op, at::ArrayRef<Tensor> in, at::ArrayRef<Tensor> index) {
+    if (!oeq_conv_has_double_backward(op.conv)) return {};
+    variable_list c, out, idx;
+    for (const Tensor& t : in) c.push_back(t.contiguous());
+    for (const Tensor& t : index) idx.push_back(t.contiguous());
+    c10::cuda::CUDAGuard guard(c[0].device());
+    for (int i = 0; i < 4; ++i) out.push_back(at::empty_like(c[i]));
+    const int64_t nodes = c[0].size(0), edges = idx[0].size(0);
+    Tensor ws = op.deterministic ? backward_scratch(op, nodes, edges, c[0].options()) : Tensor();
+    const int rc = oeq_conv_double_backward(
+        op.conv, nodes, edges, c[0].const_data_ptr(), c[1].const_data_ptr(), c[2].const_data_ptr(), c[3].const_data_ptr(),
+        c[4].const_data_ptr(), c[5].const_data_ptr(), c[6].const_data_ptr(), index_ptr(idx[0]), index_ptr(idx[1]),
+        op.deterministic ? index_ptr(idx[2]) : nullptr, out[0].mutable_data_ptr(), out[1].mutable_data_ptr(), out[2].mutable_data_ptr(),
+        out[3].mutable_data_ptr(), ws.defined() ? ws.mutable_data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
+        c10::cuda::getCurrentCUDAStream().stream());
+    if (rc == OEQ_ERR_UNSUPPORTED) return {};
+    check(rc);
+    return out;
+}
+
 // ---------------------------------------------------------------- autograd
 
 Tensor call_forward(const Op& op, at::ArrayRef<Tensor> in) {
@@ -241,8 +266,9 @@ struct GradientFn : torch::autograd::Function<GradientFn> {
             // nothing differentiates through this result: launches that read a row's arrays once
             if (op.tp && oeq_tp_has_double_backward(op.tp)) return per_argument(tp_second(op, {x, y, w, dz, e[0], e[1], e[2]}), op);
         }
-        if (op.second && !at::GradMode::is_enabled()) {
-            variable_list all = call_list(*op.second, joined({x, y, w, dz, e[0], e[1], e[2]}, idx));
+        if (op.conv && !at::GradMode::is_enabled()) {
+            variable_list all = op.second && op.call_second ? call_list(*op.second, joined({x, y, w, dz, e[0], e[1], e[2]}, idx))
+                                                            : conv_second(op, {x, y, w, dz, e[0], e[1], e[2]}, idx);
             if (all.size() == 4) return per_argument(std::move(all), op);
         }
         variable_list a = call_list(*op.gradient, joined({e[0], e[1], w, dz}, idx));    // dX(ey, w), dY(ex, w)
@@ -282,6 +308,10 @@ std::deque<torch::Library>& libraries() {
     static auto* l = new std::deque<torch::Library>();      // ops stay registered until the process ends
     return *l;
 }
+std::map<std::string, Op*>& operators() {       // by the name of their forward op
+    static auto* m = new std::map<std::string, Op*>();
+    return *m;
+}
 std::mutex register_mutex;
 thread_local std::string register_error;
 
@@ -292,7 +322,8 @@ extern "C" {
 const char* oeq_torch_error() { return register_error.c_str(); }
 
 // Registers the forward op and the gradient op of one operator (`tp` or `conv`) in the namespace
-// openequivariance_b200.  `second`: name of an op (registered by the caller) for second derivatives, or null.
+// openequivariance_b200.  `second`: name of an op (registered by the caller) that may replace the fused second
+// derivatives (oeq_torch_call_second), or null.
 int oeq_torch_register(const char* forward, const char* gradient, const char* second, oeq_tp* tp, oeq_conv* conv, int deterministic,
                        int shared, int has_weights, int f64, int64_t x_dim, int64_t y_dim, int64_t z_dim, int64_t w_numel) {
     try {
@@ -325,11 +356,22 @@ int oeq_torch_register(const char* forward, const char* gradient, const char* se
         op->forward = dispatcher.findSchemaOrThrow((ns + "::" + forward).c_str(), "");
         op->gradient = dispatcher.findSchemaOrThrow((ns + "::" + gradient).c_str(), "");
         if (second) op->second = dispatcher.findSchemaOrThrow((ns + "::" + second).c_str(), "");
+        operators()[forward] = op;
         return 0;
     } catch (const std::exception& e) {
         register_error = e.what();
         return 1;
     }
+}
+
+// Whether the second backward pass of the operator with this forward op calls its op `second` (see oeq_torch_register)
+// instead of the library's fused launches.
+int oeq_torch_call_second(const char* forward, int call) {
+    std::lock_guard<std::mutex> lock(register_mutex);
+    auto it = operators().find(forward);
+    if (it == operators().end()) return 1;
+    it->second->call_second = call != 0;
+    return 0;
 }
 
 }  // extern "C"

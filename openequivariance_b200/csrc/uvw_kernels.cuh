@@ -386,7 +386,8 @@ extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     oeqd::T s = (oeqd::T)0;
-    for (long long g = 0; g < groups; ++g) s += ws[g * n + i];
+#pragma unroll 8        // (the loads go out together; the sum keeps its order)
+    for (int g = 0; g < (int)groups; ++g) s += ws[(long long)g * n + i];
     out[i] = s;
 }
 #else

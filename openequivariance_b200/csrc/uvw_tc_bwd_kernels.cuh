@@ -391,6 +391,7 @@ extern "C" __global__ void oeq_reduce_partials(const float* ws, float* out, int 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.f;
-    for (long long g = 0; g < groups; ++g) s += ws[g * n + i];
+#pragma unroll 8        // (the loads go out together; the sum keeps its order)
+    for (int g = 0; g < (int)groups; ++g) s += ws[(long long)g * n + i];
     out[i] = s;
 }

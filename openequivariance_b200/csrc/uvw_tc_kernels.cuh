@@ -117,15 +117,6 @@ struct TcBars {
     }
 };
 
-// Offset of W[u, w] (mu x mw, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks, u-chunk
-// major, each chunk [u][w].
-__device__ __forceinline__ int tc_weight_offset(int mu, int mw, int u, int w) {
-    const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
-    const int ulen = (mu - (uc << 5)) < 32 ? (mu - (uc << 5)) : 32;
-    const int wlen = (mw - (wc << 5)) < 32 ? (mw - (wc << 5)) : 32;
-    return (uc << 5) * mw + ulen * (wc << 5) + ul * wlen + wl;
-}
-
 // rows of the batch owned by this CTA
 __device__ __forceinline__ void tc_row_range(long long batch, long long& lo, long long& hi) {
     lo = batch * blockIdx.x / gridDim.x;
@@ -580,6 +571,7 @@ extern "C" __global__ void oeq_uvw_pack_weights(const float* __restrict__ W, flo
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     oeq::sfor<0, N_INSTR>([&](auto p_) {
         constexpr int P = p_;
+        if (blockIdx.y != P) return;
         constexpr int O = I_OUT[P], MU = IN1_MUL[I_IN1[P]], MW = OUT_MUL[O], MWP = oeq::tc_mwp(O);
         constexpr int KH = oeq::tc_khalves(P), BLOCK = oeq::tc_block_bytes(O);
         unsigned char* base = reinterpret_cast<unsigned char*>(packed) + oeq::tc_w_offset(O) +
@@ -594,10 +586,10 @@ extern "C" __global__ void oeq_uvw_pack_weights(const float* __restrict__ W, flo
                     oeq::sfor<SUB_BEGIN[P], SUB_BEGIN[P + 1]>([&](auto q_) {
                         constexpr int q = q_;
                         if (w >= SUB_START[q] && w < SUB_START[q] + SUB_MUL[q])
-                            v = W[SUB_WOFF[q] + oeq::tc_weight_offset(SUB_MUL[q], MU, w - SUB_START[q], u)];
+                            v = W[SUB_WOFF[q] + oeq::weight_offset_v1(SUB_MUL[q], MU, w - SUB_START[q], u)];
                     });
                 } else {
-                    v = W[W_OFF[P] + oeq::tc_weight_offset(MU, MW, u, w)];
+                    v = W[W_OFF[P] + oeq::weight_offset_v1(MU, MW, u, w)];
                 }
             }
             const float hi = oeq::tf32_round(v), lo = oeq::tf32_round(v - hi);

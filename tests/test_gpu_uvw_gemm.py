@@ -1,0 +1,39 @@
+"""Shared-weight 'uvw': the FP64 GEMM kernels and the joined products of the FP32 backward pass at remainders of their
+tiles (64 channels, 64 row-component pairs, 32 deep), one row, several shares of the rows, and paths that do not all fit
+one joined block."""
+import numpy as np
+import pytest
+import torch
+
+import openequivariance_b200 as oeq
+from oracle import tp_oracle as orc
+from helpers import REL_TOL, rel_err, tp_inputs, to_e3nn, to_oeq
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e", 1),
+    ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e", 300),
+    ("16x0e+80x1o", "0e+1o", "65x0e+16x1o+33x2e", 63),          # (33 and 65: not on the tensor cores)
+    ("48x1o+16x3o", "1o+2e", "16x0e+64x2e+32x4e", 130),
+    ("128x0e+128x1o", "0e+1o+2e", "128x0e+128x1o", 70),          # joined blocks of one path each
+    ("16x0e+16x1o", "0e+1o", "16x0e+16x1o+16x4e", 40),           # an output irrep without paths
+]
+
+
+@pytest.mark.parametrize("in1,in2,out,batch", CASES)
+@pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
+def test_shared_weights(in1, in2, out, batch, dtype):
+    p = oeq.FullyConnectedTPProblem(in1, in2, out, irrep_dtype=dtype, weight_dtype=dtype)
+    x, y, w, dz = tp_inputs(p, batch, 17)
+    w = (w / 8).astype(dtype)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
+    tp = oeq.TensorProduct(p, torch_op=True)
+    got = [tp(*dev[:3]), *tp.backward_helper(*dev)]
+    again = tp.backward_helper(*dev)
+    tp.check_device_status()
+    assert all(torch.equal(a, b) for a, b in zip(got[1:], again))
+    want = [orc.tp_forward(p, x, y, w), *orc.tp_backward(p, x, y, w, dz)]
+    for g, r in zip(got[:3], want):
+        assert rel_err(g.cpu().numpy(), r) < REL_TOL[dtype]
+    assert rel_err(to_e3nn(p, got[3].cpu().numpy()), want[3]) < REL_TOL[dtype]
