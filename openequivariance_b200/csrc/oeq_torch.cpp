@@ -9,7 +9,9 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/library.h>
 
 #include <atomic>
@@ -27,7 +29,6 @@ namespace {
 using at::Tensor;
 using c10::OperatorHandle;
 using c10::Stack;
-using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 struct Op {
@@ -46,23 +47,23 @@ struct Op {
 
 void check(int rc) { TORCH_CHECK(rc == OEQ_OK, "oeq_b200: ", oeq_last_error()); }
 
-// Argument i of the n on top of the stack.
-const Tensor& arg(const Stack& stack, int n, int i) { return stack[stack.size() - n + i].toTensor(); }
+typedef at::ArrayRef<Tensor> Args;
 
-void check_inputs(const Op& op, const Stack& stack, int n) {
-    for (int i = 0; i < n; ++i)
-        TORCH_CHECK(arg(stack, n, i).is_cuda(), "openequivariance_b200 runs on CUDA tensors only (there is no CPU fallback)");
-    const Tensor &x = arg(stack, n, 0), &y = arg(stack, n, 1);
+void check_inputs(const Op& op, Args in) {
+    const int n = (int)in.size();
+    for (const Tensor& t : in)
+        TORCH_CHECK(t.is_cuda(), "openequivariance_b200 runs on CUDA tensors only (there is no CPU fallback)");
+    const Tensor &x = in[0], &y = in[1];
     TORCH_CHECK_VALUE(x.dim() == 2 && x.size(1) == op.x_dim, op.conv ? "node features must be [nodes, " : "first input must be [batch, ",
                       op.x_dim, "], got ", x.sizes());
     int64_t rows_n = x.size(0);
     if (op.conv) {
-        const Tensor &rows = arg(stack, n, n - op.index), &cols = arg(stack, n, n - op.index + 1);
+        const Tensor &rows = in[n - op.index], &cols = in[n - op.index + 1];
         TORCH_CHECK_VALUE(rows.dim() == 1 && cols.sizes() == rows.sizes(), "rows and cols must be 1-D and of equal length");
         TORCH_CHECK_VALUE(rows.scalar_type() == at::kLong && cols.scalar_type() == at::kLong, "rows and cols must be int64");
         rows_n = rows.size(0);
         if (op.deterministic) {
-            const Tensor& perm = arg(stack, n, n - 1);
+            const Tensor& perm = in[n - 1];
             TORCH_CHECK_VALUE(perm.sizes() == rows.sizes() && perm.scalar_type() == at::kLong, "sender_perm must be int64 and as long as rows");
         }
     }
@@ -70,7 +71,7 @@ void check_inputs(const Op& op, const Stack& stack, int n) {
                       rows_n, ", ", op.y_dim, "], got ", y.sizes());
     TORCH_CHECK_VALUE(x.scalar_type() == op.dtype && y.scalar_type() == op.dtype, "tensors must be ", op.dtype);
     if (op.inputs == 3) {
-        const Tensor& w = arg(stack, n, 2);
+        const Tensor& w = in[2];
         TORCH_CHECK_VALUE(op.shared ? (w.dim() == 1 && w.size(0) == op.w_numel) : (w.dim() == 2 && w.size(0) == rows_n && w.size(1) == op.w_numel),
                           "weights must be [", op.shared ? "" : std::to_string(rows_n) + ", ", op.w_numel, "], got ", w.sizes());
         TORCH_CHECK_VALUE(w.scalar_type() == op.dtype, "tensors must be ", op.dtype);
@@ -81,29 +82,24 @@ const int64_t* index_ptr(const Tensor& t) { return static_cast<const int64_t*>(t
 
 // ---------------------------------------------------------------- CUDA kernels
 
-struct ForwardKernel final : c10::OperatorKernel {
-    Op* op;
-    explicit ForwardKernel(Op* o) : op(o) {}
-    void operator()(const OperatorHandle&, c10::DispatchKeySet, Stack* stack) {
-        const int n = op->inputs + op->index;
-        check_inputs(*op, *stack, n);
-        const Tensor x = arg(*stack, n, 0).contiguous(), y = arg(*stack, n, 1).contiguous();
-        const Tensor w = op->inputs == 3 ? arg(*stack, n, 2).contiguous() : Tensor();
-        const void* wp = op->inputs == 3 ? w.const_data_ptr() : nullptr;
-        c10::cuda::CUDAGuard guard(x.device());
-        Tensor z = at::empty({x.size(0), op->z_dim}, x.options());
-        void* st = c10::cuda::getCurrentCUDAStream().stream();
-        if (op->tp) {
-            check(oeq_tp_forward(op->tp, x.size(0), x.const_data_ptr(), y.const_data_ptr(), wp, z.mutable_data_ptr(), st));
-        } else {
-            const Tensor rows = arg(*stack, n, op->inputs).contiguous(), cols = arg(*stack, n, op->inputs + 1).contiguous();
-            check(oeq_conv_forward(op->conv, x.size(0), rows.size(0), x.const_data_ptr(), y.const_data_ptr(), wp, index_ptr(rows),
-                                   index_ptr(cols), z.mutable_data_ptr(), nullptr, 0, st));
-        }
-        torch::jit::drop(*stack, n);
-        stack->emplace_back(std::move(z));
+// Operands x, y[, w], then the index arrays.
+Tensor forward_cuda(const Op& op, Args in) {
+    check_inputs(op, in);
+    const auto x = in[0].expect_contiguous(), y = in[1].expect_contiguous();
+    const auto w = in[op.inputs == 3 ? 2 : 0].expect_contiguous();
+    const void* wp = op.inputs == 3 ? w->const_data_ptr() : nullptr;
+    c10::cuda::CUDAGuard guard(x->device());
+    Tensor z = at::empty({x->size(0), op.z_dim}, x->options());
+    void* st = c10::cuda::getCurrentCUDAStream().stream();
+    if (op.tp) {
+        check(oeq_tp_forward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, z.mutable_data_ptr(), st));
+    } else {
+        const auto rows = in[op.inputs].expect_contiguous(), cols = in[op.inputs + 1].expect_contiguous();
+        check(oeq_conv_forward(op.conv, x->size(0), rows->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, index_ptr(*rows),
+                               index_ptr(*cols), z.mutable_data_ptr(), nullptr, 0, st));
     }
-};
+    return z;
+}
 
 // Scratch of the deterministic backward pass.  Up to 256 MB come from the caching allocator call by call, safe with
 // any number of streams; more is kept on the operator (allocating it again and again would flush a full device's
@@ -129,43 +125,57 @@ Tensor backward_scratch(Op& op, int64_t nodes, int64_t edges, const at::TensorOp
     return kept;
 }
 
+// Operands x, y[, w], the output gradient, then the index arrays.
+variable_list gradient_cuda(Op& op, Args in) {
+    check_inputs(op, in);
+    const auto x = in[0].expect_contiguous(), y = in[1].expect_contiguous();
+    const auto w = in[op.inputs == 3 ? 2 : 0].expect_contiguous();
+    const auto dz = in[op.inputs].expect_contiguous();
+    TORCH_CHECK_VALUE(dz->dim() == 2 && dz->size(0) == x->size(0) && dz->size(1) == op.z_dim && dz->scalar_type() == op.dtype,
+                      "output gradient must be [", x->size(0), ", ", op.z_dim, "] of ", op.dtype, ", got ", dz->sizes());
+    c10::cuda::CUDAGuard guard(x->device());
+    variable_list out{at::empty_like(*x), at::empty_like(*y)};
+    if (op.inputs == 3) out.push_back(at::empty_like(*w));
+    const void* wp = op.inputs == 3 ? w->const_data_ptr() : nullptr;
+    void *dxp = out[0].mutable_data_ptr(), *dyp = out[1].mutable_data_ptr(), *dwp = op.inputs == 3 ? out[2].mutable_data_ptr() : nullptr;
+    void* st = c10::cuda::getCurrentCUDAStream().stream();
+    Tensor ws;
+    if (op.tp) {
+        const size_t bytes = oeq_tp_workspace_bytes(op.tp, x->size(0));
+        if (bytes) ws = at::empty({(int64_t)bytes}, x->options().dtype(at::kByte));
+        check(oeq_tp_backward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(), dxp, dyp, dwp,
+                              bytes ? ws.mutable_data_ptr() : nullptr, bytes, st));
+    } else {
+        const auto rows = in[op.inputs + 1].expect_contiguous(), cols = in[op.inputs + 2].expect_contiguous();
+        const auto perm = in[op.inputs + (op.deterministic ? 3 : 1)].expect_contiguous();
+        if (op.deterministic) ws = backward_scratch(op, x->size(0), rows->size(0), x->options());
+        check(oeq_conv_backward(op.conv, x->size(0), rows->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(),
+                                index_ptr(*rows), index_ptr(*cols), op.deterministic ? index_ptr(*perm) : nullptr, dxp, dyp, dwp,
+                                ws.defined() ? ws.mutable_data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0, st));
+    }
+    return out;
+}
+
+// The arguments on top of the stack.
+variable_list pop(Stack* stack, int n) {
+    variable_list in;
+    in.reserve(n);
+    for (auto it = stack->end() - n; it != stack->end(); ++it) in.push_back(std::move(*it).toTensor());
+    torch::jit::drop(*stack, n);
+    return in;
+}
+struct ForwardKernel final : c10::OperatorKernel {
+    Op* op;
+    explicit ForwardKernel(Op* o) : op(o) {}
+    void operator()(const OperatorHandle&, c10::DispatchKeySet, Stack* stack) {
+        stack->emplace_back(forward_cuda(*op, pop(stack, op->inputs + op->index)));
+    }
+};
 struct GradientKernel final : c10::OperatorKernel {
     Op* op;
     explicit GradientKernel(Op* o) : op(o) {}
     void operator()(const OperatorHandle&, c10::DispatchKeySet, Stack* stack) {
-        const int n = op->inputs + 1 + op->index;
-        check_inputs(*op, *stack, n);
-        const Tensor x = arg(*stack, n, 0).contiguous(), y = arg(*stack, n, 1).contiguous();
-        const Tensor w = op->inputs == 3 ? arg(*stack, n, 2).contiguous() : Tensor();
-        const Tensor dz = arg(*stack, n, op->inputs).contiguous();
-        TORCH_CHECK_VALUE(dz.dim() == 2 && dz.size(0) == x.size(0) && dz.size(1) == op->z_dim && dz.scalar_type() == op->dtype,
-                          "output gradient must be [", x.size(0), ", ", op->z_dim, "] of ", op->dtype, ", got ", dz.sizes());
-        c10::cuda::CUDAGuard guard(x.device());
-        Tensor dx = at::empty_like(x), dy = at::empty_like(y), dw = op->inputs == 3 ? at::empty_like(w) : Tensor();
-        const void* wp = op->inputs == 3 ? w.const_data_ptr() : nullptr;
-        void* dwp = op->inputs == 3 ? dw.mutable_data_ptr() : nullptr;
-        void* st = c10::cuda::getCurrentCUDAStream().stream();
-        Tensor ws;
-        if (op->tp) {
-            const size_t bytes = oeq_tp_workspace_bytes(op->tp, x.size(0));
-            if (bytes) ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
-            check(oeq_tp_backward(op->tp, x.size(0), x.const_data_ptr(), y.const_data_ptr(), wp, dz.const_data_ptr(), dx.mutable_data_ptr(),
-                                  dy.mutable_data_ptr(), dwp, bytes ? ws.mutable_data_ptr() : nullptr, bytes, st));
-        } else {
-            const Tensor rows = arg(*stack, n, op->inputs + 1).contiguous(), cols = arg(*stack, n, op->inputs + 2).contiguous();
-            const Tensor perm = op->deterministic ? arg(*stack, n, op->inputs + 3).contiguous() : Tensor();
-            ws = op->deterministic ? backward_scratch(*op, x.size(0), rows.size(0), x.options()) : Tensor();
-            check(oeq_conv_backward(op->conv, x.size(0), rows.size(0), x.const_data_ptr(), y.const_data_ptr(), wp, dz.const_data_ptr(),
-                                    index_ptr(rows), index_ptr(cols), perm.defined() ? index_ptr(perm) : nullptr, dx.mutable_data_ptr(),
-                                    dy.mutable_data_ptr(), dwp, ws.defined() ? ws.mutable_data_ptr() : nullptr,
-                                    ws.defined() ? (size_t)ws.numel() : 0, st));
-        }
-        torch::jit::drop(*stack, n);
-        c10::List<Tensor> out;
-        out.push_back(std::move(dx));
-        out.push_back(std::move(dy));
-        if (op->inputs == 3) out.push_back(std::move(dw));
-        stack->emplace_back(std::move(out));
+        stack->emplace_back(c10::List<Tensor>(gradient_cuda(*op, pop(stack, op->inputs + 1 + op->index))));
     }
 };
 
@@ -206,78 +216,113 @@ variable_list conv_second(Op& op, at::ArrayRef<Tensor> in, at::ArrayRef<Tensor> 
 
 // ---------------------------------------------------------------- autograd
 
-Tensor call_forward(const Op& op, at::ArrayRef<Tensor> in) {
+// The gradients that an autograd node computes.  Plain CUDA tensors that nothing differentiates go straight to the
+// kernels; anything else (tracing modes, tensor subclasses, derivatives of the derivative) through the dispatcher.
+bool direct(Args in) {
+    const auto tls = c10::impl::tls_local_dispatch_key_set().included_;
+    if (at::GradMode::is_enabled() || tls.has(c10::DispatchKey::Python) || tls.has(c10::DispatchKey::PythonTLSSnapshot) ||
+        tls.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || tls.has(c10::DispatchKey::Functionalize))
+        return false;
+    for (const Tensor& t : in)
+        if (!t.defined() || !t.is_cuda() || t.key_set().has(c10::DispatchKey::Python) || t.key_set().has(c10::DispatchKey::Functionalize) ||
+            t.key_set().has(c10::DispatchKey::FuncTorchBatched) || t.key_set().has(c10::DispatchKey::FuncTorchGradWrapper))
+            return false;
+    return true;
+}
+Tensor call_forward(const Op& op, Args in) {
+    if (direct(in)) return forward_cuda(op, in);
     Stack stack(in.begin(), in.end());
     op.forward->callBoxed(stack);
     return stack.back().toTensor();
 }
-variable_list call_list(const OperatorHandle& handle, at::ArrayRef<Tensor> in) {
+variable_list call_boxed(const OperatorHandle& handle, Args in) {
     Stack stack(in.begin(), in.end());
     handle.callBoxed(stack);
     return stack.back().toTensorVector();
 }
-variable_list joined(std::initializer_list<Tensor> a, at::ArrayRef<Tensor> index) {
-    variable_list v(a);
+variable_list call_gradient(Op& op, Args in) { return direct(in) ? gradient_cuda(op, in) : call_boxed(*op.gradient, in); }
+variable_list joined(std::initializer_list<Tensor> a, Args index) {
+    variable_list v;
+    v.reserve(a.size() + index.size());
+    v.insert(v.end(), a.begin(), a.end());
     v.insert(v.end(), index.begin(), index.end());
     return v;
 }
-// One gradient per forward argument: none for the operator, the given ones, none for the index arrays.
-variable_list per_argument(variable_list grads, const Op& op) {
-    grads.insert(grads.begin(), Tensor());
-    grads.resize(grads.size() + op.index);
-    return grads;
-}
 
-struct ForwardFn : torch::autograd::Function<ForwardFn> {
-    static Tensor forward(AutogradContext* ctx, Op* op, at::TensorList in) {
-        ctx->saved_data["op"] = reinterpret_cast<int64_t>(op);
-        ctx->save_for_backward(in.vec());
-        at::AutoDispatchBelowADInplaceOrView guard;
-        return call_forward(*op, in);
+// Saved operands (the index arrays among them), and next edges for the differentiable ones alone: a good deal less per
+// call than torch::autograd::Function, which wraps every argument.
+struct OpNode : torch::autograd::Node {
+    Op* op;
+    std::vector<torch::autograd::SavedVariable> saved;
+    OpNode(Op* o, const variable_list& in, int diff) : op(o) {
+        saved.reserve(in.size());
+        for (const Tensor& t : in) saved.emplace_back(t, false);
+        set_next_edges(torch::autograd::collect_next_edges(Args(in.data(), (size_t)diff)));
     }
-    static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        Op& op = *reinterpret_cast<Op*>(ctx->saved_data["op"].toInt());
-        variable_list in = ctx->get_saved_variables();
-        in.insert(in.begin() + op.inputs, grads[0]);
-        return per_argument(call_list(*op.gradient, in), op);
+    variable_list operands() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        TORCH_CHECK(!saved.empty(), "Trying to backward through the graph a second time: specify retain_graph=True");
+        variable_list v;
+        v.reserve(saved.size() + 1);
+        for (const auto& s : saved) v.push_back(s.unpack());
+        return v;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        saved.clear();
     }
 };
 
-struct GradientFn : torch::autograd::Function<GradientFn> {
-    static variable_list forward(AutogradContext* ctx, Op* op, at::TensorList in) {
-        ctx->saved_data["op"] = reinterpret_cast<int64_t>(op);
-        ctx->save_for_backward(in.vec());
-        at::AutoDispatchBelowADInplaceOrView guard;
-        return call_list(*op->gradient, in);
+struct ForwardNode final : OpNode {
+    using OpNode::OpNode;
+    std::string name() const override { return "OeqForwardBackward"; }
+    variable_list apply(variable_list&& grads) override {
+        if (!grads[0].defined()) return variable_list(op->inputs);
+        variable_list in = operands();
+        in.insert(in.begin() + op->inputs, std::move(grads[0]));
+        return call_gradient(*op, in);
     }
+};
+
+struct GradientNode final : OpNode {
+    using OpNode::OpNode;
+    std::string name() const override { return "OeqGradientBackward"; }
     // The product is trilinear in (x, y, w).  With cotangents (ex, ey, ew) of (dX, dY, dW):
     //   d/d(dz) = f(ex, y, w) + f(x, ey, w) + f(x, y, ew);  d/dx = dX(ey, w, dz) + dX(y, ew, dz), likewise y and w.
-    static variable_list backward(AutogradContext* ctx, variable_list e) {
-        Op& op = *reinterpret_cast<Op*>(ctx->saved_data["op"].toInt());
-        const variable_list s = ctx->get_saved_variables();
-        const at::ArrayRef<Tensor> idx(s.data() + op.inputs + 1, (size_t)op.index);
-        const Tensor &x = s[0], &y = s[1], &dz = s[op.inputs];
-        if (op.inputs == 2) {
-            variable_list a = call_list(*op.gradient, joined({e[0], e[1], dz}, idx));
-            return per_argument({a[0], a[1], call_forward(op, joined({e[0], y}, idx)) + call_forward(op, joined({x, e[1]}, idx))}, op);
+    variable_list apply(variable_list&& e) override {
+        Op& o = *op;
+        const variable_list s = operands();
+        bool any = false;
+        for (int i = 0; i < o.inputs; ++i) {
+            any |= e[i].defined();
+            if (!e[i].defined()) e[i] = at::zeros_like(s[i]);
+        }
+        if (!any) return variable_list(o.inputs + 1);
+        const Args idx(s.data() + o.inputs + 1, (size_t)o.index);
+        const Tensor &x = s[0], &y = s[1], &dz = s[o.inputs];
+        if (o.inputs == 2) {
+            variable_list a = call_gradient(o, joined({e[0], e[1], dz}, idx));
+            return {a[0], a[1], call_forward(o, joined({e[0], y}, idx)) + call_forward(o, joined({x, e[1]}, idx))};
         }
         const Tensor& w = s[2];
         if (!at::GradMode::is_enabled()) {
             // nothing differentiates through this result: launches that read a row's arrays once
-            if (op.tp && oeq_tp_has_double_backward(op.tp)) return per_argument(tp_second(op, {x, y, w, dz, e[0], e[1], e[2]}), op);
+            const variable_list all_in{x, y, w, dz, e[0], e[1], e[2]};
+            if (o.tp && oeq_tp_has_double_backward(o.tp) && direct(all_in)) return tp_second(o, all_in);
+            if (o.conv) {
+                variable_list all;
+                if (o.second && o.call_second) all = call_boxed(*o.second, joined({x, y, w, dz, e[0], e[1], e[2]}, idx));
+                else if (direct(all_in)) all = conv_second(o, all_in, idx);
+                if (all.size() == 4) return all;
+            }
         }
-        if (op.conv && !at::GradMode::is_enabled()) {
-            variable_list all = op.second && op.call_second ? call_list(*op.second, joined({x, y, w, dz, e[0], e[1], e[2]}, idx))
-                                                            : conv_second(op, {x, y, w, dz, e[0], e[1], e[2]}, idx);
-            if (all.size() == 4) return per_argument(std::move(all), op);
-        }
-        variable_list a = call_list(*op.gradient, joined({e[0], e[1], w, dz}, idx));    // dX(ey, w), dY(ex, w)
-        variable_list b = call_list(*op.gradient, joined({x, y, e[2], dz}, idx));       // dX(y, ew), dY(x, ew)
-        variable_list c = call_list(*op.gradient, joined({e[0], y, w, dz}, idx));       // dW(ex, y)
-        variable_list d = call_list(*op.gradient, joined({x, e[1], w, dz}, idx));       // dW(x, ey)
-        Tensor gz = call_forward(op, joined({e[0], y, w}, idx)) + call_forward(op, joined({x, e[1], w}, idx)) +
-                    call_forward(op, joined({x, y, e[2]}, idx));
-        return per_argument({a[0] + b[0], a[1] + b[1], c[2] + d[2], gz}, op);
+        variable_list a = call_gradient(o, joined({e[0], e[1], w, dz}, idx));    // dX(ey, w), dY(ex, w)
+        variable_list b = call_gradient(o, joined({x, y, e[2], dz}, idx));       // dX(y, ew), dY(x, ew)
+        variable_list c = call_gradient(o, joined({e[0], y, w, dz}, idx));       // dW(ex, y)
+        variable_list d = call_gradient(o, joined({x, e[1], w, dz}, idx));       // dW(x, ey)
+        Tensor gz = call_forward(o, joined({e[0], y, w}, idx)) + call_forward(o, joined({x, e[1], w}, idx)) +
+                    call_forward(o, joined({x, y, e[2]}, idx));
+        return {a[0] + b[0], a[1] + b[1], c[2] + d[2], gz};
     }
 };
 
@@ -289,7 +334,7 @@ struct AutogradKernel final : c10::OperatorKernel {
         const int diff = op->inputs + (GRADIENT ? 1 : 0), n = diff + op->index;
         bool needed = false;
         if (at::GradMode::is_enabled())
-            for (int i = 0; i < diff; ++i) needed |= arg(*stack, n, i).requires_grad();
+            for (int i = 0; i < diff; ++i) needed |= (*stack)[stack->size() - n + i].toTensor().requires_grad();
         if (!needed) {
             at::AutoDispatchBelowADInplaceOrView guard;
             handle.redispatchBoxed(keys & c10::after_autograd_keyset, stack);
@@ -297,10 +342,22 @@ struct AutogradKernel final : c10::OperatorKernel {
         }
         variable_list in;
         in.reserve(n);
-        for (int i = 0; i < n; ++i) in.push_back(arg(*stack, n, i));
-        torch::jit::drop(*stack, n);
-        if constexpr (GRADIENT) stack->emplace_back(c10::List<Tensor>(GradientFn::apply(op, at::TensorList(in))));
-        else stack->emplace_back(ForwardFn::apply(op, at::TensorList(in)));
+        for (auto it = stack->end() - n; it != stack->end(); ++it) in.push_back(it->toTensor());
+        typedef std::conditional_t<GRADIENT, GradientNode, ForwardNode> NodeT;
+        auto node = std::shared_ptr<NodeT>(new NodeT(op, in, diff), torch::autograd::deleteNode);
+        {
+            at::AutoDispatchBelowADInplaceOrView guard;
+            handle.redispatchBoxed(keys & c10::after_autograd_keyset, stack);
+        }
+        if constexpr (GRADIENT) {
+            variable_list out = stack->back().toTensorVector();
+            for (Tensor& t : out) torch::autograd::set_history(t, node);
+            stack->back() = c10::List<Tensor>(std::move(out));
+        } else {
+            Tensor z = stack->back().toTensor();
+            torch::autograd::set_history(z, node);
+            stack->back() = std::move(z);
+        }
     }
 };
 
