@@ -193,4 +193,25 @@ __device__ __forceinline__ int weight_offset_v1(int mu, int mw, int u, int w) {
     return (uc << 5) * mw + ulen * (wc << 5) + ul * wlen + wl;
 }
 
+// out[i] = sum_g ws[g][i] in a fixed order, by blocks of 256 threads for 32 values: eight threads take every eighth
+// partial each (with one thread per value 148 partials of 45 056 weights took 12.5 us, a chain of loads), then their
+// sums are added up.
+template <class T>
+__device__ __forceinline__ void reduce_partials(const T* __restrict__ ws, T* __restrict__ out, int n, long long groups) {
+    __shared__ T part[8][32];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    T s = (T)0;
+    if (i < n) {
+#pragma unroll 4
+        for (long long g = row; g < groups; g += 8) s += ws[g * n + i];
+    }
+    part[row][lane] = s;
+    __syncthreads();
+    if (row == 0 && i < n) {
+#pragma unroll
+        for (int r = 1; r < 8; ++r) s += part[r][lane];
+        out[i] = s;
+    }
+}
+
 }  // namespace oeq

@@ -1299,6 +1299,7 @@ constexpr int K_UVW_TC_FWD = 20;
 struct TcGeometry {
     size_t packed_bytes = 0;
     int smem = 0;
+    unsigned outputs = 1;
     unsigned paths = 1;                     // instructions (the weights of each are packed by blocks of their own)
     int producers = 16, epilogues = 1;      // producer warps, groups of four epilogue warps
     int threads() const { return 32 * (producers + 1 + 4 * epilogues); }
@@ -1335,6 +1336,7 @@ bool uvw_tc_geometry(const Problem& p, TcGeometry& g, bool pad = false) {
     g.smem = off_bar + (2 * 2 + 2 * 32 + 2) * 8 + 16 + 1024;
     g.packed_bytes = total;
     g.paths = (unsigned)p.instr.size();
+    g.outputs = (unsigned)p.out.size();
     return g.smem <= SMEM_LIMIT;
 }
 
@@ -1958,12 +1960,13 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
         tp{X, Y, packed, Z, batch, status, nullptr};
     void* args[] = {&tp};
     const long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
+    const unsigned split = grid * geo.outputs <= k.sm_count ? geo.outputs : 1;     // output irreps over CTAs
 #ifdef OEQ_DEV_PROFILE
     if (env_int("OEQ_B200_TC_PROFILE", 0)) {
         // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr
         OEQ_CUDA(cudaMalloc(&tp.prof, 32 * 8));
         OEQ_CUDA(cudaMemsetAsync(tp.prof, 0, 32 * 8, st));
-        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid, split), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
         unsigned long long hb[32];
         OEQ_CUDA(cudaMemcpyAsync(hb, tp.prof, sizeof hb, cudaMemcpyDeviceToHost, st));
         OEQ_CUDA(cudaStreamSynchronize(st));
@@ -1973,7 +1976,7 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
         return OEQ_OK;
     }
 #endif
-    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid, split), dim3((unsigned)geo.threads()), args, (size_t)k.smem, st));
     return OEQ_OK;
 }
 
@@ -2110,7 +2113,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         if (shares > 1) {
             const void* ws = workspace;
             void* rargs[] = {&ws, &dW, &n, &shares};
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
         }
         return gradients_from_dt(block, [&](long long, long long rows, const void* dz) {
             return launch_gemm(h->grad_product_k, h->grad_product, rows, dz, nullptr, W, workspace, st);
@@ -2149,11 +2152,20 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; }
                 tp{X, Y, dZ, workspace, batch, h->d_status};
             void* targs[] = {&tp};
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas), dim3(21 * 32), targs, (size_t)k.smem, st));
+            // groups of paths that fill the 128 rows of an MMA (tb_groups in the kernel); few rows: dealt over CTAs
+            unsigned dw_groups = 0;
+            for (size_t o = 0; o < p.out.size(); ++o) {
+                unsigned paths = 0, per = 2;
+                for (const Instr& t : p.instr)
+                    if (t.io == (int)o) { ++paths; if (p.in1[t.i1].mul > 64) per = 1; }
+                dw_groups += (paths + per - 1) / per;
+            }
+            if (dw_ctas * dw_groups > k.sm_count) dw_groups = 1;
+            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3(21 * 32), targs, (size_t)k.smem, st));
             int n = p.w_numel;
             const void* ws = workspace;
             void* rargs[] = {&ws, &dW, &n, &dw_ctas};
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
             up.skip_dw = 1;
             up.ws = nullptr;
             // dX and dY in two steps over dT rows, which take the partial gradients' place in the workspace
@@ -2174,7 +2186,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             int n = p.w_numel;
             const void* ws = workspace;
             void* rargs[] = {&ws, &dW, &n, &ctas};
-            OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+            OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
         }
         return OEQ_OK;
     }
@@ -2197,7 +2209,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         int n = p.w_numel;
         const void* ws = workspace;
         void* args[] = {&ws, &dW, &n, &groups};
-        OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 127) / 128), dim3(128), args, 0, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 31) / 32), dim3(256), args, 0, st));
     }
     return OEQ_OK;
 }
@@ -2325,7 +2337,7 @@ int oeq_tp_backward_noalloc(oeq_tp* h, int64_t batch, const void* X, const void*
         int n = p.w_numel;
         const void* ws = scratch;
         void* rargs[] = {&ws, &dW, &n, &ctas};
-        OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
         return OEQ_OK;
     }
     if ((rc = load_kernel(h->bwd, "oeq_uvu_kernel", true))) return rc;
@@ -2342,7 +2354,7 @@ int oeq_tp_backward_noalloc(oeq_tp* h, int64_t batch, const void* X, const void*
     int n = p.w_numel;
     const void* ws = scratch;
     void* rargs[] = {&ws, &dW, &n, &groups};
-    OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 127) / 128), dim3(128), rargs, 0, st));
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
     return OEQ_OK;
 }
 

@@ -2128,14 +2128,9 @@ extern "C" __global__ void __launch_bounds__(oeq::NTHREADS, oeqd::MIN_CTAS) oeq_
 #endif
 }
 
-// Fixed-order sum of the per-group partial weight gradients (shared weights):
-// dW[i] = sum_g ws[g][i], g ascending, one thread per weight.
-extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, int n, long long groups) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    oeqd::T s = (oeqd::T)0;
-    for (long long g = 0; g < groups; ++g) s += ws[g * n + i];
-    out[i] = s;
+// Fixed-order sum of the partial weight gradients.
+extern "C" __global__ void __launch_bounds__(256) oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, int n, long long groups) {
+    oeq::reduce_partials(ws, out, n, groups);
 }
 
 #endif  // OEQ_UVU_NO_ENTRY

@@ -241,12 +241,7 @@ extern "C" __global__ void __launch_bounds__(oeq::G_THREADS, 2) oeq_uvw_gemm_ker
 #endif
 }
 
-// Fixed-order sum of the shares' weight gradients: dW[i] = sum_s ws[s][i].
-extern "C" __global__ void oeq_reduce_partials(const oeqd::T* __restrict__ ws, oeqd::T* __restrict__ out, int n, long long groups) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    oeqd::T s = (oeqd::T)0;
-#pragma unroll 8
-    for (int g = 0; g < (int)groups; ++g) s += ws[(long long)g * n + i];
-    out[i] = s;
+// Fixed-order sum of the partial weight gradients.
+extern "C" __global__ void __launch_bounds__(256) oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, int n, long long groups) {
+    oeq::reduce_partials(ws, out, n, groups);
 }

@@ -381,14 +381,9 @@ extern "C" __global__ void __launch_bounds__(oeq::NT, 1) oeq_uvw_kernel(const oe
 #endif
 }
 
-// Fixed-order sum of the per-CTA partial weight gradients: dW[i] = sum_c ws[c][i].
-extern "C" __global__ void oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, int n, long long groups) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    oeqd::T s = (oeqd::T)0;
-#pragma unroll 8        // (the loads go out together; the sum keeps its order)
-    for (int g = 0; g < (int)groups; ++g) s += ws[(long long)g * n + i];
-    out[i] = s;
+// Fixed-order sum of the partial weight gradients.
+extern "C" __global__ void __launch_bounds__(256) oeq_reduce_partials(const oeqd::T* ws, oeqd::T* out, int n, long long groups) {
+    oeq::reduce_partials(ws, out, n, groups);
 }
 #else
 }  // namespace oeq

@@ -308,6 +308,13 @@ __device__ __forceinline__ bool dw_epilogue(const UvwTcBwdParams& p, const DwBar
     return true;
 }
 
+// Small batches: the groups of paths are dealt over the grid's y dimension.
+constexpr int dw_groups_before(int o) {
+    int n = 0;
+    for (int q = 0; q < o; ++q) n += tb_groups(q);
+    return n;
+}
+
 __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -344,6 +351,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
             constexpr int O = o_;
             sfor<0, tb_groups(O)>([&](auto g_) {
                 constexpr int GRP = g_;
+                if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
                 if (ok) ok = dw_produce<O, GRP>(p, smem, bars, row_lo, row_hi, stage_it, tid);
             });
         });
@@ -355,6 +363,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
                 constexpr int O = o_;
                 sfor<0, tb_groups(O)>([&](auto g_) {
                     constexpr int GRP = g_;
+                if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
                     if (ok) ok = dw_mma<O, GRP>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, tmem_base);
                 });
             });
@@ -367,6 +376,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
             constexpr int O = o_;
             sfor<0, tb_groups(O)>([&](auto g_) {
                 constexpr int GRP = g_;
+                if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
                 if (ok) ok = dw_epilogue<O, GRP>(p, bars, row_lo, row_hi, acc_it, tmem_base, warp & 3, lane);
             });
         });
@@ -386,12 +396,7 @@ extern "C" __global__ void __launch_bounds__(oeq::TB_THREADS, 1) oeq_uvw_tc_dw_k
     oeq::uvw_tc_dw(p);
 }
 
-// Fixed-order sum of the per-CTA partial weight gradients: dW[i] = sum_c ws[c][i].
-extern "C" __global__ void oeq_reduce_partials(const float* ws, float* out, int n, long long groups) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.f;
-#pragma unroll 8        // (the loads go out together; the sum keeps its order)
-    for (int g = 0; g < (int)groups; ++g) s += ws[(long long)g * n + i];
-    out[i] = s;
+// Fixed-order sum of the partial weight gradients.
+extern "C" __global__ void __launch_bounds__(256) oeq_reduce_partials(const float* ws, float* out, int n, long long groups) {
+    oeq::reduce_partials(ws, out, n, groups);
 }

@@ -478,6 +478,10 @@ constexpr bool tc_output_has_paths(int o) {
     return false;
 }
 
+// Small batches: the output irreps are dealt over the grid's y dimension (a CTA that took all of them would load their
+// weights one after the other while most of the machine is idle).
+__device__ __forceinline__ bool tc_mine(int o) { return gridDim.y == 1 || (int)blockIdx.y == o; }
+
 __device__ void uvw_tc_forward(const UvwTcParams& p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // the 128-byte swizzle pattern repeats every 1024 bytes: operand tiles must start on that boundary
@@ -516,6 +520,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
         bool ok = true;
         sfor<0, N_OUT>([&](auto o_) {
             constexpr int O = o_;
+            if (!tc_mine(O)) return;
             if constexpr (tc_output_has_paths(O)) {
                 if (ok) ok = tc_produce_output<O>(p, smem, bars, row_lo, row_hi, stage_it, warp, lane);
             } else {
@@ -531,6 +536,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
             bool ok = true;
             sfor<0, N_OUT>([&](auto o_) {
                 constexpr int O = o_;
+                if (!tc_mine(O)) return;
                 if constexpr (tc_output_has_paths(O)) {
                     if (ok) ok = tc_mma_output<O>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, w_use, tmem_base);
                 }
@@ -542,6 +548,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
         bool ok = true;
         sfor<0, N_OUT>([&](auto o_) {
             constexpr int O = o_;
+            if (!tc_mine(O)) return;
             if constexpr (tc_output_has_paths(O)) {
                 // a warp may only read the TMEM lanes of its own quarter: 32 * (warp index mod 4)
                 if (ok) ok = tc_epilogue_output<O>(p, smem, bars, row_lo, row_hi, acc_it, tmem_base, warp & 3, lane, (warp - TC_PRODUCER_WARPS - 1) / TC_EPILOGUE_WARPS);

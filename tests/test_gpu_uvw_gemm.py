@@ -14,6 +14,7 @@ pytestmark = pytest.mark.gpu
 CASES = [
     ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e", 1),
     ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e", 300),
+    ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e", 1900),  # too many rows to deal the outputs over CTAs
     ("16x0e+80x1o", "0e+1o", "65x0e+16x1o+33x2e", 63),          # (33 and 65: not on the tensor cores)
     ("48x1o+16x3o", "1o+2e", "16x0e+64x2e+32x4e", 130),
     ("128x0e+128x1o", "0e+1o+2e", "128x0e+128x1o", 70),          # joined blocks of one path each
