@@ -105,7 +105,9 @@ int64_t oeq_tp_weight_numel(const oeq_tp* h);
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z,
                    void* stream);
 
-/* Scratch needed by oeq_tp_backward for `batch` rows (0 unless weights are shared). */
+/* Scratch needed by oeq_tp_backward for `batch` rows (0 unless weights are shared): partial weight gradients,
+ * packed weights and, for 'uvw' with second-input multiplicity 1, the products of the weights with dZ for blocks
+ * of at most 1 GiB. */
 size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch);
 
 /* dX, dY, dW from X, Y, W, dZ.  Replaces JITTPImpl::backward (tensorproducts.hpp:87-95).
@@ -178,7 +180,7 @@ int oeq_conv_check(oeq_conv* h);
 /* Number of kernels the most recent oeq_conv_backward on this handle launched: 1 for the sender-order kernel
  * and for the atomic receiver-order kernel; for the deterministic receiver-order pass the kernel that clears dX,
  * one launch per block of edges (each sums the previous block's rows as well when the blocks are pipelined)
- * and the row-sum launches.  Benchmarks report it; it has no counterpart in the reference. */
+ * and the row-sum launches (with one block nothing is cleared: the row sum writes every row of dX).  Benchmarks report it; it has no counterpart in the reference. */
 int oeq_conv_last_backward_launches(const oeq_conv* h);
 
 /* Second derivatives of the convolution in two fused launches (plus the row sum of the deterministic variant).

@@ -11,6 +11,8 @@
 //   * Products x_i y_j are formed once for all paths that share the two input irreps (E_* tables).
 //   * FP64: the same code with one edge at a time.
 // The walk deals chunks of consecutive edges round robin, so that gathered rows are shared in L2.
+// Measured against the group kernels: 32x(0e+1o+2e) on 20 000 nodes / 800 k edges, atomic, forward 463 -> 262 us and
+// backward 796 -> 585 us; 128x(0e+1o+2e) x (0e..3o) on 5 000 nodes / 150 k edges, deterministic, 446 -> 297 and 854 -> 585.
 #pragma once
 #define OEQ_UVU_NO_ENTRY
 #include "uvu_kernels.cuh"
