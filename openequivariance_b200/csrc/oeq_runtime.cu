@@ -1956,11 +1956,19 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
         void* args[] = {(void*)&W, &packed};
         OEQ_CUDA(cudaLaunchKernel((const void*)pack_fn, dim3(16, geo.paths), dim3(256), args, 0, st));
     }
-    struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; unsigned long long* prof; }
-        tp{X, Y, packed, Z, batch, status, nullptr};
+    struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; int dealt; unsigned long long* prof; }
+        tp{X, Y, packed, Z, batch, status, 0, nullptr};
     void* args[] = {&tp};
-    const long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
-    const unsigned split = grid * geo.outputs <= k.sm_count ? geo.outputs : 1;     // output irreps over CTAs
+    // Up to a chunk per CTA and output: output irreps over the grid's y dimension.  Up to 200 rows per SM: chunks of all
+    // outputs dealt (64x(0e+1o+2e), forward / W dZ: 1 500 rows 31 -> 17 / 20 -> 14 us, 10 007 rows 73 -> 62 / 46 -> 39,
+    // 30 000 rows 154 -> 151 / 99 -> 92).  Above, a share of the rows each: its balance does not depend on the costs
+    // that the deal assumes (100 000 rows: 443 against 504 us).
+    long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
+    const unsigned split = grid * geo.outputs <= k.sm_count ? geo.outputs : 1;
+    if (split == 1 && geo.outputs > 1 && batch <= 200LL * k.sm_count) {
+        tp.dealt = 1;
+        grid = k.sm_count;
+    }
 #ifdef OEQ_DEV_PROFILE
     if (env_int("OEQ_B200_TC_PROFILE", 0)) {
         // cycle accounting of the roles of CTA 0 (development aid): synchronous, prints to stderr

@@ -33,6 +33,7 @@ struct UvwTcParams {
     float* Z;
     long long batch;
     int* status;
+    int dealt;                  // chunks of all output irreps dealt to the CTAs, instead of a share of the rows each
     unsigned long long* prof;   // optional cycle accounting of CTA 0 (development aid), else null
 };
 
@@ -117,11 +118,6 @@ struct TcBars {
     }
 };
 
-// rows of the batch owned by this CTA
-__device__ __forceinline__ void tc_row_range(long long batch, long long& lo, long long& hi) {
-    lo = batch * blockIdx.x / gridDim.x;
-    hi = batch * (blockIdx.x + 1) / gridDim.x;
-}
 
 // Batch rows of a chunk and the accumulator row of (batch row r, component k): k-major, with the rows rounded down to
 // a multiple of eight where that costs at most an eighth of the tile.  A producer warp then keeps its row of the
@@ -136,6 +132,47 @@ constexpr int tc_first_path(int o) {
         if (I_OUT[p] == o) return p;
     return 0;
 }
+// Relative time of a chunk of output o.  Forward: the producers, about one instruction per input and output component and
+// coefficient and row, but no stage is shorter than its MMAs.  The product W dZ: draining its columns.
+constexpr int tc_chunk_cost(int o) {
+    int n = 16;
+    for (int p = 0; p < N_INSTR; ++p) {
+        if (I_OUT[p] != o) continue;
+        int ops = 8 + 4 * IN1_D[I_IN1[p]] + 6 * OUT_D[o] + CG_BEGIN[p + 1] - CG_BEGIN[p];
+        for (int c = CG_BEGIN[p]; c < CG_BEGIN[p + 1]; ++c)
+            if (c == CG_BEGIN[p] || CG_I[c] != CG_I[c - 1] || CG_J[c] != CG_J[c - 1]) ++ops;
+        const int stage = tc_rpc(o) * ops / 64;
+        n += tc_khalves(p) * (stage > 12 ? stage : 12);
+    }
+    return UNIT_Y ? 16 + OUT_MUL[o] / 4 : n;
+}
+
+// Rows of the batch that this CTA forms for output O.  Large batches: the same share of the rows for every output.  Where
+// a share is a few chunks, rounding it up to whole chunks for every output (and loading all weights) costs more than the
+// work: the chunks of all outputs, in one list, are cut into one run per CTA (at most two outputs in most of them).
+template <int O>
+__device__ __forceinline__ void tc_row_range(const UvwTcParams& p, long long& lo, long long& hi) {
+    if (!p.dealt) {
+        lo = p.batch * blockIdx.x / gridDim.x;
+        hi = p.batch * (blockIdx.x + 1) / gridDim.x;
+        return;
+    }
+    int total = 0, before = 0;                  // (a dealt batch is small)
+    sfor<0, N_OUT>([&](auto o_) {
+        constexpr int o = o_;
+        const int n = ((int)p.batch + tc_rpc(o) - 1) / tc_rpc(o) * tc_chunk_cost(o);
+        total += n;
+        if constexpr (o < O) before += n;
+    });
+    constexpr int COST = tc_chunk_cost(O), RPC = tc_rpc(O);
+    const int from = (int)((long long)total * blockIdx.x / gridDim.x) - before;
+    const int to = (int)((long long)total * (blockIdx.x + 1) / gridDim.x) - before;
+    const long long a = from > 0 ? (long long)((from + COST - 1) / COST) * RPC : 0;
+    const long long b = to > 0 ? (long long)((to + COST - 1) / COST) * RPC : 0;
+    lo = a < p.batch ? a : p.batch;
+    hi = b < p.batch ? b : p.batch;
+}
+
 constexpr int tc_d1_max(int o) {
     int m = 1;
     for (int p = 0; p < N_INSTR; ++p)
@@ -489,7 +526,6 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
     const TcBars bars(smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     long long row_lo, row_hi;
-    tc_row_range(p.batch, row_lo, row_hi);
 
     if (tid == 0) {
         for (int i = 0; i < TC_NA; ++i) {
@@ -521,6 +557,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
         sfor<0, N_OUT>([&](auto o_) {
             constexpr int O = o_;
             if (!tc_mine(O)) return;
+            tc_row_range<O>(p, row_lo, row_hi);
             if constexpr (tc_output_has_paths(O)) {
                 if (ok) ok = tc_produce_output<O>(p, smem, bars, row_lo, row_hi, stage_it, warp, lane);
             } else {
@@ -537,6 +574,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
             sfor<0, N_OUT>([&](auto o_) {
                 constexpr int O = o_;
                 if (!tc_mine(O)) return;
+                tc_row_range<O>(p, row_lo, row_hi);
                 if constexpr (tc_output_has_paths(O)) {
                     if (ok) ok = tc_mma_output<O>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, w_use, tmem_base);
                 }
@@ -549,6 +587,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
         sfor<0, N_OUT>([&](auto o_) {
             constexpr int O = o_;
             if (!tc_mine(O)) return;
+            tc_row_range<O>(p, row_lo, row_hi);
             if constexpr (tc_output_has_paths(O)) {
                 // a warp may only read the TMEM lanes of its own quarter: 32 * (warp index mod 4)
                 if (ok) ok = tc_epilogue_output<O>(p, smem, bars, row_lo, row_hi, acc_it, tmem_base, warp & 3, lane, (warp - TC_PRODUCER_WARPS - 1) / TC_EPILOGUE_WARPS);
