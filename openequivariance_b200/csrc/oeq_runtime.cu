@@ -1688,10 +1688,13 @@ void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes,
     grid = std::max<long long>(1, std::min(most, (chunks + per_cta - 1) / per_cta));
 }
 
-// Row sum: a warp takes a chunk of the sender-ordered edge list and 512 bytes of the rows.  64 edges per chunk, fewer
+// Row sum: a warp takes a chunk of the sender-ordered edge list and 512 bytes (rows of 8 KB and more: 2 KB) of the rows.  64 edges per chunk, fewer
 // when that would leave warps idle.
 constexpr int SUM_WARPS_PER_SM = 48;
-long long row_sum_blocks(const Problem& p) { return (pad16(p.x_dim * p.elem()) + 511) / 512; }
+long long row_sum_blocks(const Problem& p) {
+    const int row = pad16(p.x_dim * p.elem()), piece = (row + 511) / 512 >= 16 ? 2048 : 512;
+    return (row + piece - 1) / piece;
+}
 int row_sum_chunk(const Kernel& k, const Problem& p, long long edges) {
     int chunk = env_int("OEQ_B200_SUM_CHUNK", 0);
     if (chunk > 0) return chunk;

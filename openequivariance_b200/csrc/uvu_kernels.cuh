@@ -2160,7 +2160,8 @@ extern "C" __global__ void oeq_clear(unsigned int* ptr, unsigned long long words
 // The row sum of the deterministic receiver-order backward pass as a launch of its own (the last block of
 // edges, or every block when the launches carry no helper warps): see sum_sender_rows.
 extern "C" __global__ void __launch_bounds__(256) oeq_sum_sender_rows(const oeq::UvuParams p) {
-    oeq::sum_sender_rows<1, 8>(reinterpret_cast<const oeqd::T*>(p.ws), p.dX, p.cols, p.perm, p.n_items, p.e_lo, p.e_hi,
+    // (rows of 8 KB and more have blocks enough at 2 KB each: MACE-large, last of four scratch blocks, 670 -> 477 us)
+    oeq::sum_sender_rows<(oeq::ROW_PIECES >= 16 ? 4 : 1), (oeq::ROW_PIECES >= 16 ? 4 : 8)>(reinterpret_cast<const oeqd::T*>(p.ws), p.dX, p.cols, p.perm, p.n_items, p.e_lo, p.e_hi,
                          (p.flags & 64) != 0, p.chunk, (p.flags & 128) ? p.n_nodes : 0, (long long)gridDim.x * (blockDim.x >> 5),
                          (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31);
 }
