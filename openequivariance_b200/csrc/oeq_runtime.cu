@@ -1358,7 +1358,7 @@ int build_uvw_tc(const Problem& p, const TcGeometry& g, Kernel& k) {
 // ---- tensor-core backward for 'uvw': the weight gradient (mirrors the constexpr geometry of uvw_tc_bwd_kernels.cuh)
 constexpr int K_UVW_TC_DW = 21;
 
-bool uvw_tc_dw_geometry(const Problem& p, int& smem) {
+bool uvw_tc_dw_geometry(const Problem& p, int& smem, int& threads) {
     TcGeometry fwd;
     if (!uvw_tc_geometry(p, fwd)) return false;          // same class of problems as the forward pass
     if (!env_int("OEQ_B200_UVW_TC_BWD", 1)) return false;
@@ -1374,6 +1374,7 @@ bool uvw_tc_dw_geometry(const Problem& p, int& smem) {
     const int stages = std::min(4, (200 * 1024) / stage);
     if (stages < 2) return false;
     smem = stages * stage + (2 * stages + 4) * 8 + 16 + 1024;
+    threads = 32 * (4 * stages + 1 + 4);                 // four producer warps per stage, MMA issuer, epilogue
     return smem <= SMEM_LIMIT;
 }
 
@@ -1739,7 +1740,7 @@ struct oeq_tp {
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
     bool has_bwd_tc = false;
-    int dw_smem = 0;
+    int dw_smem = 0, dw_threads = 0;
     // dX and dY of the same class of problems: dT = W dZ on the tensor cores, then the channel-wise backward pass
     Problem grad_product, grad_channels;
     Kernel grad_product_k, grad_channels_k;
@@ -1820,9 +1821,9 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if ((rc = build_tp(p, true, b))) return rc;
         TcGeometry g;
         if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, g, tc))) return rc;
-        int smem = 0;
+        int smem = 0, threads = 0;
         Kernel dw, product, channels;
-        if (uvw_tc_dw_geometry(p, smem)) {
+        if (uvw_tc_dw_geometry(p, smem, threads)) {
             if ((rc = build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
             Problem pp, pc;
             rc = build_uvw_gradients(p, pp, pc, g, product, channels);
@@ -1892,7 +1893,7 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
         rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
         h->has_tc = rc == OEQ_OK;
     }
-    if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem)) {
+    if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem, h->dw_threads)) {
         rc = build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
         h->has_bwd_tc = rc == OEQ_OK;
         if (!rc) {
@@ -2172,7 +2173,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
                 dw_groups += (paths + per - 1) / per;
             }
             if (dw_ctas * dw_groups > k.sm_count) dw_groups = 1;
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3(21 * 32), targs, (size_t)k.smem, st));
+            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3((unsigned)h->dw_threads), targs, (size_t)k.smem, st));
             int n = p.w_numel;
             const void* ws = workspace;
             void* rargs[] = {&ws, &dW, &n, &dw_ctas};

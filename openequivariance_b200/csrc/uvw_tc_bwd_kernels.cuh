@@ -30,9 +30,7 @@ struct UvwTcBwdParams {
     int* status;
 };
 
-constexpr int TB_PRODUCER_WARPS = 16;
 constexpr int TB_EPILOGUE_WARPS = 4;
-constexpr int TB_THREADS = (TB_PRODUCER_WARPS + 1 + TB_EPILOGUE_WARPS) * 32;
 constexpr int TB_TILE = 128 * 128;             // one [128 rows x 32 tf32] swizzled tile
 constexpr int ERR_TB_EMPTY = 31, ERR_TB_FULL = 32, ERR_TB_ACC_EMPTY = 33, ERR_TB_ACC_FULL = 34;
 
@@ -93,6 +91,11 @@ constexpr int TB_MW_MAX = tb_mw_max();
 constexpr int DW_B_HALF = TB_MW_MAX * 128;                       // [MW x 32] tile
 constexpr int DW_STAGE_BYTES = 2 * TB_TILE + 2 * DW_B_HALF;      // A hi, A lo, B hi, B lo
 constexpr int DW_STAGES = (200 * 1024) / DW_STAGE_BYTES < 4 ? (200 * 1024) / DW_STAGE_BYTES : 4;
+// One set of four producer warps per stage of the ring: a set builds the same slot every time, so it meets every phase of
+// that slot's `empty` barrier.  (A set that changed slots would wait for the parity of a phase without having seen the one
+// before it: the wait can pass one phase early, while the tensor core still reads the slot.)
+constexpr int TB_PRODUCER_WARPS = 4 * DW_STAGES;
+constexpr int TB_THREADS = (TB_PRODUCER_WARPS + 1 + TB_EPILOGUE_WARPS) * 32;
 constexpr int DW_ACC_COLS = 2 * TB_MW_MAX;                       // [hi.hi + lo.hi | hi.lo]
 constexpr int DW_TMEM_COLS = 2 * DW_ACC_COLS <= 32 ? 32 : 2 * DW_ACC_COLS <= 64 ? 64 : 2 * DW_ACC_COLS <= 128 ? 128
                              : 2 * DW_ACC_COLS <= 256 ? 256 : 512;
@@ -134,7 +137,7 @@ __device__ __forceinline__ void dw_store4(unsigned char* hi_row, int lo_off, int
 }
 
 // Bound by issue: with a thread per (slot row, every fourth batch row) each element paid a swizzled address and two
-// 4-byte stores.  Four warps now build a whole stage (the four sets take the stages in turn): a thread keeps one slot
+// 4-byte stores.  Four warps now build a whole stage (one set of warps per slot of the ring): a thread keeps one slot
 // row and walks the stage's batch rows four at a time, whose values fill whole 16-byte pieces.
 template <int O, int GRP>
 __device__ __forceinline__ bool dw_produce(const UvwTcBwdParams& p, unsigned char* smem, const DwBars& bars,
@@ -146,9 +149,9 @@ __device__ __forceinline__ bool dw_produce(const UvwTcBwdParams& p, unsigned cha
     const int which = t / SLOT, u = t % SLOT;
     bool ok = true;
     for (long long b0 = row_lo; b0 < row_hi && ok; b0 += RB, ++stage_it) {
-        if ((int)(stage_it & 3) != set) continue;
-        const int rows = (int)(row_hi - b0 < RB ? row_hi - b0 : RB);
         const int s = (int)(stage_it % DW_STAGES);
+        if (s != set) continue;
+        const int rows = (int)(row_hi - b0 < RB ? row_hi - b0 : RB);
         const long long use = stage_it / DW_STAGES;
         if (use > 0) ok = mbar_wait(bars.empty + s, (unsigned)((use - 1) & 1), p.status, ERR_TB_EMPTY);
         if (!ok) break;
@@ -324,7 +327,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
     tb_row_range(p.batch, row_lo, row_hi);
     if (tid == 0) {
         for (int i = 0; i < DW_STAGES; ++i) {
-            mbar_init(bars.full + i, TB_PRODUCER_WARPS / 4);
+            mbar_init(bars.full + i, 4);
             mbar_init(bars.empty + i, 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -363,7 +366,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
                 constexpr int O = o_;
                 sfor<0, tb_groups(O)>([&](auto g_) {
                     constexpr int GRP = g_;
-                if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
+                    if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
                     if (ok) ok = dw_mma<O, GRP>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, tmem_base);
                 });
             });
