@@ -94,14 +94,16 @@ def build_torch_library(force: bool = False, verbose: bool = False) -> str:
     cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
     source = os.path.join(CSRC, "oeq_torch.cpp")
 
+    # The host compiler that nvcc uses, not $CXX: the library hands C++ objects to and from torch and has to share its
+    # libstdc++.  With a second copy linked in, the first number written to a stream (an error message) ends the process.
     def command(out):
-        return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+        return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
                 f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + include,
                 "-I" + os.path.join(include, "torch", "csrc", "api", "include"), "-I" + cuda, source, "-o", out,
                 "-L" + os.path.join(root, "lib"), "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
                 "-L" + HERE, "-l:" + os.path.basename(lib), "-Wl,-rpath,$ORIGIN"]
 
-    return _build(torch_library_path(), [source, HEADER], command, verbose, force)
+    return _build(torch_library_path(), [source, HEADER, os.path.abspath(__file__)], command, verbose, force)
 
 
 if __name__ == "__main__":

@@ -26,6 +26,19 @@ def test_library_exports_every_declared_symbol():
     assert b"sm_100a" in lib.oeq_version()
 
 
+def test_torch_library_shares_the_cxx_runtime(monkeypatch, tmp_path):
+    """A private copy of libstdc++ (what a compiler named by $CXX may link) crashes on the first formatted message."""
+    import subprocess
+    from openequivariance_b200 import build
+    fake = tmp_path / "cxx"
+    fake.write_text("#!/bin/sh\nexec g++ -static-libstdc++ \"$@\"\n")
+    fake.chmod(0o755)
+    monkeypatch.setenv("CXX", str(fake))
+    monkeypatch.setattr(build, "torch_library_path", lambda: str(tmp_path / "lib.so"))
+    out = subprocess.run(["readelf", "-d", build.build_torch_library()], capture_output=True, text=True, check=True).stdout
+    assert "libstdc++.so" in out
+
+
 def test_descriptor_errors_are_reported_not_fatal():
     from openequivariance_b200 import _native
     lib = _native.lib()

@@ -68,3 +68,29 @@ def test_convolution_ops(deterministic):
     z_c.backward(dzt)
     dx_e = conv.backward_helper(xt, yt, wt, dzt, *index)[0]
     assert (xg.grad - dx_e).abs().max().item() <= 1e-5 * dx_e.abs().max().item()
+
+
+@pytest.mark.parametrize("op", ["product", "convolution"])
+def test_wrong_arguments_raise(op):
+    """Messages name the shapes; the process lives on."""
+    p = problem_by_name("nequip_32")
+    rows, cols = random_graph(7, 40, seed=1)
+    rows, cols, _, perm = orc.coord_graph(rows, cols)
+    if op == "product":
+        call, (x, y, w, dz), index = oeq.TensorProduct(p, torch_op=True), _cuda(*tp_inputs(p, 9, 1)), ()
+    else:
+        call = oeq.TensorProductConv(p, torch_op=True, deterministic=True)
+        (x, y, w, dz), index = _cuda(*conv_inputs(p, 7, 40, 1)), _cuda(rows, cols, perm)
+    for bad in ((x[:, 1:], y, w), (x, y[1:], w), (x, y, w[:, 1:]), (x.double(), y, w), (x, y, w.double())):
+        with pytest.raises(ValueError, match=r"must be"):
+            call.forward(*bad, *index)
+    with pytest.raises(ValueError, match=r"output gradient must be \[\d+, 1120\]"):
+        call.backward_helper(x, y, w, dz[:, 1:], *index)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        call.forward(x, y.cpu(), w, *index)
+    if index:
+        with pytest.raises(ValueError, match="int64"):
+            call.forward(x, y, w, index[0].int(), *index[1:])
+        with pytest.raises(ValueError, match="sender_perm"):
+            call.forward(x, y, w, *index[:2], index[2][1:])
+    assert torch.isfinite(call.forward(x, y, w, *index)).all()
