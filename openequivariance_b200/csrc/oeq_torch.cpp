@@ -261,16 +261,13 @@ struct OpNode : torch::autograd::Node {
     }
     variable_list operands() {
         std::lock_guard<std::mutex> lock(mutex_);
-        TORCH_CHECK(!saved.empty(), "Trying to backward through the graph a second time: specify retain_graph=True");
         variable_list v;
         v.reserve(saved.size() + 1);
         for (const auto& s : saved) v.push_back(s.unpack());
         return v;
     }
-    void release_variables() override {
-        std::lock_guard<std::mutex> lock(mutex_);
-        saved.clear();
-    }
+    // (release_variables is not overridden: the operands live as long as the graph, so that a second backward pass through
+    // a result needs no retain_graph, as with the reference's nodes, which keep their operands as attributes.)
 };
 
 struct ForwardNode final : OpNode {

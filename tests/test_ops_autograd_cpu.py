@@ -1,0 +1,59 @@
+"""Autograd of the registered ops without a GPU: the nodes (csrc/oeq_torch.cpp) dispatch tensors that are not plain CUDA
+tensors through the registered ops, which have CPU kernels here (x * sum(y) * w, trilinear like the product)."""
+import pytest
+import torch
+
+import openequivariance_b200 as oeq
+
+N = 5
+
+
+def _forward(x, y, w):
+    return x * y.sum(1, keepdim=True) * w
+
+
+def _gradient(x, y, w, dz):
+    s = y.sum(1, keepdim=True)
+    return [dz * w * s, (dz * x * w).sum(1, keepdim=True).expand_as(y).contiguous(), dz * x * s]
+
+
+@pytest.fixture(scope="module")
+def product():
+    """An operator with x, weight and output rows of 3 values and second-input rows of 3."""
+    p = oeq.TPProblem("3x0e", "3x0e", "3x0e", [(0, 0, 0, "uvu", True)], shared_weights=False, internal_weights=False)
+    tp = oeq.TensorProduct(p, torch_op=True)
+    lib = torch.library.Library("openequivariance_b200", "IMPL")
+    lib.impl(f"tp_forward{tp.tp_id}", lambda x, y, w: _forward(x, y, w[:, :3]), "CPU")
+    lib.impl(f"tp_grad_helper{tp.tp_id}", lambda x, y, w, dz: [g if g.shape == t.shape else torch.cat([g, torch.zeros(N, 6, dtype=g.dtype)], 1)
+                                                             for g, t in zip(_gradient(x, y, w[:, :3], dz), (x, y, w))], "CPU")
+    yield tp
+    lib._destroy()
+
+
+def _inputs(grad=True):
+    gen = torch.Generator().manual_seed(1)
+    x, y, w = (torch.randn(N, k, generator=gen).requires_grad_(grad) for k in (3, 3, 9))
+    return x, y, w, torch.randn(N, 3, generator=gen).requires_grad_(grad)
+
+
+def _wanted(x, y, w, dz):
+    return torch.autograd.grad(_forward(x, y, w[:, :3]), (x, y, w), dz)
+
+
+def test_a_second_pass_without_retained_graph(product):
+    """Saved operands are kept with the graph, as the reference's nodes keep them: two backward passes through one result
+    need no retain_graph."""
+    x, y, w, dz = _inputs()
+    z = product.forward(x, y, w)
+    for _ in range(2):
+        for got, want in zip(torch.autograd.grad(z, (x, y, w), dz.detach()), _wanted(x, y, w, dz.detach())):
+            torch.testing.assert_close(got, want)
+    first = torch.autograd.grad(z, (x, y, w), dz, create_graph=True)
+    for _ in range(2):
+        got, = torch.autograd.grad(first[0], y, torch.ones(N, 3))
+        want, = torch.autograd.grad(_wanted_graph(x, y, w, dz), y, torch.ones(N, 3))
+        torch.testing.assert_close(got, want)
+
+
+def _wanted_graph(x, y, w, dz):
+    return torch.autograd.grad(_forward(x, y, w[:, :3]), x, dz, create_graph=True)[0]
