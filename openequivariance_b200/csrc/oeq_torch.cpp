@@ -274,8 +274,9 @@ struct ForwardNode final : OpNode {
     using OpNode::OpNode;
     std::string name() const override { return "OeqForwardBackward"; }
     variable_list apply(variable_list&& grads) override {
-        if (!grads[0].defined()) return variable_list(op->inputs);
         variable_list in = operands();
+        // (nothing flows in from a later node that gave no gradient: zeros, and zero gradients out)
+        if (!grads[0].defined()) grads[0] = in[0].new_zeros_symint({in[0].sym_size(0), op->z_dim});
         in.insert(in.begin() + op->inputs, std::move(grads[0]));
         return call_gradient(*op, in);
     }
@@ -289,12 +290,8 @@ struct GradientNode final : OpNode {
     variable_list apply(variable_list&& e) override {
         Op& o = *op;
         const variable_list s = operands();
-        bool any = false;
-        for (int i = 0; i < o.inputs; ++i) {
-            any |= e[i].defined();
+        for (int i = 0; i < o.inputs; ++i)
             if (!e[i].defined()) e[i] = at::zeros_like(s[i]);
-        }
-        if (!any) return variable_list(o.inputs + 1);
         const Args idx(s.data() + o.inputs + 1, (size_t)o.index);
         const Tensor &x = s[0], &y = s[1], &dz = s[o.inputs];
         if (o.inputs == 2) {

@@ -57,3 +57,26 @@ def test_a_second_pass_without_retained_graph(product):
 
 def _wanted_graph(x, y, w, dz):
     return torch.autograd.grad(_forward(x, y, w[:, :3]), x, dz, create_graph=True)[0]
+
+
+class _NoGradient(torch.autograd.Function):
+    """A later layer that returns no gradient for its first input."""
+
+    @staticmethod
+    def forward(ctx, z, other):
+        return other * 1
+
+    @staticmethod
+    def backward(ctx, g):
+        return None, g
+
+
+def test_undefined_gradients_count_as_zeros(product):
+    other = torch.ones(2, requires_grad=True)
+    x, y, w, dz = _inputs()
+    z = product.forward(x, y, w)
+    for g, t in zip(torch.autograd.grad(_NoGradient.apply(z, other).sum(), (x, y, w)), (x, y, w)):
+        assert g.shape == t.shape and torch.count_nonzero(g) == 0
+    first = torch.autograd.grad(z, (x, y, w), dz, create_graph=True)
+    for g, t in zip(torch.autograd.grad(_NoGradient.apply(first[1], other).sum(), (x, y, w, dz)), (x, y, w, dz)):
+        assert g.shape == t.shape and torch.count_nonzero(g) == 0
