@@ -326,6 +326,10 @@ struct AutogradKernel final : c10::OperatorKernel {
     explicit AutogradKernel(Op* o) : op(o) {}
     void operator()(const OperatorHandle& handle, c10::DispatchKeySet keys, Stack* stack) {
         const int diff = op->inputs + (GRADIENT ? 1 : 0), n = diff + op->index;
+        // no tangents: below this kernel they would be dropped, and the derivative would come out as zero
+        for (int i = 0; i < diff; ++i)
+            TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined((*stack)[stack->size() - n + i].toTensor()),
+                                        "openequivariance_b200: the operators have no forward-mode derivative");
         bool needed = false;
         if (at::GradMode::is_enabled())
             for (int i = 0; i < diff; ++i) needed |= (*stack)[stack->size() - n + i].toTensor().requires_grad();

@@ -80,3 +80,23 @@ def test_undefined_gradients_count_as_zeros(product):
     first = torch.autograd.grad(z, (x, y, w), dz, create_graph=True)
     for g, t in zip(torch.autograd.grad(_NoGradient.apply(first[1], other).sum(), (x, y, w, dz)), (x, y, w, dz)):
         assert g.shape == t.shape and torch.count_nonzero(g) == 0
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_forward_mode_is_refused(product, grad):
+    """A tangent is not dropped in silence."""
+    import torch.autograd.forward_ad as fwad
+    x, y, w, dz = _inputs(grad)
+    with fwad.dual_level():
+        for i in range(3):
+            args = [x, y, w]
+            args[i] = fwad.make_dual(args[i], torch.ones_like(args[i]))
+            with pytest.raises(NotImplementedError, match="forward-mode"):
+                product.forward(*args)
+            with pytest.raises(NotImplementedError, match="forward-mode"):
+                product.backward_helper(*args, dz)
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            product.backward_helper(x, y, w, fwad.make_dual(dz, dz.detach()))
+    with pytest.raises(NotImplementedError, match="forward-mode"):
+        torch.func.jvp(lambda t: product.forward(t, y.detach(), w.detach()), (x.detach(),), (x.detach(),))
+    assert torch.isfinite(product.forward(x, y, w)).all()
