@@ -400,8 +400,10 @@ int oeq_torch_register(const char* forward, const char* gradient, const char* se
         const std::string ns = "openequivariance_b200";
         libraries().emplace_back(torch::Library::FRAGMENT, ns, std::nullopt, __FILE__, __LINE__);
         torch::Library& lib = libraries().back();
-        lib.def((std::string(forward) + "(" + in + idx + ") -> Tensor").c_str());
-        lib.def((std::string(gradient) + "(" + in + ", Tensor L3_grad" + idx + ") -> Tensor[]").c_str());
+        // (fake kernels and autograd are registered: a graph may hold these ops even where only such ops are allowed)
+        const std::vector<at::Tag> tags{at::Tag::pt2_compliant_tag};
+        lib.def((std::string(forward) + "(" + in + idx + ") -> Tensor").c_str(), tags);
+        lib.def((std::string(gradient) + "(" + in + ", Tensor L3_grad" + idx + ") -> Tensor[]").c_str(), tags);
         auto boxed = [](auto functor) { return torch::CppFunction::makeFromBoxedFunctor(std::move(functor)); };
         lib.impl(forward, torch::dispatch(c10::DispatchKey::CUDA, boxed(std::make_unique<ForwardKernel>(op))));
         lib.impl(gradient, torch::dispatch(c10::DispatchKey::CUDA, boxed(std::make_unique<GradientKernel>(op))));

@@ -100,3 +100,9 @@ def test_forward_mode_is_refused(product, grad):
     with pytest.raises(NotImplementedError, match="forward-mode"):
         torch.func.jvp(lambda t: product.forward(t, y.detach(), w.detach()), (x.detach(),), (x.detach(),))
     assert torch.isfinite(product.forward(x, y, w)).all()
+
+
+def test_ops_are_marked_for_compilation(product):
+    """torch.compile with only_allow_pt2_compliant_ops takes them."""
+    for op in (product.forward, product.backward_helper):
+        assert torch.Tag.pt2_compliant_tag in op.tags
