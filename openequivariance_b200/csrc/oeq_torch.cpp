@@ -217,16 +217,18 @@ variable_list conv_second(Op& op, at::ArrayRef<Tensor> in, at::ArrayRef<Tensor> 
 // ---------------------------------------------------------------- autograd
 
 // The gradients that an autograd node computes.  Plain CUDA tensors that nothing differentiates go straight to the
-// kernels; anything else (tracing modes, tensor subclasses, derivatives of the derivative) through the dispatcher.
+// kernels; anything else (tracing modes, tensor subclasses, batched tensors, negated or zero tensors whose memory does not
+// hold their values, derivatives of the derivative) through the dispatcher.
 bool direct(Args in) {
+    using c10::DispatchKey;
     const auto tls = c10::impl::tls_local_dispatch_key_set().included_;
-    if (at::GradMode::is_enabled() || tls.has(c10::DispatchKey::Python) || tls.has(c10::DispatchKey::PythonTLSSnapshot) ||
-        tls.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || tls.has(c10::DispatchKey::Functionalize))
+    if (at::GradMode::is_enabled() || tls.has(DispatchKey::Python) || tls.has(DispatchKey::PythonTLSSnapshot) ||
+        tls.has(DispatchKey::FuncTorchDynamicLayerFrontMode) || tls.has(DispatchKey::Functionalize))
         return false;
+    // keys of a dense CUDA tensor; a tensor with any other one is not plain
+    static const uint64_t plain = c10::DispatchKeySet({DispatchKey::CUDA, DispatchKey::ADInplaceOrView, DispatchKey::AutogradCUDA, DispatchKey::AutocastCUDA}).raw_repr();
     for (const Tensor& t : in)
-        if (!t.defined() || !t.is_cuda() || t.key_set().has(c10::DispatchKey::Python) || t.key_set().has(c10::DispatchKey::Functionalize) ||
-            t.key_set().has(c10::DispatchKey::FuncTorchBatched) || t.key_set().has(c10::DispatchKey::FuncTorchGradWrapper))
-            return false;
+        if (!t.defined() || !t.is_cuda() || (t.key_set().raw_repr() & ~plain) != 0) return false;
     return true;
 }
 Tensor call_forward(const Op& op, Args in) {

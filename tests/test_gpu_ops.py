@@ -94,3 +94,37 @@ def test_wrong_arguments_raise(op):
         with pytest.raises(ValueError, match="sender_perm"):
             call.forward(x, y, w, *index[:2], index[2][1:])
     assert torch.isfinite(call.forward(x, y, w, *index)).all()
+
+
+@pytest.mark.parametrize("op", ["product", "convolution"])
+def test_operands_whose_memory_does_not_hold_their_values(op):
+    """Lazily negated operands and gradients give the gradients of their values; batched gradients are refused by name."""
+    p = problem_by_name("nequip_32")
+    rows, cols = random_graph(7, 40, seed=1)
+    rows, cols, _, perm = orc.coord_graph(rows, cols)
+    if op == "product":
+        call, (x, y, w, dz), index = oeq.TensorProduct(p, torch_op=True), _cuda(*tp_inputs(p, 9, 1)), ()
+    else:
+        call = oeq.TensorProductConv(p, torch_op=True, deterministic=True)
+        (x, y, w, dz), index = _cuda(*conv_inputs(p, 7, 40, 1)), _cuda(rows, cols, perm)
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    cotangents = [torch.randn(t.shape, device="cuda", generator=gen) for t in (x, y, w)]
+
+    def gradients(wrap_x, wrap_dz, second=False):
+        ins = [t.clone().requires_grad_(True) for t in (x, y, w)]
+        z = call.forward(wrap_x(ins[0]), *ins[1:], *index)
+        if not second:
+            return torch.autograd.grad(z, ins, wrap_dz(dz))
+        first = torch.autograd.grad(z, ins, wrap_dz(dz), create_graph=True)
+        return torch.autograd.grad(first, ins, (wrap_dz(cotangents[0]), *cotangents[1:]))
+
+    negated, plain = torch._neg_view, torch.neg
+    for second in (False, True):
+        for wraps in ((negated, lambda t: t), (lambda t: t, negated), (negated, negated)):
+            same = tuple(plain if f is negated else f for f in wraps)
+            for got, want in zip(gradients(*wraps, second), gradients(*same, second)):
+                assert (got - want).abs().max().item() <= 1e-5 * want.abs().max().item()
+    z = call.forward(x.requires_grad_(True), y, w, *index)
+    with pytest.raises(RuntimeError, match="Batching rule"):
+        torch.autograd.grad(z, x, torch.stack([dz, dz]), is_grads_batched=True)
