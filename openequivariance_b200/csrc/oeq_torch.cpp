@@ -101,27 +101,33 @@ Tensor forward_cuda(const Op& op, Args in) {
     return z;
 }
 
-// Scratch of the deterministic backward pass.  Up to 256 MB come from the caching allocator call by call, safe with
-// any number of streams; more is kept on the operator (allocating it again and again would flush a full device's
-// cache): a quarter of it when the device cannot spare the whole, none when not even that.
+// Memory for the library to use as scratch: a quarter of what it wants when the device cannot spare the whole, none when
+// not even that.
+Tensor scratch_memory(size_t want, const at::TensorOptions& bytes) {
+    for (size_t size : {want, want / 4}) {
+        try {
+            return at::empty({(int64_t)size}, bytes);
+        } catch (const c10::OutOfMemoryError&) {
+        }
+    }
+    return Tensor();
+}
+
+// Scratch of the deterministic backward pass, which runs without it too.  Up to 256 MB come from the caching allocator
+// call by call, safe with any number of streams; more is kept on the operator (allocating it again and again would flush
+// a full device's cache).
 Tensor backward_scratch(Op& op, int64_t nodes, int64_t edges, const at::TensorOptions& options) {
     const size_t want = oeq_conv_workspace_bytes(op.conv, nodes, edges);
     if (want == 0) return Tensor();
     const auto bytes = options.dtype(at::kByte);
-    if (want <= (256u << 20)) return at::empty({(int64_t)want}, bytes);
+    if (want <= (256u << 20)) return scratch_memory(want, bytes);
     const size_t device = (size_t)options.device().index();
     std::lock_guard<std::mutex> lock(op.mutex);
     if (op.scratch.size() <= device) op.scratch.resize(device + 1);
     Tensor& kept = op.scratch[device];
     if (kept.defined() && (size_t)kept.numel() >= want) return kept;
     kept = Tensor();
-    for (size_t size : {want, want / 4}) {
-        try {
-            kept = at::empty({(int64_t)size}, bytes);
-            break;
-        } catch (const c10::OutOfMemoryError&) {
-        }
-    }
+    kept = scratch_memory(want, bytes);
     return kept;
 }
 
