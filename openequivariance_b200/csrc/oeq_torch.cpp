@@ -7,6 +7,7 @@
 // differentiable.  All arguments are tensors: `inputs` operands, for the gradient op the output gradient, then the
 // index arrays of a convolution, so that one boxed kernel serves every operator.
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -41,8 +42,13 @@ struct Op {
     at::ScalarType dtype = at::kFloat;
     std::optional<OperatorHandle> forward, gradient, second;
     std::atomic<bool> call_second{false};   // the caller replaced the fused second derivatives by the op `second`
+    struct Kept {
+        Tensor memory;
+        std::optional<c10::cuda::CUDAStream> stream;    // whose work uses it
+        size_t wanted = 0;          // size that was asked for (the device may have had less)
+    };
     std::mutex mutex;
-    std::vector<Tensor> scratch;    // large backward scratch, per device
+    std::map<c10::DeviceIndex, Kept> kept;  // large backward scratch
 };
 
 void check(int rc) { TORCH_CHECK(rc == OEQ_OK, "oeq_b200: ", oeq_last_error()); }
@@ -114,21 +120,34 @@ Tensor scratch_memory(size_t want, const at::TensorOptions& bytes) {
 }
 
 // Scratch of the deterministic backward pass, which runs without it too.  Up to 256 MB come from the caching allocator
-// call by call, safe with any number of streams; more is kept on the operator (allocating it again and again would flush
-// a full device's cache).
-Tensor backward_scratch(Op& op, int64_t nodes, int64_t edges, const at::TensorOptions& options) {
+// call by call; more is kept on the operator (allocating it again and again would flush a full device's cache).  Kept
+// memory serves one stream, the last to ask: another stream's call gives it back to the pool of the former one, whose
+// allocations come after its pending work, and takes memory of its own.  The lock is held until the launches that use kept
+// memory are on the stream, so that the launches of two threads on one stream do not mix.  A captured call, whose graph may
+// run at any time on any stream, takes memory from the graph's pool.
+struct Scratch {
+    std::unique_lock<std::mutex> lock;
+    Tensor memory;
+    void* data() const { return memory.defined() ? memory.mutable_data_ptr() : nullptr; }
+    size_t bytes() const { return memory.defined() ? (size_t)memory.numel() : 0; }
+};
+Scratch backward_scratch(Op& op, int64_t nodes, int64_t edges, const at::TensorOptions& options) {
     const size_t want = oeq_conv_workspace_bytes(op.conv, nodes, edges);
-    if (want == 0) return Tensor();
+    if (want == 0) return {};
     const auto bytes = options.dtype(at::kByte);
-    if (want <= (256u << 20)) return scratch_memory(want, bytes);
-    const size_t device = (size_t)options.device().index();
-    std::lock_guard<std::mutex> lock(op.mutex);
-    if (op.scratch.size() <= device) op.scratch.resize(device + 1);
-    Tensor& kept = op.scratch[device];
-    if (kept.defined() && (size_t)kept.numel() >= want) return kept;
-    kept = Tensor();
-    kept = scratch_memory(want, bytes);
-    return kept;
+    if (want <= (256u << 20) || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+        return {{}, scratch_memory(want, bytes)};
+    const auto stream = c10::cuda::getCurrentCUDAStream();
+    std::unique_lock<std::mutex> lock(op.mutex);
+    Op::Kept& kept = op.kept[stream.device_index()];
+    const bool enough = kept.memory.defined() && ((size_t)kept.memory.numel() >= want || kept.wanted == want);
+    if (!enough || kept.stream != stream) {
+        kept.memory = Tensor();
+        kept.memory = scratch_memory(want, bytes);
+        kept.stream = stream;
+        kept.wanted = want;
+    }
+    return {std::move(lock), kept.memory};
 }
 
 // Operands x, y[, w], the output gradient, then the index arrays.
@@ -145,8 +164,8 @@ variable_list gradient_cuda(Op& op, Args in) {
     const void* wp = op.inputs == 3 ? w->const_data_ptr() : nullptr;
     void *dxp = out[0].mutable_data_ptr(), *dyp = out[1].mutable_data_ptr(), *dwp = op.inputs == 3 ? out[2].mutable_data_ptr() : nullptr;
     void* st = c10::cuda::getCurrentCUDAStream().stream();
-    Tensor ws;
     if (op.tp) {
+        Tensor ws;
         const size_t bytes = oeq_tp_workspace_bytes(op.tp, x->size(0));
         if (bytes) ws = at::empty({(int64_t)bytes}, x->options().dtype(at::kByte));
         check(oeq_tp_backward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(), dxp, dyp, dwp,
@@ -154,10 +173,10 @@ variable_list gradient_cuda(Op& op, Args in) {
     } else {
         const auto rows = in[op.inputs + 1].expect_contiguous(), cols = in[op.inputs + 2].expect_contiguous();
         const auto perm = in[op.inputs + (op.deterministic ? 3 : 1)].expect_contiguous();
-        if (op.deterministic) ws = backward_scratch(op, x->size(0), rows->size(0), x->options());
+        const Scratch ws = op.deterministic ? backward_scratch(op, x->size(0), rows->size(0), x->options()) : Scratch();
         check(oeq_conv_backward(op.conv, x->size(0), rows->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(),
                                 index_ptr(*rows), index_ptr(*cols), op.deterministic ? index_ptr(*perm) : nullptr, dxp, dyp, dwp,
-                                ws.defined() ? ws.mutable_data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0, st));
+                                ws.data(), ws.bytes(), st));
     }
     return out;
 }
@@ -208,12 +227,12 @@ variable_list conv_second(Op& op, at::ArrayRef<Tensor> in, at::ArrayRef<Tensor> 
     c10::cuda::CUDAGuard guard(c[0].device());
     for (int i = 0; i < 4; ++i) out.push_back(at::empty_like(c[i]));
     const int64_t nodes = c[0].size(0), edges = idx[0].size(0);
-    Tensor ws = op.deterministic ? backward_scratch(op, nodes, edges, c[0].options()) : Tensor();
+    const Scratch ws = op.deterministic ? backward_scratch(op, nodes, edges, c[0].options()) : Scratch();
     const int rc = oeq_conv_double_backward(
         op.conv, nodes, edges, c[0].const_data_ptr(), c[1].const_data_ptr(), c[2].const_data_ptr(), c[3].const_data_ptr(),
         c[4].const_data_ptr(), c[5].const_data_ptr(), c[6].const_data_ptr(), index_ptr(idx[0]), index_ptr(idx[1]),
         op.deterministic ? index_ptr(idx[2]) : nullptr, out[0].mutable_data_ptr(), out[1].mutable_data_ptr(), out[2].mutable_data_ptr(),
-        out[3].mutable_data_ptr(), ws.defined() ? ws.mutable_data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
+        out[3].mutable_data_ptr(), ws.data(), ws.bytes(),
         c10::cuda::getCurrentCUDAStream().stream());
     if (rc == OEQ_ERR_UNSUPPORTED) return {};
     check(rc);

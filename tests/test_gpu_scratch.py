@@ -1,6 +1,7 @@
-"""Scratch memory of the deterministic convolution: a device that has none to spare."""
+"""Scratch memory of the deterministic convolution: a device that has none to spare; several streams, threads and graphs."""
 import contextlib
 import gc
+import threading
 
 import numpy as np
 import pytest
@@ -57,3 +58,77 @@ def test_a_full_device(edges, share, launches, entry):
         assert conv.internal.last_backward_launches() == launches
     for g, r in zip(got, want):
         assert (g - r).abs().max().item() <= 1e-5 * r.abs().max().item()
+
+
+def test_a_full_device_is_asked_once():
+    """The size that did not fit is not tried again on every call (each try empties the allocator's cache)."""
+    conv, (x, y, w, dz), index = _case(300_000)
+    outputs = sum(-(-t.numel() * 4 // (2 * MB)) * 2 * MB for t in (x, y, w))
+    with _memory_left(outputs + 8 * MB + int(0.3 * len(y) * conv.L1.dim * 4)):
+        got = conv.backward_helper(x, y, w, dz, *index)
+        failed = torch.cuda.memory_stats()["num_ooms"]
+        for _ in range(3):
+            got = None
+            got = conv.backward_helper(x, y, w, dz, *index)
+            assert conv.internal.last_backward_launches() == 9
+        assert torch.cuda.memory_stats()["num_ooms"] == failed
+
+
+# 300 000 edges: 346 MB, kept between calls; 100 000: from the allocator
+@pytest.mark.parametrize("edges", [300_000, 100_000])
+def test_two_streams(edges):
+    """Backward passes of one operator on two streams at a time."""
+    conv, first, index = _case(edges, seed=3)
+    _, second, _ = _case(edges, seed=4)
+    want = [[t.clone() for t in conv.backward_helper(*arrays, *index)] for arrays in (first, second)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = []
+        for s, arrays in zip(streams, (first, second)):
+            with torch.cuda.stream(s):
+                got.append(conv.backward_helper(*arrays, *index))
+        torch.cuda.synchronize()
+        for g, r in zip(got, want):
+            assert all(torch.equal(a, b) for a, b in zip(g, r))
+
+
+def test_two_threads_on_one_stream():
+    conv, first, index = _case(300_000, seed=3)
+    _, second, _ = _case(300_000, seed=4)
+    want = [[t.clone() for t in conv.backward_helper(*arrays, *index)] for arrays in (first, second)]
+    same = [True, True]
+
+    def run(i, arrays):
+        for _ in range(10):
+            got = conv.backward_helper(*arrays, *index)
+            same[i] &= all(torch.equal(a, b) for a, b in zip(got, want[i]))
+
+    threads = [threading.Thread(target=run, args=(i, a)) for i, a in enumerate((first, second))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert same == [True, True]
+
+
+def test_a_captured_pass_has_scratch_of_its_own():
+    """A graph that replays beside other calls of the operator."""
+    conv, first, index = _case(300_000, seed=3)
+    _, second, _ = _case(300_000, seed=4)
+    want = [[t.clone() for t in conv.backward_helper(*arrays, *index)] for arrays in (first, second)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = conv.backward_helper(*first, *index)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for t in captured:
+            t.zero_()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            graph.replay()
+        got = conv.backward_helper(*second, *index)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(captured, want[0]))
+        assert all(torch.equal(a, b) for a, b in zip(got, want[1]))
