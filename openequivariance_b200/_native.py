@@ -124,6 +124,7 @@ def register_ops(forward, gradient, handle, *, deterministic=False, shared=False
             t.oeq_torch_error.restype = C.c_char_p
             t.oeq_torch_register.argtypes = [C.c_char_p] * 3 + [_P, _P] + [_INT] * 4 + [_I64] * 4
             t.oeq_torch_call_second.argtypes = [C.c_char_p, _INT]
+            t.oeq_torch_conv_gradients.argtypes = [C.c_char_p] + [_I64] * 2 + [_P] * 14 + [C.POINTER(_I64), C.POINTER(_P)]
             _torch_lib = t
     is_conv = isinstance(handle, ConvHandle)
     code = _torch_lib.oeq_torch_register(forward.encode(), gradient.encode(), second.encode() if second else None,
@@ -150,6 +151,17 @@ def register_ops(forward, gradient, handle, *, deterministic=False, shared=False
 def call_second(forward, call: bool):
     """Let the second backward pass of the operator with this forward op call its registered ``second`` op."""
     _torch_lib.oeq_torch_call_second(forward.encode(), int(call))
+
+
+def conv_gradients(forward, nodes, edges, *pointers):
+    """First (``EX``, ``EY``, ``EW``, ``GdZ`` 0) or second derivatives on the current device and stream, with the scratch
+    memory that the ops of the operator with this forward op keep.  Returns that memory's size and address."""
+    size, address = _I64(0), _P(None)
+    code = _torch_lib.oeq_torch_conv_gradients(forward.encode(), nodes, edges, *pointers, C.byref(size), C.byref(address))
+    if code < 0:
+        raise RuntimeError(_torch_lib.oeq_torch_error().decode(errors="replace"))
+    check(code)
+    return size.value, address.value or 0
 
 
 def check(code: int):

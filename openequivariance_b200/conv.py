@@ -107,7 +107,6 @@ class TensorProductConv(TensorProductBase):
         self.idx_dtype = idx_dtype
         self.deterministic = deterministic
         self.conv_id = next(_conv_ids)
-        self._scratch = {}
         self._second_replacement = None
         self.workspace_size = 0
         self.workspace_ptr = 0
@@ -119,9 +118,9 @@ class TensorProductConv(TensorProductBase):
             assert inst.connection_mode == "uvu", "the fused convolution supports 'uvu', or 'uvw' with shared weights"
         assert not config.shared_weights, "the fused convolution needs per-edge weights"
         self.internal = _native.ConvHandle(config, deterministic)
-        # The forward pass needs no scratch (node-aligned segmented reduction).  The deterministic backward
-        # pass takes optional scratch (one dX row per edge, capped); it is allocated on first use, per
-        # device, and kept (the reference keeps its workspace on the object too: ConvolutionBase.py:93-99).
+        # The forward pass needs no scratch (node-aligned segmented reduction).  The deterministic backward pass takes
+        # optional scratch (one dX row per edge, capped); large scratch is allocated on first use, per device, and kept
+        # with the ops (the reference keeps its workspace on the object: ConvolutionBase.py:93-99).
         self.setup_torch_module()
 
     @staticmethod
@@ -202,31 +201,9 @@ class TensorProductConv(TensorProductBase):
                                   torch.cuda.current_stream().cuda_stream)
         return z
 
-    def _backward_scratch(self, device, nodes, edges):
-        """(pointer, bytes) of the backward scratch for this call, growing the cached buffer if needed.
-        When the device cannot spare the preferred size a quarter of it is tried, then none (the library
-        then runs its scratch-free kernel)."""
-        want = self.internal.workspace_bytes(nodes, edges) if self.deterministic else 0
-        if want == 0:
-            return 0, 0
-        buf = self._scratch.get(device)
-        if buf is None or buf.numel() < want:
-            self._scratch.pop(device, None)
-            buf = None
-            for size in (want, want // 4):
-                try:
-                    buf = torch.empty(size, dtype=torch.uint8, device=device)
-                    break
-                except torch.OutOfMemoryError:
-                    continue
-            if buf is None:
-                return 0, 0
-            self._scratch[device] = buf
-        self.workspace_size, self.workspace_ptr = buf.numel(), buf.data_ptr()
-        return buf.data_ptr(), buf.numel()
-
     def _backward_impl(self, x, y, w, dz, rows, cols, perm=None, scratch=True):
-        """``scratch=False`` runs the deterministic pass without scratch memory (the sender-order kernel)."""
+        """``scratch=False`` runs the deterministic pass without scratch memory (the sender-order kernel); otherwise it
+        takes what the registered ops keep."""
         self._check(x, y, w, rows, cols, perm)
         if self.deterministic and perm is None:
             raise ValueError("the deterministic convolution needs sender_perm")
@@ -235,11 +212,15 @@ class TensorProductConv(TensorProductBase):
         perm_ptr = perm.contiguous().data_ptr() if (perm is not None and self.deterministic) else 0
         dx, dy, dw = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w)
         with torch.cuda.device(x.device):
-            ws_ptr, ws_bytes = self._backward_scratch(x.device, x.shape[0], rows.shape[0]) if scratch else (0, 0)
-            self.internal.backward(x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(),
-                                   dz.data_ptr(), rows.data_ptr(), cols.data_ptr(), perm_ptr,
-                                   dx.data_ptr(), dy.data_ptr(), dw.data_ptr(), ws_ptr, ws_bytes,
-                                   torch.cuda.current_stream().cuda_stream)
+            if scratch:
+                self.workspace_size, self.workspace_ptr = _native.conv_gradients(
+                    f"conv_forward{self.conv_id}", x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(),
+                    dz.data_ptr(), 0, 0, 0, rows.data_ptr(), cols.data_ptr(), perm_ptr, dx.data_ptr(), dy.data_ptr(),
+                    dw.data_ptr(), 0)
+            else:
+                self.internal.backward(x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(),
+                                       dz.data_ptr(), rows.data_ptr(), cols.data_ptr(), perm_ptr, dx.data_ptr(),
+                                       dy.data_ptr(), dw.data_ptr(), 0, 0, torch.cuda.current_stream().cuda_stream)
         return dx, dy, dw
 
     def _has_fused_double_backward(self):
@@ -267,13 +248,11 @@ class TensorProductConv(TensorProductBase):
         perm_ptr = perm.contiguous().data_ptr() if (perm is not None and self.deterministic) else 0
         gx, gy, gw, gdz = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w), torch.empty_like(dz)
         with torch.cuda.device(x.device):
-            ws_ptr, ws_bytes = self._backward_scratch(x.device, x.shape[0], rows.shape[0])
             try:
-                self.internal.double_backward(x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(),
-                                              dz.data_ptr(), ex.data_ptr(), ey.data_ptr(), ew.data_ptr(),
-                                              rows.data_ptr(), cols.data_ptr(), perm_ptr, gx.data_ptr(),
-                                              gy.data_ptr(), gw.data_ptr(), gdz.data_ptr(), ws_ptr, ws_bytes,
-                                              torch.cuda.current_stream().cuda_stream)
+                self.workspace_size, self.workspace_ptr = _native.conv_gradients(
+                    f"conv_forward{self.conv_id}", x.shape[0], rows.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(),
+                    dz.data_ptr(), ex.data_ptr(), ey.data_ptr(), ew.data_ptr(), rows.data_ptr(), cols.data_ptr(), perm_ptr,
+                    gx.data_ptr(), gy.data_ptr(), gw.data_ptr(), gdz.data_ptr())
             except _native.OeqError as err:
                 if err.code == _native.OEQ_ERR_UNSUPPORTED:
                     return None

@@ -458,4 +458,31 @@ int oeq_torch_call_second(const char* forward, int call) {
     return 0;
 }
 
+// The gradient passes of a convolution's object on raw pointers (any number of receivers), with the scratch that its ops
+// keep: `forward` names its forward op; the current device and stream are those of the calling thread.  Returns the
+// library's code; `scratch`: the memory used.  EX null: first derivatives into dX, dY, dW (and no dZ gradient).
+int oeq_torch_conv_gradients(const char* forward, int64_t nodes, int64_t edges, const void* X, const void* Y, const void* W, const void* dZ,
+                             const void* EX, const void* EY, const void* EW, const int64_t* rows, const int64_t* cols, const int64_t* perm,
+                             void* dX, void* dY, void* dW, void* GdZ, int64_t* scratch_bytes, void** scratch) {
+    try {
+        Op* op = nullptr;
+        {
+            std::lock_guard<std::mutex> lock(register_mutex);
+            auto it = operators().find(forward);
+            TORCH_CHECK(it != operators().end(), "no such operator");
+            op = it->second;
+        }
+        const auto stream = c10::cuda::getCurrentCUDAStream();
+        const Scratch ws = op->deterministic ? backward_scratch(*op, nodes, edges, at::TensorOptions().device(stream.device())) : Scratch();
+        *scratch_bytes = (int64_t)ws.bytes();
+        *scratch = ws.data();
+        if (EX) return oeq_conv_double_backward(op->conv, nodes, edges, X, Y, W, dZ, EX, EY, EW, rows, cols, perm, dX, dY, dW, GdZ,
+                                                ws.data(), ws.bytes(), stream.stream());
+        return oeq_conv_backward(op->conv, nodes, edges, X, Y, W, dZ, rows, cols, perm, dX, dY, dW, ws.data(), ws.bytes(), stream.stream());
+    } catch (const std::exception& e) {
+        register_error = e.what();
+        return -1;
+    }
+}
+
 }  // extern "C"

@@ -132,3 +132,15 @@ def test_a_captured_pass_has_scratch_of_its_own():
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(captured, want[0]))
         assert all(torch.equal(a, b) for a, b in zip(got, want[1]))
+
+
+def test_one_kept_buffer_for_all_entry_points():
+    conv, (x, y, w, dz), index = _case(300_000)
+    conv.backward_helper(x, y, w, dz, *index)
+    held = torch.cuda.memory_allocated()
+    conv._backward_impl(x, y, w, dz, *index)
+    assert conv.workspace_size == len(y) * conv.L1.dim * 4
+    address = conv.workspace_ptr
+    conv._double_backward_impl(x, y, w, dz, x, y, w, *index)
+    assert conv.workspace_ptr == address
+    assert torch.cuda.memory_allocated() == held
