@@ -209,7 +209,8 @@ class TensorProductConv(TensorProductBase):
             raise ValueError("the deterministic convolution needs sender_perm")
         x, y, w, dz = x.contiguous(), y.contiguous(), w.contiguous(), dz.contiguous()
         rows, cols = rows.contiguous(), cols.contiguous()
-        perm_ptr = perm.contiguous().data_ptr() if (perm is not None and self.deterministic) else 0
+        perm = perm.contiguous() if (perm is not None and self.deterministic) else None   # (held until the launch)
+        perm_ptr = 0 if perm is None else perm.data_ptr()
         dx, dy, dw = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w)
         with torch.cuda.device(x.device):
             if scratch:
@@ -245,7 +246,8 @@ class TensorProductConv(TensorProductBase):
             raise ValueError("the deterministic convolution needs sender_perm")
         x, y, w, dz, ex, ey, ew = (t.contiguous() for t in (x, y, w, dz, ex, ey, ew))
         rows, cols = rows.contiguous(), cols.contiguous()
-        perm_ptr = perm.contiguous().data_ptr() if (perm is not None and self.deterministic) else 0
+        perm = perm.contiguous() if (perm is not None and self.deterministic) else None   # (held until the launch)
+        perm_ptr = 0 if perm is None else perm.data_ptr()
         gx, gy, gw, gdz = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w), torch.empty_like(dz)
         with torch.cuda.device(x.device):
             try:

@@ -484,3 +484,19 @@ def test_backward_without_scratch_uses_the_sender_order_kernel():
     rx, ry, rw = orc.conv_backward(p, x, y, w, dz, rows, cols)
     assert rel_err(dx.cpu().numpy(), rx) < 1e-5 and rel_err(dy.cpu().numpy(), ry) < 1e-5
     assert rel_err(dw.cpu().numpy(), rw) < 1e-5
+
+
+def test_strided_sender_order():
+    """A sender order that has to be copied first: the copy outlives the allocation of the results."""
+    p = problem_by_name("nequip_32")
+    nodes, edges = 500, 20000
+    rows, cols = random_graph(nodes, edges, seed=61)
+    rows, cols, _, perm = orc.coord_graph(rows, cols)
+    xt, yt, wt, dzt, r, c, pm = cuda(*conv_inputs(p, nodes, edges, 62), rows, cols, perm)
+    conv = oeq.TensorProductConv(p, torch_op=True, deterministic=True)
+    want = conv._backward_impl(xt, yt, wt, dzt, r, c, pm)
+    strided = torch.stack([pm, torch.zeros_like(pm)], 1)[:, 0]
+    assert not strided.is_contiguous()
+    for call in (conv._backward_impl, conv.backward_helper):
+        for a, b in zip(call(xt, yt, wt, dzt, r, c, strided), want):
+            assert torch.equal(a, b)
