@@ -1734,6 +1734,7 @@ long long uvu_grid(const Kernel& k, long long n_items) {
 // ====================================================================== C ABI
 
 struct oeq_tp {
+    std::mutex mutex;           // a call that launches (and loads kernels the first time) at a time
     Problem prob;
     Kernel fwd, bwd;
     Kernel fwd_tc;              // tensor-core forward ('uvw', shared FP32 weights), when the problem qualifies
@@ -1759,6 +1760,7 @@ struct oeq_tp {
     cudaStream_t last_stream = nullptr;
 };
 struct oeq_conv {
+    std::mutex mutex;           // a call that launches (and loads kernels the first time) at a time
     Problem prob;
     bool deterministic = false;
     Kernel fwd, bwd;
@@ -2031,6 +2033,7 @@ static int launch_gemm(Kernel& k, const Problem& p, long long batch, const void*
 
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
     if (batch == 0) return OEQ_OK;
     if (!X || !Y || !W || !Z) return fail(OEQ_ERR_INVALID, "null buffer");
@@ -2079,6 +2082,7 @@ size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch) {
 int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, const void* dZ, void* dX,
                     void* dY, void* dW, void* workspace, size_t workspace_bytes, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
     cudaStream_t st = (cudaStream_t)stream;
     const Problem& p = h->prob;
@@ -2232,6 +2236,7 @@ int oeq_tp_double_backward(oeq_tp* h, int64_t batch, const void* X, const void* 
                            const void* EX, const void* EY, const void* EW, void* GX, void* GY, void* GW, void* GdZ,
                            void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (!h->has_dbl) return fail(OEQ_ERR_UNSUPPORTED, "no one-pass second-derivative kernel for this problem: compose it from "
                                                       "oeq_tp_forward and oeq_tp_backward");
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
@@ -2321,6 +2326,7 @@ static int noalloc_scratch(void** out) {
 int oeq_tp_backward_noalloc(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, const void* dZ,
                             void* dX, void* dY, void* dW, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     const Problem& p = h->prob;
     if (!p.shared)
         return fail(OEQ_ERR_INVALID, "per-row weights need no scratch: call oeq_tp_backward with a null workspace");
@@ -2441,6 +2447,7 @@ int oeq_conv_forward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, c
                      void* stream) {
     (void)workspace; (void)workspace_bytes;
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (nodes < 0 || edges < 0) return fail(OEQ_ERR_INVALID, "negative size");
     cudaStream_t st = (cudaStream_t)stream;
     const Problem& p = h->prob;
@@ -2498,6 +2505,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
                       const void* dZ, const int64_t* rows, const int64_t* cols, const int64_t* perm, void* dX,
                       void* dY, void* dW, void* workspace, size_t workspace_bytes, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (nodes < 0 || edges < 0) return fail(OEQ_ERR_INVALID, "negative size");
     cudaStream_t st = (cudaStream_t)stream;
     const Problem& p = h->prob;
@@ -2665,6 +2673,7 @@ int oeq_conv_double_backward(oeq_conv* h, int64_t nodes, int64_t edges, const vo
                              const int64_t* cols, const int64_t* perm, void* GX, void* GY, void* GW, void* GdZ,
                              void* workspace, size_t workspace_bytes, void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    std::lock_guard<std::mutex> lock(h->mutex);
     if (nodes < 0 || edges < 0) return fail(OEQ_ERR_INVALID, "negative size");
     if (!oeq_conv_has_double_backward(h)) return fail(OEQ_ERR_UNSUPPORTED, "no fused second derivatives for this problem");
     cudaStream_t st = (cudaStream_t)stream;

@@ -128,3 +128,31 @@ def test_operands_whose_memory_does_not_hold_their_values(op):
     z = call.forward(x.requires_grad_(True), y, w, *index)
     with pytest.raises(RuntimeError, match="Batching rule"):
         torch.autograd.grad(z, x, torch.stack([dz, dz]), is_grads_batched=True)
+
+
+def test_first_calls_from_several_threads():
+    """The kernels of an operator are loaded by its first call; several threads may make it."""
+    import threading
+    p = problem_by_name("nequip_32")
+    rows, cols = random_graph(7, 40, seed=1)
+    rows, cols, _, perm = orc.coord_graph(rows, cols)
+    for _ in range(5):
+        cases = [(oeq.TensorProduct(p, torch_op=True), _cuda(*tp_inputs(p, 9, 1)), ()),
+                 (oeq.TensorProductConv(p, torch_op=True, deterministic=True), _cuda(*conv_inputs(p, 7, 40, 1)), _cuda(rows, cols, perm))]
+        for op, (x, y, w, dz), index in cases:
+            results, start = [None] * 6, threading.Barrier(6)
+
+            def run(i):
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    start.wait()
+                    results[i] = [op.forward(x, y, w, *index), *op.backward_helper(x, y, w, dz, *index)]
+
+            torch.cuda.synchronize()
+            threads = [threading.Thread(target=run, args=(i,)) for i in range(6)]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            torch.cuda.synchronize()
+            want = [op.forward(x, y, w, *index), *op.backward_helper(x, y, w, dz, *index)]
+            assert all(torch.equal(a, b) for got in results for a, b in zip(got, want))
