@@ -105,9 +105,18 @@ int64_t oeq_tp_weight_numel(const oeq_tp* h);
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z,
                    void* stream);
 
-/* Scratch needed by oeq_tp_backward for `batch` rows (0 unless weights are shared): partial weight gradients,
- * packed weights and, for 'uvw' with second-input multiplicity 1, the products of the weights with dZ for blocks
- * of at most 1 GiB. */
+/* The same with device memory for what a call prepares (shared FP32 'uvw' weights in the operand layout of the tensor
+ * cores; oeq_tp_forward_workspace_bytes is 0 for all else), 16-byte aligned, free again after the call's launches.  Calls on
+ * several streams may then overlap.  Without it the prepared weights are in memory that the handle allocates at its first
+ * such call and writes in every one: oeq_tp_forward calls on one handle belong on one stream. */
+size_t oeq_tp_forward_workspace_bytes(const oeq_tp* h);
+int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* workspace,
+                      size_t workspace_bytes, void* stream);
+
+/* Scratch of oeq_tp_backward for `batch` rows (0 unless weights are shared): partial weight gradients and, for 'uvw' with
+ * second-input multiplicity 1, the products of the weights with dZ for blocks of at most 1 GiB and (FP32) the packed
+ * weights behind them.  Less is taken as long as it holds the partial gradients; the packed weights are then in memory of
+ * the handle's, as for oeq_tp_forward, or other kernels run. */
 size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch);
 
 /* dX, dY, dW from X, Y, W, dZ.  Replaces JITTPImpl::backward (tensorproducts.hpp:87-95).

@@ -62,6 +62,8 @@ SYMBOLS = {
     "oeq_tp_destroy": (_INT, [_P]),
     "oeq_tp_weight_numel": (_I64, [_P]),
     "oeq_tp_forward": (_INT, [_P, _I64, _P, _P, _P, _P, _P]),
+    "oeq_tp_forward_workspace_bytes": (_SZ, [_P]),
+    "oeq_tp_forward_ws": (_INT, [_P, _I64, _P, _P, _P, _P, _P, _SZ, _P]),
     "oeq_tp_workspace_bytes": (_SZ, [_P, _I64]),
     "oeq_tp_backward": (_INT, [_P, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _SZ, _P]),
     "oeq_tp_backward_noalloc": (_INT, [_P, _I64, _P, _P, _P, _P, _P, _P, _P, _P]),
@@ -250,8 +252,11 @@ class TPHandle(_Handle):
         self.desc = Descriptor(problem)
         check(lib().oeq_tp_create(self.desc.ref(), C.byref(self.ptr)))
 
-    def forward(self, batch, x, y, w, z, stream):
-        check(lib().oeq_tp_forward(self.ptr, batch, x, y, w, z, stream))
+    def forward_workspace_bytes(self):
+        return lib().oeq_tp_forward_workspace_bytes(self.ptr)
+
+    def forward(self, batch, x, y, w, z, stream, ws=0, ws_bytes=0):
+        check(lib().oeq_tp_forward_ws(self.ptr, batch, x, y, w, z, ws, ws_bytes, stream))
 
     def workspace_bytes(self, batch):
         return lib().oeq_tp_workspace_bytes(self.ptr, batch)

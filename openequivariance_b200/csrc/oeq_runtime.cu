@@ -1747,14 +1747,14 @@ struct oeq_tp {
     Kernel grad_product_k, grad_channels_k;
     TcGeometry grad_tc;
     bool has_grad_tc = false;
-    void* d_packed_t = nullptr; // the transposed weights, split and swizzled
+    void* d_packed_t = nullptr; // the transposed weights, split and swizzled (calls whose workspace does not hold them)
     cudaKernel_t pack_t_fn = nullptr;
     Kernel gemm, gemm_dw;       // FP64 with shared weights: the product and the weight gradient as GEMMs
     bool has_gemm = false, has_gemm_bwd = false;
     Kernel dbl;                 // one-pass second derivatives ('uvu', per-row weights)
     bool has_dbl = false;
     TcGeometry tc;
-    void* d_packed = nullptr;   // weights split and swizzled for the tensor cores (owned by the handle)
+    void* d_packed = nullptr;   // weights split and swizzled for the tensor cores (calls without a workspace)
     cudaKernel_t pack_fn = nullptr;
     int* d_status = nullptr;
     cudaStream_t last_stream = nullptr;
@@ -1937,7 +1937,17 @@ static int ensure_status(int** d_status) {
     return OEQ_OK;
 }
 
-static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack, void*& packed) {
+// Weights in the operand layout: at `workspace` when it holds them, else in memory of the handle's own (`own`), which
+// every call that has no workspace writes anew: such calls are for one stream at a time.
+static int packed_weights(const TcGeometry& geo, void* workspace, size_t workspace_bytes, void*& own, void*& packed) {
+    packed = workspace;
+    if (workspace && workspace_bytes >= geo.packed_bytes && aligned16(workspace)) return OEQ_OK;
+    if (!own) OEQ_CUDA(cudaMalloc(&own, geo.packed_bytes));
+    packed = own;
+    return OEQ_OK;
+}
+
+static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack) {
     if (k.loaded) return OEQ_OK;
     OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
     OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_tc_kernel"));
@@ -1950,7 +1960,6 @@ static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack, voi
     cudaFuncAttributes attr;
     if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
     else (void)cudaGetLastError();
-    OEQ_CUDA(cudaMalloc(&packed, geo.packed_bytes));
     k.loaded = true;
     return OEQ_OK;
 }
@@ -2031,7 +2040,14 @@ static int launch_gemm(Kernel& k, const Problem& p, long long batch, const void*
     return OEQ_OK;
 }
 
+size_t oeq_tp_forward_workspace_bytes(const oeq_tp* h) { return h && h->has_tc ? h->tc.packed_bytes : 0; }
+
 int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* stream) {
+    return oeq_tp_forward_ws(h, batch, X, Y, W, Z, nullptr, 0, stream);
+}
+
+int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, const void* W, void* Z, void* workspace, size_t workspace_bytes,
+                      void* stream) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
     std::lock_guard<std::mutex> lock(h->mutex);
     if (batch < 0) return fail(OEQ_ERR_INVALID, "negative batch");
@@ -2041,8 +2057,10 @@ int oeq_tp_forward(oeq_tp* h, int64_t batch, const void* X, const void* Y, const
     if (rc) return rc;
     h->last_stream = (cudaStream_t)stream;
     if (h->has_tc) {
-        if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed))) return rc;
-        return launch_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, h->d_packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
+        void* packed = nullptr;
+        if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn)) || (rc = packed_weights(h->tc, workspace, workspace_bytes, h->d_packed, packed)))
+            return rc;
+        return launch_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     }
     if (h->has_gemm) return launch_gemm(h->gemm, h->prob, batch, X, Y, W, Z, (cudaStream_t)stream);
     if (h->prob.mode == OEQ_MODE_UVW) {
@@ -2075,7 +2093,7 @@ size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch) {
     if (h->has_gemm_bwd)
         return std::max((size_t)gemm_shares(h->prob, batch, 256) * h->prob.w_numel * 8, std::min((size_t)batch * h->grad_product.z_dim * 8, UVW_DT_BYTES));
     size_t bytes = (size_t)groups * h->prob.w_numel * h->prob.elem();
-    if (h->has_grad_tc) bytes = std::max(bytes, std::min((size_t)batch * h->grad_product.z_dim * 4, UVW_DT_BYTES));
+    if (h->has_grad_tc) bytes = std::max(bytes, std::min((size_t)batch * h->grad_product.z_dim * 4, UVW_DT_BYTES) + h->grad_tc.packed_bytes + 256);
     return bytes;
 }
 
@@ -2185,12 +2203,18 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             up.skip_dw = 1;
             up.ws = nullptr;
             // dX and dY in two steps over dT rows, which take the partial gradients' place in the workspace
-            const size_t row = (size_t)h->grad_product.z_dim * 4;
-            const long long block = h->has_grad_tc && aligned16(workspace) ? (long long)std::min<size_t>((size_t)batch, workspace_bytes / row) : 0;
+            const size_t row = (size_t)h->grad_product.z_dim * 4, tail = h->grad_tc.packed_bytes;
+            // (their weights at the end of the workspace, unless it is too small to hold them beside the rows)
+            const size_t least = (size_t)std::min<long long>(batch, 4096) * row;
+            const size_t room = workspace_bytes >= least + tail + 256 ? (workspace_bytes - tail) / 256 * 256 : workspace_bytes;
+            const long long block = h->has_grad_tc && aligned16(workspace) ? (long long)std::min<size_t>((size_t)batch, room / row) : 0;
             if (block > 0 && (block == batch || block >= 4096)) {
-                if ((rc = load_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t))) return rc;
+                void* packed = nullptr;
+                if ((rc = load_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn)) ||
+                    (rc = packed_weights(h->grad_tc, (char*)workspace + room, workspace_bytes - room, h->d_packed_t, packed)))
+                    return rc;
                 return gradients_from_dt(block, [&](long long b0, long long rows, const void* dz) {
-                    return launch_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, h->d_packed_t, b0 == 0, rows, dz, nullptr, W, workspace,
+                    return launch_uvw_tc(h->grad_product_k, h->grad_tc, h->pack_t_fn, packed, b0 == 0, rows, dz, nullptr, W, workspace,
                                          h->d_status, st);
                 });
             }

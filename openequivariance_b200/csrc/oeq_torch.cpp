@@ -98,7 +98,11 @@ Tensor forward_cuda(const Op& op, Args in) {
     Tensor z = at::empty({x->size(0), op.z_dim}, x->options());
     void* st = c10::cuda::getCurrentCUDAStream().stream();
     if (op.tp) {
-        check(oeq_tp_forward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, z.mutable_data_ptr(), st));
+        Tensor ws;      // of this call: safe with any number of streams
+        const size_t bytes = oeq_tp_forward_workspace_bytes(op.tp);
+        if (bytes) ws = at::empty({(int64_t)bytes}, x->options().dtype(at::kByte));
+        check(oeq_tp_forward_ws(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, z.mutable_data_ptr(),
+                                bytes ? ws.mutable_data_ptr() : nullptr, bytes, st));
     } else {
         const auto rows = in[op.inputs].expect_contiguous(), cols = in[op.inputs + 1].expect_contiguous();
         check(oeq_conv_forward(op.conv, x->size(0), rows->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, index_ptr(*rows),

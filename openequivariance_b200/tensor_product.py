@@ -87,7 +87,6 @@ class TensorProduct(TensorProductBase):
         self.tp_id = next(_op_ids)
         self.internal = _native.TPHandle(problem)
         self._has_fused_double_backward = self.internal.has_double_backward()
-        self._workspace = None
         # both modes need torch to drive device memory and streams
         self.setup_torch_custom_op()
 
@@ -118,9 +117,10 @@ class TensorProduct(TensorProductBase):
         self._check_shapes(x, y, w)
         x, y, w = x.contiguous(), y.contiguous(), w.contiguous()
         z = torch.empty((x.shape[0], self.L3.dim), dtype=x.dtype, device=x.device)
+        ws = torch.empty(self.internal.forward_workspace_bytes(), dtype=torch.uint8, device=x.device)
         with torch.cuda.device(x.device):
             self.internal.forward(x.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(), z.data_ptr(),
-                                  torch.cuda.current_stream().cuda_stream)
+                                  torch.cuda.current_stream().cuda_stream, ws.data_ptr(), ws.numel())
         return z
 
     def _backward_impl(self, x, y, w, dz):
@@ -128,16 +128,10 @@ class TensorProduct(TensorProductBase):
         self._check_shapes(x, y, w)
         x, y, w, dz = x.contiguous(), y.contiguous(), w.contiguous(), dz.contiguous()
         dx, dy, dw = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w)
-        ws_bytes = self.internal.workspace_bytes(x.shape[0])
-        ws_ptr = 0
-        if ws_bytes:
-            ws = self._workspace
-            if ws is None or ws.numel() < ws_bytes or ws.device != x.device:
-                ws = self._workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
-            ws_ptr = ws.data_ptr()
+        ws = torch.empty(self.internal.workspace_bytes(x.shape[0]), dtype=torch.uint8, device=x.device)
         with torch.cuda.device(x.device):
             self.internal.backward(x.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(), dz.data_ptr(),
-                                   dx.data_ptr(), dy.data_ptr(), dw.data_ptr(), ws_ptr, ws_bytes,
+                                   dx.data_ptr(), dy.data_ptr(), dw.data_ptr(), ws.data_ptr(), ws.numel(),
                                    torch.cuda.current_stream().cuda_stream)
         return dx, dy, dw
 
