@@ -169,11 +169,23 @@ variable_list gradient_cuda(Op& op, Args in) {
     void *dxp = out[0].mutable_data_ptr(), *dyp = out[1].mutable_data_ptr(), *dwp = op.inputs == 3 ? out[2].mutable_data_ptr() : nullptr;
     void* st = c10::cuda::getCurrentCUDAStream().stream();
     if (op.tp) {
-        Tensor ws;
-        const size_t bytes = oeq_tp_workspace_bytes(op.tp, x->size(0));
-        if (bytes) ws = at::empty({(int64_t)bytes}, x->options().dtype(at::kByte));
-        check(oeq_tp_backward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(), dxp, dyp, dwp,
-                              bytes ? ws.mutable_data_ptr() : nullptr, bytes, st));
+        // Half of the workspace, a quarter ... when the device cannot spare the whole: the library then goes through the
+        // batch in blocks or with other kernels, as long as the partial weight gradients fit.
+        const size_t want = oeq_tp_workspace_bytes(op.tp, x->size(0));
+        for (size_t bytes = want;; bytes /= 2) {
+            Tensor ws;
+            try {
+                if (bytes) ws = at::empty({(int64_t)bytes}, x->options().dtype(at::kByte));
+            } catch (const c10::OutOfMemoryError&) {
+                if (bytes / 2 < want / 64) throw;
+                continue;
+            }
+            const int rc = oeq_tp_backward(op.tp, x->size(0), x->const_data_ptr(), y->const_data_ptr(), wp, dz->const_data_ptr(), dxp, dyp,
+                                           dwp, bytes ? ws.mutable_data_ptr() : nullptr, bytes, st);
+            TORCH_CHECK_WITH(OutOfMemoryError, rc != OEQ_ERR_INVALID || bytes == want, "out of memory: ", want, " bytes of workspace");
+            check(rc);
+            break;
+        }
     } else {
         const auto rows = in[op.inputs + 1].expect_contiguous(), cols = in[op.inputs + 2].expect_contiguous();
         const auto perm = in[op.inputs + (op.deterministic ? 3 : 1)].expect_contiguous();

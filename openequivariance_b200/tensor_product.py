@@ -128,11 +128,23 @@ class TensorProduct(TensorProductBase):
         self._check_shapes(x, y, w)
         x, y, w, dz = x.contiguous(), y.contiguous(), w.contiguous(), dz.contiguous()
         dx, dy, dw = torch.empty_like(x), torch.empty_like(y), torch.empty_like(w)
-        ws = torch.empty(self.internal.workspace_bytes(x.shape[0]), dtype=torch.uint8, device=x.device)
-        with torch.cuda.device(x.device):
-            self.internal.backward(x.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(), dz.data_ptr(),
-                                   dx.data_ptr(), dy.data_ptr(), dw.data_ptr(), ws.data_ptr(), ws.numel(),
-                                   torch.cuda.current_stream().cuda_stream)
+        size = want = self.internal.workspace_bytes(x.shape[0])
+        while True:     # half of the workspace, a quarter ... when the device cannot spare the whole
+            try:
+                ws = torch.empty(size, dtype=torch.uint8, device=x.device)
+                with torch.cuda.device(x.device):
+                    self.internal.backward(x.shape[0], x.data_ptr(), y.data_ptr(), w.data_ptr(), dz.data_ptr(),
+                                           dx.data_ptr(), dy.data_ptr(), dw.data_ptr(), ws.data_ptr(), size,
+                                           torch.cuda.current_stream().cuda_stream)
+                break
+            except torch.OutOfMemoryError:
+                size //= 2
+                if size < want // 64:
+                    raise
+            except _native.OeqError as err:
+                if err.code == _native.OEQ_ERR_INVALID and size < want:     # less than the partial weight gradients
+                    raise torch.OutOfMemoryError(f"out of memory: {want} bytes of workspace") from err
+                raise
         return dx, dy, dw
 
     def _double_backward_impl(self, x, y, w, dz, ex, ey, ew):

@@ -1,5 +1,7 @@
 """Shared-weight 'uvw' products of one operator on several streams at a time, each with weights of its own: what a call
 prepares (weights in the operand layout of the tensor cores) belongs to the call."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -52,3 +54,30 @@ def test_less_workspace_than_stated():
         tp.internal.backward(batch, *(t.data_ptr() for t in (x, y, w, dz, *got, ws)), size, stream)
         for g, r in zip(got, want):
             assert (g - r).abs().max().item() <= 1e-5 * r.abs().max().item()
+
+
+@pytest.mark.parametrize("entry", ["op", "python"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
+def test_a_full_device(dtype, entry):
+    """The products of the weights with dZ (360 and 720 MB here) shrink to what there is."""
+    p = oeq.FullyConnectedTPProblem("64x0e+64x1o", "0e+1o", "64x0e+64x1o", irrep_dtype=dtype, weight_dtype=dtype)
+    tp = oeq.TensorProduct(p, torch_op=True)
+    batch, mb = 100_000, 1 << 20
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x, y, w, dz = (torch.randn(*s, device="cuda", dtype=torch.float32 if dtype is np.float32 else torch.float64, generator=gen)
+                   for s in ((batch, p.irreps_in1.dim), (batch, p.irreps_in2.dim), (p.weight_numel,), (batch, p.irreps_out.dim)))
+    call = tp.backward_helper if entry == "op" else tp._backward_impl
+    want = call(x, y, w, dz)
+    outputs = sum(-(-t.numel() * t.element_size() // (2 * mb)) * 2 * mb for t in (x, y)) + 22 * mb
+    torch.cuda.synchronize()
+    gc.collect()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + outputs + 130 * mb) / total)
+    try:
+        got = call(x, y, w, dz)
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for g, r in zip(got, want):
+        assert (g - r).abs().max().item() <= (1e-5 if dtype is np.float32 else 1e-12) * r.abs().max().item()
