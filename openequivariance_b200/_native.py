@@ -18,6 +18,7 @@ import numpy as np
 from .wigner import cg_nonzeros
 
 OEQ_OK = 0
+OEQ_ERR_INVALID = 1
 OEQ_ERR_UNSUPPORTED = 2
 ERR_NAMES = {1: "invalid argument", 2: "unsupported problem", 3: "kernel specialisation failed",
              4: "CUDA error", 5: "device-side wait abandoned"}
