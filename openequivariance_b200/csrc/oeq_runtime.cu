@@ -2129,11 +2129,10 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         }
         return r;
     };
-    if (h->has_gemm_bwd) {
-        const size_t wbytes = (size_t)p.w_numel * 8;
-        const long long block = workspace ? (long long)std::min<size_t>((size_t)batch, workspace_bytes / ((size_t)h->grad_product.z_dim * 8)) : 0;
-        if (workspace_bytes < wbytes || block < 1 || !aligned16(workspace))
-            return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
+    // (a workspace that does not hold a partial gradient and a dT row each, 16-byte aligned, is for the tiled kernel)
+    const size_t wbytes = (size_t)p.w_numel * 8, dt_row = (size_t)h->grad_product.z_dim * 8;
+    if (h->has_gemm_bwd && workspace && aligned16(workspace) && workspace_bytes >= std::max(wbytes, dt_row)) {
+        const long long block = (long long)std::min<size_t>((size_t)batch, workspace_bytes / dt_row);
         if ((rc = load_gemm(h->gemm_dw))) return rc;
         h->last_stream = st;
         Kernel& k = h->gemm_dw;

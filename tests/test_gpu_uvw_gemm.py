@@ -38,3 +38,18 @@ def test_shared_weights(in1, in2, out, batch, dtype):
     for g, r in zip(got[:3], want):
         assert rel_err(g.cpu().numpy(), r) < REL_TOL[dtype]
     assert rel_err(to_e3nn(p, got[3].cpu().numpy()), want[3]) < REL_TOL[dtype]
+
+
+def test_fp64_workspace_off_the_16_byte_rule():
+    """A workspace at an odd multiple of 8 bytes is taken: the tiled kernel."""
+    p = oeq.FullyConnectedTPProblem("16x0e+16x1o", "0e+1o", "16x0e+16x1o", irrep_dtype=np.float64, weight_dtype=np.float64)
+    x, y, w, dz = tp_inputs(p, 50, 17)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
+    handle = oeq.TensorProduct(p).internal
+    size = handle.workspace_bytes(50)
+    got = [torch.empty_like(t) for t in dev[:3]]
+    ws = torch.empty(size + 8, dtype=torch.uint8, device="cuda")
+    handle.backward(50, *(t.data_ptr() for t in (*dev, *got)), ws.data_ptr() + 8, size, torch.cuda.current_stream().cuda_stream)
+    want = orc.tp_backward(p, x, y, w, dz)
+    for g, r in zip((got[0].cpu().numpy(), got[1].cpu().numpy(), to_e3nn(p, got[2].cpu().numpy())), want):
+        assert rel_err(g, r) < REL_TOL[np.float64]
