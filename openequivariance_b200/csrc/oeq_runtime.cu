@@ -1469,6 +1469,32 @@ bool uvw_row_supported(const Problem& p) {
     return uvw_row_smem(p, true) <= 100 * 1024;
 }
 
+// Rows per SM up to which the row kernel is the faster one (0: always).  It pays a CTA's barriers and phases per row, the
+// tiled kernel shares them among 16 rows; with few weights a row that is what counts once every SM has rows enough.
+// Measured, tiled against row kernel in us (30 000 rows unless stated, second input 0e+1o...):
+//   forward: FP32 by the input channels of all paths: 8x(0e+1o) (32) 51 / 84, 12x(0e+1o) (48) 121 / 141, 8 -> 64 channels (32)
+//     74 / 102, but 16x(0e+1o) (64) 225 / 127, 4x(0e..3o) (136) 199 / 174; 2 000 rows 12 / 12 and 14 / 16.  FP64, whose tiled
+//     kernel is slower: 1x(0e+1o) (4) 20 / 45, but 4x(0e+1o) (16) 74 / 66; one tile of output channels keeps one warp of eight
+//     busy: 128x0e -> 4x0e 317 / 504.
+//   backward: by the weights per path: FP32 4x(0e+1o) (16) 53 / 123, 4x(0e..3o) (16) 657 / 1000, 8x(0e+1o+2e) (64) 260 / 299,
+//     but 12x(0e+1o) (144) 215 / 131; FP64 4x(0e..3o) 961 / 3029 (1 000 rows 92 / 123), 8x(0e+1o+2e) (64) 668 / 897, but without
+//     l = 2 8x(0e+1o) (64) 221 / 154; fewer than eight output channels leave most lanes idle: 128x0e -> 4x0e 88 / 113.
+int uvw_row_limit(const Problem& p, bool bwd) {
+    long long uv = 0, tiles = 0;
+    int dim = 1, width = 0;
+    for (const Instr& t : p.instr) uv += (long long)p.in1[t.i1].mul * p.in2[t.i2].mul;
+    for (const Irrep& r : p.out) {
+        tiles += (r.mul + 31) / 32;
+        dim = std::max(dim, r.dim);
+        width = std::max(width, r.mul);
+    }
+    const bool f64 = p.dtype == OEQ_F64;
+    if (!bwd) return (f64 ? uv < 8 || tiles == 1 : uv < 64) ? 24 : 0;
+    const long long per_path = p.w_numel / (long long)p.instr.size();
+    if (per_path >= (f64 && dim <= 3 ? 48 : 144) && width >= 8) return 0;
+    return per_path < 32 ? 8 : 64;
+}
+
 int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
     k.is_uvw = k.is_uvw_row = true;
     k.uvw.tile_r = 1;       // (the tiled kernel's bodies are not compiled)
@@ -1538,8 +1564,14 @@ long long gemm_shares(const Problem& p, long long batch, long long sm_count) {
     return std::max<long long>(1, std::min((6 * sm_count + tiles - 1) / std::max<long long>(1, tiles), batch / 64));
 }
 
-int build_tp(const Problem& p, bool bwd, Kernel& k) {
-    if (uvw_row_supported(p)) return build_uvw_row(p, bwd, k);
+// `row`: kernel with one row per CTA, where the problem has one; the kernel for the other batches is then optional.
+int build_tp(const Problem& p, bool bwd, Kernel& k, Kernel& row) {
+    if (uvw_row_supported(p)) {
+        const int rc = build_uvw_row(p, bwd, row);
+        if (rc || uvw_row_limit(p, bwd) == 0) return rc;
+        const int tiled = build_uvw(p, bwd ? K_UVW_BWD : K_UVW_FWD, k);
+        return tiled == OEQ_ERR_UNSUPPORTED ? OEQ_OK : tiled;
+    }
     if (p.mode == OEQ_MODE_UVW) return build_uvw(p, bwd ? K_UVW_BWD : K_UVW_FWD, k);
     return build_uvu(p, bwd ? K_BWD_BATCH : K_FWD_BATCH, k);
 }
@@ -1577,6 +1609,12 @@ struct UvwParams {
     int* status;
     int skip_dw;      // the shared-weight gradient comes from the tensor-core kernel
 };
+
+// The kernel that a batch takes.
+Kernel& uvw_kernel(Kernel& tiled, Kernel& row, const Problem& p, bool bwd, long long batch) {
+    if (!row.compiled) return tiled;
+    return tiled.compiled && row.loaded && batch > (long long)uvw_row_limit(p, bwd) * row.sm_count ? tiled : row;
+}
 
 long long uvw_grid(const Kernel& k, long long batch) {
     const long long tiles = (batch + k.uvw.tile_r - 1) / k.uvw.tile_r;
@@ -1737,6 +1775,7 @@ struct oeq_tp {
     std::mutex mutex;           // a call that launches (and loads kernels the first time) at a time
     Problem prob;
     Kernel fwd, bwd;
+    Kernel fwd_row, bwd_row;    // 'uvw' with per-row weights: one row per CTA (then fwd / bwd are for the batches of uvw_row_limit, if any)
     Kernel fwd_tc;              // tensor-core forward ('uvw', shared FP32 weights), when the problem qualifies
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
@@ -1810,17 +1849,17 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
     if (rc) return rc;
     if (p.mode == OEQ_MODE_UVW) {
         if (kinds & 6) return fail(OEQ_ERR_UNSUPPORTED, "fused convolution supports 'uvu' problems only");
-        Kernel f, b, tc;
+        Kernel f, b, fr, br, tc;
         if (uvw_gemm_supported(p)) {
             Problem pp, pc;
             Kernel dw, kp, kc;
             if ((rc = build_uvw_gemm(p, K_UVW_GEMM, f))) return rc;
             rc = build_uvw_gemm_backward(p, pp, pc, dw, kp, kc);
             if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
-        } else if ((rc = build_tp(p, false, f))) {
+        } else if ((rc = build_tp(p, false, f, fr))) {
             return rc;
         }
-        if ((rc = build_tp(p, true, b))) return rc;
+        if ((rc = build_tp(p, true, b, br))) return rc;
         TcGeometry g;
         if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, g, tc))) return rc;
         int smem = 0, threads = 0;
@@ -1889,8 +1928,8 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
             if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
         }
     }
-    if (!rc && !h->has_gemm) rc = build_tp(h->prob, false, h->fwd);
-    if (!rc) rc = build_tp(h->prob, true, h->bwd);
+    if (!rc && !h->has_gemm) rc = build_tp(h->prob, false, h->fwd, h->fwd_row);
+    if (!rc) rc = build_tp(h->prob, true, h->bwd, h->bwd_row);
     if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
         rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
         h->has_tc = rc == OEQ_OK;
@@ -1922,7 +1961,7 @@ int oeq_tp_destroy(oeq_tp* h) {
     if (h->d_status) cudaFree(h->d_status);
     if (h->d_packed) cudaFree(h->d_packed);
     if (h->d_packed_t) cudaFree(h->d_packed_t);
-    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
+    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_row, &h->bwd_row, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
         if (k->lib) cudaLibraryUnload(k->lib);
     delete h;
     return OEQ_OK;
@@ -2064,12 +2103,14 @@ int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, co
     }
     if (h->has_gemm) return launch_gemm(h->gemm, h->prob, batch, X, Y, W, Z, (cudaStream_t)stream);
     if (h->prob.mode == OEQ_MODE_UVW) {
-        if ((rc = load_uvw(h->fwd, h->prob, false))) return rc;
+        if (h->fwd_row.compiled && (rc = load_uvw(h->fwd_row, h->prob, false))) return rc;
+        Kernel& k = uvw_kernel(h->fwd, h->fwd_row, h->prob, false, batch);
+        if ((rc = load_uvw(k, h->prob, false))) return rc;
         UvwParams up{};
         up.X = X; up.Y = Y; up.W = W; up.Z = Z; up.batch = batch; up.status = h->d_status;
         void* args[] = {&up};
-        OEQ_CUDA(cudaLaunchKernel((const void*)h->fwd.fn, dim3((unsigned)uvw_grid(h->fwd, batch)),
-                                  dim3((unsigned)h->fwd.uvw.threads), args, (size_t)h->fwd.smem, (cudaStream_t)stream));
+        OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)uvw_grid(k, batch)), dim3((unsigned)k.uvw.threads), args, (size_t)k.smem,
+                                  (cudaStream_t)stream));
         return OEQ_OK;
     }
     if ((rc = load_kernel(h->fwd, "oeq_uvu_kernel", false))) return rc;
@@ -2153,8 +2194,10 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         });
     }
     if (p.mode == OEQ_MODE_UVW) {
-        if ((rc = load_uvw(h->bwd, p, true))) return rc;
-        long long ctas = uvw_grid(h->bwd, batch);
+        if (h->bwd_row.compiled && (rc = load_uvw(h->bwd_row, p, true))) return rc;
+        Kernel& main = uvw_kernel(h->bwd, h->bwd_row, p, true, batch);
+        if ((rc = load_uvw(main, p, true))) return rc;
+        long long ctas = uvw_grid(main, batch);
         if (p.shared) {
             const size_t need = (size_t)ctas * p.w_numel * p.elem();
             if (!workspace || workspace_bytes < need)
@@ -2219,8 +2262,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             }
         }
         void* args[] = {&up};
-        OEQ_CUDA(cudaLaunchKernel((const void*)h->bwd.fn, dim3((unsigned)ctas), dim3((unsigned)h->bwd.uvw.threads), args,
-                                  (size_t)h->bwd.smem, st));
+        OEQ_CUDA(cudaLaunchKernel((const void*)main.fn, dim3((unsigned)ctas), dim3((unsigned)main.uvw.threads), args, (size_t)main.smem, st));
         if (p.shared && !h->has_bwd_tc) {
             int n = p.w_numel;
             const void* ws = workspace;
@@ -2318,7 +2360,8 @@ int oeq_tp_launch_info(const oeq_tp* h, int which, int* threads, int* ng, int* p
         if (regs) *regs = h->fwd_tc.regs;
         return OEQ_OK;
     }
-    return launch_info(which ? h->bwd : h->fwd, threads, ng, ps, stages, smem, regs);
+    const Kernel& row = which ? h->bwd_row : h->fwd_row;
+    return launch_info(row.compiled ? row : which ? h->bwd : h->fwd, threads, ng, ps, stages, smem, regs);
 }
 
 // ---------------------------------------------------------------- backward pass that allocates nothing

@@ -1,5 +1,6 @@
 """'uvw' with per-row weights: the one-row-per-CTA kernels at chunk remainders of every multiplicity, second inputs of
-multiplicity above one, one row, and more rows than CTAs; a problem whose row does not fit them (tiled kernel)."""
+multiplicity above one, one row, and more rows than CTAs; a problem whose row does not fit them, and large batches of rows
+with few weights (tiled kernel)."""
 import numpy as np
 import pytest
 import torch
@@ -30,3 +31,14 @@ def test_row_weights(irreps, batch, dtype):
     for got, ref in zip((z, dx, dy), want):
         assert rel_err(got.cpu().numpy()[some], ref) < REL_TOL[dtype]
     assert rel_err(to_e3nn(p, dw.cpu().numpy()[some]), want[3]) < REL_TOL[dtype]
+
+
+FEW = [("4x0e+4x1o", "0e+1o", "4x0e+4x1o"), ("8x0e+8x1o", "0e+1o", "8x0e+8x1o"), ("128x0e", "0e", "4x0e"), ("8x0e+8x1o+8x2e", "0e+1o+2e", "8x0e+8x1o+8x2e")]
+
+
+# (on both sides of 8, 24 and 64 rows per SM, where batches of rows with few weights go over to the tiled kernel)
+@pytest.mark.parametrize("batch", [1185, 3552, 3553, 9473])
+@pytest.mark.parametrize("irreps", FEW, ids=["mul4", "mul8", "one_tile", "mul8_l2"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
+def test_few_weights(irreps, batch, dtype):
+    test_row_weights(irreps, batch, dtype)
