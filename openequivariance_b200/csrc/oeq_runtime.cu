@@ -1533,6 +1533,40 @@ bool uvw_gemm_supported(const Problem& p) {
     return true;
 }
 
+// Batches that the tiled kernel computes faster than the GEMMs, whose chain of chunks of 32 channels, each with a barrier,
+// and whose three launches backward show where there is little to do.  Measured, tiled / GEMM in us:
+//   forward, up to one wave of 16-row tiles (2 368 rows) and 8 192 products a row: 300 rows of 32x0e 8 / 12, 128x0e -> 64x0e
+//     12 / 25, 16x(0e+1o) 12 / 14; above either line 128x0e -> 64x0e 5 000 rows 27 / 22, 16x(0e+1o+2e) (8 960) 27 / 18.
+//     Half-filled tiles with l = 2 lose at many rows: 20x(0e+1o+2e), 60 000 rows 428 / 504, 20 000 rows 158 / 160;
+//     28x(0e+1o+2e) 617 / 606.  16x0e alone never fills a tile: 60 000 rows 29 / 33.
+//   backward, from the 128 rows on that take two shares of the rows (and their sum): 300 rows of 16x(0e+1o) (2 048) 36 / 46,
+//     32x0e 22 / 32; 64x0e (4 096) 46 / 38, one row of 16x(0e+1o) 32 / 17.
+constexpr int GEMM_SMALL_FWD = 8192, GEMM_SMALL_BWD = 2048, GEMM_SMALL_ROWS_PER_SM = 16;
+
+long long uvw_row_products(const Problem& p) {
+    long long n = 0;
+    for (const Instr& t : p.instr) n += (long long)p.in1[t.i1].mul * p.in2[t.i2].mul * p.out[t.io].mul * p.out[t.io].dim;
+    return n;
+}
+// Rows per SM from which multiplicities below 28 with l >= 2 are for the tiled kernel (0: not one of them).
+int gemm_narrow_rows_per_sm(const Problem& p) {
+    int mul = 0, dim = 0;
+    for (const std::vector<Irrep>* v : {&p.in1, &p.out})
+        for (const Irrep& r : *v) mul = std::max(mul, r.mul);
+    for (const Irrep& r : p.out) dim = std::max(dim, r.dim);
+    return mul < 28 && dim >= 5 ? 200 : 0;
+}
+bool gemm_forward_tiled(const Problem& p, long long batch, long long sms) {
+    const long long n = uvw_row_products(p);
+    if (n <= 256 || (n <= GEMM_SMALL_FWD && batch <= GEMM_SMALL_ROWS_PER_SM * sms)) return true;
+    return gemm_narrow_rows_per_sm(p) && batch > gemm_narrow_rows_per_sm(p) * sms;
+}
+bool gemm_backward_tiled(const Problem& p, long long batch, long long sms) {
+    return uvw_row_products(p) <= GEMM_SMALL_BWD && batch >= 128 && batch <= GEMM_SMALL_ROWS_PER_SM * sms;
+}
+// Whether any batch takes the tiled forward kernel (the backward one is there anyway, for small workspaces).
+bool gemm_keeps_tiled(const Problem& p) { return uvw_row_products(p) <= GEMM_SMALL_FWD || gemm_narrow_rows_per_sm(p) > 0; }
+
 int build_uvw_gemm(const Problem& p, int kernel_id, Kernel& k) {
     k.is_uvw = true;
     k.map.part_of_out.assign(p.out.size(), 0);
@@ -1856,6 +1890,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
             if ((rc = build_uvw_gemm(p, K_UVW_GEMM, f))) return rc;
             rc = build_uvw_gemm_backward(p, pp, pc, dw, kp, kc);
             if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
+            if (gemm_keeps_tiled(p) && (rc = build_tp(p, false, fr, fr))) return rc;
         } else if ((rc = build_tp(p, false, f, fr))) {
             return rc;
         }
@@ -1928,7 +1963,7 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
             if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
         }
     }
-    if (!rc && !h->has_gemm) rc = build_tp(h->prob, false, h->fwd, h->fwd_row);
+    if (!rc && (!h->has_gemm || gemm_keeps_tiled(h->prob))) rc = build_tp(h->prob, false, h->fwd, h->fwd_row);
     if (!rc) rc = build_tp(h->prob, true, h->bwd, h->bwd_row);
     if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
         rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
@@ -2101,7 +2136,10 @@ int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, co
             return rc;
         return launch_uvw_tc(h->fwd_tc, h->tc, h->pack_fn, packed, true, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     }
-    if (h->has_gemm) return launch_gemm(h->gemm, h->prob, batch, X, Y, W, Z, (cudaStream_t)stream);
+    if (h->has_gemm) {
+        if ((rc = load_gemm(h->gemm))) return rc;
+        if (!h->fwd.compiled || !gemm_forward_tiled(h->prob, batch, h->gemm.sm_count)) return launch_gemm(h->gemm, h->prob, batch, X, Y, W, Z, (cudaStream_t)stream);
+    }
     if (h->prob.mode == OEQ_MODE_UVW) {
         if (h->fwd_row.compiled && (rc = load_uvw(h->fwd_row, h->prob, false))) return rc;
         Kernel& k = uvw_kernel(h->fwd, h->fwd_row, h->prob, false, batch);
@@ -2131,8 +2169,10 @@ size_t oeq_tp_workspace_bytes(const oeq_tp* h, int64_t batch) {
     } else {
         groups = 256ll * 4 * h->bwd.map.ng;
     }
-    if (h->has_gemm_bwd)
-        return std::max((size_t)gemm_shares(h->prob, batch, 256) * h->prob.w_numel * 8, std::min((size_t)batch * h->grad_product.z_dim * 8, UVW_DT_BYTES));
+    if (h->has_gemm_bwd) {
+        const size_t partial = (size_t)h->prob.w_numel * 8, tiled = gemm_backward_tiled(h->prob, batch, 256) ? (size_t)groups * partial : 0;
+        return std::max({(size_t)gemm_shares(h->prob, batch, 256) * partial, tiled, std::min((size_t)batch * h->grad_product.z_dim * 8, UVW_DT_BYTES)});
+    }
     size_t bytes = (size_t)groups * h->prob.w_numel * h->prob.elem();
     if (h->has_grad_tc) bytes = std::max(bytes, std::min((size_t)batch * h->grad_product.z_dim * 4, UVW_DT_BYTES) + h->grad_tc.packed_bytes + 256);
     return bytes;
@@ -2172,9 +2212,11 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
     };
     // (a workspace that does not hold a partial gradient and a dT row each, 16-byte aligned, is for the tiled kernel)
     const size_t wbytes = (size_t)p.w_numel * 8, dt_row = (size_t)h->grad_product.z_dim * 8;
-    if (h->has_gemm_bwd && workspace && aligned16(workspace) && workspace_bytes >= std::max(wbytes, dt_row)) {
+    if (h->has_gemm_bwd && (rc = load_gemm(h->gemm_dw))) return rc;
+    const bool gemm_tiled = h->has_gemm_bwd && gemm_backward_tiled(p, batch, h->gemm_dw.sm_count) &&
+                            workspace_bytes / wbytes >= (size_t)std::min<long long>((batch + 3) / 4, 2ll * h->gemm_dw.sm_count);
+    if (h->has_gemm_bwd && workspace && aligned16(workspace) && workspace_bytes >= std::max(wbytes, dt_row) && !gemm_tiled) {
         const long long block = (long long)std::min<size_t>((size_t)batch, workspace_bytes / dt_row);
-        if ((rc = load_gemm(h->gemm_dw))) return rc;
         h->last_stream = st;
         Kernel& k = h->gemm_dw;
         long long shares = std::min<long long>(gemm_shares(p, batch, k.sm_count), (long long)(workspace_bytes / wbytes));

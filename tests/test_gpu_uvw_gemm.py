@@ -53,3 +53,23 @@ def test_fp64_workspace_off_the_16_byte_rule():
     want = orc.tp_backward(p, x, y, w, dz)
     for g, r in zip((got[0].cpu().numpy(), got[1].cpu().numpy(), to_e3nn(p, got[2].cpu().numpy())), want):
         assert rel_err(g, r) < REL_TOL[np.float64]
+
+
+# one path or few products a row: small batches (and some large ones) are for the tiled kernel; both sides of each line
+@pytest.mark.parametrize("irreps", [("16x0e", "0e", "16x0e"), ("32x0e", "0e", "32x0e"), ("128x0e", "0e", "64x0e"),
+                                    ("16x0e+16x1o", "0e+1o", "16x0e+16x1o"), ("20x0e+20x1o+20x2e", "0e+1o+2e", "20x0e+20x1o+20x2e")],
+                         ids=["16", "32", "128_64", "16_l1", "20_l2"])
+@pytest.mark.parametrize("batch", [127, 128, 2368, 2369, 29601])
+def test_fp64_lines_between_the_kernels(irreps, batch):
+    p = oeq.FullyConnectedTPProblem(*irreps, irrep_dtype=np.float64, weight_dtype=np.float64)
+    x, y, w, dz = tp_inputs(p, batch, 23)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
+    tp = oeq.TensorProduct(p, torch_op=True)
+    got = [tp(*dev[:3]), *tp.backward_helper(*dev)]
+    tp.check_device_status()
+    some = np.r_[0:3, batch // 2, batch - 3:batch]                 # (the oracle is slow)
+    want = [orc.tp_forward(p, x[some], y[some], w), *orc.tp_backward(p, x[some], y[some], w, dz[some])[:2]]
+    for g, r in zip(got[:3], want):
+        assert rel_err(g.cpu().numpy()[some], r) < REL_TOL[np.float64]
+    parts = sum(orc.tp_backward(p, x[i:i + 5000], y[i:i + 5000], w, dz[i:i + 5000])[2] for i in range(0, batch, 5000))
+    assert rel_err(to_e3nn(p, got[3].cpu().numpy()), parts) < REL_TOL[np.float64]
