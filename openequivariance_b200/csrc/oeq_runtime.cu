@@ -2095,6 +2095,9 @@ static int load_gemm(Kernel& k) {
     OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
     k.smem = GEMM_SMEM;
     OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
+    else (void)cudaGetLastError();
     k.loaded = true;
     return OEQ_OK;
 }
@@ -2402,6 +2405,7 @@ int oeq_tp_launch_info(const oeq_tp* h, int which, int* threads, int* ng, int* p
         if (regs) *regs = h->fwd_tc.regs;
         return OEQ_OK;
     }
+    if (which ? h->has_gemm_bwd : h->has_gemm) return launch_info(which ? h->gemm_dw : h->gemm, threads, ng, ps, stages, smem, regs);
     const Kernel& row = which ? h->bwd_row : h->fwd_row;
     return launch_info(row.compiled ? row : which ? h->bwd : h->fwd, threads, ng, ps, stages, smem, regs);
 }

@@ -25,6 +25,8 @@ def test_row_weights(irreps, batch, dtype):
     z = tp(x, y, w)
     dx, dy, dw = tp.backward_helper(x, y, w, dz)
     tp.check_device_status()
+    if irreps is ODD:       # (the row kernels are those that ran: eight warps without a tile)
+        assert all(tp.internal.launch_info(which)["threads"] == 256 and tp.internal.launch_info(which)["regs"] > 0 for which in (0, 1))
     some = slice(0, batch) if batch < 100 else np.r_[0:3, batch // 2, batch - 3:batch]     # (the oracle is slow)
     sub = [a[some] for a in arrays]
     want = [orc.tp_forward(p, *sub[:3]), *orc.tp_backward(p, *sub)]
