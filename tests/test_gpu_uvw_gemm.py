@@ -35,8 +35,8 @@ def test_shared_weights(in1, in2, out, batch, dtype):
     tp.check_device_status()
     assert all(torch.equal(a, b) for a, b in zip(got[1:], again))
     if dtype is np.float64:     # (the GEMM kernels are those that ran: two buffers of two 32 x 66 tiles)
-        assert [tp.internal.launch_info(which)["smem"] for which in (0, 1)] == [4 * 32 * 66 * 8] * 2
-        assert tp.internal.launch_info(1)["regs"] > 0
+        assert [tp.internal.launch_info(which)["smem_bytes"] for which in (0, 1)] == [4 * 32 * 66 * 8] * 2
+        assert tp.internal.launch_info(1)["registers"] > 0
     want = [orc.tp_forward(p, x, y, w), *orc.tp_backward(p, x, y, w, dz)]
     for g, r in zip(got[:3], want):
         assert rel_err(g.cpu().numpy(), r) < REL_TOL[dtype]
