@@ -1677,9 +1677,107 @@ __device__ __forceinline__ long long align_sender(const long long* cols, const l
     return n;
 }
 
-// A warp takes NV 16-byte pieces per lane of every row: one 512-byte block of columns with eight rows in flight where a
-// launch has warps to spare (with whole rows a warp has one 4.6 KB row in flight: 56 k rows took 80 us, now 58), whole
-// rows for the few helper warps of a receiver-order launch.
+// The helper warps of a receiver-order launch: whole rows, a row (or as many short ones as fit 16 to 32 values per lane) in
+// flight.  With the loop of the launch of its own below in its place (vector flushes), MACE-large at 6.0 M edges takes 66.3
+// instead of 61.9 ms (one box, in turn); with its blocks of columns the helper warps' launch went from 2.8 to 6.9 ms at
+// 300 k rows.
+__device__ void sum_sender_rows_beside(const T* __restrict__ temp, T* __restrict__ dX, const long long* __restrict__ cols,
+                                       const long long* __restrict__ perm, long long n_items, long long e_lo, long long e_hi,
+                                       bool first, int chunk, long long warps, long long wid, int lane) {
+    constexpr int VEC = 16 / ELEM;                                  // elements per 16-byte load
+    constexpr int XS = XB / ELEM;
+    constexpr int NV = (XS / VEC + 31) / 32;                        // 16-byte pieces per lane
+    T acc[NV * VEC];
+#pragma unroll
+    for (int i = 0; i < NV * VEC; ++i) acc[i] = (T)0;
+    auto flush = [&](long long node) {
+        T* xrow = dX + node * (long long)X_DIM;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int base = (lane + 32 * v) * VEC;
+            if (base < X_DIM) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q)
+                    if (base + q < X_DIM) {
+                        if (first) xrow[base + q] = acc[v * VEC + q];
+                        else xrow[base + q] += acc[v * VEC + q];
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NV * VEC; ++i) acc[i] = (T)0;
+    };
+    const long long n_chunks = (n_items + chunk - 1) / chunk;
+    for (long long c = wid; c < n_chunks; c += warps) {
+        const long long pos = align_sender(cols, perm, n_items, c * chunk, lane);
+        const long long end = c + 1 >= n_chunks ? n_items : align_sender(cols, perm, n_items, (c + 1) * chunk, lane);
+        long long prev = -1;
+        for (long long base = pos; base < end; base += 32) {
+            const long long k = base + lane;
+            long long e = -1, s = -1;
+            if (k < end) e = perm[k];
+            const bool in_block = e >= e_lo && e < e_hi;
+            unsigned mask = __ballot_sync(0xffffffffu, in_block);
+            if (mask == 0) continue;
+            if (in_block) s = cols[e];
+            // Short rows: the loads of up to U rows go out together (a row at a time would pay the DRAM latency
+            // per row); the rows are still added one after the other, in order.
+            constexpr int U = (NV * VEC <= 16) ? 4 : (NV * VEC <= 32 ? 2 : 1);
+            while (mask) {
+                long long ej[U], sj[U];
+                T val[U][NV * VEC];
+                int n = 0;
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    ej[q] = 0; sj[q] = -1;
+                    if (mask) {
+                        const int src = __ffs(mask) - 1;
+                        mask &= mask - 1;
+                        ej[q] = __shfl_sync(0xffffffffu, e, src);
+                        sj[q] = __shfl_sync(0xffffffffu, s, src);
+                        n = q + 1;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    if (q < n) {
+                        const T* row = temp + (ej[q] - e_lo) * (long long)XS;
+#pragma unroll
+                        for (int v = 0; v < NV; ++v) {
+                            const int b4 = (lane + 32 * v) * VEC;
+                            if (b4 < XS) {
+                                if constexpr (ELEM == 4) {
+                                    const float4 t = __ldcs(reinterpret_cast<const float4*>(row + b4));
+                                    val[q][v * VEC + 0] = t.x; val[q][v * VEC + 1] = t.y; val[q][v * VEC + 2] = t.z; val[q][v * VEC + 3] = t.w;
+                                } else {
+                                    const double2 t = __ldcs(reinterpret_cast<const double2*>(row + b4));
+                                    val[q][v * VEC + 0] = t.x; val[q][v * VEC + 1] = t.y;
+                                }
+                            } else {
+#pragma unroll
+                                for (int c = 0; c < VEC; ++c) val[q][v * VEC + c] = (T)0;
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    if (q < n) {
+                        if (prev >= 0 && sj[q] != prev) flush(prev);
+                        prev = sj[q];
+#pragma unroll
+                        for (int i = 0; i < NV * VEC; ++i) acc[i] += val[q][i];
+                    }
+                }
+            }
+        }
+        if (prev >= 0) flush(prev);
+    }
+}
+
+// The row sum as a launch of its own.  A warp takes NV 16-byte pieces per lane of every row: one 512-byte block of columns
+// with eight rows in flight where a launch has warps to spare (with whole rows a warp has one 4.6 KB row in flight: 56 k
+// rows took 80 us, now 58).
 template <int NV, int U>
 __device__ void sum_sender_rows(const T* __restrict__ temp, T* __restrict__ dX, const long long* __restrict__ cols,
                                 const long long* __restrict__ perm, long long n_items, long long e_lo, long long e_hi,
@@ -1803,9 +1901,9 @@ __device__ __forceinline__ void uvu_body_recv(const UvuParams& p) {
     if (tid >= NCONSUMERS + NSTAGING) {
         if constexpr (HELPER_WARPS > 0) {
             if (p.sum_items > 0)
-                sum_sender_rows<ROW_PIECES, (ROW_PIECES <= 4 ? 4 : ROW_PIECES <= 8 ? 2 : 1)>(p.sum_ws, p.dX, p.sum_cols, p.sum_perm, p.sum_items, p.sum_e_lo, p.sum_e_hi, p.sum_first != 0,
-                                p.sum_chunk, 0, (long long)gridDim.x * HELPER_WARPS,
-                                (long long)blockIdx.x * HELPER_WARPS + ((tid - NCONSUMERS - NSTAGING) >> 5), tid & 31);
+                sum_sender_rows_beside(p.sum_ws, p.dX, p.sum_cols, p.sum_perm, p.sum_items, p.sum_e_lo, p.sum_e_hi, p.sum_first != 0,
+                                       p.sum_chunk, (long long)gridDim.x * HELPER_WARPS,
+                                       (long long)blockIdx.x * HELPER_WARPS + ((tid - NCONSUMERS - NSTAGING) >> 5), tid & 31);
         }
         return;
     }
