@@ -1735,8 +1735,12 @@ int launch_uvu(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream,
         chunk = 128;
         const long long groups = grid * k.map.ng;
         while (chunk > k.map.chunk_floor && prm.n_items / (groups * chunk) < 8) chunk /= 2;
-        // a short list: smaller chunks while groups would be left without one
-        while (chunk > 8 && prm.n_items < groups * chunk) chunk /= 2;
+        // A short list: smaller chunks while groups would be left without one.  Deterministic walks, whose chunks move to
+        // the next boundary (two dependent index reads) or meet a receiver's dZ anew, wait until half of the groups would
+        // be: 64x0e+32x1o, 59 k edges, forward 137 us with chunks of 32 (as many as groups), 111 with 64; 30 k edges 92 with
+        // 16, 80 with 32; 32x(0e..3o) FP64 backward, 6 k edges, 162 with 8, 109 with 16 (forward 131 and 148).
+        const int slack = prm.rows && (k.map.chunk_floor > 32 || prm.ws) ? 2 : 1;
+        while (chunk > 8 && prm.n_items * slack < groups * chunk) chunk /= 2;
     }
     prm.chunk = std::max(1, chunk);
     void* args[] = {&prm};
