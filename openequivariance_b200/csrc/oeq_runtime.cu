@@ -1751,15 +1751,20 @@ int launch_uvu(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream,
 
 // Edges per chunk and CTAs of a slice kernel.  Node rows that fit in L2 are gathered from there whatever the order:
 // each walker then takes one run of the edge list (at least 8 edges), which needs its ends aligned once.  Larger graphs
-// are dealt in chunks of 128 edges, so that the walkers stay in one neighbourhood of the list.
-void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes, long long& grid, int& chunk) {
+// are dealt in chunks of 128 edges, so that the walkers stay in one neighbourhood of the list.  A walk that adds to the
+// rows it gathers (`adds_mb` > 0, atomic backward) has both in L2, up to that many MB.  FP64, whose additions are by eight
+// bytes, 32x(0e+1o+2e): one run each / chunks of 128, 10 000 nodes (2 x 23 MB) 476 / 466 us, 15 000 822 / 769, 20 000
+// 1187 / 1002; 128x(0e+1o+2e), 3 000 nodes (2 x 28 MB) 771 / 874.  FP32: 32x(0e+1o+2e), 40 000 nodes (2 x 46 MB) 1006 / 1054;
+// 128x(0e+1o+2e), 20 000 nodes (2 x 92 MB) 2817 / 2696.
+void slice_launch_shape(const Kernel& k, long long edges, size_t gathered_bytes, int adds_mb, long long& grid, int& chunk) {
     const int per_cta = k.map.slice_warps / k.map.n_slice;
     const long long most = (long long)k.sm_count * k.ctas_per_sm;
     const long long walkers = most * per_cta;
+    const bool runs = adds_mb ? 2 * gathered_bytes <= ((size_t)adds_mb << 20) : gathered_bytes <= (48u << 20) || edges < walkers * 512;
     chunk = env_int("OEQ_B200_CHUNK", 0);
     if (chunk <= 0) {
         chunk = 128;
-        if (gathered_bytes <= (48u << 20) || edges < walkers * 512) chunk = (int)std::max<long long>(8, (edges + walkers - 1) / walkers);
+        if (runs || edges < walkers * chunk) chunk = (int)std::max<long long>(8, (edges + walkers - 1) / walkers);
     }
     const long long chunks = (edges + chunk - 1) / chunk;
     grid = std::max<long long>(1, std::min(most, (chunks + per_cta - 1) / per_cta));
@@ -1794,7 +1799,7 @@ int launch_slice(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t strea
     if (prm.dX ? ((full || (p.x_dim * e) % 16 == 0) && aligned16(prm.ws ? prm.ws : prm.dX)) : aligned16(prm.Z)) flags |= 8;
     prm.flags = flags & ~clear_flags;
     long long grid = 1;
-    slice_launch_shape(k, prm.n_items, (size_t)prm.n_nodes * p.x_dim * e, grid, prm.chunk);
+    slice_launch_shape(k, prm.n_items, (size_t)prm.n_nodes * p.x_dim * e, prm.dX && !prm.ws ? (e == 8 ? 64 : 128) : 0, grid, prm.chunk);
     void* args[] = {&prm};
     OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)grid), dim3((unsigned)k.threads()), args, (size_t)k.smem, stream));
     return OEQ_OK;
