@@ -1236,6 +1236,12 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
 bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || slice.map.slice_regs > 200; }
 constexpr long long RECV_MIN_EDGES = 65536;
 
+// Wide FP64 rows in the forward pass: the slice kernel gathers every row once per slice of 32 channels, which
+// costs once the rows no longer fit in L2.  128x(0e+1o+2e), group / slice kernel, atomic: 5 000 nodes (46 MB) 695 / 636 us,
+// 10 000 (92 MB) 1252 / 1277, 20 000 2422 / 2730; deterministic 659 / 592, 1159 / 1171, 2330 / 2422.
+bool group_forward_beside_slice(const Problem& p, const Kernel& slice) { return p.dtype == OEQ_F64 && slice.map.slice_regs > 160 && slice.map.n_slice > 2; }
+constexpr size_t GROUP_FORWARD_BYTES = 64u << 20;
+
 // Problems for which fused second derivatives may exist (whether they fit is known once they are built).
 bool conv_second_possible(const Problem& p) {
     Mapping m;
@@ -1940,7 +1946,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         const int rf = build_slice_fwd(p, det != 0, f), rb = build_slice_bwd(p, det != 0, b);
         if (rf && rf != OEQ_ERR_UNSUPPORTED) return rf;
         if (rb && rb != OEQ_ERR_UNSUPPORTED) return rb;
-        if (rf && (rc = one(det ? K_FWD_DET : K_FWD_ATOMIC))) return rc;
+        if ((rf || group_forward_beside_slice(p, f)) && (rc = one(det ? K_FWD_DET : K_FWD_ATOMIC))) return rc;
         if ((rc = one(det ? K_BWD_DET : K_BWD_ATOMIC))) return rc;
         if (tc && (rc = build_uvu_tc(p, det != 0, k))) return rc;
         if (recv && recv_beside_slice(!rb, b) && (rc = build_uvu_recv(p, det != 0, kr))) return rc;
@@ -2513,7 +2519,8 @@ int oeq_conv_create(const oeq_problem_desc* desc, int deterministic, oeq_conv** 
         if (rc2 != OEQ_OK && rc2 != OEQ_ERR_UNSUPPORTED) rc = rc2;
     };
     if (!rc) optional(build_slice_fwd(h->prob, h->deterministic, h->fwd_slice), h->has_fwd_slice);
-    if (!rc && !h->has_fwd_slice) rc = build_uvu(h->prob, deterministic ? K_FWD_DET : K_FWD_ATOMIC, h->fwd);
+    if (!rc && (!h->has_fwd_slice || group_forward_beside_slice(h->prob, h->fwd_slice)))
+        rc = build_uvu(h->prob, deterministic ? K_FWD_DET : K_FWD_ATOMIC, h->fwd);
     if (!rc) rc = build_uvu(h->prob, deterministic ? K_BWD_DET : K_BWD_ATOMIC, h->bwd);
     UvuTcGeometry geo;
     if (!rc && uvu_tc_geometry(h->prob, geo)) {
@@ -2582,7 +2589,8 @@ int oeq_conv_forward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, c
     const bool tc = h->has_fwd_tc && aligned16(X) && aligned16(W) && !env_int("OEQ_B200_NO_BULK", 0);
     int rc = ensure_status(&h->d_status);
     // (the slice kernels count nodes and edges in 32 bits)
-    if (!rc && !tc && h->has_fwd_slice && edges < (1ll << 31) - 4096 && nodes < (1ll << 31) - 4096) {
+    const bool group = h->has_fwd_slice && group_forward_beside_slice(p, h->fwd_slice) && (size_t)nodes * p.x_dim * p.elem() > GROUP_FORWARD_BYTES;
+    if (!rc && !tc && h->has_fwd_slice && !group && edges < (1ll << 31) - 4096 && nodes < (1ll << 31) - 4096) {
         if ((rc = load_kernel(h->fwd_slice, "oeq_uvu_kernel", false))) return rc;
         UvuParams prm{};
         prm.X = X; prm.Y = Y; prm.W = W; prm.Z = Z;
