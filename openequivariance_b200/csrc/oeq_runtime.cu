@@ -1230,11 +1230,14 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
     return OEQ_OK;
 }
 
-// Where a thread of the backward slice kernel needs more than 200 registers (two warps per scheduler) and the edges
-// fill the machine, the receiver-order group kernel with its staging warps is the faster one: MACE-large, 600 k edges
-// 5.1 against 5.6 ms atomic, but at 15 k edges 178 against 152 us.
-bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || slice.map.slice_regs > 200; }
-constexpr long long RECV_MIN_EDGES = 65536;
+// Where a thread of the backward slice kernel needs more than 200 registers (two warps per scheduler) for rows of several
+// slices, the receiver-order group kernel with its staging warps is the faster one once the edges fill the machine.
+// MACE-large, group / slice kernel in us: atomic 30 k edges 374 / 325, 65 k 601 / 636, 1.2 M 10211 / 11278; deterministic, with
+// the row sum beside later launches on large lists only, 65 k 886 / 736, 131 k 1451 / 1434, 263 k 2751 / 2828, 1.2 M
+// 11987 / 13138.  128x(0e+1o+2e) in FP64 is within 2 % from 15 k to 66 k edges and 131 k on 1154 / 1256 (atomic).  A row
+// of one slice is the slice kernel's at every size: 32x(0e..3o), 65 k edges 202 / 173, 1.2 M 3552 / 2804.
+bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || (slice.map.slice_regs > 200 && slice.map.n_slice > 1); }
+long long recv_min_edges(bool deterministic) { return env_int("OEQ_B200_RECV_MIN_EDGES", deterministic ? 196608 : 49152); }
 
 // Wide FP64 rows in the forward pass: the slice kernel gathers every row once per slice of 32 channels, which
 // costs once the rows no longer fit in L2.  128x(0e+1o+2e), group / slice kernel, atomic: 5 000 nodes (46 MB) 695 / 636 us,
@@ -2657,7 +2660,7 @@ int oeq_conv_backward(oeq_conv* h, int64_t nodes, int64_t edges, const void* X, 
     long long block_edges = 0;
     // (slice kernels count edges and nodes in 32 bits)
     const bool sliced = h->has_bwd_slice && edges < (1ll << 31) - 4096 && nodes < (1ll << 31) - 4096 &&
-                        !(h->has_bwd_recv && edges >= RECV_MIN_EDGES);
+                        !(h->has_bwd_recv && edges >= recv_min_edges(h->deterministic));
     if (h->has_bwd_recv || sliced) {
         if (!h->deterministic) block_edges = edges;
         else if (workspace && aligned16(workspace)) {

@@ -59,12 +59,13 @@ def test_fp64(deterministic):
 @pytest.mark.parametrize("name,dtype,deterministic,epi", [("nequip_32", np.float32, True, 4), ("nequip_32", np.float32, False, 3),
                                                          ("readme", np.float64, True, 3), ("readme", np.float32, False, 4)])
 def test_edges_per_item(name, dtype, deterministic, epi, monkeypatch):
-    """Narrow problems stage runs of consecutive edges as one item (two by default); other run lengths, ragged
+    """Narrow problems on the group kernels stage runs of consecutive edges as one item (two by default); other run lengths, ragged
     runs at chunk ends, rows that do not qualify for bulk copies, and bit-equality with one edge per item in the
     deterministic variant."""
     p = problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype)
     nodes = 57
     rows, cols = random_graph(nodes, 1003, seed=41)
+    monkeypatch.setenv("OEQ_B200_SLICE", "0")       # (the slice kernels, which take these problems, have no such runs)
     monkeypatch.setenv("OEQ_B200_EPI", str(epi))
     monkeypatch.setenv("OEQ_B200_EPI_STAGES", "3")
     conv, inputs, got = check_conv(p, nodes, rows, cols, 42, deterministic, dtype=dtype)
@@ -366,12 +367,18 @@ def test_tensor_core_forward(name, deterministic, monkeypatch):
             assert torch.equal(conv.forward(*args), first)
 
 
+@pytest.mark.parametrize("kernels", ["slice", "receiver_order", "sender_order"])
 @pytest.mark.parametrize("chunk", [16, 128])
-def test_widest_rows_many_chunks_per_group(chunk, monkeypatch):
-    """MACE-large rows on a graph large enough that every group walks several work chunks (small chunks make
-    that happen at a size the oracle can follow): chunk boundaries moved to node boundaries, the phased
-    backward stages and the ring of dY partials all wrap many times."""
+def test_widest_rows_many_chunks_per_group(chunk, kernels, monkeypatch):
+    """MACE-large rows on a graph large enough that every walker takes several work chunks (small chunks make that happen
+    at a size the oracle can follow): chunk boundaries moved to node boundaries; group kernels: the dZ slice in shared
+    memory (receiver order), the phased backward stages and the ring of dY partials (sender order) wrap many times."""
     monkeypatch.setenv("OEQ_B200_CHUNK", str(chunk))
+    if kernels == "receiver_order":
+        monkeypatch.setenv("OEQ_B200_RECV_MIN_EDGES", "1")
+    if kernels == "sender_order":
+        monkeypatch.setenv("OEQ_B200_SLICE", "0")
+        monkeypatch.setenv("OEQ_B200_BWD_RECV", "0")
     p = problem_by_name("mace_large_128")
     nodes = 700
     rows, cols = random_graph(nodes, 20000, seed=31)
@@ -439,21 +446,26 @@ def test_periodic_radius_graph(name, nodes, lmax, deterministic):
             assert torch.equal(z, z2) and torch.equal(dx, dx2) and torch.equal(dy, dy2) and torch.equal(dw, dw2)
 
 
-@pytest.mark.parametrize("name", ["nequip_32", "mace_128"])
+@pytest.mark.parametrize("name", ["nequip_32", "mace_128", "mace_large_128"])
 def test_deterministic_backward_in_edge_blocks(name, monkeypatch):
     """The receiver-order backward pass with scratch for only a part of the edges: it then runs block by block
     (receiver-order launch + row sum per block, later blocks adding into dX).  Same results as the oracle, the
     same bits run to run, and agreement with the scratch-free sender-order kernel."""
     monkeypatch.setenv("OEQ_B200_BWD_SCRATCH_MB", "1")      # 1 MiB of scratch: a few hundred rows per block
     monkeypatch.setenv("OEQ_B200_BWD_MIN_BLOCK", "1")
-    if name == "mace_128":
+    if name == "mace_large_128":                                # the receiver-order group kernel, whatever the size:
+        monkeypatch.setenv("OEQ_B200_RECV_MIN_EDGES", "1")
         monkeypatch.setenv("OEQ_B200_PIPELINE_BLOCK_MB", "1")   # blocks of a few hundred edges are pipelined too:
         # each launch's helper warps sum the previous block while the consumers work on the current one
     p = problem_by_name(name)
     nodes = 300
     rows, cols = random_graph(nodes, 4000, seed=41)
     conv, (xt, yt, wt, dzt, index), (z, dx, dy, dw) = check_conv(p, nodes, rows, cols, 42, True)
-    assert conv.internal.last_backward_launches() >= 6        # several blocks, two launches each
+    row = p.irreps_in1.dim * 4
+    if name == "mace_large_128":        # the clearing of dX, a launch per half-scratch block, the last block's row sum
+        assert conv.internal.last_backward_launches() == 2 + -(-len(rows) // ((1 << 20) // row // 2))
+    else:                               # the clearing of dX, two launches per block
+        assert conv.internal.last_backward_launches() == 1 + 2 * -(-len(rows) // ((1 << 20) // row))
     dx2, dy2, dw2 = conv.backward_helper(xt, yt, wt, dzt, *index)
     assert torch.equal(dx, dx2) and torch.equal(dy, dy2) and torch.equal(dw, dw2)
     monkeypatch.setenv("OEQ_B200_BWD_SCRATCH_MB", "8192")
