@@ -1546,8 +1546,8 @@ bool uvw_gemm_supported(const Problem& p) {
 // and whose three launches backward show where there is little to do.  Measured, tiled / GEMM in us:
 //   forward, up to one wave of 16-row tiles (2 368 rows) and 8 192 products a row: 300 rows of 32x0e 8 / 12, 128x0e -> 64x0e
 //     12 / 25, 16x(0e+1o) 12 / 14; above either line 128x0e -> 64x0e 5 000 rows 27 / 22, 16x(0e+1o+2e) (8 960) 27 / 18.
-//     Half-filled tiles with l = 2 lose at many rows: 20x(0e+1o+2e), 60 000 rows 428 / 504, 20 000 rows 158 / 160;
-//     28x(0e+1o+2e) 617 / 606.  16x0e alone never fills a tile: 60 000 rows 29 / 33.
+//     Half-filled tiles with l = 2 lose at many rows: 20x(0e+1o+2e), 60 000 rows 428 / 504, 25 000 rows 188 / 199, 20 000
+//     158 / 160; 28x(0e+1o+2e) 617 / 606.  16x0e alone never fills a tile: 60 000 rows 29 / 33.
 //   backward, from the 128 rows on that take two shares of the rows (and their sum): 300 rows of 16x(0e+1o) (2 048) 36 / 46,
 //     32x0e 22 / 32; 64x0e (4 096) 46 / 38, one row of 16x(0e+1o) 32 / 17.
 constexpr int GEMM_SMALL_FWD = 8192, GEMM_SMALL_BWD = 2048, GEMM_SMALL_ROWS_PER_SM = 16;
@@ -1563,7 +1563,7 @@ int gemm_narrow_rows_per_sm(const Problem& p) {
     for (const std::vector<Irrep>* v : {&p.in1, &p.out})
         for (const Irrep& r : *v) mul = std::max(mul, r.mul);
     for (const Irrep& r : p.out) dim = std::max(dim, r.dim);
-    return mul < 28 && dim >= 5 ? 200 : 0;
+    return mul < 28 && dim >= 5 ? 150 : 0;
 }
 bool gemm_forward_tiled(const Problem& p, long long batch, long long sms) {
     const long long n = uvw_row_products(p);
@@ -2235,7 +2235,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
     const size_t wbytes = (size_t)p.w_numel * 8, dt_row = (size_t)h->grad_product.z_dim * 8;
     if (h->has_gemm_bwd && (rc = load_gemm(h->gemm_dw))) return rc;
     const bool gemm_tiled = h->has_gemm_bwd && gemm_backward_tiled(p, batch, h->gemm_dw.sm_count) &&
-                            workspace_bytes / wbytes >= (size_t)std::min<long long>((batch + 3) / 4, 2ll * h->gemm_dw.sm_count);
+                            workspace_bytes / wbytes >= (size_t)std::min<long long>((batch + h->bwd.uvw.tile_r - 1) / h->bwd.uvw.tile_r, 2ll * h->gemm_dw.sm_count);
     if (h->has_gemm_bwd && workspace && aligned16(workspace) && workspace_bytes >= std::max(wbytes, dt_row) && !gemm_tiled) {
         const long long block = (long long)std::min<size_t>((size_t)batch, workspace_bytes / dt_row);
         h->last_stream = st;
