@@ -1486,8 +1486,8 @@ bool uvw_row_supported(const Problem& p) {
 //     kernel is slower: 1x(0e+1o) (4) 20 / 45, but 4x(0e+1o) (16) 74 / 66; one tile of output channels keeps one warp of eight
 //     busy: 128x0e -> 4x0e 317 / 504.
 //   backward: by the weights per path: FP32 4x(0e+1o) (16) 53 / 123, 4x(0e..3o) (16) 657 / 1000, 8x(0e+1o+2e) (64) 260 / 299,
-//     but 12x(0e+1o) (144) 215 / 131; FP64 4x(0e..3o) 961 / 3029 (1 000 rows 92 / 123), 8x(0e+1o+2e) (64) 668 / 897, but without
-//     l = 2 8x(0e+1o) (64) 221 / 154; fewer than eight output channels leave most lanes idle: 128x0e -> 4x0e 88 / 113.
+//     but 12x(0e+1o) (144) 215 / 131; FP64 4x(0e..3o) 961 / 3029 (1 000 rows 92 / 123), 8x(0e+1o+2e) (64) 668 / 897 (2 000 rows
+//     57 / 70, 1 000 rows 55 / 41), but without l = 2 8x(0e+1o) (64) 221 / 154; fewer than eight output channels leave most lanes idle: 128x0e -> 4x0e 88 / 113.
 int uvw_row_limit(const Problem& p, bool bwd) {
     long long uv = 0, tiles = 0;
     int dim = 1, width = 0;
@@ -1501,6 +1501,7 @@ int uvw_row_limit(const Problem& p, bool bwd) {
     if (!bwd) return (f64 ? uv < 8 || tiles == 1 : uv < 64) ? 24 : 0;
     const long long per_path = p.w_numel / (long long)p.instr.size();
     if (per_path >= (f64 && dim <= 3 ? 48 : 144) && width >= 8) return 0;
+    if (f64 && dim >= 5) return per_path < 32 ? 5 : 8;
     return per_path < 32 ? 8 : 64;
 }
 
