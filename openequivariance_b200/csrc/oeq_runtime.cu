@@ -1311,6 +1311,7 @@ struct TcGeometry {
     unsigned outputs = 1;
     unsigned paths = 1;                     // instructions (the weights of each are packed by blocks of their own)
     int producers = 16, epilogues = 1;      // producer warps, groups of four epilogue warps
+    int dealt_rows_per_sm = 200;            // batches whose chunks are dealt over the CTAs (launch_uvw_tc)
     int threads() const { return 32 * (producers + 1 + 4 * epilogues); }
 };
 
@@ -1336,6 +1337,8 @@ bool uvw_tc_geometry(const Problem& p, TcGeometry& g, bool pad = false) {
         total += bytes;
     }
     if (total == 0) return false;
+    for (const Irrep& r : p.in1)
+        if (r.mul > 32) g.dealt_rows_per_sm = 160;
     g.producers = p.unit_y ? 8 : 16;
     g.epilogues = p.unit_y ? 2 : 1;
     const int off_w = 2 * 2 * 128 * 128;
@@ -2067,13 +2070,14 @@ static int launch_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t pack_fn,
     struct { const void* X; const void* Y; const void* Wp; void* Z; long long batch; int* status; int dealt; unsigned long long* prof; }
         tp{X, Y, packed, Z, batch, status, 0, nullptr};
     void* args[] = {&tp};
-    // Up to a chunk per CTA and output: output irreps over the grid's y dimension.  Up to 200 rows per SM: chunks of all
-    // outputs dealt (64x(0e+1o+2e), forward / W dZ: 1 500 rows 31 -> 17 / 20 -> 14 us, 10 007 rows 73 -> 62 / 46 -> 39,
-    // 30 000 rows 154 -> 151 / 99 -> 92).  Above, a share of the rows each: its balance does not depend on the costs
-    // that the deal assumes (100 000 rows: 443 against 504 us).
+    // Up to a chunk per CTA and output: output irreps over the grid's y dimension.  Then, up to some rows per SM, chunks of
+    // all outputs dealt; above, a share of the rows each, whose balance does not depend on the costs that the deal assumes.
+    // Shares / dealt in us, forward and W dZ: 64x(0e+1o+2e), 8 000 rows 72 / 58 and 43 / 35, 16 000 98 / 98 and 60 / 58, 24 000
+    // 139 / 136 and 85 / 82, 26 000 146 / 146 and 90 / 91, 29 600 156 / 166 and 97 / 101; 32x(0e+1o+2e), 29 600 77 / 73 and
+    // 52 / 52.
     long long grid = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 23) / 24));
     const unsigned split = grid * geo.outputs <= k.sm_count ? geo.outputs : 1;
-    if (split == 1 && geo.outputs > 1 && batch <= 200LL * k.sm_count) {
+    if (split == 1 && geo.outputs > 1 && batch <= (long long)geo.dealt_rows_per_sm * k.sm_count) {
         tp.dealt = 1;
         grid = k.sm_count;
     }

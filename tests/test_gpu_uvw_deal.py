@@ -11,10 +11,10 @@ from helpers import REL_TOL, rel_err, tp_inputs, to_oeq
 
 pytestmark = pytest.mark.gpu
 
-PER_SM = 200        # rows per SM up to which a batch is dealt
+PER_SM = 160        # rows per SM up to which a batch is dealt (more than 32 input channels; 200 below)
 
 
-@pytest.mark.parametrize("rows", [1177, 1200, 4001, PER_SM * 148, PER_SM * 148 + 1])
+@pytest.mark.parametrize("rows", [1177, 1200, 4001, PER_SM * 148, PER_SM * 148 + 1, 200 * 148])
 @pytest.mark.parametrize("irreps", [("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
                                     ("16x0e+48x1o", "0e+1o", "32x0e+16x1o+48x2e+16x4e")],   # (4e: no paths)
                          ids=["even", "uneven"])
