@@ -1548,13 +1548,14 @@ bool uvw_gemm_supported(const Problem& p) {
 
 // Batches that the tiled kernel computes faster than the GEMMs, whose chain of chunks of 32 channels, each with a barrier,
 // and whose three launches backward show where there is little to do.  Measured, tiled / GEMM in us:
-//   forward, up to one wave of 16-row tiles (2 368 rows) and 8 192 products a row: 300 rows of 32x0e 8 / 12, 128x0e -> 64x0e
-//     12 / 25, 16x(0e+1o) 12 / 14; above either line 128x0e -> 64x0e 5 000 rows 27 / 22, 16x(0e+1o+2e) (8 960) 27 / 18.
+//   forward, up to one wave of 16-row tiles (2 368 rows) and 4 096 products a row (8 192 with one path): 300 rows of 32x0e
+//     8 / 12, 128x0e -> 64x0e 12 / 25, 16x(0e+1o) 12 / 14, but one row of 64 -> 16x(0e+1o) (8 192, four paths) 26 / 20; above
+//     either line 128x0e -> 64x0e 5 000 rows 27 / 22, 16x(0e+1o+2e) (8 960) 27 / 18.
 //     Half-filled tiles with l = 2 lose at many rows: 20x(0e+1o+2e), 60 000 rows 428 / 504, 25 000 rows 188 / 199, 20 000
-//     158 / 160; 28x(0e+1o+2e) 617 / 606.  16x0e alone never fills a tile: 60 000 rows 29 / 33.
+//     158 / 160; 16 and 24 channels, 25 000 rows 180 / 174 and 233 / 221; 28x(0e+1o+2e) 617 / 606.  16x0e alone never fills a tile: 60 000 rows 29 / 33.
 //   backward, from the 128 rows on that take two shares of the rows (and their sum): 300 rows of 16x(0e+1o) (2 048) 36 / 46,
 //     32x0e 22 / 32; 64x0e (4 096) 46 / 38, one row of 16x(0e+1o) 32 / 17.
-constexpr int GEMM_SMALL_FWD = 8192, GEMM_SMALL_BWD = 2048, GEMM_SMALL_ROWS_PER_SM = 16;
+constexpr int GEMM_SMALL_FWD = 4096, GEMM_SMALL_FWD_ONE_PATH = 8192, GEMM_SMALL_BWD = 2048, GEMM_SMALL_ROWS_PER_SM = 16;
 
 long long uvw_row_products(const Problem& p) {
     long long n = 0;
@@ -1567,18 +1568,18 @@ int gemm_narrow_rows_per_sm(const Problem& p) {
     for (const std::vector<Irrep>* v : {&p.in1, &p.out})
         for (const Irrep& r : *v) mul = std::max(mul, r.mul);
     for (const Irrep& r : p.out) dim = std::max(dim, r.dim);
-    return mul < 28 && dim >= 5 ? 150 : 0;
+    return mul < 28 && dim >= 5 ? 200 : 0;
 }
+bool gemm_small_forward(const Problem& p) { return uvw_row_products(p) <= (p.instr.size() == 1 ? GEMM_SMALL_FWD_ONE_PATH : GEMM_SMALL_FWD); }
 bool gemm_forward_tiled(const Problem& p, long long batch, long long sms) {
-    const long long n = uvw_row_products(p);
-    if (n <= 256 || (n <= GEMM_SMALL_FWD && batch <= GEMM_SMALL_ROWS_PER_SM * sms)) return true;
+    if (uvw_row_products(p) <= 256 || (gemm_small_forward(p) && batch <= GEMM_SMALL_ROWS_PER_SM * sms)) return true;
     return gemm_narrow_rows_per_sm(p) && batch > gemm_narrow_rows_per_sm(p) * sms;
 }
 bool gemm_backward_tiled(const Problem& p, long long batch, long long sms) {
     return uvw_row_products(p) <= GEMM_SMALL_BWD && batch >= 128 && batch <= GEMM_SMALL_ROWS_PER_SM * sms;
 }
 // Whether any batch takes the tiled forward kernel (the backward one is there anyway, for small workspaces).
-bool gemm_keeps_tiled(const Problem& p) { return uvw_row_products(p) <= GEMM_SMALL_FWD || gemm_narrow_rows_per_sm(p) > 0; }
+bool gemm_keeps_tiled(const Problem& p) { return gemm_small_forward(p) || gemm_narrow_rows_per_sm(p) > 0; }
 
 int build_uvw_gemm(const Problem& p, int kernel_id, Kernel& k) {
     k.is_uvw = true;
@@ -1749,11 +1750,11 @@ int launch_uvu(Kernel& k, const Problem& p, UvuParams& prm, cudaStream_t stream,
         const long long groups = grid * k.map.ng;
         while (chunk > k.map.chunk_floor && prm.n_items / (groups * chunk) < 8) chunk /= 2;
         // A short list: smaller chunks while groups would be left without one.  Deterministic walks, whose chunks move to
-        // the next boundary (two dependent index reads) or meet a receiver's dZ anew, wait until half of the groups would
-        // be: 64x0e+32x1o, 59 k edges, forward 137 us with chunks of 32 (as many as groups), 111 with 64; 30 k edges 92 with
-        // 16, 80 with 32; 32x(0e..3o) FP64 backward, 6 k edges, 162 with 8, 109 with 16 (forward 131 and 148).
-        const int slack = prm.rows && (k.map.chunk_floor > 32 || prm.ws) ? 2 : 1;
-        while (chunk > 8 && prm.n_items * slack < groups * chunk) chunk /= 2;
+        // the next boundary (two dependent index reads) or meet a receiver's dZ anew, wait until three in seven would be:
+        // 64x0e+32x1o, 59 k edges, forward 137 us with chunks of 32 (as many as groups), 111 with 64; 20 k edges 68 with 32,
+        // 63 with 16; 32x(0e..3o) FP64 backward, 6 k edges, 162 with 8, 109 with 16 (forward 131 and 148).
+        const bool aligned = prm.rows && (k.map.chunk_floor > 32 || prm.ws);
+        while (chunk > 8 && (aligned ? prm.n_items * 7 / 4 : prm.n_items) < groups * chunk) chunk /= 2;
     }
     prm.chunk = std::max(1, chunk);
     void* args[] = {&prm};

@@ -62,7 +62,7 @@ def test_fp64_workspace_off_the_16_byte_rule():
 @pytest.mark.parametrize("irreps", [("16x0e", "0e", "16x0e"), ("32x0e", "0e", "32x0e"), ("128x0e", "0e", "64x0e"),
                                     ("16x0e+16x1o", "0e+1o", "16x0e+16x1o"), ("20x0e+20x1o+20x2e", "0e+1o+2e", "20x0e+20x1o+20x2e")],
                          ids=["16", "32", "128_64", "16_l1", "20_l2"])
-@pytest.mark.parametrize("batch", [127, 128, 2368, 2369, 22201])
+@pytest.mark.parametrize("batch", [127, 128, 2368, 2369, 29601])
 def test_fp64_lines_between_the_kernels(irreps, batch):
     p = oeq.FullyConnectedTPProblem(*irreps, irrep_dtype=np.float64, weight_dtype=np.float64)
     x, y, w, dz = tp_inputs(p, batch, 23)
