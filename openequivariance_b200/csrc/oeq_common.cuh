@@ -185,8 +185,9 @@ __device__ __forceinline__ void red_add(T* addr, T v) {
 }
 
 // Offset of W[u, w] (mu x mw, second-input multiplicity 1) in the kernel weight layout: 32-wide (u, w) chunks, u-chunk
-// major, each chunk [u][w].
+// major, each chunk [u][w] (reference: openequivariance/implementations/ComputationSchedule.py:146-230,427-471).
 __device__ __forceinline__ int weight_offset_v1(int mu, int mw, int u, int w) {
+    if (mu <= 32 && mw <= 32) return u * mw + w;        // (multiplicities are constants)
     const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
     const int ulen = (mu - (uc << 5)) < 32 ? (mu - (uc << 5)) : 32;
     const int wlen = (mw - (wc << 5)) < 32 ? (mw - (wc << 5)) : 32;

@@ -34,21 +34,6 @@ constexpr int TB_EPILOGUE_WARPS = 4;
 constexpr int TB_TILE = 128 * 128;             // one [128 rows x 32 tf32] swizzled tile
 constexpr int ERR_TB_EMPTY = 31, ERR_TB_FULL = 32, ERR_TB_ACC_EMPTY = 33, ERR_TB_ACC_FULL = 34;
 
-// Offset of W_p[u, w] (second-input multiplicity 1) in the kernel weight layout: 32-wide chunks, u-chunk major,
-// each chunk stored [u][w] (reference: openequivariance/implementations/ComputationSchedule.py:146-230,427-471).
-template <int P>
-__device__ __forceinline__ int tb_weight_offset(int u, int w) {
-    constexpr int MU = IN1_MUL[I_IN1[P]], MW = OUT_MUL[I_OUT[P]];
-    if constexpr (MU <= 32 && MW <= 32) {
-        return W_OFF[P] + u * MW + w;
-    } else {
-        const int uc = u >> 5, ul = u & 31, wc = w >> 5, wl = w & 31;
-        const int ulen = (MU - (uc << 5)) < 32 ? (MU - (uc << 5)) : 32;
-        const int wlen = (MW - (wc << 5)) < 32 ? (MW - (wc << 5)) : 32;
-        return W_OFF[P] + (uc << 5) * MW + ulen * (wc << 5) + ul * wlen + wl;
-    }
-}
-
 // rows of the batch owned by this CTA
 __device__ __forceinline__ void tb_row_range(long long batch, long long& lo, long long& hi) {
     lo = batch * blockIdx.x / gridDim.x;
@@ -276,7 +261,7 @@ __device__ __forceinline__ bool dw_epilogue(const UvwTcBwdParams& p, const DwBar
             constexpr int P = tb_nth_path(O, GRP * PER + j_);
             if constexpr (P >= 0) {
                 if (which == j_ && u < IN1_MUL[I_IN1[P]])
-                    for (int w = 0; w < MW; ++w) out[tb_weight_offset<P>(u, w)] = 0.f;
+                    for (int w = 0; w < MW; ++w) out[W_OFF[P] + weight_offset_v1(IN1_MUL[I_IN1[P]], MW, u, w)] = 0.f;
             }
         });
         return true;
@@ -299,7 +284,7 @@ __device__ __forceinline__ bool dw_epilogue(const UvwTcBwdParams& p, const DwBar
                 if (which == j_ && u < IN1_MUL[I_IN1[P]]) {
 #pragma unroll
                     for (int c = 0; c < 16; ++c)
-                        out[tb_weight_offset<P>(u, c0 + c)] = __uint_as_float(v[c]) + __uint_as_float(v2[c]);
+                        out[W_OFF[P] + weight_offset_v1(IN1_MUL[I_IN1[P]], MW, u, c0 + c)] = __uint_as_float(v[c]) + __uint_as_float(v2[c]);
                 }
             }
         });
