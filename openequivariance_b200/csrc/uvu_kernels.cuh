@@ -1679,7 +1679,7 @@ __device__ __forceinline__ long long align_sender(const long long* cols, const l
 
 // The helper warps of a receiver-order launch: whole rows, a row (or as many short ones as fit 16 to 32 values per lane) in
 // flight.  With the loop of the launch of its own below in its place (vector flushes), MACE-large at 6.0 M edges takes 66.3
-// instead of 61.9 ms (one box, in turn); with its blocks of columns the helper warps' launch went from 2.8 to 6.9 ms at
+// instead of 61.9 ms; with its blocks of columns the helper warps' launch went from 2.8 to 6.9 ms at
 // 300 k rows.
 __device__ void sum_sender_rows_beside(const T* __restrict__ temp, T* __restrict__ dX, const long long* __restrict__ cols,
                                        const long long* __restrict__ perm, long long n_items, long long e_lo, long long e_hi,
