@@ -26,6 +26,7 @@
 #include <cstring>
 #include <fstream>
 #include <mutex>
+#include <set>
 #include <sstream>
 #include <string>
 #include <tuple>
@@ -228,6 +229,7 @@ struct Mapping {
     int chunk_floor = 32;                     // smallest chunk of consecutive edges a launch may deal out
     int slice_warps = 0, n_slice = 1;         // slice kernels (uvu_slice_kernels.cuh): warps per CTA (0: not one of them)
     bool slice_full = false;
+    bool slice_outer = false;       // no weights: sums of products per receiver
     int slice_stages = 2, slice_smem = 0, slice_regs = 0;
     int threads() const { return ng * mulg * ps + 32 * ng * producer + 32 * helper_warps; }
     int fixed_bytes(int stages) const { return ng * stages * (16 + 8 * (epi > 1 ? 4 + 2 * epi : 4)) + ng * 128 + sw_bytes; }
@@ -673,9 +675,9 @@ bool uvu_tc_geometry(const Problem& p, UvuTcGeometry& g, int npad = 0) {
 // Clebsch-Gordan entries of a group ordered by (i, j), so that a product x_i y_j is formed once for all its paths.
 void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m) {
     struct Entry { int i, j, path, k; double v; };
-    std::vector<int> ga, gb, ge = {0}, gp = {0}, plist, toff(p.instr.size(), 0), ei, ej, et, enew, efirst;
+    std::vector<int> ga, gb, g0, ge = {0}, gp = {0}, plist, toff(p.instr.size(), 0), ei, ej, et, enew, efirst;
     std::vector<double> ev;
-    int tmax = 1;
+    int tmax = 1, products = 0;
     for (size_t a = 0; a < p.in1.size(); ++a)
         for (size_t b = 0; b < p.in2.size(); ++b) {
             std::vector<Entry> es;
@@ -701,13 +703,15 @@ void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m
                 efirst.push_back(!seen[tt]);
                 seen[tt] = 1;
             }
-            ga.push_back((int)a); gb.push_back((int)b);
+            ga.push_back((int)a); gb.push_back((int)b); g0.push_back(products);
+            products += p.in1[a].dim * p.in2[b].dim;
             ge.push_back((int)ei.size()); gp.push_back((int)plist.size());
         }
     auto put_int = [](std::ostringstream& o, int v) { o << v; };
     s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages
-      << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ";\n";
-    s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ";\n";
+      << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ", N_OUTER = " << products << ";\n";
+    s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ", SLICE_OUTER = " << (m.slice_outer ? "true" : "false") << ";\n";
+    emit_array(s, "int", "GRP_B0", g0, put_int);
     emit_array(s, "int", "GRP_A", ga, put_int);
     emit_array(s, "int", "GRP_B", gb, put_int);
     emit_array(s, "int", "GRP_E", ge, put_int);
@@ -1145,6 +1149,17 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
     return false;
 }
 
+constexpr int OUTER_REGS = 240;
+
+// Products of first- and second-input components that a channel needs (pairs of irreps with a path).
+int outer_products(const Problem& p) {
+    std::set<std::pair<int, int>> seen;
+    int n = 0;
+    for (const Instr& i : p.instr)
+        if (seen.insert({i.i1, i.i2}).second) n += p.in1[i.i1].dim * p.in2[i.i2].dim;
+    return n;
+}
+
 int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
     Mapping& m = k.map;
     if (!slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
@@ -1159,7 +1174,10 @@ int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
             tmax = std::max(tmax, t);
         }
     const int w = p.elem() / 4;
-    const int regs = zpc * w + 2 * (p.y_dim + d1 + tmax) + 24;
+    int regs = zpc * w + 2 * (p.y_dim + d1 + tmax) + 24;
+    const int outer = w * (outer_products(p) + p.y_dim + d1) + 28;
+    m.slice_outer = p.unit && outer <= OUTER_REGS;
+    if (m.slice_outer) regs = outer;
     if (!slice_fit(p, m, regs, pad16(32 * d3 * p.elem()), 0)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
     m.mulg = 32;
     m.z_ph_begin = {0, p.z_dim};
@@ -1180,7 +1198,10 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
     for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
     const int e = p.elem(), w = e / 4, per = 3 - w;         // registers of a value, edges computed together
-    const int regs = w * (zpc + per * (2 * p.y_dim + 3 * d1 + d2)) + 12;
+    int regs = w * (zpc + per * (2 * p.y_dim + 3 * d1 + d2)) + 12;
+    const int outer = w * (outer_products(p) + per * (2 * p.y_dim + 2 * d1)) + 24;
+    m.slice_outer = p.unit && outer <= OUTER_REGS;
+    if (m.slice_outer) regs = outer;
     int pitch = 8;
     while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
     if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;

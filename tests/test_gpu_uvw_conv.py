@@ -8,6 +8,7 @@ import openequivariance_b200 as oeq
 from oracle import tp_oracle as orc
 from conftest import problem_by_name
 from helpers import REL_TOL, rel_err, random_graph, to_oeq, to_e3nn
+from test_gpu_slice_conv import DEGREES
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,28 @@ def test_second_derivatives():
 def test_rejects_per_edge_uvw_weights():
     with pytest.raises(AssertionError):
         oeq.TensorProductConv(problem_by_name("diffdock_l1"), torch_op=True)
+
+
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("name,dtype", [("uvw_64", np.float32), ("uvw_64", np.float64), ("tetris_poly_2", np.float32)],
+                         ids=["uvw_64", "uvw_64_f64", "tetris_poly_2"])
+@pytest.mark.parametrize("graph", ["runs", "one_edge", "many"])
+def test_edge_sum_walk(name, dtype, graph, deterministic):
+    """The edge sums keep products per receiver: runs of no, one, odd and even numbers of edges."""
+    p = problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype)
+    degrees = np.array(DEGREES[graph])
+    nodes, edges = len(degrees), int(degrees.sum())
+    rng = np.random.default_rng(edges)
+    rows, cols, _, perm = orc.coord_graph(np.repeat(np.arange(nodes), degrees), rng.integers(0, nodes, edges))
+    x, y, w, dz = _inputs(p, nodes, edges, 8)
+    conv = oeq.TensorProductConv(p, torch_op=True, deterministic=deterministic)
+    xt, yt, dzt, *index = _cuda(x, y, dz, rows, cols, *([perm] if deterministic else []))
+    wt = torch.from_numpy(to_oeq(p, w)).cuda()
+    z = conv.forward(xt, yt, wt, *index)
+    dx, dy, dw = conv.backward_helper(xt, yt, wt, dzt, *index)
+    conv.check_device_status()
+    rx, ry, rw = orc.conv_backward(p, x, y, w, dz, rows, cols)
+    tol = REL_TOL[dtype]
+    assert rel_err(z.cpu().numpy(), orc.conv_forward(p, x, y, w, rows, cols)) < tol
+    assert rel_err(dx.cpu().numpy(), rx) < tol and rel_err(dy.cpu().numpy(), ry) < tol
+    assert rel_err(to_e3nn(p, dw.cpu().numpy()), rw) < tol
