@@ -257,6 +257,37 @@ __device__ __forceinline__ void cg_backward(const XA& x, const YA& y, const GA& 
 
 // Second-derivative form of the above (convolution): with r = w ex + ew x,
 //   ay_i += y_j P_ij;  aey_i += ey_j P_ij;  b_j += r_i P_ij.
+// The same with the weight on the smaller input: with w x in dY's sums, s_i = sum_j y_j P_ij gives dW = <x, s> and
+// dX += w s, three operations per value of the first input (two for each and one per value of the second input otherwise);
+// the inputs exchanged where the second one is smaller.  128x(0e..3o), receiver-order pass, 300 k edges: 2.68 -> 2.52 ms.
+template <int P, class XA, class YA, class GA, class DX, class DY>
+__device__ __forceinline__ T cg_backward_w(T w, const XA& x, const YA& y, const GA& g, DX& dx, DY& dy) {
+    constexpr bool W1 = IN1_D[I_IN1[P]] <= IN2_D[I_IN2[P]];
+    constexpr int DM = W1 ? IN1_D[I_IN1[P]] : IN2_D[I_IN2[P]];
+    T v[DM], s[DM], pij = (T)0, tw = (T)0;
+#pragma unroll
+    for (int i = 0; i < DM; ++i) {
+        v[i] = w * (W1 ? x[W1 ? i : 0] : y[W1 ? 0 : i]);
+        s[i] = (T)0;
+    }
+    sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n) {
+        constexpr int N = n, I = CG_I[N], J = CG_J[N], M = W1 ? I : J;
+        if constexpr (cg_pair_first<P, N>()) pij = (T)CG_V[N] * g[CG_K[N]];
+        else pij = fma((T)CG_V[N], g[CG_K[N]], pij);
+        if constexpr (cg_pair_last<P, N>()) {
+            s[M] = fma(W1 ? y[J] : x[I], pij, s[M]);
+            T& d = W1 ? dy[J] : dx[I];
+            d = fma(v[M], pij, d);
+        }
+    });
+#pragma unroll
+    for (int i = 0; i < DM; ++i) {
+        tw = fma(W1 ? x[W1 ? i : 0] : y[W1 ? 0 : i], s[i], tw);
+        T& d = W1 ? dx[W1 ? i : 0] : dy[W1 ? 0 : i];
+        d = fma(w, s[i], d);
+    }
+    return tw;
+}
 template <int P, class RA, class YA, class EA, class GA, class AA, class BA>
 __device__ __forceinline__ void cg_backward_dbl(const RA& r, const YA& y, const EA& ey, const GA& g, AA& ay, AA& aey, BA& b) {
     T pij = (T)0;
@@ -1573,33 +1604,25 @@ __device__ void run_backward_recv(const UvuParams& p, const Smem<true, MODE, tru
                         for (int j = 0; j < D2; ++j) dyreg[IN2_OFF[b] + j] += bv[j];
                     } else if constexpr (I_IN1[P] == a) {
                         constexpr int b = I_IN2[P], o = I_OUT[P];
-                        constexpr int D2 = IN2_D[b];
-                        T av[D1], bv[D2];
-    #pragma unroll
-                        for (int i = 0; i < D1; ++i) av[i] = (T)0;
-    #pragma unroll
-                        for (int j = 0; j < D2; ++j) bv[j] = (T)0;
-                        const T w = live ? (UNIT_W ? (T)1 : sWt[weight_offset<P>(u, 0)]) : (T)0;
+                        auto path = [&](const auto& gs) {
+                            T* dyb = dyreg + IN2_OFF[b];
+                            if constexpr (UNIT_W) {
+                                cg_backward<P>(x, &yr[IN2_OFF[b]], gs, dxa, dyb);
+                            } else {
+                                const T w = live ? sWt[weight_offset<P>(u, 0)] : (T)0;
+                                const T tw = cg_backward_w<P>(w, x, &yr[IN2_OFF[b]], gs, dxa, dyb);
+                                if (live) __stcs(dwrow + weight_offset<P>(u, 0), tw);
+                            }
+                        };
                         if constexpr (out_reg_off(o) < GZ_REGS) {
-                            cg_backward<P>(x, &yr[IN2_OFF[b]], &gz[out_reg_off(o)], av, bv);
+                            path(&gz[out_reg_off(o)]);
                         } else {
                             // this output irrep's slice of dZ is parked in shared memory ([value][channel]: no conflicts)
                             T gs[OUT_D[o]];
     #pragma unroll
                             for (int k = 0; k < OUT_D[o]; ++k) gs[k] = gzs[(out_reg_off(o) - GZ_FIRST_SMEM + k) * G + u];
-                            cg_backward<P>(x, &yr[IN2_OFF[b]], gs, av, bv);
+                            path(gs);
                         }
-                        T tw = (T)0;
-    #pragma unroll
-                        for (int i = 0; i < D1; ++i) {
-                            tw = fma(x[i], av[i], tw);
-                            dxa[i] = fma(w, av[i], dxa[i]);
-                        }
-                        if constexpr (!UNIT_W) {
-                            if (live) __stcs(dwrow + weight_offset<P>(u, 0), tw);
-                        }
-    #pragma unroll
-                        for (int j = 0; j < D2; ++j) dyreg[IN2_OFF[b] + j] = fma(w, bv[j], dyreg[IN2_OFF[b] + j]);
                     }
                 });
                 if (live) {

@@ -53,3 +53,26 @@ def test_walk(name, dtype, graph, deterministic):
         if deterministic and plain is not None:     # copies in pieces or in elements: the same sums
             assert all(torch.equal(a, b) for a, b in zip(got, plain))
         plain = got
+
+
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("name", ["nequip_32", "mace_128"])
+def test_missing_second_edge(name, deterministic):
+    """Receivers with an odd number of edges: the place of the edge that is not there holds zeros, not what an earlier edge
+    left there (infinities and NaN of other receivers stay where they belong)."""
+    p = problem_by_name(name, irrep_dtype=np.float32, weight_dtype=np.float32)
+    degrees = np.array([2, 1, 4, 3, 2, 1, 1, 5] * 40)
+    nodes, edges = len(degrees), int(degrees.sum())
+    rng = np.random.default_rng(3)
+    rows, cols, _, perm = orc.coord_graph(np.repeat(np.arange(nodes), degrees), rng.integers(0, nodes, edges))
+    x, y, w, _ = conv_inputs(p, nodes, edges, 11)
+    want = orc.conv_forward(p, x, y, w, rows, cols)
+    w, y = w.copy(), y.copy()
+    bad = degrees[rows] == 2
+    w[bad] = np.nan
+    y[bad] = np.inf
+    index = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in ((rows, cols, perm) if deterministic else (rows, cols))]
+    conv = oeq.TensorProductConv(p, torch_op=True, deterministic=deterministic)
+    got = conv.forward(*(torch.from_numpy(a).cuda() for a in (x, y, w)), *index).cpu().numpy()
+    assert rel_err(got[degrees != 2], want[degrees != 2]) < REL_TOL[np.float32]
+    assert np.isnan(got[degrees == 2]).all()
