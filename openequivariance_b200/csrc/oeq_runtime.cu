@@ -230,6 +230,7 @@ struct Mapping {
     int slice_warps = 0, n_slice = 1;         // slice kernels (uvu_slice_kernels.cuh): warps per CTA (0: not one of them)
     bool slice_full = false;
     bool slice_outer = false;       // no weights: sums of products per receiver
+    int slice_cpl = 1;              // channels per lane
     int slice_stages = 2, slice_smem = 0, slice_regs = 0;
     int threads() const { return ng * mulg * ps + 32 * ng * producer + 32 * helper_warps; }
     int fixed_bytes(int stages) const { return ng * stages * (16 + 8 * (epi > 1 ? 4 + 2 * epi : 4)) + ng * 128 + sw_bytes; }
@@ -708,7 +709,7 @@ void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m
             ge.push_back((int)ei.size()); gp.push_back((int)plist.size());
         }
     auto put_int = [](std::ostringstream& o, int v) { o << v; };
-    s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages
+    s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages << ", SLICE_CPL = " << m.slice_cpl
       << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ", N_OUTER = " << products << ";\n";
     s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ", SLICE_OUTER = " << (m.slice_outer ? "true" : "false") << ";\n";
     emit_array(s, "int", "GRP_B0", g0, put_int);
@@ -1128,7 +1129,7 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
     const int e = p.elem();
     int xch = 0;
     for (const Irrep& r : p.in1) xch += r.dim;
-    const int xs = pad16((m.slice_full ? 32 * xch : p.x_dim) * e);
+    const int xs = pad16((m.slice_full ? 32 * m.slice_cpl * xch : p.x_dim) * e);
     const int ws = p.unit ? 0 : pad16((m.slice_full ? 32 * (int)p.instr.size() : p.w_numel) * e);
     const int stage = 16 + (second ? 2 : 1) * (pad16(2 * p.y_dim * e) + 2 * xs + 2 * ws);     // (rows and cotangent rows)
     if (regs > 256) return false;
@@ -1190,6 +1191,16 @@ int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
     return OEQ_OK;
 }
 
+// Backward edge sums of rows of 64, 128 ... channels: two channels per lane share the walk, the second input and the sum of dY.
+// 64x(0e+1o+2e), 400 k edges, forward and backward 1 028 -> 1 010 us; the forward pass alone gains 9 of 269 us there but loses
+// 2 of 30 us on graphs of some hundred edges (fewer, longer walks) and keeps one channel.
+bool two_channels_per_lane(Mapping& m, int regs) {
+    if (!m.slice_full || m.n_slice % 2 || regs > OUTER_REGS) return false;
+    m.slice_cpl = 2;
+    m.n_slice /= 2;
+    return true;
+}
+
 int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     Mapping& m = k.map;
     if (!env_int("OEQ_B200_BWD_RECV", 1) || !slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
@@ -1197,11 +1208,17 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     for (const Irrep& r : p.out) zpc += r.dim;
     for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
     for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
-    const int e = p.elem(), w = e / 4, per = 3 - w;         // registers of a value, edges computed together
+    const int e = p.elem(), w = e / 4;      // registers of a value
+    int per = 3 - w;                        // edges computed together
     int regs = w * (zpc + per * (2 * p.y_dim + 3 * d1 + d2)) + 12;
     const int outer = w * (outer_products(p) + per * (2 * p.y_dim + 2 * d1)) + 24;
     m.slice_outer = p.unit && outer <= OUTER_REGS;
     if (m.slice_outer) regs = outer;
+    const int two = w * (2 * outer_products(p) + 2 * p.y_dim + 4 * d1) + 24;
+    if (m.slice_outer && two_channels_per_lane(m, two)) {
+        regs = two;
+        per = 1;
+    }
     int pitch = 8;
     while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
     if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;

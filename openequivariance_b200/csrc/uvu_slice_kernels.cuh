@@ -27,8 +27,9 @@ namespace oeq {
 
 constexpr int SL_S = SLICE_STAGES;              // stages per warp
 constexpr int SL_WARPS = SLICE_WARPS;           // warps per CTA, a multiple of N_SLICE
-constexpr int N_SLICE = NSLICE;                 // slices of 32 channels of a row (1: the whole row, at most 32 wide)
-constexpr bool FULL = SLICE_FULL;               // every multiplicity is 32 * NSLICE
+constexpr int CPL = SLICE_CPL, CH = 32 * CPL;   // channels per lane and of a slice
+constexpr int N_SLICE = NSLICE;                 // slices of a row (1: the whole row)
+constexpr bool FULL = SLICE_FULL;               // every multiplicity is CH * NSLICE
 
 // Without weights (UNIT_W) the coefficients are the same for all edges of a receiver, so a run of edges needs only the
 // products of the two inputs per edge: forward, the sums B_ij = sum_e x_i y_j are kept and contracted once per receiver;
@@ -36,6 +37,7 @@ constexpr bool FULL = SLICE_FULL;               // every multiplicity is 32 * NS
 // Edge sums of 64x(0e+1o+2e) x (0e+1o+2e), 10 007 nodes / 400 k edges: forward 265 -> 211 us, backward 433 -> 393 us (81 and
 // 162 FMAs per channel and edge; the walk, the copies and the sum of dY take 110 and 200 instructions beside them).
 constexpr bool OUTER = SLICE_OUTER;
+static_assert(CPL == 1 || (OUTER && FULL), "several channels per lane: backward edge sums of full slices");
 
 // ---- two edges in one register pair (FP32), or one edge (FP64, and the forward sums of products)
 #if OEQ_KERNEL == OEQ_K_SLICE_FWD_DET || OEQ_KERNEL == OEQ_K_SLICE_FWD_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_DET || OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_ATOMIC
@@ -43,7 +45,7 @@ constexpr bool FORWARD = true;                  // the walk that sums rows of Z
 constexpr bool ONE_EDGE = OUTER || ELEM == 8;   // (packing saves nothing where every product goes into a sum of its own)
 #else
 constexpr bool FORWARD = false;
-constexpr bool ONE_EDGE = ELEM == 8;
+constexpr bool ONE_EDGE = CPL > 1 || ELEM == 8;
 #endif
 template <class U, bool ONE> struct Pack;
 template <> struct Pack<float, false> {
@@ -76,11 +78,11 @@ typedef PK::V V2;
 // ---- slice layout of a staged pair: X and W of both edges, Y (FP32: interleaved, element j of edge h at 2j + h)
 __host__ __device__ constexpr int sum_in1_d(int n) { int s = 0; for (int a = 0; a < n; ++a) s += IN1_D[a]; return s; }
 constexpr int X_CH = sum_in1_d(N_IN1);                              // X values per channel
-constexpr int XS_ELEMS = FULL ? 32 * X_CH : X_DIM;                  // X values of a slice
+constexpr int XS_ELEMS = FULL ? CH * X_CH : X_DIM;                  // X values of a slice
 constexpr int WS_ELEMS = UNIT_W ? 0 : (FULL ? 32 * N_INSTR : W_NUMEL);
 constexpr int XSB = pad16(XS_ELEMS * ELEM), WSB = pad16(WS_ELEMS * ELEM), YSB = pad16(2 * Y_DIM * ELEM);
 // where irrep a of X, weight p of a slice start
-template <int A> __host__ __device__ constexpr int xs_off() { return FULL ? 32 * sum_in1_d(A) : IN1_OFF[A]; }
+template <int A> __host__ __device__ constexpr int xs_off() { return FULL ? CH * sum_in1_d(A) : IN1_OFF[A]; }
 template <int P> __host__ __device__ constexpr int ws_off() { return FULL ? 32 * P : W_OFF[P]; }
 
 struct SliceStage {
@@ -250,7 +252,7 @@ struct SliceCopies {
                 int o = 0;
                 sfor<0, N_IN1>([&](auto a_) {
                     constexpr int a = a_;
-                    constexpr int lo = xs_off<a>(), n = 32 * IN1_D[a];
+                    constexpr int lo = xs_off<a>(), n = CH * IN1_D[a];
                     if (el >= lo && el < lo + n) o = IN1_OFF[a] + slice * n + (el - lo);
                 });
                 xo[i] = o;
@@ -271,7 +273,7 @@ struct SliceCopies {
         } else if constexpr (FULL && N_SLICE > 1) {
             sfor<0, N_IN1>([&](auto a_) {
                 constexpr int a = a_;
-                constexpr int n = 32 * IN1_D[a];
+                constexpr int n = CH * IN1_D[a];
                 for (int i = lane; i < n; i += 32)
                     cp_async_elem_fill((T*)dst + xs_off<a>() + i, row + IN1_OFF[a] + slice * n + i, be);
             });
@@ -316,7 +318,7 @@ struct SliceCopies {
             } else {
                 sfor<0, N_IN1>([&](auto a_) {
                     constexpr int a = a_;
-                    constexpr int n = 32 * IN1_D[a];
+                    constexpr int n = CH * IN1_D[a];
                     for (int i = lane; i < n; i += 32) elem_out<ADD>(row + IN1_OFF[a] + slice * n + i, src[xs_off<a>() + i]);
                 });
             }
@@ -492,9 +494,10 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
     const bool z_vec = p.flags & 8;
 
     // the receiver's row, or (OUTER) its sums of products
-    T z[OUTER ? N_OUTER : ZPC_ALL];
+    constexpr int NZ = OUTER ? N_OUTER : ZPC_ALL;
+    T z[NZ];
 #pragma unroll
-    for (int k = 0; k < (OUTER ? N_OUTER : ZPC_ALL); ++k) z[k] = (T)0;
+    for (int k = 0; k < NZ; ++k) z[k] = (T)0;
 
     auto flush = [&](int node) {
         T* zrow = p.Z + (long long)node * Z_DIM;
@@ -527,7 +530,7 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
             }
         });
 #pragma unroll
-        for (int k = 0; k < (OUTER ? N_OUTER : ZPC_ALL); ++k) z[k] = (T)0;
+        for (int k = 0; k < NZ; ++k) z[k] = (T)0;
     };
 
     bool more = true;
@@ -585,7 +588,10 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
                     for (int i = 0; i < D1; ++i) {
                         const T x = live ? load_pair(sx, XSB, xs_off<a>() + lane * D1 + i, e) : (T)0;
 #pragma unroll
-                        for (int j = 0; j < D2; ++j) z[GRP_B0[g] + i * D2 + j] = fma(x, y[IN2_OFF[b] + j], z[GRP_B0[g] + i * D2 + j]);
+                        for (int j = 0; j < D2; ++j) {
+                            T& s = z[GRP_B0[g] + i * D2 + j];
+                            s = fma(x, y[IN2_OFF[b] + j], s);
+                        }
                     }
                 });
             }
@@ -703,7 +709,8 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
     T* dyg = reinterpret_cast<T*>(smem + (long long)SL_WARPS * (SL_S * L::BYTES + DYB) + grp * DYG);
     const bool dx_vec = p.flags & 8;
 
-    T gz[OUTER ? N_OUTER : ZPC_ALL];            // the receiver's dZ, or (OUTER) its G
+    T gzc[CPL][OUTER ? N_OUTER : ZPC_ALL];      // the receiver's dZ, or (OUTER) its G
+    auto& gz = gzc[0];
     bool more = true;
     int fill = 0, prev = -2, use = 0, ahead = 1 - SL_S, step = 0;
     for (;;) {
@@ -733,21 +740,21 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
             const T* zrow = p.dZ + (long long)prev * Z_DIM;
             if constexpr (OUTER) {
 #pragma unroll
-                for (int k = 0; k < N_OUTER; ++k) gz[k] = (T)0;
+                for (int k = 0; k < CPL * N_OUTER; ++k) gzc[k / N_OUTER][k % N_OUTER] = (T)0;
             }
-            sfor<0, N_OUT>([&](auto o_) {
-                constexpr int o = o_;
+            sfor<0, N_OUT * CPL>([&](auto oc_) {
+                constexpr int o = oc_ / CPL, c = oc_ % CPL;
                 const bool live = FULL || lane < OUT_MUL[o];
                 T v[OUT_D[o]];
 #pragma unroll
-                for (int k = 0; k < OUT_D[o]; ++k) v[k] = live ? __ldg(zrow + OUT_OFF[o] + (slice * 32 + lane) * OUT_D[o] + k) : (T)0;
+                for (int k = 0; k < OUT_D[o]; ++k) v[k] = live ? __ldg(zrow + OUT_OFF[o] + (slice * CH + 32 * c + lane) * OUT_D[o] + k) : (T)0;
                 if constexpr (OUTER) {
                     sfor<0, N_INSTR>([&](auto p_) {
                         constexpr int P = p_;
                         if constexpr (I_OUT[P] == o) {
                             sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
                                 constexpr int n = n_;
-                                T& g = gz[outer_off<P>() + CG_I[n] * IN2_D[I_IN2[P]] + CG_J[n]];
+                                T& g = gzc[c][outer_off<P>() + CG_I[n] * IN2_D[I_IN2[P]] + CG_J[n]];
                                 g = fma((T)CG_V[n], v[CG_K[n]], g);
                             });
                         }
@@ -783,8 +790,8 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                 sw[q] = reinterpret_cast<const T*>(st + L::OFF_W + (e + q) * WSB);
                 dw[q] = p.dW + (long long)(h.x + e + q) * W_NUMEL;
             }
-            sfor<0, N_IN1>([&](auto a_) {
-                constexpr int a = a_;
+            sfor<0, N_IN1 * CPL>([&](auto ac_) {
+                constexpr int a = ac_ / CPL, c = ac_ % CPL, X0 = xs_off<a>() + 32 * c * IN1_D[a];
                 constexpr int D1 = IN1_D[a];
                 const bool live = FULL || lane < IN1_MUL[a];
                 T x[NE][D1], dx[NE][D1], ex[DBLC ? NE : 1][D1];
@@ -792,7 +799,7 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                 for (int q = 0; q < NE; ++q)
 #pragma unroll
                     for (int i = 0; i < D1; ++i) {
-                        x[q][i] = live ? sx[q][xs_off<a>() + lane * D1 + i] : (T)0;
+                        x[q][i] = live ? sx[q][X0 + lane * D1 + i] : (T)0;
                         dx[q][i] = (T)0;
                         if constexpr (DBLC) ex[q][i] = live ? sx[q][(L::OFF_EX - L::OFF_X) / ELEM + xs_off<a>() + lane * D1 + i] : (T)0;
                     }
@@ -805,7 +812,7 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                             for (int i = 0; i < D1; ++i)
 #pragma unroll
                                 for (int j = 0; j < D2; ++j) {
-                                    const T v = gz[GRP_B0[g] + i * D2 + j];
+                                    const T v = gzc[c][GRP_B0[g] + i * D2 + j];
 #pragma unroll
                                     for (int q = 0; q < NE; ++q) {
                                         dx[q][i] = fma(y[q][IN2_OFF[b] + j], v, dx[q][i]);
@@ -919,7 +926,7 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
 #pragma unroll
                     for (int q = 0; q < NE; ++q)
 #pragma unroll
-                        for (int i = 0; i < D1; ++i) sx[q][xs_off<a>() + lane * D1 + i] = dx[q][i];
+                        for (int i = 0; i < D1; ++i) sx[q][X0 + lane * D1 + i] = dx[q][i];
                 }
             });
             // dY: transpose through shared memory, lane v then owns value v (edge-major) of all 32 channels
