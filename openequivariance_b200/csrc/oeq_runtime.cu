@@ -231,6 +231,7 @@ struct Mapping {
     bool slice_full = false;
     bool slice_outer = false;       // no weights: sums of products per receiver
     int slice_cpl = 1;              // channels per lane
+    bool slice_one = false;         // one edge at a time, and per stage
     int slice_stages = 2, slice_smem = 0, slice_regs = 0;
     int threads() const { return ng * mulg * ps + 32 * ng * producer + 32 * helper_warps; }
     int fixed_bytes(int stages) const { return ng * stages * (16 + 8 * (epi > 1 ? 4 + 2 * epi : 4)) + ng * 128 + sw_bytes; }
@@ -709,7 +710,7 @@ void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m
             ge.push_back((int)ei.size()); gp.push_back((int)plist.size());
         }
     auto put_int = [](std::ostringstream& o, int v) { o << v; };
-    s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages << ", SLICE_CPL = " << m.slice_cpl
+    s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages << ", SLICE_CPL = " << m.slice_cpl << ", SLICE_ONE = " << (m.slice_one ? 1 : 0)
       << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ", N_OUTER = " << products << ";\n";
     s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ", SLICE_OUTER = " << (m.slice_outer ? "true" : "false") << ";\n";
     emit_array(s, "int", "GRP_B0", g0, put_int);
@@ -1131,7 +1132,8 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
     for (const Irrep& r : p.in1) xch += r.dim;
     const int xs = pad16((m.slice_full ? 32 * m.slice_cpl * xch : p.x_dim) * e);
     const int ws = p.unit ? 0 : pad16((m.slice_full ? 32 * (int)p.instr.size() : p.w_numel) * e);
-    const int stage = 16 + (second ? 2 : 1) * (pad16(2 * p.y_dim * e) + 2 * xs + 2 * ws);     // (rows and cotangent rows)
+    const int ep = m.slice_one ? 1 : 2;     // edges of a stage
+    const int stage = 16 + (second ? 2 : 1) * (pad16(ep * p.y_dim * e) + ep * xs + ep * ws);     // (rows and cotangent rows)
     if (regs > 256) return false;
     m.slice_regs = regs;
     const int target = env_int("OEQ_B200_SLICE_WARPS_SM", regs <= 124 ? 16 : (regs <= 164 ? 12 : 8));
@@ -1247,15 +1249,30 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
     for (const Irrep& r : p.out) { zpc += r.dim; d3 = std::max(d3, r.dim); }
     for (const Irrep& r : p.in1) d1 = std::max(d1, r.dim);
     for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
-    const int e = p.elem(), w = e / 4, per = 3 - w;
-    const int regs = w * (zpc + per * (grads ? 2 * p.y_dim + 6 * d1 + d2 : 2 * p.y_dim + 4 * d1 + 2)) + 12;
-    int pitch = 8;
-    while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
-    if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;
-    const int groups = m.n_slice >= 4 ? 1 : 4 / m.n_slice;
-    const int dyg = m.n_slice > 1 ? 2 * m.n_slice * pitch * e : 0;
-    if (!slice_fit(p, m, regs, grads ? 32 * pitch * e : pad16(32 * d3 * e), grads ? groups * dyg : 0, true))
-        return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+    const int e = p.elem(), w = e / 4;
+    // A stage of two edges and their cotangents, or of one: where two leave shared memory for fewer warps than the registers do
+    // (FP64), or computing two together takes too many registers (FP32).  FP64, deterministic, forward and both derivatives:
+    // 128x(0e+1o+2e) x (0e..3o), 1 000 nodes / 28 k edges 1 308 -> 1 157 us; 32x(0e+1o+2e), 3 000 / 111 k 980 -> 889.  FP32
+    // 128x(0e..3o), group kernel before: 1 000 / 30 k 1 954 -> 1 418, 6 000 / 180 k 9 535 -> 7 887.  Where two edges fit with the
+    // same warps they are faster: 8x(0e+1o) 482 against 521, FP64 270 against 286; FP32 128x(0e+1o+2e) 1 133 against 1 136.
+    auto fit = [&](bool one) {
+        const int per = one ? 1 : 3 - w;        // edges computed together
+        m.slice_one = one;
+        const int regs = w * (zpc + per * (grads ? 2 * p.y_dim + 6 * d1 + d2 : 2 * p.y_dim + 4 * d1 + 2)) + 12;
+        int pitch = 8;
+        while (pitch < 32 && pitch < per * p.y_dim) pitch *= 2;
+        if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;
+        const int groups = m.n_slice >= 4 ? 1 : 4 / m.n_slice;
+        const int dyg = m.n_slice > 1 ? 2 * m.n_slice * pitch * e : 0;
+        return slice_fit(p, m, regs, grads ? 32 * pitch * e : pad16(32 * d3 * e), grads ? groups * dyg : 0, true);
+    };
+    const bool pair = fit(false);
+    if (!pair || w == 2) {
+        const Mapping two = m;
+        const bool one = fit(true);
+        if (!one && !pair) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+        if (!one || (pair && m.min_ctas * m.slice_warps <= two.min_ctas * two.slice_warps)) m = two;
+    }
     m.mulg = 32;
     m.z_ph_begin = {0, p.z_dim};
     m.w_ph_begin = {0, p.w_numel};

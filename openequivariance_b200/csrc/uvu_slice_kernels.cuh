@@ -42,10 +42,10 @@ static_assert(CPL == 1 || (OUTER && FULL), "several channels per lane: backward 
 // ---- two edges in one register pair (FP32), or one edge (FP64, and the forward sums of products)
 #if OEQ_KERNEL == OEQ_K_SLICE_FWD_DET || OEQ_KERNEL == OEQ_K_SLICE_FWD_ATOMIC || OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_DET || OEQ_KERNEL == OEQ_K_SLICE_DBL_Z_ATOMIC
 constexpr bool FORWARD = true;                  // the walk that sums rows of Z
-constexpr bool ONE_EDGE = OUTER || ELEM == 8;   // (packing saves nothing where every product goes into a sum of its own)
+constexpr bool ONE_EDGE = OUTER || SLICE_ONE || ELEM == 8;   // (packing saves nothing where every product goes into a sum of its own)
 #else
 constexpr bool FORWARD = false;
-constexpr bool ONE_EDGE = CPL > 1 || ELEM == 8;
+constexpr bool ONE_EDGE = CPL > 1 || SLICE_ONE || ELEM == 8;
 #endif
 template <class U, bool ONE> struct Pack;
 template <> struct Pack<float, false> {
@@ -77,10 +77,11 @@ typedef PK::V V2;
 
 // ---- slice layout of a staged pair: X and W of both edges, Y (FP32: interleaved, element j of edge h at 2j + h)
 __host__ __device__ constexpr int sum_in1_d(int n) { int s = 0; for (int a = 0; a < n; ++a) s += IN1_D[a]; return s; }
+constexpr int EP = SLICE_ONE ? 1 : 2;                               // edges of a stage
 constexpr int X_CH = sum_in1_d(N_IN1);                              // X values per channel
 constexpr int XS_ELEMS = FULL ? CH * X_CH : X_DIM;                  // X values of a slice
 constexpr int WS_ELEMS = UNIT_W ? 0 : (FULL ? 32 * N_INSTR : W_NUMEL);
-constexpr int XSB = pad16(XS_ELEMS * ELEM), WSB = pad16(WS_ELEMS * ELEM), YSB = pad16(2 * Y_DIM * ELEM);
+constexpr int XSB = pad16(XS_ELEMS * ELEM), WSB = pad16(WS_ELEMS * ELEM), YSB = pad16(EP * Y_DIM * ELEM);
 // where irrep a of X, weight p of a slice start
 template <int A> __host__ __device__ constexpr int xs_off() { return FULL ? CH * sum_in1_d(A) : IN1_OFF[A]; }
 template <int P> __host__ __device__ constexpr int ws_off() { return FULL ? 32 * P : W_OFF[P]; }
@@ -90,10 +91,10 @@ struct SliceStage {
     static constexpr int OFF_Y = 16;
     static constexpr int OFF_EY = OFF_Y + YSB;  // (second derivatives: the cotangent rows beside the rows)
     static constexpr int OFF_X = OFF_EY + (DBLC ? YSB : 0);     // two rows
-    static constexpr int OFF_EX = OFF_X + 2 * XSB;
-    static constexpr int OFF_W = OFF_EX + (DBLC ? 2 * XSB : 0);
-    static constexpr int OFF_EW = OFF_W + 2 * WSB;
-    static constexpr int BYTES = OFF_EW + (DBLC ? 2 * WSB : 0);
+    static constexpr int OFF_EX = OFF_X + EP * XSB;
+    static constexpr int OFF_W = OFF_EX + (DBLC ? EP * XSB : 0);
+    static constexpr int OFF_EW = OFF_W + EP * WSB;
+    static constexpr int BYTES = OFF_EW + (DBLC ? EP * WSB : 0);
 };
 constexpr int MAX_OUT_D = []() { int m = 1; for (int o = 0; o < N_OUT; ++o) m = OUT_D[o] > m ? OUT_D[o] : m; return m; }();
 constexpr int SL_FLUSH = pad16(32 * MAX_OUT_D * ELEM);              // transposition buffer of one output irrep
@@ -191,7 +192,7 @@ struct PairWalker {
         row = __shfl_sync(0xffffffffu, wr, src);
         s0 = __shfl_sync(0xffffffffu, wc, src);
         const int r1 = __shfl_sync(0xffffffffu, wr, src + 1), c1 = __shfl_sync(0xffffffffu, wc, src + 1);
-        const bool two = r1 == row;         // (a lane past the chunk holds -1)
+        const bool two = EP == 2 && r1 == row;      // (a lane past the chunk holds -1)
         s1 = two ? c1 : -1;
         e0 = pos;
         pos += two ? 2 : 1;

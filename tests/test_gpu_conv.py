@@ -214,6 +214,15 @@ def test_fused_second_derivatives(name, dtype, tol, deterministic):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("deterministic", [True, False])
+@pytest.mark.parametrize("name,dtype,tol", [("mace_large_128", np.float32, 2e-5), ("mace_128", np.float64, 1e-11),
+                                            ("nequip_32", np.float64, 1e-11), ("interaction_8", np.float64, 1e-11)])
+def test_fused_second_derivatives_one_edge(name, dtype, tol, deterministic):
+    """Rows whose second derivatives take one edge at a time: wide ones, and FP64 where that leaves room for more warps (the
+    last problem keeps two edges per stage)."""
+    test_fused_second_derivatives(name, dtype, tol, deterministic)
+
+
 def test_fused_second_derivatives_staging_variants(monkeypatch):
     """Cotangent rows at addresses that rule out bulk copies, and bulk copies switched off altogether: same bits as
     the aligned run of the deterministic variant (only the way rows reach shared memory differs)."""
