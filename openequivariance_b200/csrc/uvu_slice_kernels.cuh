@@ -448,6 +448,9 @@ __device__ __forceinline__ void slice_second_z(const unsigned char* st, int e, i
 // to the row.  With the zeros for a missing second edge: 32x(0e+1o+2e), 800 k edges, forward 281 -> 271 us; 128x(0e+1o+2e) x
 // (0e..3o), 150 k edges, 313 -> 296; 128x(0e..3o), 1.2 M edges, 5.07 -> 4.86 ms.
 enum class Place { IN1, IN2, OUT };
+// FP64 with few sums: the coefficient FMAs of a path would follow one another on the same values of the row, at the FP64 FMA's
+// latency.  8x(0e+1o), 8 sums, 4 000 nodes: 48 us with the weight on an input, 45 on the output; 32x(0e+1o+2e), 35 sums: 97 / 98.
+constexpr bool FEW_SUMS = ELEM == 8 && ZPC_ALL < 16;
 __host__ __device__ constexpr Place weight_place(int p) {
     const int d1 = IN1_D[I_IN1[p]], d2 = IN2_D[I_IN2[p]], d3 = OUT_D[I_OUT[p]];
     return d1 <= d2 && d1 <= d3 ? Place::IN1 : (d2 <= d3 ? Place::IN2 : Place::OUT);
@@ -608,7 +611,7 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
                         constexpr int g = g_;
                         if constexpr (GRP_A[g] == a) {
                             constexpr int b = GRP_B[g], P0 = P_LIST[GRP_P[g]];
-                            constexpr Place PL = UNIT_W || GRP_P[g + 1] - GRP_P[g] > 1 ? Place::OUT : weight_place(P0);
+                            constexpr Place PL = UNIT_W || FEW_SUMS || GRP_P[g + 1] - GRP_P[g] > 1 ? Place::OUT : weight_place(P0);
                             if constexpr (PL == Place::OUT) {
                                 V2 t[T_MAX], xy;
                                 sfor<GRP_E[g], GRP_E[g + 1]>([&](auto n_) {
