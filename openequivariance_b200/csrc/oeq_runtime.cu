@@ -676,10 +676,11 @@ bool uvu_tc_geometry(const Problem& p, UvuTcGeometry& g, int npad = 0) {
 // Tables of the slice kernels: the paths grouped by their two input irreps (first-input major), and the
 // Clebsch-Gordan entries of a group ordered by (i, j), so that a product x_i y_j is formed once for all its paths.
 void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m) {
-    struct Entry { int i, j, path, k; double v; };
-    std::vector<int> ga, gb, g0, ge = {0}, gp = {0}, plist, toff(p.instr.size(), 0), ei, ej, et, enew, efirst;
+    struct Entry { int i, j, path, k, n; double v; };
+    std::vector<int> ga, gb, g0 = {0}, pri, prj, ge = {0}, gp = {0}, plist, toff(p.instr.size(), 0), ei, ej, et, enew, efirst;
+    std::vector<std::vector<int>> pr(p.instr.size());       // the products of a path's coefficients
     std::vector<double> ev;
-    int tmax = 1, products = 0;
+    int tmax = 1;
     for (size_t a = 0; a < p.in1.size(); ++a)
         for (size_t b = 0; b < p.in2.size(); ++b) {
             std::vector<Entry> es;
@@ -690,7 +691,8 @@ void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m
                 plist.push_back((int)q);
                 toff[q] = t;
                 t += p.out[ins.io].dim;
-                for (size_t z = 0; z < ins.cv.size(); ++z) es.push_back({ins.ci[z], ins.cj[z], (int)q, ins.ck[z], ins.cv[z]});
+                for (size_t z = 0; z < ins.cv.size(); ++z) es.push_back({ins.ci[z], ins.cj[z], (int)q, ins.ck[z], (int)z, ins.cv[z]});
+                pr[q].assign(ins.cv.size(), 0);
             }
             if (t == 0) continue;
             tmax = std::max(tmax, t);
@@ -702,18 +704,24 @@ void emit_slice_tables(std::ostringstream& s, const Problem& p, const Mapping& m
                 const int tt = toff[es[n].path] + es[n].k;
                 ei.push_back(es[n].i); ej.push_back(es[n].j); et.push_back(tt); ev.push_back(es[n].v);
                 enew.push_back(n == 0 || es[n].i != es[n - 1].i || es[n].j != es[n - 1].j);
+                if (enew.back()) { pri.push_back(es[n].i); prj.push_back(es[n].j); }
+                pr[es[n].path][es[n].n] = (int)pri.size() - 1;
                 efirst.push_back(!seen[tt]);
                 seen[tt] = 1;
             }
-            ga.push_back((int)a); gb.push_back((int)b); g0.push_back(products);
-            products += p.in1[a].dim * p.in2[b].dim;
+            ga.push_back((int)a); gb.push_back((int)b); g0.push_back((int)pri.size());
             ge.push_back((int)ei.size()); gp.push_back((int)plist.size());
         }
     auto put_int = [](std::ostringstream& o, int v) { o << v; };
     s << "constexpr int NSLICE = " << m.n_slice << ", SLICE_WARPS = " << m.slice_warps << ", SLICE_STAGES = " << m.slice_stages << ", SLICE_CPL = " << m.slice_cpl << ", SLICE_ONE = " << (m.slice_one ? 1 : 0)
-      << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ", N_OUTER = " << products << ";\n";
+      << ", N_GROUPS = " << ga.size() << ", T_MAX = " << tmax << ", N_OUTER = " << pri.size() << ";\n";
     s << "constexpr bool SLICE_FULL = " << (m.slice_full ? "true" : "false") << ", SLICE_OUTER = " << (m.slice_outer ? "true" : "false") << ";\n";
-    emit_array(s, "int", "GRP_B0", g0, put_int);
+    std::vector<int> cgpr;
+    for (const std::vector<int>& v : pr) cgpr.insert(cgpr.end(), v.begin(), v.end());
+    emit_array(s, "int", "GRP_PR", g0, put_int);
+    emit_array(s, "int", "PR_I", pri, put_int);
+    emit_array(s, "int", "PR_J", prj, put_int);
+    emit_array(s, "int", "CG_PR", cgpr, put_int);
     emit_array(s, "int", "GRP_A", ga, put_int);
     emit_array(s, "int", "GRP_B", gb, put_int);
     emit_array(s, "int", "GRP_E", ge, put_int);
@@ -1154,8 +1162,10 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
 
 constexpr int OUTER_REGS = 240;
 
-// Products of first- and second-input components that a channel needs (pairs of irreps with a path).
-int outer_products(const Problem& p) {
+// Pairs of first- and second-input components of a channel, of the irreps that have a path: the measure of the register
+// estimates.  (The pairs with a coefficient are what the kernels keep, but as a measure they give some kernels four warps per
+// scheduler where three are faster: 64x(0e+1o) x (0e+1o+2e) -> 64x(0e+1o+2e), 800 k edges, backward 351 -> 376 us.)
+int outer_pairs(const Problem& p) {
     std::set<std::pair<int, int>> seen;
     int n = 0;
     for (const Instr& i : p.instr)
@@ -1178,7 +1188,7 @@ int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
         }
     const int w = p.elem() / 4;
     int regs = zpc * w + 2 * (p.y_dim + d1 + tmax) + 24;
-    const int outer = w * (outer_products(p) + p.y_dim + d1) + 28;
+    const int outer = w * (outer_pairs(p) + p.y_dim + d1) + 28;
     m.slice_outer = p.unit && outer <= OUTER_REGS;
     if (m.slice_outer) regs = outer;
     if (!slice_fit(p, m, regs, pad16(32 * d3 * p.elem()), 0)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
@@ -1213,10 +1223,10 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     const int e = p.elem(), w = e / 4;      // registers of a value
     int per = 3 - w;                        // edges computed together
     int regs = w * (zpc + per * (2 * p.y_dim + 3 * d1 + d2)) + 12;
-    const int outer = w * (outer_products(p) + per * (2 * p.y_dim + 2 * d1)) + 24;
+    const int outer = w * (outer_pairs(p) + per * (2 * p.y_dim + 2 * d1)) + 24;
     m.slice_outer = p.unit && outer <= OUTER_REGS;
     if (m.slice_outer) regs = outer;
-    const int two = w * (2 * outer_products(p) + 2 * p.y_dim + 4 * d1) + 24;
+    const int two = w * (2 * outer_pairs(p) + 2 * p.y_dim + 4 * d1) + 24;
     if (m.slice_outer && two_channels_per_lane(m, two)) {
         regs = two;
         per = 1;

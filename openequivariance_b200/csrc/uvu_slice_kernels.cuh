@@ -33,9 +33,12 @@ constexpr bool FULL = SLICE_FULL;               // every multiplicity is CH * NS
 
 // Without weights (UNIT_W) the coefficients are the same for all edges of a receiver, so a run of edges needs only the
 // products of the two inputs per edge: forward, the sums B_ij = sum_e x_i y_j are kept and contracted once per receiver;
-// backward, G_ij = sum_k C_ijk dZ_k is formed once per receiver.  (GRP_B0: where a pair of irreps starts in B and G.)
-// Edge sums of 64x(0e+1o+2e) x (0e+1o+2e), 10 007 nodes / 400 k edges: forward 265 -> 211 us, backward 433 -> 393 us (81 and
-// 162 FMAs per channel and edge; the walk, the copies and the sum of dY take 110 and 200 instructions beside them).
+// backward, G_ij = sum_k C_ijk dZ_k is formed once per receiver.  B and G hold the pairs (i, j) that have a coefficient (PR_I,
+// PR_J; GRP_PR: where a pair of irreps starts, CG_PR: the place of a coefficient's pair): a component times the zeros of
+// other pairs would be work for nothing, and NaN where it is infinite.
+// Edge sums of 64x(0e+1o+2e) x (0e+1o+2e), 10 007 nodes / 400 k edges: forward 265 -> 211 us, backward 433 -> 393 us.  Per
+// channel and edge 71 and 142 FMAs instead of 71 products, 83 coefficient FMAs and 35 additions forward, 83 coefficient FMAs for
+// two edges and 158 for each backward; the walk, the copies and the sum of dY take 110 and 200 instructions beside them.
 constexpr bool OUTER = SLICE_OUTER;
 static_assert(CPL == 1 || (OUTER && FULL), "several channels per lane: backward edge sums of full slices");
 
@@ -461,12 +464,6 @@ __host__ __device__ constexpr bool same_coefficient(int p) {
     return true;
 }
 
-// where the products of the irreps of path P start in the sums of products
-template <int P> __host__ __device__ constexpr int outer_off() {
-    for (int g = 0; g < N_GROUPS; ++g)
-        if (GRP_A[g] == I_IN1[P] && GRP_B[g] == I_IN2[P]) return GRP_B0[g];
-    return 0;
-}
 // Output irrep O of a channel from its sums of products.
 template <int O, class BA>
 __device__ __forceinline__ void outer_contract(const BA& b, T (&v)[OUT_D[O]]) {
@@ -477,14 +474,12 @@ __device__ __forceinline__ void outer_contract(const BA& b, T (&v)[OUT_D[O]]) {
         if constexpr (I_OUT[P] == O) {
             sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
                 constexpr int n = n_;
-                v[CG_K[n]] = fma((T)CG_V[n], b[outer_off<P>() + CG_I[n] * IN2_D[I_IN2[P]] + CG_J[n]], v[CG_K[n]]);
+                v[CG_K[n]] = fma((T)CG_V[n], b[CG_PR[n]], v[CG_K[n]]);
             });
         }
     });
 }
 
-// Without weights: 81 sums of products for two inputs 0e+1o+2e.  An edge then takes 81 FMAs of a channel instead of 81
-// products, 101 coefficient FMAs and 35 additions.
 template <int MODE>
 __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp, int lane) {
     using L = SliceStage;
@@ -584,24 +579,9 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
             V2 y[Y_DIM];
             load_y(st + L::OFF_Y, e, y);
             if constexpr (DBLC) slice_second_z(st, e, lane, y, z);
-            if constexpr (OUTER) {
-                sfor<0, N_GROUPS>([&](auto g_) {
-                    constexpr int g = g_, a = GRP_A[g], b = GRP_B[g], D1 = IN1_D[a], D2 = IN2_D[b];
-                    const bool live = FULL || lane < IN1_MUL[a];
-#pragma unroll
-                    for (int i = 0; i < D1; ++i) {
-                        const T x = live ? load_pair(sx, XSB, xs_off<a>() + lane * D1 + i, e) : (T)0;
-#pragma unroll
-                        for (int j = 0; j < D2; ++j) {
-                            T& s = z[GRP_B0[g] + i * D2 + j];
-                            s = fma(x, y[IN2_OFF[b] + j], s);
-                        }
-                    }
-                });
-            }
             sfor<0, N_IN1>([&](auto a_) {
                 constexpr int a = a_;
-                if constexpr (any_part_uses_in1(a) && !DBLC && !OUTER) {
+                if constexpr (any_part_uses_in1(a) && !DBLC) {
                     constexpr int D1 = IN1_D[a];
                     const bool live = FULL || lane < IN1_MUL[a];
                     V2 x[D1];
@@ -609,7 +589,12 @@ __device__ void slice_forward(const UvuParams& p, unsigned char* smem, int warp,
                     for (int i = 0; i < D1; ++i) x[i] = live ? load_pair(sx, XSB, xs_off<a>() + lane * D1 + i, e) : PK::all((T)0);
                     sfor<0, N_GROUPS>([&](auto g_) {
                         constexpr int g = g_;
-                        if constexpr (GRP_A[g] == a) {
+                        if constexpr (GRP_A[g] == a && OUTER) {
+                            sfor<GRP_PR[g], GRP_PR[g + 1]>([&](auto s_) {
+                                constexpr int s = s_;
+                                z[s] = fma(x[PR_I[s]], y[IN2_OFF[GRP_B[g]] + PR_J[s]], z[s]);
+                            });
+                        } else if constexpr (GRP_A[g] == a) {
                             constexpr int b = GRP_B[g], P0 = P_LIST[GRP_P[g]];
                             constexpr Place PL = UNIT_W || FEW_SUMS || GRP_P[g + 1] - GRP_P[g] > 1 ? Place::OUT : weight_place(P0);
                             if constexpr (PL == Place::OUT) {
@@ -758,8 +743,7 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                         if constexpr (I_OUT[P] == o) {
                             sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
                                 constexpr int n = n_;
-                                T& g = gzc[c][outer_off<P>() + CG_I[n] * IN2_D[I_IN2[P]] + CG_J[n]];
-                                g = fma((T)CG_V[n], v[CG_K[n]], g);
+                                gzc[c][CG_PR[n]] = fma((T)CG_V[n], v[CG_K[n]], gzc[c][CG_PR[n]]);
                             });
                         }
                     });
@@ -811,19 +795,14 @@ __device__ void slice_backward(const UvuParams& p, unsigned char* smem, int warp
                     sfor<0, N_GROUPS>([&](auto g_) {
                         constexpr int g = g_;
                         if constexpr (GRP_A[g] == a) {
-                            constexpr int b = GRP_B[g], D2 = IN2_D[b];
+                            sfor<GRP_PR[g], GRP_PR[g + 1]>([&](auto s_) {
+                                constexpr int s = s_, i = PR_I[s], j = IN2_OFF[GRP_B[g]] + PR_J[s];
 #pragma unroll
-                            for (int i = 0; i < D1; ++i)
-#pragma unroll
-                                for (int j = 0; j < D2; ++j) {
-                                    const T v = gzc[c][GRP_B0[g] + i * D2 + j];
-#pragma unroll
-                                    for (int q = 0; q < NE; ++q) {
-                                        dx[q][i] = fma(y[q][IN2_OFF[b] + j], v, dx[q][i]);
-                                        T& d = dy[q][IN2_OFF[b] + j];
-                                        d = fma(x[q][i], v, d);
-                                    }
+                                for (int q = 0; q < NE; ++q) {
+                                    dx[q][i] = fma(y[q][j], gzc[c][s], dx[q][i]);
+                                    dy[q][j] = fma(x[q][i], gzc[c][s], dy[q][j]);
                                 }
+                            });
                         }
                     });
                 }

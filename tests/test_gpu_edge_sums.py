@@ -1,0 +1,66 @@
+"""The edge sums of a shared-weight 'uvw' convolution (channel-wise, without weights): sums of products per receiver."""
+import numpy as np
+import pytest
+import torch
+
+import openequivariance_b200 as oeq
+from openequivariance_b200.conv import UVWConvPlan, _UnitWeightConv
+from openequivariance_b200.wigner import cg_nonzeros
+from oracle import tp_oracle as orc
+from helpers import REL_TOL, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _edge_sum(mul, in1, in2, out, dtype=np.float32):
+    wide = lambda irreps: "+".join(f"{mul}x{ir}" for ir in irreps.split("+"))
+    return UVWConvPlan(oeq.FullyConnectedTPProblem(wide(in1), in2, wide(out), irrep_dtype=dtype, weight_dtype=dtype)).edge_sum
+
+
+def _cuda(*arrays):
+    return [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in arrays]
+
+
+def _pairs(p):
+    """[components of a channel of the first input, components of the second]: pairs with a coefficient."""
+    d1 = np.cumsum([0] + [2 * ir.l + 1 for _, ir in p.irreps_in1])
+    d2 = np.cumsum([0] + [2 * ir.l + 1 for _, ir in p.irreps_in2])
+    has = np.zeros((d1[-1], d2[-1]), bool)
+    for t in p.instructions:
+        for i, j, _, _ in cg_nonzeros(p.irreps_in1[t.i_in1].ir.l, p.irreps_in2[t.i_in2].ir.l, p.irreps_out[t.i_out].ir.l):
+            has[d1[t.i_in1] + i, d2[t.i_in2] + j] = True
+    return has
+
+
+def _components(p):
+    """Component of its channel that each value of a first-input row is."""
+    out, d = [], 0
+    for mul, ir in p.irreps_in1:
+        out.append(np.tile(d + np.arange(2 * ir.l + 1), mul))
+        d += 2 * ir.l + 1
+    return np.concatenate(out)
+
+
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("mul,dtype", [(64, np.float32), (32, np.float32), (8, np.float64)])
+def test_infinite_components_stay_with_their_pairs(mul, dtype, deterministic):
+    """An infinite component of one input reaches the gradients of the components that share a coefficient with it only."""
+    p = _edge_sum(mul, "0e+1o+2e", "0e+1o+2e", "0e+1o+2e", dtype)
+    has, comp = _pairs(p), _components(p)
+    nodes, rng = 40, np.random.default_rng(5)
+    rows, cols = np.arange(nodes), np.arange(nodes)[::-1].copy()        # one edge per receiver and per sender
+    x, y, dz = (rng.normal(size=(nodes, r.dim)).astype(dtype) for r in (p.irreps_in1, p.irreps_in2, p.irreps_out))
+    ones = np.ones((nodes, p.weight_numel), dtype)
+    conv = _UnitWeightConv(p, deterministic)
+    index = _cuda(rows, cols) + (_cuda(cols) if deterministic else [])
+    assert not has.all()
+    i0, j0 = np.argwhere(~has)[0]
+    for where, kept_x, kept_y in (("y", ~has[:, j0][comp], np.arange(has.shape[1]) != j0),
+                                  ("x", comp != i0, ~has[i0])):
+        hot, zeroed = {"x": x.copy(), "y": y.copy()}, {"x": x.copy(), "y": y.copy()}
+        at = (slice(None), comp == i0) if where == "x" else (slice(None), j0)
+        hot[where][at], zeroed[where][at] = np.inf, 0
+        dx, dy = conv.backward_helper(*_cuda(hot["x"], hot["y"], dz), *index)
+        rx, ry, _ = orc.conv_backward(p, zeroed["x"], zeroed["y"], ones, dz, rows, cols)
+        assert rel_err(dx.cpu().numpy()[:, kept_x], rx[:, kept_x]) < REL_TOL[dtype]
+        assert rel_err(dy.cpu().numpy()[:, kept_y], ry[:, kept_y]) < REL_TOL[dtype]
