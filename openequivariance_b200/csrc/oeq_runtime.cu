@@ -1173,6 +1173,14 @@ int outer_pairs(const Problem& p) {
     return n;
 }
 
+// Pairs of components that have a coefficient: the products that the edge sums keep.
+int coefficient_pairs(const Problem& p) {
+    std::set<std::tuple<int, int, int, int>> seen;
+    for (const Instr& t : p.instr)
+        for (size_t n = 0; n < t.cv.size(); ++n) seen.insert(std::make_tuple(t.i1, t.i2, t.ci[n], t.cj[n]));
+    return (int)seen.size();
+}
+
 int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
     Mapping& m = k.map;
     if (!slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
@@ -1301,13 +1309,30 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
 // the row sum beside later launches on large lists only, 65 k 886 / 736, 131 k 1451 / 1434, 263 k 2751 / 2828, 1.2 M
 // 11987 / 13138.  128x(0e+1o+2e) in FP64 is within 2 % from 15 k to 66 k edges and 131 k on 1154 / 1256 (atomic).  A row
 // of one slice is the slice kernel's at every size: 32x(0e..3o), 65 k edges 202 / 173, 1.2 M 3552 / 2804.
-bool recv_beside_slice(bool has_slice, const Kernel& slice) { return !has_slice || (slice.map.slice_regs > 200 && slice.map.n_slice > 1); }
+// Edge sums of products (no weights) stay with the slice kernel whatever their registers: 128x(0e+1o+2e) with 0e+1o+2e, 200 k
+// edges atomic 558 / 368, deterministic 792 / 541, 256 channels 992 / 773, 64x(0e..3o) 753 / 310, 128x(0e..3o) 1096 / 658.
+// But FP64 rows of more than 64 channels with few products per value of the row are bound by the additions of an atomic pass,
+// 8 bytes each (the group kernel adds whole rows): 200 k edges, group ~ 130 + 32 x + 6.5 products us for x values per channel of
+// 128, slices ~ 88 x.  128x(0e+1o+2e) with 0e+1o (32 products) 574 / 798, to 0e (4) 433 / 775, with 0e+1o+2e to 0e+1o (37)
+// 638 / 781, 128x(0e+2e) with 0e+2e (34) 499 / 517, 256x(0e+1o) with 0e+1o (10) 628 / 738; on the other side 128x(0e+1o+2e) with
+// 0e+1o+2e (71) 941 / 929, 256x(0e+1o) with 0e+1o+2e (21) 830 / 724, 256x0e (1) 387 / 270.
+bool recv_beside_slice(const Problem& p, bool has_slice, const Kernel& slice, bool deterministic) {
+    if (!has_slice) return true;
+    const Mapping& m = slice.map;
+    if (!m.slice_outer) return m.slice_regs > 200 && m.n_slice > 1;
+    int x = 0;
+    for (const Irrep& r : p.in1) x += r.dim;
+    return !deterministic && p.dtype == OEQ_F64 && m.n_slice * m.slice_cpl > 2 && coefficient_pairs(p) <= 9 * x - 20;
+}
 long long recv_min_edges(bool deterministic) { return env_int("OEQ_B200_RECV_MIN_EDGES", deterministic ? 196608 : 49152); }
 
 // Wide FP64 rows in the forward pass: the slice kernel gathers every row once per slice of 32 channels, which
 // costs once the rows no longer fit in L2.  128x(0e+1o+2e), group / slice kernel, atomic: 5 000 nodes (46 MB) 695 / 636 us,
 // 10 000 (92 MB) 1252 / 1277, 20 000 2422 / 2730; deterministic 659 / 592, 1159 / 1171, 2330 / 2422.
-bool group_forward_beside_slice(const Problem& p, const Kernel& slice) { return p.dtype == OEQ_F64 && slice.map.slice_regs > 160 && slice.map.n_slice > 2; }
+// (Edge sums of products read rows once per 32 channels too, but compute less: 128x(0e+1o+2e), 20 000 nodes, 2508 / 1373.)
+bool group_forward_beside_slice(const Problem& p, const Kernel& slice) {
+    return p.dtype == OEQ_F64 && !slice.map.slice_outer && slice.map.slice_regs > 160 && slice.map.n_slice > 2;
+}
 constexpr size_t GROUP_FORWARD_BYTES = 64u << 20;
 
 // Problems for which fused second derivatives may exist (whether they fit is known once they are built).
@@ -2022,7 +2047,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if ((rf || group_forward_beside_slice(p, f)) && (rc = one(det ? K_FWD_DET : K_FWD_ATOMIC))) return rc;
         if ((rc = one(det ? K_BWD_DET : K_BWD_ATOMIC))) return rc;
         if (tc && (rc = build_uvu_tc(p, det != 0, k))) return rc;
-        if (recv && recv_beside_slice(!rb, b) && (rc = build_uvu_recv(p, det != 0, kr))) return rc;
+        if (recv && recv_beside_slice(p, !rb, b, det != 0) && (rc = build_uvu_recv(p, det != 0, kr))) return rc;
     }
     if ((kinds & 8) && (kinds & 6) && conv_second_possible(p)) {
         for (int det = 0; det < 2; ++det) {
@@ -2602,7 +2627,7 @@ int oeq_conv_create(const oeq_problem_desc* desc, int deterministic, oeq_conv** 
         h->has_fwd_tc = !rc;
     }
     if (!rc) optional(build_slice_bwd(h->prob, h->deterministic, h->bwd_slice), h->has_bwd_slice);
-    if (!rc && recv_beside_slice(h->has_bwd_slice, h->bwd_slice) && recv_backward_supported(h->prob)) {
+    if (!rc && recv_beside_slice(h->prob, h->has_bwd_slice, h->bwd_slice, h->deterministic) && recv_backward_supported(h->prob)) {
         rc = build_uvu_recv(h->prob, h->deterministic, h->bwd_recv);
         h->has_bwd_recv = !rc;
     }

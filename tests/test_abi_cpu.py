@@ -81,3 +81,29 @@ def test_kernels_specialise_without_a_gpu(tmp_path):
         assert sorted(os.listdir(tmp_path)) == files
     finally:
         lib.oeq_set_cache_dir(os.path.join(os.path.dirname(_native.library_path()), "_kcache").encode())
+
+
+@pytest.mark.parametrize("mul,in1,in2,dtype,atomic,kernels", [
+    (128, "0e+1o+2e", "0e+1o+2e", "float32", True, 3),      # forward and backward in slices, the sender-order kernel behind
+    (128, "0e+1o+2e", "0e+1o+2e", "float32", False, 3),
+    (64, "0e+1o+2e+3o", "0e+1o+2e", "float32", False, 3),
+    (128, "0e+1o+2e", "0e+1o+2e", "float64", False, 3),
+    (128, "0e+1o+2e", "0e+1o", "float64", False, 3),
+    (128, "0e+1o+2e", "0e+1o", "float64", True, 4),         # the additions of wide FP64 rows: receiver-order kernel for large lists
+    (64, "0e+1o+2e", "0e+1o", "float64", True, 3),
+    (128, "0e+1o", "0e+1o+2e", "float64", True, 3),
+])
+def test_edge_sums_leave_large_lists_to_the_slice_kernels(tmp_path, mul, in1, in2, dtype, atomic, kernels):
+    """Group kernels for large lists are specialised where they are the faster ones, which sums of products hardly ever are."""
+    import openequivariance_b200 as oeq
+    from openequivariance_b200 import _native
+    from openequivariance_b200.conv import UVWConvPlan
+    wide, dt = "+".join(f"{mul}x{ir}" for ir in in1.split("+")), getattr(np, dtype)
+    p = oeq.FullyConnectedTPProblem(wide, in2, wide, irrep_dtype=dt, weight_dtype=dt)
+    lib = _native.lib()
+    lib.oeq_set_cache_dir(str(tmp_path).encode())
+    try:
+        _native.precompile(UVWConvPlan(p).edge_sum, _native.KIND_CONV_ATOMIC if atomic else _native.KIND_CONV_DET, unit_weights=True)
+        assert len(os.listdir(tmp_path)) == kernels
+    finally:
+        lib.oeq_set_cache_dir(os.path.join(os.path.dirname(_native.library_path()), "_kcache").encode())
