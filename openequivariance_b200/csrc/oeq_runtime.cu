@@ -1160,6 +1160,9 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
     return false;
 }
 
+// Estimated registers up to which edge sums keep products per receiver, though that may leave fewer warps than the per-edge form:
+// 800 k edges, per edge / sums, forward, 64x(0e+1o+2e) with 0e..3o (16 against 8 warps per SM) 681 / 534 us, FP64 with 0e+1o+2e
+// (12 against 8) 878 / 705; backward, FP64 32x(0e+1o+2e) with 0e+1o 842 / 847, 128x(0e+1o) with 0e+1o+2e 1736 / 1422.
 constexpr int OUTER_REGS = 240;
 
 // Pairs of first- and second-input components of a channel, of the irreps that have a path: the measure of the register
@@ -1181,6 +1184,18 @@ int coefficient_pairs(const Problem& p) {
     return (int)seen.size();
 }
 
+// The forward sums of products save the coefficient FMAs and the additions to the row, but take one edge at a time where the
+// per-edge form of FP32 packs two: twice the reads of Y and about 20 operations per edge are lost.  800 k edges of 64 channels,
+// per edge / sums of products: 64x(0e+1o+2e) to a scalar 220 / 261 us (12 operations saved), 0e+1o with 0e+1o 171 / 187 (18), with
+// 0e+1o+2e to 0e+1o 206 / 228 (32, and 9 values of Y), 0e+1o+2e with 0e 226 / 240 (18); 0e+1o with 0e+1o to 0e+1o+2e 204 / 202 (34),
+// 0e+1o+2e with 0e+1o+2e to 0e+1o 306 / 308 (52), with 0e+1o 314 / 292 (58).  FP64 has no packed form: 0e+1o 240 / 225.
+bool outer_forward_pays(const Problem& p) {
+    if (p.dtype == OEQ_F64) return true;
+    int saved = 0;
+    for (const Instr& t : p.instr) saved += (int)t.cv.size() + p.out[t.io].dim;
+    return saved > 2 * p.y_dim + 20;
+}
+
 int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
     Mapping& m = k.map;
     if (!slice_shape(p, m)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not have the shape of the slice kernels");
@@ -1197,7 +1212,7 @@ int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
     const int w = p.elem() / 4;
     int regs = zpc * w + 2 * (p.y_dim + d1 + tmax) + 24;
     const int outer = w * (outer_pairs(p) + p.y_dim + d1) + 28;
-    m.slice_outer = p.unit && outer <= OUTER_REGS;
+    m.slice_outer = p.unit && outer <= OUTER_REGS && outer_forward_pays(p);
     if (m.slice_outer) regs = outer;
     if (!slice_fit(p, m, regs, pad16(32 * d3 * p.elem()), 0)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
     m.mulg = 32;

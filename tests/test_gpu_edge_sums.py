@@ -8,6 +8,7 @@ from openequivariance_b200.conv import UVWConvPlan, _UnitWeightConv
 from openequivariance_b200.wigner import cg_nonzeros
 from oracle import tp_oracle as orc
 from helpers import REL_TOL, rel_err
+from test_gpu_slice_conv import DEGREES, _unaligned
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,37 @@ def test_infinite_components_stay_with_their_pairs(mul, dtype, deterministic):
         rx, ry, _ = orc.conv_backward(p, zeroed["x"], zeroed["y"], ones, dz, rows, cols)
         assert rel_err(dx.cpu().numpy()[:, kept_x], rx[:, kept_x]) < REL_TOL[dtype]
         assert rel_err(dy.cpu().numpy()[:, kept_y], ry[:, kept_y]) < REL_TOL[dtype]
+
+
+# Both sides of the lines between the forms: per edge or sums of products, one or two channels per lane, rows of at most 32
+# channels, one slice and several; FP64 with and without sums in the backward pass.
+E1, E2, E3 = "0e+1o", "0e+1o+2e", "0e+1o+2e+3o"
+WALKS = [(8, E1, E1, E1, np.float32), (20, E2, E2, E2, np.float32), (32, E1, E1, E2, np.float32), (64, E2, E2, "0e", np.float32),
+         (64, E3, E2, E3, np.float32), (96, E2, E2, E2, np.float32), (128, E2, E2, E2, np.float32), (256, E2, E2, E2, np.float32),
+         (8, E1, E1, E1, np.float64), (24, E2, E2, E2, np.float64), (64, E1, E1, E1, np.float64), (128, E1, E2, E1, np.float64)]
+
+
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("graph", ["one_edge", "runs", "many"])
+@pytest.mark.parametrize("mul,in1,in2,out,dtype", WALKS)
+def test_walk(mul, in1, in2, out, dtype, graph, deterministic):
+    p = _edge_sum(mul, in1, in2, out, dtype)
+    degrees = np.array(DEGREES[graph] if graph != "many" else DEGREES[graph][:90])
+    nodes, edges = len(degrees), int(degrees.sum())
+    rng = np.random.default_rng(edges)
+    rows, cols, _, perm = orc.coord_graph(np.repeat(np.arange(nodes), degrees), rng.integers(0, nodes, edges))
+    x, y, dz = (rng.normal(size=(n, r.dim)).astype(dtype) for n, r in ((nodes, p.irreps_in1), (edges, p.irreps_in2), (nodes, p.irreps_out)))
+    ones = np.ones((edges, p.weight_numel), dtype)
+    want = [orc.conv_forward(p, x, y, ones, rows, cols), *orc.conv_backward(p, x, y, ones, dz, rows, cols)[:2]]
+    conv = _UnitWeightConv(p, deterministic)
+    index = _cuda(rows, cols) + (_cuda(perm) if deterministic else [])
+    plain = None
+    for wrap in (lambda t: t, _unaligned):
+        xt, yt, dzt = (wrap(t) for t in _cuda(x, y, dz))
+        got = [conv.forward(xt, yt, *index), *conv.backward_helper(xt, yt, dzt, *index)]
+        conv.internal.check()
+        for g, r in zip(got, want):
+            assert rel_err(g.cpu().numpy(), r) < REL_TOL[dtype]
+        if deterministic and plain is not None:     # copies in pieces or in elements: the same sums
+            assert all(torch.equal(a, b) for a, b in zip(got, plain))
+        plain = got
