@@ -1133,8 +1133,8 @@ bool slice_shape(const Problem& p, Mapping& m) {
 }
 
 // Warps per SM by the registers a thread needs (65 536 over the warps, in steps of the warps that share a
-// scheduler), stages by shared memory.
-bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_bytes, bool second = false) {
+// scheduler), stages by shared memory.  `room`: registers to leave room for, where the estimate falls short.
+bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_bytes, bool second = false, int room = 0) {
     const int e = p.elem();
     int xch = 0;
     for (const Irrep& r : p.in1) xch += r.dim;
@@ -1144,7 +1144,7 @@ bool slice_fit(const Problem& p, Mapping& m, int regs, int warp_bytes, int cta_b
     const int stage = 16 + (second ? 2 : 1) * (pad16(ep * p.y_dim * e) + ep * xs + ep * ws);     // (rows and cotangent rows)
     if (regs > 256) return false;
     m.slice_regs = regs;
-    const int target = env_int("OEQ_B200_SLICE_WARPS_SM", regs <= 124 ? 16 : (regs <= 164 ? 12 : 8));
+    const int target = env_int("OEQ_B200_SLICE_WARPS_SM", std::max(regs, room) <= 124 ? 16 : (std::max(regs, room) <= 164 ? 12 : 8));
     m.slice_warps = m.n_slice * std::max(1, 4 / m.n_slice);
     if (m.slice_warps > 8) m.slice_warps = m.n_slice;
     for (int ctas = std::max(1, target / m.slice_warps); ctas >= 1; --ctas)
@@ -1259,7 +1259,15 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     if (per * p.y_dim > 32) pitch = (per * p.y_dim + 31) / 32 * 32;
     const int groups = m.n_slice >= 4 ? 1 : 4 / m.n_slice;
     const int dyg = m.n_slice > 1 ? 2 * m.n_slice * pitch * e : 0;
-    if (!slice_fit(p, m, regs, 32 * pitch * e, groups * dyg)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+    // FP64 rows with weights of their own take up to 1.6 times the estimate; with more warps they spill to an L1 that shared memory
+    // leaves little of (16x(0e+1o+2e) with 0e+1o+2e: 108 bytes a thread).  200 k edges, atomic, 16 / 12 / 8 warps per SM (what
+    // narrow rows have the shared memory for): 8x(0e+1o+2e) with 0e+1o+2e (estimate 158, 35 sums of the receiver)
+    // 499 / 316 / 237 us, 8x(0e..3o) with 0e+1o (156, 40) 546 / 290 / 230, 8x(1o+2e) with 0e+1o+2e (136, 24) 280 / 210 / 179; with
+    // 0e..3o to 8x(0e+1o) (156, 18) 359 / 196 / 208; 8x(0e+1o) with 0e+1o+2e to 8x(0e+1o+2e) (118, 21) 206 / 140 / 159, 8x(0e+2e)
+    // with 0e+2e (110, 17) 177 / 138 / 157; 8x(0e+1o+2e) with 0e+1o (106, 21) 138 / 146 / 165.
+    int room = 0;
+    if (e == 8 && !p.unit) room = regs > 134 && zpc >= 24 ? 256 : (regs > 108 ? 126 : 0);
+    if (!slice_fit(p, m, regs, 32 * pitch * e, groups * dyg, false, room)) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
     m.mulg = 32;
     m.z_ph_begin = {0, p.z_dim};
     m.w_ph_begin = {0, p.w_numel};

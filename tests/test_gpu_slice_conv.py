@@ -33,7 +33,22 @@ def _unaligned(t):
                                         ("nequip_32", np.float64), ("mace_128", np.float32), ("mace_large_128", np.float32)])
 @pytest.mark.parametrize("graph", sorted(DEGREES))
 def test_walk(name, dtype, graph, deterministic):
-    p = problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype)
+    _check_walk(problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype), dtype, graph, deterministic)
+
+
+# eight warps per SM, twelve (two estimates), sixteen
+NARROW = [("16x0e+16x1o+16x2e", "0e+1o+2e", "16x0e+16x1o+16x2e"), ("8x0e+8x1o", "0e+1o+2e", "8x0e+8x1o+8x2e"),
+          ("8x0e+8x1o+8x2e", "0e+1o+2e+3o", "8x0e+8x1o"), ("8x0e+8x1o+8x2e", "0e+1o", "8x0e+8x1o+8x2e")]
+
+
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("irreps", NARROW, ids=[" ".join(i) for i in NARROW])
+def test_narrow_double_rows(irreps, deterministic):
+    p = oeq.ChannelwiseTPP(*irreps, irrep_dtype=np.float64, weight_dtype=np.float64)
+    _check_walk(p, np.float64, "many", deterministic)
+
+
+def _check_walk(p, dtype, graph, deterministic):
     degrees = np.array(DEGREES[graph])
     nodes, edges = len(degrees), int(degrees.sum())
     rng = np.random.default_rng(edges)
