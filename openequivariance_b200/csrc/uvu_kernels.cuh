@@ -262,6 +262,20 @@ __device__ __forceinline__ void cg_backward(const XA& x, const YA& y, const GA& 
 // the inputs exchanged where the second one is smaller.  128x(0e..3o), receiver-order pass, 300 k edges: 2.68 -> 2.52 ms.
 template <int P, class XA, class YA, class GA, class DX, class DY>
 __device__ __forceinline__ T cg_backward_w(T w, const XA& x, const YA& y, const GA& g, DX& dx, DY& dy) {
+    if constexpr (ELEM == 8) {
+        // FP64, whose registers are short: the sums of the two inputs side by side, the weight on both.  128x0e+64x1o+32x2e with
+        // 0e+1o+2e, deterministic, 200 k edges 2 086 us, with the weight on the smaller input 2 319; 30 k edges 452 / 499.
+        T av[IN1_D[I_IN1[P]]] = {}, bv[IN2_D[I_IN2[P]]] = {}, tw = (T)0;
+        cg_backward<P>(x, y, g, av, bv);
+#pragma unroll
+        for (int i = 0; i < IN1_D[I_IN1[P]]; ++i) {
+            tw = fma(x[i], av[i], tw);
+            dx[i] = fma(w, av[i], dx[i]);
+        }
+#pragma unroll
+        for (int j = 0; j < IN2_D[I_IN2[P]]; ++j) dy[j] = fma(w, bv[j], dy[j]);
+        return tw;
+    }
     constexpr bool W1 = IN1_D[I_IN1[P]] <= IN2_D[I_IN2[P]];
     constexpr int DM = W1 ? IN1_D[I_IN1[P]] : IN2_D[I_IN2[P]];
     T v[DM], s[DM], pij = (T)0, tw = (T)0;

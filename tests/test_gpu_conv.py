@@ -56,6 +56,15 @@ def test_fp64(deterministic):
     check_conv(p, 40, rows, cols, 10, deterministic, dtype=np.float64)
 
 
+@pytest.mark.parametrize("deterministic", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_unequal_multiplicities(dtype, deterministic):
+    """Rows that no slice kernel takes: the receiver-order kernel, whose FP32 and FP64 forms place the weight differently."""
+    p = oeq.ChannelwiseTPP("48x0e+32x1o+16x2e", "0e+1o+2e", "48x0e+32x1o+16x2e", irrep_dtype=dtype, weight_dtype=dtype)
+    rows, cols = random_graph(31, 400, seed=4)
+    check_conv(p, 31, rows, cols, 11, deterministic, dtype=dtype)
+
+
 @pytest.mark.parametrize("name,dtype,deterministic,epi", [("nequip_32", np.float32, True, 4), ("nequip_32", np.float32, False, 3),
                                                          ("readme", np.float64, True, 3), ("readme", np.float32, False, 4)])
 def test_edges_per_item(name, dtype, deterministic, epi, monkeypatch):
