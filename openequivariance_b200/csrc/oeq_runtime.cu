@@ -1292,10 +1292,15 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
     for (const Irrep& r : p.in2) d2 = std::max(d2, r.dim);
     const int e = p.elem(), w = e / 4;
     // A stage of two edges and their cotangents, or of one: where two leave shared memory for fewer warps than the registers do
-    // (FP64), or computing two together takes too many registers (FP32).  FP64, deterministic, forward and both derivatives:
-    // 128x(0e+1o+2e) x (0e..3o), 1 000 nodes / 28 k edges 1 308 -> 1 157 us; 32x(0e+1o+2e), 3 000 / 111 k 980 -> 889.  FP32
-    // 128x(0e..3o), group kernel before: 1 000 / 30 k 1 954 -> 1 418, 6 000 / 180 k 9 535 -> 7 887.  Where two edges fit with the
-    // same warps they are faster: 8x(0e+1o) 482 against 521, FP64 270 against 286; FP32 128x(0e+1o+2e) 1 133 against 1 136.
+    // (FP64), or computing two together takes too many registers (FP32).  Forward and both derivatives, FP64, deterministic:
+    // 128x(0e+1o+2e) x (0e..3o), 1 000 nodes / 28 k edges 1 304 -> 1 162 us; 32x(0e+1o+2e), 3 000 / 111 k 977 -> 894; FP32
+    // 128x(0e..3o), group kernel before, 1 000 / 30 k 1 922 -> 1 419.  The two launches alone, FP32 128x(0e..3o), group / slices,
+    // 30 k edges 1406 / 933, 990 k 36 405 / 28 975, atomic 36 913 / 27 106; 96 channels (six warps) 30 k 1122 / 900, 600 k 15 723 / 16 962.
+    // Not where two edges have three warps per scheduler already (FP64 96x(0e+1o), 196 k edges, two / one edges 905 / 947), nor,
+    // in the deterministic forward walk of rows of one slice, two: each warp takes a run there, and twice the warps leave more of
+    // them with one receiver more than others (16x(0e+1o+2e), 28 k edges 138 / 178, 196 k 634 / 863; 20x(0e+1o+2e) x (0e+1o) 105 / 122).
+    // Nor for FP64 rows that two edges do not fit at all and one leaves with few warps: 160x(0e+1o+2e) x (0e..3o), group / one
+    // edge with five warps, 28 k edges 851 / 1151, 196 k 5947 / 8391.
     auto fit = [&](bool one) {
         const int per = one ? 1 : 3 - w;        // edges computed together
         m.slice_one = one;
@@ -1311,8 +1316,10 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
     if (!pair || w == 2) {
         const Mapping two = m;
         const bool one = fit(true);
-        if (!one && !pair) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
-        if (!one || (pair && m.min_ctas * m.slice_warps <= two.min_ctas * two.slice_warps)) m = two;
+        const int warps1 = m.min_ctas * m.slice_warps, warps2 = two.min_ctas * two.slice_warps;
+        const bool keep = pair && warps2 >= (deterministic && !grads && m.n_slice == 1 ? 8 : 12);
+        if (!pair && (!one || (w == 2 && warps1 < 8))) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+        if (!one || (pair && (keep || warps1 <= warps2))) m = two;
     }
     m.mulg = 32;
     m.z_ph_begin = {0, p.z_dim};

@@ -186,7 +186,8 @@ def test_autograd_and_double_backward():
 def test_fused_second_derivatives(name, dtype, tol, deterministic):
     """Second derivatives in two fused launches (taken when nothing differentiates through the result) against
     the oracle's autograd and against the composed path (four backward and three forward launches)."""
-    p = problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype)
+    kw = dict(irrep_dtype=dtype, weight_dtype=dtype)
+    p = problem_by_name(name, **kw) if isinstance(name, str) else oeq.ChannelwiseTPP(*name, **kw)
     nodes = 40
     rows, cols = random_graph(nodes, 700, seed=21)
     rows, cols, order, perm = orc.coord_graph(rows, cols)
@@ -230,6 +231,14 @@ def test_fused_second_derivatives_one_edge(name, dtype, tol, deterministic):
     """Rows whose second derivatives take one edge at a time: wide ones, and FP64 where that leaves room for more warps (the
     last problem keeps two edges per stage)."""
     test_fused_second_derivatives(name, dtype, tol, deterministic)
+
+
+@pytest.mark.parametrize("deterministic", [True, False])
+@pytest.mark.parametrize("mul", [16, 24, 160])
+def test_fused_second_derivatives_double_rows(mul, deterministic):
+    """FP64 on either side of the line between one and two edges per stage, and a row that the group kernel takes."""
+    irreps = f"{mul}x0e+{mul}x1o+{mul}x2e"
+    test_fused_second_derivatives((irreps, "0e+1o+2e+3o" if mul > 32 else "0e+1o+2e", irreps), np.float64, 1e-11, deterministic)
 
 
 def test_fused_second_derivatives_staging_variants(monkeypatch):
