@@ -1299,8 +1299,6 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
     // Not where two edges have three warps per scheduler already (FP64 96x(0e+1o), 196 k edges, two / one edges 905 / 947), nor,
     // in the deterministic forward walk of rows of one slice, two: each warp takes a run there, and twice the warps leave more of
     // them with one receiver more than others (16x(0e+1o+2e), 28 k edges 138 / 178, 196 k 634 / 863; 20x(0e+1o+2e) x (0e+1o) 105 / 122).
-    // Nor for FP64 rows that two edges do not fit at all and one leaves with few warps: 160x(0e+1o+2e) x (0e..3o), group / one
-    // edge with five warps, 28 k edges 851 / 1151, 196 k 5947 / 8391.
     auto fit = [&](bool one) {
         const int per = one ? 1 : 3 - w;        // edges computed together
         m.slice_one = one;
@@ -1318,7 +1316,7 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
         const bool one = fit(true);
         const int warps1 = m.min_ctas * m.slice_warps, warps2 = two.min_ctas * two.slice_warps;
         const bool keep = pair && warps2 >= (deterministic && !grads && m.n_slice == 1 ? 8 : 12);
-        if (!pair && (!one || (w == 2 && warps1 < 8))) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
+        if (!pair && !one) return fail(OEQ_ERR_UNSUPPORTED, "problem does not fit the slice kernels");
         if (!one || (pair && (keep || warps1 <= warps2))) m = two;
     }
     m.mulg = 32;

@@ -200,6 +200,7 @@ def test_fused_second_derivatives(name, dtype, tol, deterministic):
     xt, yt, wt, dzt = (t.requires_grad_(True) for t in cuda(x, y, w, dz))
     rng = np.random.default_rng(23)
     ex, ey, ew = (torch.from_numpy(rng.normal(size=a.shape).astype(dtype)).cuda() for a in (x, y, w))
+    assert conv._fused_second(*(t.detach() for t in (xt, yt, wt, dzt)), ex, ey, ew, *index) is not None
 
     def second(create_graph):
         z = conv.forward(xt, yt, wt, *index)
@@ -236,7 +237,7 @@ def test_fused_second_derivatives_one_edge(name, dtype, tol, deterministic):
 @pytest.mark.parametrize("deterministic", [True, False])
 @pytest.mark.parametrize("mul", [16, 24, 160])
 def test_fused_second_derivatives_double_rows(mul, deterministic):
-    """FP64 on either side of the line between one and two edges per stage, and a row that the group kernel takes."""
+    """FP64 on either side of the line between one and two edges per stage, and a row that two edges do not fit at all."""
     irreps = f"{mul}x0e+{mul}x1o+{mul}x2e"
     test_fused_second_derivatives((irreps, "0e+1o+2e+3o" if mul > 32 else "0e+1o+2e", irreps), np.float64, 1e-11, deterministic)
 
