@@ -260,11 +260,12 @@ __device__ __forceinline__ void cg_backward(const XA& x, const YA& y, const GA& 
 // The same with the weight on the smaller input: with w x in dY's sums, s_i = sum_j y_j P_ij gives dW = <x, s> and
 // dX += w s, three operations per value of the first input (two for each and one per value of the second input otherwise);
 // the inputs exchanged where the second one is smaller.  128x(0e..3o), receiver-order pass, 300 k edges: 2.68 -> 2.52 ms.
-template <int P, class XA, class YA, class GA, class DX, class DY>
+// BOTH: sums of either input side by side, the weight on both (for FP64 in the deterministic kernel, whose helper warps leave the
+// fewest registers: 128x0e+64x1o+32x2e with 0e+1o+2e, 200 k edges 2 086 us, with the weight on the smaller input 2 319; atomic, without
+// helper warps, 1 428 and 1 398).
+template <int P, bool BOTH, class XA, class YA, class GA, class DX, class DY>
 __device__ __forceinline__ T cg_backward_w(T w, const XA& x, const YA& y, const GA& g, DX& dx, DY& dy) {
-    if constexpr (ELEM == 8) {
-        // FP64, whose registers are short: the sums of the two inputs side by side, the weight on both.  128x0e+64x1o+32x2e with
-        // 0e+1o+2e, deterministic, 200 k edges 2 086 us, with the weight on the smaller input 2 319; 30 k edges 452 / 499.
+    if constexpr (BOTH) {
         T av[IN1_D[I_IN1[P]]] = {}, bv[IN2_D[I_IN2[P]]] = {}, tw = (T)0;
         cg_backward<P>(x, y, g, av, bv);
 #pragma unroll
@@ -1624,7 +1625,7 @@ __device__ void run_backward_recv(const UvuParams& p, const Smem<true, MODE, tru
                                 cg_backward<P>(x, &yr[IN2_OFF[b]], gs, dxa, dyb);
                             } else {
                                 const T w = live ? sWt[weight_offset<P>(u, 0)] : (T)0;
-                                const T tw = cg_backward_w<P>(w, x, &yr[IN2_OFF[b]], gs, dxa, dyb);
+                                const T tw = cg_backward_w<P, ELEM == 8 && MODE == MODE_DET>(w, x, &yr[IN2_OFF[b]], gs, dxa, dyb);
                                 if (live) __stcs(dwrow + weight_offset<P>(u, 0), tw);
                             }
                         };
