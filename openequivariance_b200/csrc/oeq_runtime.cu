@@ -1184,6 +1184,15 @@ int coefficient_pairs(const Problem& p) {
     return (int)seen.size();
 }
 
+// FP64 edge sums with few products per value of the row: an atomic backward pass is bound by its additions, 8 bytes each.  For
+// x values per channel (128 channels, 200 k edges) it takes ~ 88 x us, the group kernel, which adds whole rows, ~ 130 + 32 x + 6.5
+// per product.
+bool bound_by_additions(const Problem& p) {
+    int x = 0;
+    for (const Irrep& r : p.in1) x += r.dim;
+    return p.dtype == OEQ_F64 && coefficient_pairs(p) <= 9 * x - 20;
+}
+
 // The forward sums of products save the coefficient FMAs and the additions to the row, but take one edge at a time where the
 // per-edge form of FP32 packs two: twice the reads of Y and about 20 operations per edge are lost.  800 k edges of 64 channels,
 // per edge / sums of products: 64x(0e+1o+2e) to a scalar 220 / 261 us (12 operations saved), 0e+1o with 0e+1o 171 / 187 (18), with
@@ -1228,7 +1237,10 @@ int build_slice_fwd(const Problem& p, bool deterministic, Kernel& k) {
 
 // Backward edge sums of rows of 64, 128 ... channels: two channels per lane share the walk, the second input and the sum of dY.
 // 64x(0e+1o+2e), 400 k edges, forward and backward 1 028 -> 1 010 us; the forward pass alone gains 9 of 269 us there but loses
-// 2 of 30 us on graphs of some hundred edges (fewer, longer walks) and keeps one channel.
+// 2 of 30 us on graphs of some hundred edges (fewer, longer walks) and keeps one channel.  One / two channels, 800 k edges: FP32
+// 256x(0e+1o+2e) 3947 / 3085, 64x(0e+1o) 357 / 290; FP64 64x(0e+1o) with 0e+1o, deterministic, 935 / 753, 128x(0e+1o) with 0e+1o+2e,
+// atomic, 1760 / 1422, 64x(0e+1o+2e) with 0e+1o, deterministic, 1707 / 1595.  Not where an atomic pass waits for its additions and
+// would have fewer warps to wait with: the last one, atomic, 1607 / 1687; with 0e+1o+2e to 0e+1o, 200 k edges, 390 / 415.
 bool two_channels_per_lane(Mapping& m, int regs) {
     if (!m.slice_full || m.n_slice % 2 || regs > OUTER_REGS) return false;
     m.slice_cpl = 2;
@@ -1250,7 +1262,8 @@ int build_slice_bwd(const Problem& p, bool deterministic, Kernel& k) {
     m.slice_outer = p.unit && outer <= OUTER_REGS;
     if (m.slice_outer) regs = outer;
     const int two = w * (2 * outer_pairs(p) + 2 * p.y_dim + 4 * d1) + 24;
-    if (m.slice_outer && two_channels_per_lane(m, two)) {
+    const bool waits = !deterministic && two > 164 && bound_by_additions(p);
+    if (m.slice_outer && !waits && two_channels_per_lane(m, two)) {
         regs = two;
         per = 1;
     }
@@ -1339,18 +1352,15 @@ int build_slice_dbl(const Problem& p, bool deterministic, bool grads, Kernel& k)
 // of one slice is the slice kernel's at every size: 32x(0e..3o), 65 k edges 202 / 173, 1.2 M 3552 / 2804.
 // Edge sums of products (no weights) stay with the slice kernel whatever their registers: 128x(0e+1o+2e) with 0e+1o+2e, 200 k
 // edges atomic 558 / 368, deterministic 792 / 541, 256 channels 992 / 773, 64x(0e..3o) 753 / 310, 128x(0e..3o) 1096 / 658.
-// But FP64 rows of more than 64 channels with few products per value of the row are bound by the additions of an atomic pass,
-// 8 bytes each (the group kernel adds whole rows): 200 k edges, group ~ 130 + 32 x + 6.5 products us for x values per channel of
-// 128, slices ~ 88 x.  128x(0e+1o+2e) with 0e+1o (32 products) 574 / 798, to 0e (4) 433 / 775, with 0e+1o+2e to 0e+1o (37)
+// But FP64 rows of more than 64 channels that are bound by their additions: 128x(0e+1o+2e) with 0e+1o (32 products) 574 / 798,
+// to 0e (4) 433 / 775, with 0e+1o+2e to 0e+1o (37)
 // 638 / 781, 128x(0e+2e) with 0e+2e (34) 499 / 517, 256x(0e+1o) with 0e+1o (10) 628 / 738; on the other side 128x(0e+1o+2e) with
 // 0e+1o+2e (71) 941 / 929, 256x(0e+1o) with 0e+1o+2e (21) 830 / 724, 256x0e (1) 387 / 270.
 bool recv_beside_slice(const Problem& p, bool has_slice, const Kernel& slice, bool deterministic) {
     if (!has_slice) return true;
     const Mapping& m = slice.map;
     if (!m.slice_outer) return m.slice_regs > 200 && m.n_slice > 1;
-    int x = 0;
-    for (const Irrep& r : p.in1) x += r.dim;
-    return !deterministic && p.dtype == OEQ_F64 && m.n_slice * m.slice_cpl > 2 && coefficient_pairs(p) <= 9 * x - 20;
+    return !deterministic && m.n_slice * m.slice_cpl > 2 && bound_by_additions(p);
 }
 long long recv_min_edges(bool deterministic) { return env_int("OEQ_B200_RECV_MIN_EDGES", deterministic ? 196608 : 49152); }
 
