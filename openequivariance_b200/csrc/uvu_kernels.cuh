@@ -255,9 +255,7 @@ __device__ __forceinline__ void cg_backward(const XA& x, const YA& y, const GA& 
     });
 }
 
-// Second-derivative form of the above (convolution): with r = w ex + ew x,
-//   ay_i += y_j P_ij;  aey_i += ey_j P_ij;  b_j += r_i P_ij.
-// The same with the weight on the smaller input: with w x in dY's sums, s_i = sum_j y_j P_ij gives dW = <x, s> and
+// The first derivatives with the weight on the smaller input: with w x in dY's sums, s_i = sum_j y_j P_ij gives dW = <x, s> and
 // dX += w s, three operations per value of the first input (two for each and one per value of the second input otherwise);
 // the inputs exchanged where the second one is smaller.  128x(0e..3o), receiver-order pass, 300 k edges: 2.68 -> 2.52 ms.
 // BOTH: sums of either input side by side, the weight on both (for FP64 in the deterministic kernel, whose helper warps leave the
@@ -303,6 +301,9 @@ __device__ __forceinline__ T cg_backward_w(T w, const XA& x, const YA& y, const 
     }
     return tw;
 }
+
+// Second-derivative form of the above (convolution): with r = w ex + ew x,
+//   ay_i += y_j P_ij;  aey_i += ey_j P_ij;  b_j += r_i P_ij.
 template <int P, class RA, class YA, class EA, class GA, class AA, class BA>
 __device__ __forceinline__ void cg_backward_dbl(const RA& r, const YA& y, const EA& ey, const GA& g, AA& ay, AA& aey, BA& b) {
     T pij = (T)0;

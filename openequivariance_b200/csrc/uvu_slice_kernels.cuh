@@ -5,9 +5,10 @@
 // warp is on its own: it walks edges in receiver order, copies *its* 32 channels of the rows ahead with 16-byte
 // cp.async (no staging warp, no barrier wider than a warp, so no third warp on a scheduler caps the registers) and
 // takes two edges of one receiver at a time.
-//   * FP32: the two edges are the two halves of packed registers (fma.rn.f32x2).  A product x_i y_j and a
-//     coefficient FMA are one issue slot for both edges, coefficients stay immediates, and a packed operand always
-//     reads one register of either bank, so the bank conflicts of the scalar code disappear.
+//   * FP32: the two edges are the two halves of packed registers.  Products, and the coefficient FMAs of paths that take their
+//     weight on the result, are one packed instruction for both edges (fma.rn.f32x2, two cycles of a scheduler's dispatch);
+//     where the weight is on an input the coefficient FMAs go straight to the receiver's row, one scalar FMA with an immediate
+//     for each edge.
 //   * Products x_i y_j are formed once for all paths that share the two input irreps (E_* tables).
 //   * FP64: the same code with one edge at a time.
 // The walk deals chunks of consecutive edges round robin, so that gathered rows are shared in L2.
@@ -78,7 +79,7 @@ template <class U> struct Pack<U, true> {
 typedef Pack<T, ONE_EDGE> PK;
 typedef PK::V V2;
 
-// ---- slice layout of a staged pair: X and W of both edges, Y (FP32: interleaved, element j of edge h at 2j + h)
+// ---- slice layout of a stage: X and W of its two edges, or one, and Y (packed pairs: interleaved, element j of edge h at 2j + h)
 __host__ __device__ constexpr int sum_in1_d(int n) { int s = 0; for (int a = 0; a < n; ++a) s += IN1_D[a]; return s; }
 constexpr int EP = SLICE_ONE ? 1 : 2;                               // edges of a stage
 constexpr int X_CH = sum_in1_d(N_IN1);                              // X values per channel
@@ -93,7 +94,7 @@ struct SliceStage {
     static constexpr int OFF_HDR = 0;           // first edge, receiver, sender of edge 0, sender of edge 1 (-1: one edge)
     static constexpr int OFF_Y = 16;
     static constexpr int OFF_EY = OFF_Y + YSB;  // (second derivatives: the cotangent rows beside the rows)
-    static constexpr int OFF_X = OFF_EY + (DBLC ? YSB : 0);     // two rows
+    static constexpr int OFF_X = OFF_EY + (DBLC ? YSB : 0);     // a row of each edge
     static constexpr int OFF_EX = OFF_X + EP * XSB;
     static constexpr int OFF_W = OFF_EX + (DBLC ? EP * XSB : 0);
     static constexpr int OFF_EW = OFF_W + EP * WSB;
@@ -453,7 +454,9 @@ __device__ __forceinline__ void slice_second_z(const unsigned char* st, int e, i
 // (0e..3o), 150 k edges, 313 -> 296; 128x(0e..3o), 1.2 M edges, 5.07 -> 4.86 ms.
 enum class Place { IN1, IN2, OUT };
 // FP64 with few sums: the coefficient FMAs of a path would follow one another on the same values of the row, at the FP64 FMA's
-// latency.  8x(0e+1o), 8 sums, 4 000 nodes: 48 us with the weight on an input, 45 on the output; 32x(0e+1o+2e), 35 sums: 97 / 98.
+// latency.  740 k edges, weight on an input / on the output: 8x(0e+1o) with 0e+1o (8 sums) 163 / 153 us, to 0e..2e (13) 196 / 187, with
+// 0e+1o+2e to 0e+1o (11) 210 / 196, but 8x(0e+1o+2e) with 0e (9, no two of a path on one sum) 153 / 157; 8x(1o+2e) with 0e+1o (17)
+// 210 / 218, 8x(0e+2e) with 0e+2e (17) 241 / 243, 8x(0e+1o+2e) with 0e+1o (21) 247 / 249.  Rows of 32 channels: within 2 %.
 constexpr bool FEW_SUMS = ELEM == 8 && ZPC_ALL < 16;
 __host__ __device__ constexpr Place weight_place(int p) {
     const int d1 = IN1_D[I_IN1[p]], d2 = IN2_D[I_IN2[p]], d3 = OUT_D[I_OUT[p]];

@@ -100,7 +100,8 @@ def test_rejects_per_edge_uvw_weights():
                          ids=["uvw_64", "uvw_64_f64", "tetris_poly_2"])
 @pytest.mark.parametrize("graph", ["runs", "one_edge", "many"])
 def test_edge_sum_walk(name, dtype, graph, deterministic):
-    """The edge sums keep products per receiver: runs of no, one, odd and even numbers of edges."""
+    """Runs of no, one, odd and even numbers of edges through both stages: sums of products per receiver (uvw_64; in FP64 in the
+    forward pass only) and the group kernels, which take rows of unequal multiplicities (tetris_poly_2)."""
     p = problem_by_name(name, irrep_dtype=dtype, weight_dtype=dtype)
     degrees = np.array(DEGREES[graph])
     nodes, edges = len(degrees), int(degrees.sum())
