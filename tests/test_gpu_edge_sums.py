@@ -99,3 +99,21 @@ def test_walk(mul, in1, in2, out, dtype, graph, deterministic):
         if deterministic and plain is not None:     # copies in pieces or in elements: the same sums
             assert all(torch.equal(a, b) for a, b in zip(got, plain))
         plain = got
+
+
+def test_large_lists_in_edge_blocks(monkeypatch):
+    """Wide rows stay with the slice kernel on lists of every length; with scratch for a part of the edges it runs block by block."""
+    monkeypatch.setenv("OEQ_B200_BWD_SCRATCH_MB", "1")
+    monkeypatch.setenv("OEQ_B200_BWD_MIN_BLOCK", "1")
+    monkeypatch.setenv("OEQ_B200_RECV_MIN_EDGES", "1")
+    p = _edge_sum(128, E2, E2, E2)
+    nodes, edges, rng = 60, 1500, np.random.default_rng(9)
+    rows, cols, _, perm = orc.coord_graph(rng.integers(0, nodes, edges), rng.integers(0, nodes, edges))
+    x, y, dz = (rng.normal(size=(n, r.dim)).astype(np.float32) for n, r in ((nodes, p.irreps_in1), (edges, p.irreps_in2), (nodes, p.irreps_out)))
+    conv = _UnitWeightConv(p, True)
+    dx, dy = conv.backward_helper(*_cuda(x, y, dz, rows, cols, perm))
+    conv.internal.check()
+    per_block = (1 << 20) // (p.irreps_in1.dim * 4)
+    assert conv.internal.last_backward_launches() == 1 + 2 * -(-edges // per_block)
+    rx, ry, _ = orc.conv_backward(p, x, y, np.ones((edges, p.weight_numel), np.float32), dz, rows, cols)
+    assert rel_err(dx.cpu().numpy(), rx) < REL_TOL[np.float32] and rel_err(dy.cpu().numpy(), ry) < REL_TOL[np.float32]
