@@ -49,6 +49,37 @@ __device__ __forceinline__ void tc_commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
+// ---- Issue from a warp in step: every lane comes to the call and the lane whose `leader` is set issues.  Operands are then in
+// uniform registers: an MMA takes about 20 cycles of issue, from a divergent lane 88, whatever its size.
+__device__ __forceinline__ void tc_mma_if(unsigned leader, unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc,
+                                          unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
+        : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(unsigned leader, unsigned long long* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
+        : "memory");
+}
+__device__ __forceinline__ unsigned elect_lane() {
+    unsigned r;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {       // (does not wait)
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// A wait of the whole warp.
+__device__ __forceinline__ bool warp_wait(bool ok, unsigned long long* bar, unsigned parity, int* status, int code) {
+    return ok && __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
+}
 // 16 consecutive accumulator columns of the calling warp's 32 TMEM lanes (wait with tcgen05.wait::ld)
 __device__ __forceinline__ void tc_load16(unsigned taddr, unsigned* v) {
     asm volatile(

@@ -5,7 +5,7 @@
 //
 // with T_p[b,u,k] = sum_{ij} C_p[i,j,k] x[b,u,i] y[b,j] as in the forward pass.  A GEMM whose operands do not exist
 // in memory in the needed layout: producer warps build them as K-major, 128-byte-swizzled [rows x 32] tiles split into
-// TF32 hi and lo parts, one thread issues the MMAs, and epilogue warps drain tensor memory.  hi.hi and hi.lo go out as
+// TF32 hi and lo parts, one warp issues the MMAs, and epilogue warps drain tensor memory.  hi.hi and hi.lo go out as
 // one MMA over a B tile of 2 N rows (hi tile followed by lo tile), lo.hi as a second one, because issuing an MMA costs
 // more than running it.  (dX and dY: dT = W dZ with the forward kernel on the transposed weights, then the channel-wise
 // backward kernel on dT.)
@@ -216,35 +216,39 @@ __device__ __forceinline__ bool dw_produce(const UvwTcBwdParams& p, unsigned cha
 
 template <int O, int GRP>
 __device__ __forceinline__ bool dw_mma(const UvwTcBwdParams& p, unsigned char* smem, const DwBars& bars, long long row_lo,
-                                       long long row_hi, long long& stage_it, long long& acc_it, unsigned tmem_base) {
+                                       long long row_hi, long long& stage_it, long long& acc_it, unsigned tmem_base, unsigned leader) {
     constexpr int D3 = OUT_D[O], RB = 32 / D3, MW = OUT_MUL[O];
     constexpr unsigned IDESC = tc_instr_desc(MW), IDESC_WIDE = tc_instr_desc(2 * MW);
     if (row_lo >= row_hi) return true;
     const int t = (int)(acc_it & 1);
     const long long acc_use = acc_it >> 1;
-    if (acc_use > 0 && !mbar_wait(bars.acc_empty + t, (unsigned)((acc_use - 1) & 1), p.status, ERR_TB_ACC_EMPTY)) return false;
+    if (acc_use > 0 && !warp_wait(true, bars.acc_empty + t, (unsigned)((acc_use - 1) & 1), p.status, ERR_TB_ACC_EMPTY)) return false;
     tc_fence_after();
     const unsigned tmem_d = tmem_base + (unsigned)(t * DW_ACC_COLS);
     const unsigned long long desc0 = tc_smem_desc(smem_u32(smem));
     unsigned accumulate = 0;
+    bool ready = false, ahead = false;      // this stage and the next one were seen to be full, two stages ahead
     for (long long b0 = row_lo; b0 < row_hi; b0 += RB) {
         const int s = (int)(stage_it % DW_STAGES);
         const long long use = stage_it / DW_STAGES;
-        if (!mbar_wait(bars.full + s, (unsigned)(use & 1), p.status, ERR_TB_FULL)) return false;
+        if (!ready && !warp_wait(true, bars.full + s, (unsigned)(use & 1), p.status, ERR_TB_FULL)) return false;
         tc_fence_after();
         const unsigned long long da_hi = desc0 + (unsigned long long)((s * DW_STAGE_BYTES) >> 4);
         const unsigned long long da_lo = da_hi + (TB_TILE >> 4);
         const unsigned long long db = da_lo + (TB_TILE >> 4);        // hi tile, then lo tile
+        const bool asked = DW_STAGES > 2 && mbar_test(bars.full + (stage_it + 2) % DW_STAGES, (unsigned)((stage_it + 2) / DW_STAGES & 1));
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            tc_mma(tmem_d, da_hi + 2 * kk, db + 2 * kk, IDESC_WIDE, accumulate);   // [hi.hi | hi.lo]
+            tc_mma_if(leader, tmem_d, da_hi + 2 * kk, db + 2 * kk, IDESC_WIDE, accumulate);   // [hi.hi | hi.lo]
             accumulate = 1;
-            tc_mma(tmem_d, da_lo + 2 * kk, db + 2 * kk, IDESC, 1);                 // lo.hi into the first half
+            tc_mma_if(leader, tmem_d, da_lo + 2 * kk, db + 2 * kk, IDESC, 1);                 // lo.hi into the first half
         }
-        tc_commit(bars.empty + s);
+        tc_commit_if(leader, bars.empty + s);
+        ready = __all_sync(0xffffffffu, ahead);
+        ahead = asked;
         ++stage_it;
     }
-    tc_commit(bars.acc_full + t);
+    tc_commit_if(leader, bars.acc_full + t);
     ++acc_it;
     return true;
 }
@@ -307,7 +311,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const DwBars bars(smem);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     long long row_lo, row_hi;
     tb_row_range(p.batch, row_lo, row_hi);
     if (tid == 0) {
@@ -330,7 +334,7 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *reinterpret_cast<volatile unsigned*>(bars.tmem_slot);
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile unsigned*>(bars.tmem_slot), 0);
 
     if (warp < TB_PRODUCER_WARPS) {
         long long stage_it = 0;
@@ -344,18 +348,17 @@ __device__ void uvw_tc_dw(const UvwTcBwdParams& p) {
             });
         });
     } else if (warp == TB_PRODUCER_WARPS) {
-        if (lane == 0) {
-            long long stage_it = 0, acc_it = 0;
-            bool ok = true;
-            sfor<0, N_OUT>([&](auto o_) {
-                constexpr int O = o_;
-                sfor<0, tb_groups(O)>([&](auto g_) {
-                    constexpr int GRP = g_;
-                    if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
-                    if (ok) ok = dw_mma<O, GRP>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, tmem_base);
-                });
+        const unsigned leader = elect_lane();
+        long long stage_it = 0, acc_it = 0;
+        bool ok = true;
+        sfor<0, N_OUT>([&](auto o_) {
+            constexpr int O = o_;
+            sfor<0, tb_groups(O)>([&](auto g_) {
+                constexpr int GRP = g_;
+                if (gridDim.y > 1 && (int)blockIdx.y != dw_groups_before(O) + GRP) return;
+                if (ok) ok = dw_mma<O, GRP>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, tmem_base, leader);
             });
-        }
+        });
         __syncwarp();
     } else {
         long long acc_it = 0;

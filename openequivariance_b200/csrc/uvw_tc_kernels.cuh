@@ -10,7 +10,7 @@
 //
 //   * 16 producer warps form T with the Clebsch-Gordan constants unrolled, split every value into
 //     hi = tf32(t), lo = tf32(t - hi), and store both as K-major 128-byte-swizzled [128 x 32] tiles;
-//   * one thread issues tcgen05.mma (M = 128, N = mul_out, K = 8 per instruction) three times per K step
+//   * one warp issues tcgen05.mma (M = 128, N = mul_out, K = 8 per instruction) three times per K step
 //     (hi.hi + hi.lo + lo.hi) into a ring of TMEM accumulator tiles, and hands shared-memory stages
 //     and accumulators on with tcgen05.commit -> mbarrier;
 //   * 4 epilogue warps read accumulators with tcgen05.ld, transpose (row,k)-major tiles through a
@@ -315,11 +315,11 @@ __device__ __forceinline__ bool tc_produce_output(const UvwTcParams& p, unsigned
     return ok;
 }
 
-// ---------------------------------------------------------------------------- MMA issuer (one thread)
+// ---------------------------------------------------------------------------- MMA issuer (one warp, in step)
 template <int O>
 __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned char* smem, const TcBars& bars,
                                               long long row_lo, long long row_hi, long long& stage_it, long long& acc_it,
-                                              int& w_use, unsigned tmem_base) {
+                                              int& w_use, unsigned tmem_base, unsigned leader, int lane) {
     constexpr int D3 = OUT_D[O];
     constexpr int RPC = tc_rpc(O);
     constexpr int MW = tc_mwp(O);
@@ -334,11 +334,11 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
     if (row_lo >= row_hi) return true;
     // the weights of the previous output must not be overwritten while tensor cores still read them
     if (w_use > 0) {
-        tc_commit(bars.w_free);
-        if (!mbar_wait(bars.w_free, (unsigned)((w_use - 1) & 1), p.status, ERR_TC_W)) return false;
+        tc_commit_if(leader, bars.w_free);
+        if (!warp_wait(true, bars.w_free, (unsigned)((w_use - 1) & 1), p.status, ERR_TC_W)) return false;
     }
-    mbar_arrive_expect_tx(bars.w_full, (unsigned)tc_w_bytes(O));
-    {
+    if (lane == 0) {
+        mbar_arrive_expect_tx(bars.w_full, (unsigned)tc_w_bytes(O));
         const unsigned char* src = reinterpret_cast<const unsigned char*>(p.Wpacked) + tc_w_offset(O);
         constexpr int TOTAL = tc_w_bytes(O);
         for (int off = 0; off < TOTAL; off += 32768) {
@@ -346,15 +346,16 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
             bulk_g2s(smem + TC_OFF_W + off, src + off, (unsigned)n, bars.w_full);
         }
     }
-    if (!mbar_wait(bars.w_full, (unsigned)(w_use & 1), p.status, ERR_TC_W)) return false;
+    __syncwarp();
+    if (!warp_wait(true, bars.w_full, (unsigned)(w_use & 1), p.status, ERR_TC_W)) return false;
     ++w_use;
     const unsigned long long w_desc0 = tc_smem_desc(smem_u32(smem + TC_OFF_W));
     const unsigned long long a_desc0 = tc_smem_desc(smem_u32(smem + TC_OFF_A));
-    bool ok = true;
+    bool ok = true, ready = false;          // ready: the next stage was seen to be full
     for (long long b0 = row_lo; b0 < row_hi && ok; b0 += RPC) {
         const int t = (int)(acc_it % NACC);
         const long long acc_use = acc_it / NACC;
-        if (acc_use > 0) ok = mbar_wait(bars.acc_empty + t, (unsigned)((acc_use - 1) & 1), p.status, ERR_TC_ACC_EMPTY);
+        if (acc_use > 0) ok = warp_wait(ok, bars.acc_empty + t, (unsigned)((acc_use - 1) & 1), p.status, ERR_TC_ACC_EMPTY);
         if (!ok) break;
         tc_fence_after();
         const unsigned tmem_d = tmem_base + (unsigned)(t * ACC_COLS);
@@ -365,9 +366,9 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
                 for (int h = 0; h < tc_khalves(P) && ok; ++h) {
                     const int s = (int)(stage_it % TC_NA);
                     const long long use = stage_it / TC_NA;
-                    const bool prof = p.prof && blockIdx.x == 0;
+                    const bool prof = p.prof && blockIdx.x == 0 && lane == 0;
                     const long long t0 = prof ? clock64() : 0;
-                    ok = mbar_wait(bars.a_full + s, (unsigned)(use & 1), p.status, ERR_TC_A_FULL);
+                    if (!ready) ok = warp_wait(ok, bars.a_full + s, (unsigned)(use & 1), p.status, ERR_TC_A_FULL);
                     const long long t1 = prof ? clock64() : 0;
                     if (ok) {
                         tc_fence_after();
@@ -377,28 +378,30 @@ __device__ __forceinline__ bool tc_mma_output(const UvwTcParams& p, unsigned cha
                         const unsigned long long da_lo = da_hi + (TC_STAGE_HALF >> 4);
                         const unsigned long long db_hi = w_desc0 + (unsigned long long)(((tc_blocks_before(O, P) + h) * 2 * BLOCK) >> 4);
                         const unsigned long long db_lo = db_hi + (BLOCK >> 4);
+                        ready = mbar_test(bars.a_full + (stage_it + 1) % TC_NA, (unsigned)((stage_it + 1) / TC_NA & 1));
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
                             if constexpr (WIDE) {
-                                tc_mma(tmem_d, da_hi + 2 * kk, db_hi + 2 * kk, IDESC_WIDE, accumulate);
+                                tc_mma_if(leader, tmem_d, da_hi + 2 * kk, db_hi + 2 * kk, IDESC_WIDE, accumulate);
                             } else {
-                                tc_mma(tmem_d, da_hi + 2 * kk, db_hi + 2 * kk, IDESC, accumulate);
-                                tc_mma(tmem_d, da_hi + 2 * kk, db_lo + 2 * kk, IDESC, 1);
+                                tc_mma_if(leader, tmem_d, da_hi + 2 * kk, db_hi + 2 * kk, IDESC, accumulate);
+                                tc_mma_if(leader, tmem_d, da_hi + 2 * kk, db_lo + 2 * kk, IDESC, 1);
                             }
                             accumulate = 1;
-                            tc_mma(tmem_d, da_lo + 2 * kk, db_hi + 2 * kk, IDESC, 1);
+                            tc_mma_if(leader, tmem_d, da_lo + 2 * kk, db_hi + 2 * kk, IDESC, 1);
                         }
-                        tc_commit(bars.a_empty + s);   // the stage may be refilled once these MMAs have read it
+                        tc_commit_if(leader, bars.a_empty + s);   // the stage may be refilled once these MMAs have read it
                         if (prof) {
                             atomicAdd(p.prof + 8, (unsigned long long)(t1 - t0));             // wait for operands
                             atomicAdd(p.prof + 9, (unsigned long long)(clock64() - t1));      // issue
                         }
+                        ready = __all_sync(0xffffffffu, ready);
                     }
                     ++stage_it;
                 }
             }
         });
-        if (ok) tc_commit(bars.acc_full + t);
+        if (ok) tc_commit_if(leader, bars.acc_full + t);
         ++acc_it;
     }
     return ok;
@@ -524,7 +527,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
     // the 128-byte swizzle pattern repeats every 1024 bytes: operand tiles must start on that boundary
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const TcBars bars(smem);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     long long row_lo, row_hi;
 
     if (tid == 0) {
@@ -549,7 +552,7 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *reinterpret_cast<volatile unsigned*>(bars.tmem_slot);
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile unsigned*>(bars.tmem_slot), 0);
 
     if (warp < TC_PRODUCER_WARPS) {
         long long stage_it = 0;
@@ -567,19 +570,18 @@ __device__ void uvw_tc_forward(const UvwTcParams& p) {
             }
         });
     } else if (warp == TC_PRODUCER_WARPS) {
-        if (lane == 0) {
-            long long stage_it = 0, acc_it = 0;
-            int w_use = 0;
-            bool ok = true;
-            sfor<0, N_OUT>([&](auto o_) {
-                constexpr int O = o_;
-                if (!tc_mine(O)) return;
-                tc_row_range<O>(p, row_lo, row_hi);
-                if constexpr (tc_output_has_paths(O)) {
-                    if (ok) ok = tc_mma_output<O>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, w_use, tmem_base);
-                }
-            });
-        }
+        const unsigned leader = elect_lane();
+        long long stage_it = 0, acc_it = 0;
+        int w_use = 0;
+        bool ok = true;
+        sfor<0, N_OUT>([&](auto o_) {
+            constexpr int O = o_;
+            if (!tc_mine(O)) return;
+            tc_row_range<O>(p, row_lo, row_hi);
+            if constexpr (tc_output_has_paths(O)) {
+                if (ok) ok = tc_mma_output<O>(p, smem, bars, row_lo, row_hi, stage_it, acc_it, w_use, tmem_base, leader, lane);
+            }
+        });
         __syncwarp();
     } else {
         long long acc_it = 0;
