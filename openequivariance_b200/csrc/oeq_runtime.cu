@@ -1495,6 +1495,42 @@ int build_uvw_tc(const Problem& p, const TcGeometry& g, Kernel& k) {
     return OEQ_OK;
 }
 
+// ---- the same with the weights in tensor memory (mirrors the constexpr geometry of uvw_ts_kernels.cuh): at most 64 output
+// channels per irrep, 256 input channels over the paths into one, rows of X in whole 16-byte pieces of four channels.
+constexpr int K_UVW_TS_FWD = 22, TS_ROWS = 16, TS_THREADS = 21 * 32;
+
+bool uvw_ts_geometry(const Problem& p, int& smem) {
+    TcGeometry g;
+    if (p.unit_y || p.transposed_w || !uvw_tc_geometry(p, g) || p.x_dim % 4) return false;
+    int data = 0;
+    for (size_t o = 0; o < p.out.size(); ++o) {
+        int slices = 0;
+        for (const Instr& t : p.instr)
+            if (t.io == (int)o) slices += (p.in1[t.i1].mul + 31) / 32;
+        if (slices == 0) continue;
+        if (p.out[o].mul > 64 || p.out[o].dim > 8 || slices > 8) return false;
+        data = std::max(data, TS_ROWS * p.out[o].dim * (4 * 2 * 128 + 2 * p.out[o].mul * 4));      // stages, rows of Z
+    }
+    for (const Irrep& r : p.in1)
+        if (r.mul % 4 || r.off % 4) return false;
+    smem = data + 2 * TS_ROWS * (p.x_dim + p.y_dim) * 4 + (int)p.out.size() * (2 * 4 + 2 * 4 + 4) * 8 + 16 + 1024;
+    return smem <= SMEM_LIMIT;
+}
+
+int build_uvw_ts(const Problem& p, Kernel& k) {
+    k.is_uvw = true;
+    int rc = choose_uvw(p, false, k.uvw);
+    if (rc) return rc;
+    k.map.part_of_out.assign(p.out.size(), 0);
+    k.map.part_of_instr.assign(p.instr.size(), 0);
+    k.map.zr_off.assign(p.out.size(), 0);
+    k.map.xr_off.assign(p.in1.size(), 0);
+    rc = compile_kernel(descriptor_text(p, k.map, &k.uvw), "uvw_ts_kernels.cuh", K_UVW_TS_FWD, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
 // ---- tensor-core backward for 'uvw': the weight gradient (mirrors the constexpr geometry of uvw_tc_bwd_kernels.cuh)
 constexpr int K_UVW_TC_DW = 21;
 
@@ -1961,7 +1997,10 @@ struct oeq_tp {
     Problem prob;
     Kernel fwd, bwd;
     Kernel fwd_row, bwd_row;    // 'uvw' with per-row weights: one row per CTA (then fwd / bwd are for the batches of uvw_row_limit, if any)
-    Kernel fwd_tc;              // tensor-core forward ('uvw', shared FP32 weights), when the problem qualifies
+    Kernel fwd_ts;              // tensor-core forward ('uvw', shared FP32 weights) with the weights in tensor memory
+    bool has_ts = false;
+    int ts_smem = 0;
+    Kernel fwd_tc;              // the same with the weights in shared memory, for wider problems
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
     bool has_bwd_tc = false;
@@ -2047,8 +2086,10 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         }
         if ((rc = build_tp(p, true, b, br))) return rc;
         TcGeometry g;
-        if (uvw_tc_geometry(p, g) && (rc = build_uvw_tc(p, g, tc))) return rc;
         int smem = 0, threads = 0;
+        if (uvw_ts_geometry(p, smem)) rc = build_uvw_ts(p, tc);
+        else if (uvw_tc_geometry(p, g)) rc = build_uvw_tc(p, g, tc);
+        if (rc) return rc;
         Kernel dw, product, channels;
         if (uvw_tc_dw_geometry(p, smem, threads)) {
             if ((rc = build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
@@ -2116,7 +2157,10 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
     }
     if (!rc && (!h->has_gemm || gemm_keeps_tiled(h->prob))) rc = build_tp(h->prob, false, h->fwd, h->fwd_row);
     if (!rc) rc = build_tp(h->prob, true, h->bwd, h->bwd_row);
-    if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
+    if (!rc && uvw_ts_geometry(h->prob, h->ts_smem)) {
+        rc = build_uvw_ts(h->prob, h->fwd_ts);
+        h->has_ts = rc == OEQ_OK;
+    } else if (!rc && uvw_tc_geometry(h->prob, h->tc)) {
         rc = build_uvw_tc(h->prob, h->tc, h->fwd_tc);
         h->has_tc = rc == OEQ_OK;
     }
@@ -2147,7 +2191,7 @@ int oeq_tp_destroy(oeq_tp* h) {
     if (h->d_status) cudaFree(h->d_status);
     if (h->d_packed) cudaFree(h->d_packed);
     if (h->d_packed_t) cudaFree(h->d_packed_t);
-    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_row, &h->bwd_row, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
+    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_row, &h->bwd_row, &h->fwd_ts, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
         if (k->lib) cudaLibraryUnload(k->lib);
     delete h;
     return OEQ_OK;
@@ -2186,6 +2230,28 @@ static int load_uvw_tc(Kernel& k, const TcGeometry& geo, cudaKernel_t& pack) {
     if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
     else (void)cudaGetLastError();
     k.loaded = true;
+    return OEQ_OK;
+}
+
+static int launch_uvw_ts(Kernel& k, int smem, const Problem& p, long long batch, const void* X, const void* Y, const void* W, void* Z, int* status, cudaStream_t st) {
+    if (!k.loaded) {
+        OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+        OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_ts_kernel"));
+        int dev = 0;
+        OEQ_CUDA(cudaGetDevice(&dev));
+        OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
+        k.smem = smem;
+        OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
+        cudaFuncAttributes attr;
+        if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
+        else (void)cudaGetLastError();
+        k.loaded = true;
+    }
+    struct { const void* X; const void* Y; const void* W; void* Z; long long batch; int* status; int in_vec, z_vec; }
+        tp{X, Y, W, Z, batch, status, aligned16(X) && aligned16(Y), aligned16(Z)};
+    void* args[] = {&tp};
+    const long long tiles = (batch + TS_ROWS - 1) / TS_ROWS * (long long)p.out.size();
+    OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)std::min<long long>(k.sm_count, tiles)), dim3(TS_THREADS), args, (size_t)k.smem, st));
     return OEQ_OK;
 }
 
@@ -2285,6 +2351,7 @@ int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, co
     int rc = ensure_status(&h->d_status);
     if (rc) return rc;
     h->last_stream = (cudaStream_t)stream;
+    if (h->has_ts) return launch_uvw_ts(h->fwd_ts, h->ts_smem, h->prob, batch, X, Y, W, Z, h->d_status, (cudaStream_t)stream);
     if (h->has_tc) {
         void* packed = nullptr;
         if ((rc = load_uvw_tc(h->fwd_tc, h->tc, h->pack_fn)) || (rc = packed_weights(h->tc, workspace, workspace_bytes, h->d_packed, packed)))
@@ -2548,6 +2615,15 @@ static int launch_info(const Kernel& k, int* threads, int* ng, int* ps, int* sta
 }
 int oeq_tp_launch_info(const oeq_tp* h, int which, int* threads, int* ng, int* ps, int* stages, int* smem, int* regs) {
     if (!h) return fail(OEQ_ERR_INVALID, "null handle");
+    if (!which && h->has_ts) {
+        if (threads) *threads = TS_THREADS;
+        if (ng) *ng = 1;
+        if (ps) *ps = 1;
+        if (stages) *stages = 2;
+        if (smem) *smem = h->fwd_ts.smem;
+        if (regs) *regs = h->fwd_ts.regs;
+        return OEQ_OK;
+    }
     if (!which && h->has_tc) {
         if (threads) *threads = h->tc.threads();
         if (ng) *ng = 1;

@@ -1,0 +1,53 @@
+"""Shared-weight FP32 'uvw' forward with the weights in tensor memory: one row to several tiles of 16 per CTA, rows that change
+from one output irrep to the next, multiplicities that are no multiple of 32 (padded slices) and narrower than 64 (padded weight
+rows), a component count of seven, second inputs too long for registers, arrays off a 16-byte boundary, an output without paths."""
+import numpy as np
+import pytest
+import torch
+
+import openequivariance_b200 as oeq
+from oracle import tp_oracle as orc
+from helpers import rel_err, tp_inputs, to_oeq
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {"even": ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
+          "padded": ("36x0e+20x1o", "0e+1o+2e", "16x0e+48x1o+32x2e+16x4e"),     # (4e: no paths)
+          "seven": ("8x2e+32x3o", "0e+1o", "16x3o+16x2e"),
+          "long_y": ("32x0e+4x1o", "0e+1o+2e+3o+4e", "16x0e+16x1o+16x2e")}
+
+
+@pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 33, 5003])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_forward(shape, rows, offset):
+    p = oeq.FullyConnectedTPProblem(*SHAPES[shape])
+    tp = oeq.TensorProduct(p, torch_op=True)
+    x, y, w, _ = tp_inputs(p, rows, 7)
+    w = (w / np.sqrt(max(1, p.weight_numel / len(p.instructions)))).astype(np.float32)
+
+    def device(a):
+        flat = torch.from_numpy(np.ascontiguousarray(a)).cuda().flatten()
+        return torch.cat((flat.new_zeros(offset), flat))[offset:].view(a.shape)
+
+    xt, yt, wt = device(x), device(y), device(to_oeq(p, w))
+    z = tp(xt, yt, wt)
+    torch.cuda.synchronize()
+    tp.check_device_status()
+    # sums of up to 256 products in FP32, hi and lo parts of 11 bits each: 2^-22 per product, and T's rounding
+    assert rel_err(z.cpu().numpy(), orc.tp_forward(p, x, y, w)) < 5e-6
+    for n in (1, rows // 2):            # a row's sums do not depend on the batch that it is part of
+        assert torch.equal(z[:n], tp(xt[:n].contiguous(), yt[:n].contiguous(), wt))
+
+
+def test_rows_off_a_boundary():
+    """Output rows that start off a 16-byte boundary."""
+    p = oeq.FullyConnectedTPProblem(*SHAPES["even"])
+    tp = oeq.TensorProduct(p, torch_op=True)
+    x, y, w, _ = tp_inputs(p, 40, 9)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w))]
+    want = tp(*dev)
+    out = torch.zeros(want.numel() + 1, device="cuda")
+    tp.internal.forward(40, *(t.data_ptr() for t in dev), out.data_ptr() + 4, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(out[1:].view_as(want), want) and out[0] == 0
