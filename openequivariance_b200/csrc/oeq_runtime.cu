@@ -962,6 +962,7 @@ struct Kernel {
     Mapping map;
     UvwConfig uvw;
     bool is_uvw = false, is_uvw_row = false;
+    int row_smem = 0;             // is_uvw_row: shared memory of a CTA
     Compiled code;
     bool compiled = false, loaded = false;
     cudaLibrary_t lib = nullptr;
@@ -1672,7 +1673,35 @@ int uvw_row_limit(const Problem& p, bool bwd) {
     return per_path < 32 ? 8 : 64;
 }
 
+// Staged rows (uvw_row_kernels.cuh): bulk copies want rows of whole 16-byte pieces, and two stages have to leave room for a
+// second CTA on an SM.  Shared memory of a CTA, 0 where a row does not qualify.
+constexpr int K_UVW_STAGED_FWD = 14, K_UVW_STAGED_BWD = 15, UVW_STAGED_BYTES = (228 * 1024) / 2 - 1024;
+constexpr int UVW_STAGED_UNITS = 256;      // (the compiler deals them)
+
+int uvw_staged_smem(const Problem& p, bool bwd) {
+    const long long e = p.elem();
+    for (long long n : {p.x_dim, p.y_dim, p.z_dim, p.w_numel})
+        if (n * e % 16) return 0;
+    auto r4 = [](long long n) { return (n + 3) / 4 * 4; };
+    long long t = 0, parts = 0, units = 0;
+    for (const Instr& i : p.instr) {
+        const int mu = p.in1[i.i1].mul, mv = p.in2[i.i2].mul, mw = p.out[i.io].mul, d3 = p.out[i.io].dim;
+        t += (long long)mu * mv * d3;
+        for (int wc = 0; wc < mw; wc += 32) {
+            const int wlen = std::min(32, mw - wc);
+            parts += (long long)((mu + 31) / 32) * (32 / wlen) * wlen * d3;
+        }
+        units += bwd ? (long long)((mu + 15) / 16) * mv : (long long)((mu + 31) / 32) * ((mw + 31) / 32);
+    }
+    if (units > UVW_STAGED_UNITS) return 0;
+    const long long stage = (long long)p.w_numel + p.x_dim + p.y_dim + (bwd ? p.z_dim : 0);
+    const long long bytes = (2 * stage + r4(t) + r4(bwd ? r4(t) + 2 * UVW_ROW_WARPS * p.y_dim : parts)) * e + (bwd ? units * 48 : 0) + 16;
+    return bytes <= UVW_STAGED_BYTES ? (int)bytes : 0;
+}
+
 int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
+    const int staged = uvw_staged_smem(p, bwd);
+    k.row_smem = staged ? staged : uvw_row_smem(p, bwd);
     k.is_uvw = k.is_uvw_row = true;
     k.uvw.tile_r = 1;       // (the tiled kernel's bodies are not compiled)
     k.uvw.threads = 32 * UVW_ROW_WARPS;
@@ -1681,7 +1710,8 @@ int build_uvw_row(const Problem& p, bool bwd, Kernel& k) {
     k.map.zr_off.assign(p.out.size(), 0);
     k.map.xr_off.assign(p.in1.size(), 0);
     const std::string rows = "namespace oeqd { constexpr int ROW_WARPS = " + std::to_string(UVW_ROW_WARPS) + "; }\n";
-    int rc = compile_kernel(descriptor_text(p, k.map, &k.uvw) + rows, "uvw_row_kernels.cuh", bwd ? K_UVW_ROW_BWD : K_UVW_ROW_FWD, k.code);
+    int rc = compile_kernel(descriptor_text(p, k.map, &k.uvw) + rows, "uvw_row_kernels.cuh",
+                            staged ? (bwd ? K_UVW_STAGED_BWD : K_UVW_STAGED_FWD) : (bwd ? K_UVW_ROW_BWD : K_UVW_ROW_FWD), k.code);
     if (rc) return rc;
     k.compiled = true;
     return OEQ_OK;
@@ -1796,7 +1826,7 @@ int load_uvw(Kernel& k, const Problem& p, bool bwd) {
     int dev = 0;
     OEQ_CUDA(cudaGetDevice(&dev));
     OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
-    k.smem = k.is_uvw_row ? uvw_row_smem(p, bwd) : k.uvw.smem(p, bwd);
+    k.smem = k.is_uvw_row ? k.row_smem : k.uvw.smem(p, bwd);
     OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
     cudaFuncAttributes attr;
     if (cudaFuncGetAttributes(&attr, (const void*)k.fn) == cudaSuccess) k.regs = attr.numRegs;
@@ -1820,6 +1850,7 @@ struct UvwParams {
     long long batch;
     int* status;
     int skip_dw;      // the shared-weight gradient comes from the tensor-core kernel
+    int bulk;         // staged rows: all arrays start on a 16-byte boundary
 };
 
 // The kernel that a batch takes.
@@ -2368,6 +2399,7 @@ int oeq_tp_forward_ws(oeq_tp* h, int64_t batch, const void* X, const void* Y, co
         if ((rc = load_uvw(k, h->prob, false))) return rc;
         UvwParams up{};
         up.X = X; up.Y = Y; up.W = W; up.Z = Z; up.batch = batch; up.status = h->d_status;
+        up.bulk = aligned16(X) && aligned16(Y) && aligned16(W);
         void* args[] = {&up};
         OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)uvw_grid(k, batch)), dim3((unsigned)k.uvw.threads), args, (size_t)k.smem,
                                   (cudaStream_t)stream));
@@ -2470,6 +2502,7 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         UvwParams up{};
         up.X = X; up.Y = Y; up.W = W; up.dZ = dZ; up.dX = dX; up.dY = dY; up.dW = dW; up.ws = workspace;
         up.batch = batch; up.status = h->d_status;
+        up.bulk = aligned16(X) && aligned16(Y) && aligned16(W) && aligned16(dZ) && aligned16(dW);
         h->last_stream = st;
         if (h->has_bwd_tc) {
             // weight gradient on the tensor cores (per-CTA partial sums in the workspace, then the fixed-order

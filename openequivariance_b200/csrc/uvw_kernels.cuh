@@ -35,6 +35,7 @@ struct UvwParams {
     long long batch;
     int* status;
     int skip_dw;   // shared weights: the weight gradient is computed elsewhere, leave dW and ws alone
+    int bulk;      // staged rows: all arrays start on a 16-byte boundary
 };
 
 constexpr int NT = UVW_THREADS;

@@ -47,3 +47,40 @@ FEW = [("4x0e+4x1o", "0e+1o", "4x0e+4x1o"), ("8x0e+8x1o", "0e+1o", "8x0e+8x1o"),
 @pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
 def test_few_weights(irreps, batch, dtype):
     test_row_weights(irreps, batch, dtype)
+
+
+# Rows of whole 16-byte pieces: bulk copies of a row's arrays ahead of it.  Remainders of the chunks of 32 channels (33 ... 52)
+# and of the units of 16, output channels beside which four, three, two and one input channels fit a warp, second inputs of
+# multiplicity above one; more rows than two per CTA; arrays that start off a 16-byte boundary.
+STAGED = [("40x0e+12x1o+4x2e", "1x0e+1x1o", "52x0e+8x1o+12x1e+4x0o"), ("36x0e+4x1o", "4x0e+4x1o", "16x0e+20x1o"),
+          ("10x1o + 10x1e + 48x0e + 48x0o", "1x0e + 1x1o", "10x1o + 10x1e + 48x0e + 48x0o")]
+
+
+@pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
+@pytest.mark.parametrize("batch", [1, 7, 1501])
+@pytest.mark.parametrize("irreps", STAGED, ids=["tails", "mul_v", "docking"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
+def test_staged_rows(irreps, batch, offset, dtype):
+    p = oeq.FullyConnectedTPProblem(*irreps, shared_weights=False, irrep_dtype=dtype, weight_dtype=dtype)
+    assert all(n * np.dtype(dtype).itemsize % 16 == 0
+               for n in (p.irreps_in1.dim, p.irreps_in2.dim, p.irreps_out.dim, p.weight_numel))
+    arrays = tp_inputs(p, batch, 5)
+
+    def device(a):
+        flat = torch.from_numpy(np.ascontiguousarray(a)).cuda().flatten()
+        return torch.cat((flat.new_zeros(offset), flat))[offset:].view(a.shape)
+
+    x, y, w, dz = (device(a) for a in (*arrays[:2], to_oeq(p, arrays[2]), arrays[3]))
+    tp = oeq.TensorProduct(p, torch_op=True)
+    z = tp(x, y, w)
+    dx, dy, dw = tp.backward_helper(x, y, w, dz)
+    tp.check_device_status()
+    some = slice(0, batch) if batch < 100 else np.r_[0:3, batch // 2, batch - 3:batch]
+    sub = [a[some] for a in arrays]
+    want = [orc.tp_forward(p, *sub[:3]), *orc.tp_backward(p, *sub)]
+    for got, ref in zip((z, dx, dy), want):
+        assert rel_err(got.cpu().numpy()[some], ref) < REL_TOL[dtype]
+    assert rel_err(to_e3nn(p, dw.cpu().numpy()[some]), want[3]) < REL_TOL[dtype]
+    again = (tp(x, y, w), *tp.backward_helper(x, y, w, dz))         # every row, not only those compared: the same bits
+    for a, b in zip((z, dx, dy, dw), again):
+        assert torch.equal(a, b)
