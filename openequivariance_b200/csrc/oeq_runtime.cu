@@ -898,7 +898,7 @@ int compile_kernel(const std::string& descriptor, const std::string& main_header
     std::string common, body;
     if (!read_file(dir + "/oeq_common.cuh", common) || !read_file(dir + "/" + main_header, body))
         return fail(OEQ_ERR_COMPILE, "kernel headers not found in " + dir);
-    for (const char* inc : {"tc_common.cuh", "uvu_kernels.cuh", "uvw_kernels.cuh"}) {   // headers that the kernel files include
+    for (const char* inc : {"tc_common.cuh", "uvw_ts_common.cuh", "uvu_kernels.cuh", "uvw_kernels.cuh"}) {   // headers that the kernel files include
         std::string text;
         if (main_header != inc && read_file(dir + "/" + inc, text)) common += text;
     }
@@ -1532,6 +1532,39 @@ int build_uvw_ts(const Problem& p, Kernel& k) {
     return OEQ_OK;
 }
 
+// ---- weight gradient from rows formed a batch row per lane (mirrors uvw_ts_dw_kernels.cuh)
+constexpr int K_UVW_TS_DW = 23, TG_ROWS = 8;
+
+bool uvw_ts_dw_geometry(const Problem& p, int& smem) {
+    int fwd = 0;
+    if (!uvw_ts_geometry(p, fwd) || p.z_dim % 4 || !env_int("OEQ_B200_UVW_TC_BWD", 1)) return false;
+    int data = 0;
+    for (size_t o = 0; o < p.out.size(); ++o) {
+        bool paths = false;
+        for (const Instr& t : p.instr) paths |= t.io == (int)o;
+        if (!paths) continue;
+        if (p.out[o].off % 4) return false;
+        data = std::max(data, 1024 * p.out[o].dim * (2 * 8 + 2 * ((2 * p.out[o].mul + 31) / 32)) +      // slots of T, of dZ, inputs
+                                  2 * TG_ROWS * (p.x_dim + p.y_dim + p.out[o].mul * p.out[o].dim) * 4);
+    }
+    smem = std::max(data, 222 * 1024) + (int)p.out.size() * (2 * 2 + 2 * 2 + 2 * 4 + 2 * 3) * 8 + 16 + 1024;
+    return smem <= SMEM_LIMIT;
+}
+
+int build_uvw_ts_dw(const Problem& p, Kernel& k) {
+    k.is_uvw = true;
+    int rc = choose_uvw(p, true, k.uvw);
+    if (rc) return rc;
+    k.map.part_of_out.assign(p.out.size(), 0);
+    k.map.part_of_instr.assign(p.instr.size(), 0);
+    k.map.zr_off.assign(p.out.size(), 0);
+    k.map.xr_off.assign(p.in1.size(), 0);
+    rc = compile_kernel(descriptor_text(p, k.map, &k.uvw), "uvw_ts_dw_kernels.cuh", K_UVW_TS_DW, k.code);
+    if (rc) return rc;
+    k.compiled = true;
+    return OEQ_OK;
+}
+
 // ---- tensor-core backward for 'uvw': the weight gradient (mirrors the constexpr geometry of uvw_tc_bwd_kernels.cuh)
 constexpr int K_UVW_TC_DW = 21;
 
@@ -2034,7 +2067,7 @@ struct oeq_tp {
     Kernel fwd_tc;              // the same with the weights in shared memory, for wider problems
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
-    bool has_bwd_tc = false;
+    bool has_bwd_tc = false, dw_ts = false;     // dw_ts: from rows formed a batch row per lane
     int dw_smem = 0, dw_threads = 0;
     // dX and dY of the same class of problems: dT = W dZ on the tensor cores, then the channel-wise backward pass
     Problem grad_product, grad_channels;
@@ -2123,7 +2156,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if (rc) return rc;
         Kernel dw, product, channels;
         if (uvw_tc_dw_geometry(p, smem, threads)) {
-            if ((rc = build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
+            if ((rc = uvw_ts_dw_geometry(p, smem) ? build_uvw_ts_dw(p, dw) : build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
             Problem pp, pc;
             rc = build_uvw_gradients(p, pp, pc, g, product, channels);
             if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
@@ -2196,7 +2229,8 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
         h->has_tc = rc == OEQ_OK;
     }
     if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem, h->dw_threads)) {
-        rc = build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
+        h->dw_ts = uvw_ts_dw_geometry(h->prob, h->dw_smem);
+        rc = h->dw_ts ? build_uvw_ts_dw(h->prob, h->bwd_dw_tc) : build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
         h->has_bwd_tc = rc == OEQ_OK;
         if (!rc) {
             const int rc2 = build_uvw_gradients(h->prob, h->grad_product, h->grad_channels, h->grad_tc, h->grad_product_k, h->grad_channels_k);
@@ -2510,8 +2544,8 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             Kernel& k = h->bwd_dw_tc;
             if (!k.loaded) {
                 OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-                OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, "oeq_uvw_tc_dw_kernel"));
-                OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, "oeq_reduce_partials"));
+                OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, h->dw_ts ? "oeq_uvw_ts_dw_kernel" : "oeq_uvw_tc_dw_kernel"));
+                OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, h->dw_ts ? "oeq_ts_reduce" : "oeq_reduce_partials"));
                 int dev = 0;
                 OEQ_CUDA(cudaGetDevice(&dev));
                 OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
@@ -2519,26 +2553,42 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
                 OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
                 k.loaded = true;
             }
-            long long dw_ctas = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 31) / 32));
-            if ((size_t)dw_ctas * p.w_numel * p.elem() > workspace_bytes)
-                return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
-            struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; }
-                tp{X, Y, dZ, workspace, batch, h->d_status};
-            void* targs[] = {&tp};
-            // groups of paths that fill the 128 rows of an MMA (tb_groups in the kernel); few rows: dealt over CTAs
-            unsigned dw_groups = 0;
-            for (size_t o = 0; o < p.out.size(); ++o) {
-                unsigned paths = 0, per = 2;
-                for (const Instr& t : p.instr)
-                    if (t.io == (int)o) { ++paths; if (p.in1[t.i1].mul > 64) per = 1; }
-                dw_groups += (paths + per - 1) / per;
+            if (h->dw_ts) {
+                const long long tiles = (batch + TG_ROWS - 1) / TG_ROWS * (long long)p.out.size();
+                const long long slices = (long long)(workspace_bytes / ((size_t)p.w_numel * p.elem()));
+                if (slices < std::min<long long>(k.sm_count, (batch + 31) / 32))
+                    return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
+                int ctas = (int)std::min<long long>({(long long)k.sm_count, 256, tiles, slices});
+                struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; int in_vec; }
+                    tp{X, Y, dZ, workspace, batch, h->d_status, aligned16(X) && aligned16(Y) && aligned16(dZ)};
+                void* targs[] = {&tp};
+                OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)ctas), dim3(TS_THREADS), targs, (size_t)k.smem, st));
+                const void* ws = workspace;
+                long long rows = batch;
+                void* rargs[] = {&ws, &dW, &rows, &ctas};
+                OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((p.w_numel + 31) / 32), dim3(256), rargs, 0, st));
+            } else {
+                long long dw_ctas = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 31) / 32));
+                if ((size_t)dw_ctas * p.w_numel * p.elem() > workspace_bytes)
+                    return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
+                struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; }
+                    tp{X, Y, dZ, workspace, batch, h->d_status};
+                void* targs[] = {&tp};
+                // groups of paths that fill the 128 rows of an MMA (tb_groups in the kernel); few rows: dealt over CTAs
+                unsigned dw_groups = 0;
+                for (size_t o = 0; o < p.out.size(); ++o) {
+                    unsigned paths = 0, per = 2;
+                    for (const Instr& t : p.instr)
+                        if (t.io == (int)o) { ++paths; if (p.in1[t.i1].mul > 64) per = 1; }
+                    dw_groups += (paths + per - 1) / per;
+                }
+                if (dw_ctas * dw_groups > k.sm_count) dw_groups = 1;
+                OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3((unsigned)h->dw_threads), targs, (size_t)k.smem, st));
+                int n = p.w_numel;
+                const void* ws = workspace;
+                void* rargs[] = {&ws, &dW, &n, &dw_ctas};
+                OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
             }
-            if (dw_ctas * dw_groups > k.sm_count) dw_groups = 1;
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3((unsigned)h->dw_threads), targs, (size_t)k.smem, st));
-            int n = p.w_numel;
-            const void* ws = workspace;
-            void* rargs[] = {&ws, &dW, &n, &dw_ctas};
-            OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((n + 31) / 32), dim3(256), rargs, 0, st));
             up.skip_dw = 1;
             up.ws = nullptr;
             // dX and dY in two steps over dT rows, which take the partial gradients' place in the workspace

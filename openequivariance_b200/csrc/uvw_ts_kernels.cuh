@@ -18,13 +18,13 @@
 // Every wait is bounded; on expiry the role records a code in *status and goes through the rest of its barriers without
 // work, and the CTA frees its tensor memory.
 // Measured against uvw_tc_kernels.cuh (weights in shared memory, which then has no room for rows of X), 64x(0e+1o+2e) with
-// 0e+1o+2e, with the packing of the weights: 100 000 rows 430-456 -> 275 us, 20 000 120 -> 74, 8 000 60 -> 40, 1 000 27 -> 23, 20 rows
+// 0e+1o+2e, with the packing of the weights: 100 000 rows 430-456 -> 275 us, 20 000 120 -> 68, 8 000 60 -> 38, 1 000 27 -> 18, 20 rows
 // 30 -> 20; relative error against 64 bits 1.2e-6 -> 6.2e-7 (hi.lo has accumulators of its own).
 // Bound by shared memory: per batch row 140 cycles of T's stores, 140 of the MMAs reading it, 80 of x and y, 72 of the epilogue
 // and 54 of the input copies, and conflicts between them, of 700; the tensor pipe is busy for 40 %, issue slots for 45 %.
 #pragma once
 #include "oeq_common.cuh"
-#include "tc_common.cuh"
+#include "uvw_ts_common.cuh"
 
 namespace oeq {
 using namespace oeqd;
@@ -46,18 +46,7 @@ constexpr int TS_THREADS = (TS_PW + TS_EW + 1) * 32;
 constexpr int ERR_TS_EMPTY = 51, ERR_TS_FULL = 52, ERR_TS_ACC_EMPTY = 53, ERR_TS_ACC_FULL = 54, ERR_TS_IN = 55;
 
 // ---- compile-time geometry
-constexpr int ts_halves(int p) { return (IN1_MUL[I_IN1[p]] + 31) / 32; }       // slices of 32 input channels
-constexpr int ts_n(int o) { return TS_ROWS * OUT_D[o]; }                        // N of the MMA
-constexpr int ts_column(int p) {                // columns of the weights of path p in tensor memory
-    int n = 0;
-    for (int q = 0; q < p; ++q) n += I_OUT[q] == I_OUT[p] ? 32 * ts_halves(q) : 0;
-    return n;
-}
-constexpr int ts_slices(int o) {
-    int n = 0;
-    for (int p = 0; p < N_INSTR; ++p) n += I_OUT[p] == o ? ts_halves(p) : 0;
-    return n;
-}
+constexpr int ts_n(int o) { return TS_ROWS * OUT_D[o]; }                        // N of the MMA, of a hi or lo tile
 constexpr int TS_W_COLS = 256, TS_ACC_COLS = 256, TS_BUFS = 4;  // tensor memory: weights, accumulators
 constexpr int ts_bufs(int o) { return TS_ACC_COLS / (2 * ts_n(o)) < TS_BUFS ? TS_ACC_COLS / (2 * ts_n(o)) : TS_BUFS; }
 // Shared memory while the CTA works on output o (1024-byte aligned base): [stages][rows of Z from hi and from lo
@@ -86,27 +75,10 @@ struct TsBars {
     }
 };
 
-// Tiles of all outputs, in one list weighted with the time of a tile, are cut into one run per CTA: most CTAs load the
-// weights of one output.  Measured, 64x(0e+1o+2e) with 0e+1o+2e: 1 980, 3 820 and 5 290 cycles for 6, 8 and 8 slices of 1, 3 and 5
-// components.
+// Time of a tile.  Measured, 64x(0e+1o+2e) with 0e+1o+2e: 1 980, 3 820 and 5 290 cycles for 6, 8 and 8 slices of 1, 3 and 5 components.
 constexpr int ts_cost(int o) { return ts_slices(o) * (OUT_D[o] + 3); }
-template <int O>
-__device__ __forceinline__ void ts_tiles(const UvwTsParams& p, int& lo, int& hi) {
-    const long long tiles = (p.batch + TS_ROWS - 1) / TS_ROWS;
-    long long total = 0, before = 0;
-    sfor<0, N_OUT>([&](auto o_) {
-        constexpr int o = o_;
-        total += tiles * ts_cost(o);
-        if constexpr (o < O) before += tiles * ts_cost(o);
-    });
-    constexpr int COST = ts_cost(O);
-    const long long from = total * blockIdx.x / gridDim.x - before, to = total * (blockIdx.x + 1) / gridDim.x - before;
-    const long long a = from > 0 ? (from + COST - 1) / COST : 0, b = to > 0 ? (to + COST - 1) / COST : 0;
-    lo = (int)(a < tiles ? a : tiles);
-    hi = (int)(b < tiles ? b : tiles);
-}
 
-// Issued by the lane whose `leader` is set; every lane of the warp comes here.  MMA with the A operand in tensor memory.
+// MMA with the A operand in tensor memory, issued by the lane whose `leader` is set; every lane of the warp comes here.
 __device__ __forceinline__ void tc_mma_ts(unsigned leader, unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
@@ -114,45 +86,11 @@ __device__ __forceinline__ void tc_mma_ts(unsigned leader, unsigned tmem_d, unsi
         ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
         : "memory");
 }
-__device__ __forceinline__ void expect_tx_if(unsigned leader, unsigned long long* bar, unsigned bytes) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t.reg .b64 st;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-        "@q mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(leader)
-        : "memory");
-}
-__device__ __forceinline__ void bulk_g2s_if(unsigned leader, void* dst_smem, const void* src_gmem, unsigned bytes, unsigned long long* bar) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
-        "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(smem_u32(dst_smem)),
-        "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar)), "r"(leader)
-        : "memory");
-}
-// 16 columns of the calling warp's 32 TMEM lanes
-__device__ __forceinline__ void tc_store16(unsigned taddr, const unsigned* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-          "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
-        : "memory");
-}
-
 // ---------------------------------------------------------------------------- producers
-// M of a row and path, from the row's second input: entries (i, k) that have a coefficient.
-template <int P, int N> constexpr bool ts_first_entry() {
-    for (int m = CG_BEGIN[P]; m < N; ++m)
-        if (CG_I[m] == CG_I[N] && CG_K[m] == CG_K[N]) return false;
-    return true;
-}
-template <int P, int N> constexpr bool ts_first_of_k() {
-    for (int m = CG_BEGIN[P]; m < N; ++m)
-        if (CG_K[m] == CG_K[N]) return false;
-    return true;
-}
-
 template <int O>
 __device__ __forceinline__ void ts_produce(const UvwTsParams& p, unsigned char* smem, const TsBars& bars, int tile_lo, int tile_hi,
                                            bool& ok, int warp, int lane) {
-    constexpr int D3 = OUT_D[O], INS = ts_ins(O);
+    constexpr int INS = ts_ins(O);
     const int set = warp / TS_SET, r = lane & 15, r8 = r & 7;
     // Four channels of a slice: the threads of row r take them in the order j ^ L(r), where L is a product with x in GF(8): L
     // and L + 1 are invertible, so eight rows read eight places of a row (an odd number of pieces apart) and write eight pieces.
@@ -173,7 +111,7 @@ __device__ __forceinline__ void ts_produce(const UvwTsParams& p, unsigned char* 
         }
         const float* x_row = reinterpret_cast<const float*>(in) + r * X_DIM;
         const float* y_row = reinterpret_cast<const float*>(in + TS_X_BYTES) + r * Y_DIM;
-        float y_regs[Y_DIM <= 16 ? Y_DIM : 1];          // (shared memory's bandwidth bounds the kernel)
+        float y_regs[Y_DIM <= 16 ? Y_DIM : 1] = {};     // (shared memory's bandwidth bounds the kernel)
         if constexpr (Y_DIM <= 16) {
 #pragma unroll
             for (int j = 0; j < Y_DIM; ++j) y_regs[j] = y_row[j];
@@ -182,13 +120,13 @@ __device__ __forceinline__ void ts_produce(const UvwTsParams& p, unsigned char* 
         sfor<0, N_INSTR>([&](auto p_) {
             constexpr int P = p_;
             if constexpr (I_OUT[P] == O) {
-                constexpr int A = I_IN1[P], B = I_IN2[P], D1 = IN1_D[A], MU = IN1_MUL[A], KH = ts_halves(P);
+                constexpr int A = I_IN1[P], D1 = IN1_D[A], MU = IN1_MUL[A], KH = ts_halves(P);
 #pragma unroll 1
                 for (int h = (set - stage_it) & (TS_STAGES - 1); h < KH; h += TS_STAGES) {
                     const int use = (stage_it + h) / TS_STAGES;
                     if (use > 0) ok = warp_wait(ok, bars.empty + set, (unsigned)(use - 1) & 1, p.status, ERR_TS_EMPTY);
                     if (ok) {
-                        float m[D1][D3], x[4 * D1];
+                        float x[4 * D1];
                         const int u0 = 32 * h + 4 * group;
 #pragma unroll
                         for (int c = 0; c < D1; ++c) {
@@ -196,30 +134,10 @@ __device__ __forceinline__ void ts_produce(const UvwTsParams& p, unsigned char* 
                                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
                             x[4 * c] = q.x; x[4 * c + 1] = q.y; x[4 * c + 2] = q.z; x[4 * c + 3] = q.w;
                         }
-                        sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
-                            constexpr int N = n_;
-                            float& e = m[CG_I[N]][CG_K[N]];
-                            if constexpr (ts_first_entry<P, N>()) e = (float)CG_V[N] * y(IN2_OFF[B] + CG_J[N]);
-                            else e = fmaf((float)CG_V[N], y(IN2_OFF[B] + CG_J[N]), e);
-                        });
-                        sfor<0, D3>([&](auto k_) {
+                        ts_form<P>(x, y, [&](auto k_, float4 hi, float4 lo) {
                             constexpr int K = k_;
-                            float t[4] = {0.f, 0.f, 0.f, 0.f}, hi[4], lo[4];
-                            sfor<CG_BEGIN[P], CG_BEGIN[P + 1]>([&](auto n_) {
-                                constexpr int N = n_, I = CG_I[N];
-                                if constexpr (CG_K[N] == K && ts_first_entry<P, N>()) {
-#pragma unroll
-                                    for (int u = 0; u < 4; ++u)
-                                        t[u] = ts_first_of_k<P, N>() ? m[I][K] * x[u * D1 + I] : fmaf(m[I][K], x[u * D1 + I], t[u]);
-                                }
-                            });
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                hi[u] = tf32_hi(t[u]);
-                                lo[u] = t[u] - hi[u];           // exact; read as TF32 by the MMA
-                            }
-                            *reinterpret_cast<float4*>(dst + K * 2048) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                            *reinterpret_cast<float4*>(dst + K * 2048 + ts_n(O) * 128) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+                            *reinterpret_cast<float4*>(dst + K * 2048) = hi;
+                            *reinterpret_cast<float4*>(dst + K * 2048 + ts_n(O) * 128) = lo;
                         });
                         fence_async_smem();
                         __syncwarp();
@@ -432,7 +350,7 @@ __device__ void uvw_ts_forward(const UvwTsParams& p) {
         constexpr int O = o_;
         if constexpr (ts_slices(O) > 0) {
             int lo, hi;
-            ts_tiles<O>(p, lo, hi);
+            ts_deal<O, TS_ROWS, ts_cost>(p.batch, blockIdx.x, gridDim.x, lo, hi);
             if (lo < hi) {
                 const TsBars bars(smem, O);
                 // (the output before is complete: its shared and tensor memory are free)

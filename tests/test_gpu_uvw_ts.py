@@ -1,13 +1,14 @@
-"""Shared-weight FP32 'uvw' forward with the weights in tensor memory: one row to several tiles of 16 per CTA, rows that change
-from one output irrep to the next, multiplicities that are no multiple of 32 (padded slices) and narrower than 64 (padded weight
-rows), a component count of seven, second inputs too long for registers, arrays off a 16-byte boundary, an output without paths."""
+"""Shared-weight FP32 'uvw' with a batch row per lane (forward with the weights in tensor memory, weight gradient): one row to
+several tiles of 16 or 8 rows per CTA, fewer CTAs than outputs, multiplicities that are no multiple of 32 (padded slices) and
+narrower than 64 (padded weight rows), a component count of seven, second inputs too long for registers, arrays off a 16-byte
+boundary, an output without paths."""
 import numpy as np
 import pytest
 import torch
 
 import openequivariance_b200 as oeq
 from oracle import tp_oracle as orc
-from helpers import rel_err, tp_inputs, to_oeq
+from helpers import rel_err, tp_inputs, to_e3nn, to_oeq
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +52,26 @@ def test_rows_off_a_boundary():
     tp.internal.forward(40, *(t.data_ptr() for t in dev), out.data_ptr() + 4, torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert torch.equal(out[1:].view_as(want), want) and out[0] == 0
+
+
+@pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 25, 5003])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_weight_gradient(shape, rows, offset):
+    """Weight gradient from tiles of eight rows: fewer than a tile, remainders, several tiles per CTA and slot of the ring."""
+    p = oeq.FullyConnectedTPProblem(*SHAPES[shape])
+    tp = oeq.TensorProduct(p, torch_op=True)
+    x, y, w, dz = tp_inputs(p, rows, 11)
+
+    def device(a):
+        flat = torch.from_numpy(np.ascontiguousarray(a)).cuda().flatten()
+        return torch.cat((flat.new_zeros(offset), flat))[offset:].view(a.shape)
+
+    args = [device(a) for a in (x, y, to_oeq(p, w), dz)]
+    dw = tp.backward_helper(*args)[2]
+    torch.cuda.synchronize()
+    tp.check_device_status()
+    # sums over rows and components in FP32 (their order differs from CTA to CTA), products as above
+    assert rel_err(to_e3nn(p, dw.cpu().numpy()), orc.tp_backward(p, x, y, w, dz)[2]) < 5e-6
+    for _ in range(3):
+        assert torch.equal(tp.backward_helper(*args)[2], dw)
