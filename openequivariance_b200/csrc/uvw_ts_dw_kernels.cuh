@@ -7,7 +7,7 @@
 // dZ [(k, b) x w], "MN-major" tiles of 32 channels by 8 batch rows per component (128-byte rows, 32-byte atoms swizzled over four
 // rows).  That is the order in which a thread with one batch row forms them, as in uvw_ts_kernels.cuh: its matrix M serves four
 // channels, and rows of X and dZ come as bulk copies.  An MMA tile has the channels of four slices of 32 (128 rows); hi.hi
-// and hi.lo are one MMA over dZ's hi channels followed by its lo channels, lo.hi a second one.  The sums of all the CTA's
+// and hi.lo are one MMA over dZ's hi channels followed by its lo channels, lo.hi a second one into hi.hi's columns.  The sums of all the CTA's
 // rows stay in tensor memory; per CTA and output irrep they go to scratch and are added in a fixed order.
 //   * 16 warps form T, in two sets with a slot of the ring each, and drain tensor memory; 4 warps split dZ and copy the
 //     inputs; one warp, in step, issues the MMAs.
@@ -16,8 +16,7 @@
 // Every wait is bounded; on expiry the role records a code in *status and goes through the rest of its barriers without
 // work, and the CTA frees its tensor memory.
 // Measured, 64x(0e+1o+2e) with 0e+1o+2e, without the sum over CTAs, uvw_tc_bwd_kernels.cuh / this kernel: 100 000 rows 498 / 370 us,
-// 8 000 69 / 57, 1 000 55 / 28, but 20 rows 13 / 23; relative error against 64 bits at 100 000 rows 1.4e-5 / 7.8e-7, at 5 000
-// 7.8e-7 / 6.8e-7 (shorter chains of additions in tensor memory).  Issue slots are busy for 60 %, shared memory for two thirds.
+// 8 000 69 / 57, 1 000 55 / 28, but 20 rows 13 / 23.  Issue slots are busy for 60 %, shared memory for two thirds.
 #pragma once
 #include "oeq_common.cuh"
 #include "uvw_ts_common.cuh"
@@ -39,10 +38,30 @@ constexpr int TG_ROWS = 8;                      // batch rows of a tile: the K o
 constexpr int TG_SETS = 2, TG_SET = 8;          // sets of warps that form T
 constexpr int TG_ROOM = 222 * 1024;              // shared memory for operands and inputs, where it is of use
 constexpr int TG_PW = TG_SETS * TG_SET, TG_BW = 4, TG_THREADS = (TG_PW + TG_BW + 1) * 32;
-// Tiles that the MMAs sum in one accumulator: an MMA adds to it with less accuracy than a rounded sum, and the error grows with
-// the length of a chain.  Then the accumulators are added to sums, in tensor memory too, while the MMAs go on in others.  (Sums every
-// 4 or 64 tiles: 495 / 399 us at 100 000 rows.)
-constexpr int tg_segment(int o) { return 40 / OUT_D[o]; }
+// Runs of tiles that the MMAs sum in one accumulator: an MMA adds to it less exactly than a rounded sum, and the error grows with the
+// length of a chain.  After a run the accumulators are added to sums, in tensor memory too, while the MMAs go on in others.  The
+// boundaries are those of the row ranges that the CTAs of uvw_tc_bwd_kernels.cuh have, so that no chain is longer than there and the
+// two kernels round much alike: relative errors at 5 000 / 20 000 / 100 000 rows 6.5e-7 / 2.4e-6 / 1.2e-5, there 7.8e-7 / 2.8e-6 /
+// 1.4e-5, and 4.8e-6 between the two at 100 000.  (Runs of 40 / components tiles, with lo.hi beside hi.lo, cost the same and are
+// 7.8e-7 off at 100 000, but then 1.3e-5 from the other kernel.)
+struct TgSegments {
+    int i, next;                                // the next boundary
+    static __device__ unsigned tiles(long long batch) { return (unsigned)((batch + TG_ROWS - 1) / TG_ROWS); }
+    static __device__ unsigned parts(long long batch) { return min((tiles(batch) + 3) / 4, gridDim.x); }
+    __device__ TgSegments(long long batch, int tile_lo) : i((unsigned)tile_lo / (tiles(batch) / parts(batch) + 1)) {
+        do advance(batch); while (next <= tile_lo);
+    }
+    __device__ void advance(long long batch) {  // boundary i of all: tiles * i / parts
+        const unsigned t = tiles(batch), p = parts(batch);
+        ++i;
+        next = (int)(i * (t / p) + i * (t % p) / p);
+    }
+    __device__ int count(long long batch, int tile_hi) {        // segments of the CTA's run
+        int n = 1;
+        for (; next < tile_hi; ++n) advance(batch);
+        return n;
+    }
+};
 constexpr int TG_BUFS = 3, TG_COLS = 512;       // accumulators of 128 columns, then sums of 64 for each MMA tile
 constexpr int TG_B = 2, TG_IN_MAX = 4;          // slots of dZ, buffers of inputs (two to four, as they fit)
 constexpr int ERR_TG_EMPTY = 61, ERR_TG_FULL = 62, ERR_TG_IN = 63, ERR_TG_IN_EMPTY = 64, ERR_TG_ACC_FULL = 65, ERR_TG_B_EMPTY = 66, ERR_TG_B_FULL = 67, ERR_TG_ACC_EMPTY = 68;
@@ -139,7 +158,7 @@ __device__ __forceinline__ bool tg_inputs(const UvwTsDwParams& p, unsigned char*
 
 // ---------------------------------------------------------------------------- sums
 // Row l of MMA tile m is input channel l mod 32 of slice 4 m + l / 32.  Set m of the warps that form T adds the accumulators of a
-// segment, columns [hi.hi | hi.lo + lo.hi], to the sums; a warp has a quarter of the rows and every other 16 columns.
+// segment, columns [hi.hi + lo.hi | hi.lo], to the sums; a warp has a quarter of the rows and every other 16 columns.
 template <int O>
 __device__ __forceinline__ bool tg_add(const UvwTsDwParams& p, const TgBars& bars, bool ok, unsigned tmem_base, int set, int w, int lane, int segment) {
     constexpr int MW = OUT_MUL[O], MT = tg_mtiles(O);
@@ -212,6 +231,7 @@ __device__ __forceinline__ void tg_produce(const UvwTsDwParams& p, unsigned char
     const int group = (((w & 1) * 4 + (lane >> 3)) ^ r);
     unsigned char* dst = smem + set * tg_a_slot(O) + (w >> 1) * BLOCK + r * 128 + ((group * 16) ^ ((r & 3) << 5));
     int slot_it = 0;                            // slots of all sets so far
+    int segment = 0;
     for (int tile = tile_lo, it = 0; tile < tile_hi; ++tile, ++it) {
         unsigned char* in = smem + tg_off_in(O) + it % INS * tg_in(O);
         ok = tg_inputs<O>(p, in, bars, tile, it, ok, warp * 32 + lane);
@@ -256,10 +276,13 @@ __device__ __forceinline__ void tg_produce(const UvwTsDwParams& p, unsigned char
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bars.in_empty + it % INS);
-        // (the segment before this tile, so that the MMAs have this one to go on with)
-        if (it > 0 && it % tg_segment(O) == 0) ok = tg_add<O>(p, bars, ok, tmem_base, set, w, lane, it / tg_segment(O) - 1);
+        // (a segment's sums are moved when its MMAs are done: where it ends would take registers to know here, 415 us instead of 372)
+        const int n = segment * MT + set;
+        if (set < MT && __any_sync(0xffffffffu, mbar_test(bars.acc_full + n % TG_BUFS, (unsigned)(n / TG_BUFS) & 1)))
+            ok = tg_add<O>(p, bars, ok, tmem_base, set, w, lane, segment++);
     }
-    ok = tg_add<O>(p, bars, ok, tmem_base, set, w, lane, (tile_hi - tile_lo - 1) / tg_segment(O));
+    for (const int segments = TgSegments(p.batch, tile_lo).count(p.batch, tile_hi); segment < segments; ++segment)
+        ok = tg_add<O>(p, bars, ok, tmem_base, set, w, lane, segment);
     if (ok) tg_store<O>(p, tmem_base, set, w, lane);
 }
 
@@ -329,9 +352,12 @@ __device__ __forceinline__ void tg_mma(const UvwTsDwParams& p, unsigned char* sm
     const unsigned long long a0 = tg_desc(smem_u32(smem), BLOCK), b0 = tg_desc(smem_u32(smem) + tg_off_b(O), BLOCK);
     int slot_it = 0;
     bool ready = false;                         // slot `slot_it` was seen to be full
+    bool first = true;
+    int segment = 0;                            // (kept apart, and steps by votes: what the MMAs' operands depend on is uniform)
+    TgSegments segments(p.batch, tile_lo);
     for (int tile = tile_lo, it = 0; tile < tile_hi && ok; ++tile, ++it) {
-        const int s = it % TG_B, segment = it / tg_segment(O);
-        const bool first = it % tg_segment(O) == 0, last = it % tg_segment(O) == tg_segment(O) - 1 || tile + 1 == tile_hi;
+        const int s = it % TG_B;
+        const bool last = __any_sync(0xffffffffu, tile + 1 == segments.next || tile + 1 == tile_hi);
         ok = warp_wait(ok, bars.b_full + s, (unsigned)(it / TG_B) & 1, p.status, ERR_TG_B_FULL);
         const unsigned long long b = b0 + (unsigned long long)((s * tg_b_slot(O)) >> 4);
 #pragma unroll 1
@@ -347,13 +373,18 @@ __device__ __forceinline__ void tg_mma(const UvwTsDwParams& p, unsigned char* sm
 #pragma unroll
             for (int k = 0; k < D3; ++k) {
                 tc_mma_if(leader, tmem_d, a + 64 * k, b + 64 * k, IDESC_WIDE, !first || k > 0);                 // [hi.hi | hi.lo]
-                tc_mma_if(leader, tmem_d + MW, a + 64 * k + (4 * BLOCK >> 4), b + 64 * k, IDESC, 1);            // lo.hi beside hi.lo
+                tc_mma_if(leader, tmem_d, a + 64 * k + (4 * BLOCK >> 4), b + 64 * k, IDESC, 1);                 // lo.hi
             }
             tc_commit_if(leader, bars.a_empty + set);
             if (last) tc_commit_if(leader, bars.acc_full + buf);
             ready = __all_sync(0xffffffffu, ready);
         }
         if (ok) tc_commit_if(leader, bars.b_empty + s);
+        if (last) {
+            ++segment;
+            segments.advance(p.batch);
+        }
+        first = last;
     }
 }
 
