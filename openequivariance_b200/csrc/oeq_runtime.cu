@@ -1514,7 +1514,7 @@ bool uvw_ts_geometry(const Problem& p, int& smem) {
     }
     for (const Irrep& r : p.in1)
         if (r.mul % 4 || r.off % 4) return false;
-    smem = data + 2 * TS_ROWS * (p.x_dim + p.y_dim) * 4 + (int)p.out.size() * (2 * 4 + 2 * 4 + 4) * 8 + 16 + 1024;
+    smem = data + 2 * TS_ROWS * (p.x_dim + p.y_dim) * 4 + (int)p.out.size() * (2 * 4 + 2 * 4 + 2 * 4) * 8 + 16 + 1024;
     return smem <= SMEM_LIMIT;
 }
 

@@ -43,7 +43,7 @@ constexpr int TS_ROWS = 16;                     // batch rows of a tile
 constexpr int TS_STAGES = 4, TS_SET = 4;        // slots of the stage ring, producer warps of each
 constexpr int TS_PW = TS_STAGES * TS_SET, TS_EW = 4;    // producer and epilogue warps
 constexpr int TS_THREADS = (TS_PW + TS_EW + 1) * 32;
-constexpr int ERR_TS_EMPTY = 51, ERR_TS_FULL = 52, ERR_TS_ACC_EMPTY = 53, ERR_TS_ACC_FULL = 54, ERR_TS_IN = 55;
+constexpr int ERR_TS_EMPTY = 51, ERR_TS_FULL = 52, ERR_TS_ACC_EMPTY = 53, ERR_TS_ACC_FULL = 54, ERR_TS_IN = 55, ERR_TS_IN_EMPTY = 56;
 
 // ---- compile-time geometry
 constexpr int ts_n(int o) { return TS_ROWS * OUT_D[o]; }                        // N of the MMA, of a hi or lo tile
@@ -62,16 +62,20 @@ constexpr int ts_data() {
     return m;
 }
 constexpr int ts_ins(int o) { return (ts_data() - ts_off_in(o)) / TS_IN < TS_IN_MAX ? (ts_data() - ts_off_in(o)) / TS_IN : TS_IN_MAX; }
-constexpr int TS_BARS = 2 * TS_STAGES + 2 * TS_BUFS + TS_IN_MAX;            // of each output: no phase outlives an output
+// An output of fewer slices than there are sets of producers: a set without a slice in a tile reads its inputs all the same (and waits
+// for each, or it would miss a phase), and the tile's accumulator says nothing of that set.  Its input buffers have barriers of
+// their own.  With more slices every set has a part in every accumulator.
+constexpr bool ts_idle_sets(int o) { return ts_slices(o) < TS_STAGES; }
+constexpr int TS_BARS = 2 * TS_STAGES + 2 * TS_BUFS + 2 * TS_IN_MAX;        // of each output: no phase outlives an output
 constexpr int TS_OFF_BAR = ts_data();
 constexpr int TS_SMEM = TS_OFF_BAR + N_OUT * TS_BARS * 8 + 16 + 1024;           // + alignment slack
 
 struct TsBars {
-    unsigned long long *full, *empty, *acc_full, *acc_empty, *in_full;
+    unsigned long long *full, *empty, *acc_full, *acc_empty, *in_full, *in_empty;
     __device__ TsBars(unsigned char* smem, int o) {
         full = reinterpret_cast<unsigned long long*>(smem + TS_OFF_BAR) + o * TS_BARS;
         empty = full + TS_STAGES; acc_full = empty + TS_STAGES; acc_empty = acc_full + TS_BUFS;
-        in_full = acc_empty + TS_BUFS;
+        in_full = acc_empty + TS_BUFS; in_empty = in_full + TS_IN_MAX;
     }
 };
 
@@ -147,6 +151,10 @@ __device__ __forceinline__ void ts_produce(const UvwTsParams& p, unsigned char* 
                 stage_it += KH;
             }
         });
+        if constexpr (ts_idle_sets(O)) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars.in_empty + b);
+        }
         if (++b == INS) {
             b = 0;
             phase ^= 1;
@@ -248,7 +256,8 @@ __device__ __forceinline__ void ts_copy_rows(const UvwTsParams& p, unsigned char
     if (all) bulk_g2s_if(leader, in + TS_X_BYTES, p.Y + row0 * Y_DIM, TS_Y_BYTES, bars.in_full + b);
 }
 
-// The first of its warps copies the inputs: a tile's accumulator is complete, so its rows of X and Y have been read.
+// The first of its warps copies the inputs: a tile's accumulator is complete, so its rows of X and Y have been read by the sets that had
+// a slice of it; ts_idle_sets.
 template <int O>
 __device__ __forceinline__ void ts_epilogue(const UvwTsParams& p, unsigned char* smem, const TsBars& bars, int tile_lo, int tile_hi,
                                             bool& ok, unsigned tmem_base, unsigned leader, int ewarp, int lane) {
@@ -261,13 +270,19 @@ __device__ __forceinline__ void ts_epilogue(const UvwTsParams& p, unsigned char*
     if (copies)
         for (int i = 0; i < INS && tile_lo + i < tile_hi; ++i) ts_copy_rows<O>(p, smem, bars, tile_lo + i, i, leader, lane);
     int t = 0, b = 0;
-    unsigned phase = 0;
+    unsigned phase = 0, in_phase = 0;
     for (int tile = tile_lo; tile < tile_hi; ++tile) {
         const long long row0 = (long long)tile * TS_ROWS;
         const int rows = (int)(p.batch - row0 < TS_ROWS ? p.batch - row0 : TS_ROWS);
         ok = warp_wait(ok, bars.acc_full + t, phase, p.status, ERR_TS_ACC_FULL);
-        if (copies && ok && tile + INS < tile_hi) ts_copy_rows<O>(p, smem, bars, tile + INS, b, leader, lane);
-        b = b + 1 == INS ? 0 : b + 1;
+        if (copies && tile + INS < tile_hi) {
+            if constexpr (ts_idle_sets(O)) ok = warp_wait(ok, bars.in_empty + b, in_phase, p.status, ERR_TS_IN_EMPTY);
+            if (ok) ts_copy_rows<O>(p, smem, bars, tile + INS, b, leader, lane);
+        }
+        if (++b == INS) {
+            b = 0;
+            in_phase ^= 1;
+        }
         if (ok) {
             tc_fence_after();
             // column n of either half of the tile: component n / 16 of batch row n mod 16
@@ -330,7 +345,10 @@ __device__ void uvw_ts_forward(const UvwTsParams& p) {
                 mbar_init(bars.acc_full + i, 1);
                 mbar_init(bars.acc_empty + i, TS_EW);
             }
-            for (int i = 0; i < TS_IN_MAX; ++i) mbar_init(bars.in_full + i, 1);
+            for (int i = 0; i < TS_IN_MAX; ++i) {
+                mbar_init(bars.in_full + i, 1);
+                mbar_init(bars.in_empty + i, TS_PW);
+            }
         }
         fence_mbar_init();
     }

@@ -75,3 +75,26 @@ def test_weight_gradient(shape, rows, offset):
     assert rel_err(to_e3nn(p, dw.cpu().numpy()), orc.tp_backward(p, x, y, w, dz)[2]) < 5e-6
     for _ in range(3):
         assert torch.equal(tp.backward_helper(*args)[2], dw)
+
+
+@pytest.mark.parametrize("muls", [("32x0e", "32x0e"), ("64x0e+32x1o", "16x0e+48x1o"), ("96x1o", "64x1o")], ids=["one", "two_and_one", "three"])
+def test_fewer_slices_than_producer_sets(muls):
+    """One to three slices of input channels per output, of which producer sets without a slice in a tile read the inputs too:
+    hundreds of tiles per CTA, so that input buffers are filled again and again; every row against the product in FP64."""
+    p = oeq.FullyConnectedTPProblem(muls[0], "0e", muls[1])
+    rows = 1_000_003 if p.irreps_in1.dim < 100 else 300_007
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x, y, w = (torch.randn(*s, device="cuda", generator=gen) for s in ((rows, p.irreps_in1.dim), (rows, 1), (p.weight_numel,)))
+    tp = oeq.TensorProduct(p, torch_op=True)
+    z = tp(x, y, torch.from_numpy(to_oeq(p, w.cpu().numpy())).cuda())
+    tp.check_device_status()
+    first = 0
+    for i in p.instructions:            # second input 0e: a matrix product of each irrep, times the coefficient 1 / sqrt(2 l + 1)
+        a, o, d = p.irreps_in1.slices()[i.i_in1], p.irreps_out.slices()[i.i_out], p.irreps_in1[i.i_in1].ir.dim
+        u, _, v = i.path_shape
+        wi = w[first:first + u * v].double().view(u, v) * (i.path_weight / np.sqrt(d))
+        first += u * v
+        for part in range(0, rows, 100_000):
+            s = slice(part, part + 100_000)
+            want = torch.einsum("bui,uw->bwi", x[s, a].double().unflatten(1, (u, d)), wi).flatten(1) * y[s].double()
+            assert ((z[s, o] - want).abs().max() / want.abs().max()).item() < 5e-6       # (as in test_forward)
