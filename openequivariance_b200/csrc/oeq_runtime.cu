@@ -1547,8 +1547,11 @@ bool uvw_ts_dw_geometry(const Problem& p, int& smem) {
         data = std::max(data, 1024 * p.out[o].dim * (2 * 8 + 2 * ((2 * p.out[o].mul + 31) / 32)) +      // slots of T, of dZ, inputs
                                   2 * TG_ROWS * (p.x_dim + p.y_dim + p.out[o].mul * p.out[o].dim) * 4);
     }
-    smem = std::max(data, 222 * 1024) + (int)p.out.size() * (2 * 2 + 2 * 2 + 2 * 4 + 2 * 3) * 8 + 16 + 1024;
-    return smem <= SMEM_LIMIT;
+    // (`smem` is that of the wider kernel until this one is taken)
+    const int bytes = std::max(data, 222 * 1024) + (int)p.out.size() * (2 * 2 + 2 * 2 + 2 * 4 + 2 * 3) * 8 + 16 + 1024;
+    if (bytes > SMEM_LIMIT) return false;
+    smem = bytes;
+    return true;
 }
 
 int build_uvw_ts_dw(const Problem& p, Kernel& k) {

@@ -98,3 +98,16 @@ def test_fewer_slices_than_producer_sets(muls):
             s = slice(part, part + 100_000)
             want = torch.einsum("bui,uw->bwi", x[s, a].double().unflatten(1, (u, d)), wi).flatten(1) * y[s].double()
             assert ((z[s, o] - want).abs().max() / want.abs().max()).item() < 5e-6       # (as in test_forward)
+
+
+def test_gradients_of_many_outputs():
+    """The barriers of the row-per-lane weight gradient beside its operands fit for 23 output irreps; more are for the wider kernel,
+    with the shared memory of its own."""
+    p = oeq.FullyConnectedTPProblem("16x0e", "0e", " + ".join(["16x0e"] * 24))
+    tp = oeq.TensorProduct(p, torch_op=True)
+    x, y, w, dz = tp_inputs(p, 500, 13)
+    args = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
+    dx, dy, dw = tp.backward_helper(*args)
+    tp.check_device_status()
+    for got, want in zip((dx.cpu().numpy(), dy.cpu().numpy(), to_e3nn(p, dw.cpu().numpy())), orc.tp_backward(p, x, y, w, dz)):
+        assert rel_err(got, want) < 5e-6
