@@ -79,8 +79,11 @@ struct TsBars {
     }
 };
 
-// Time of a tile.  Measured, 64x(0e+1o+2e) with 0e+1o+2e: 1 980, 3 820 and 5 290 cycles for 6, 8 and 8 slices of 1, 3 and 5 components.
-constexpr int ts_cost(int o) { return ts_slices(o) * (OUT_D[o] + 3); }
+// Time of a tile.  Measured for 1 / 2 / 4 / 8 slices, in units of 6 cycles: 216 / 262 / 308 / 400 of one component, 324 / 370 / 450 / 636
+// of three, 384 / 494 / 632 / 882 of five, 462 / 614 of seven (one and two slices); 330 for six of one.  Mostly the drain, which takes as long for one
+// slice as for eight: with a cost in proportion to the slices an output of one slice got too few CTAs (64x(0e+1o+2e) + 32x0o with
+// 0e+1o+2e to 64x(1o+2e) + 16x0o, 100 000 rows: 1 002 us, now 288; 64x(0e+1o+2e) with 0e+1o 227 and 204).
+constexpr int ts_cost(int o) { return ts_slices(o) ? 140 + 40 * OUT_D[o] + ts_slices(o) * (13 + 11 * OUT_D[o]) : 0; }
 
 // MMA with the A operand in tensor memory, issued by the lane whose `leader` is set; every lane of the warp comes here.
 __device__ __forceinline__ void tc_mma_ts(unsigned leader, unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {

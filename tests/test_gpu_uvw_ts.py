@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = {"even": ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
           "padded": ("36x0e+20x1o", "0e+1o+2e", "16x0e+48x1o+32x2e+16x4e"),     # (4e: no paths)
           "seven": ("8x2e+32x3o", "0e+1o", "16x3o+16x2e"),
-          "long_y": ("32x0e+4x1o", "0e+1o+2e+3o+4e", "16x0e+16x1o+16x2e")}
+          "long_y": ("32x0e+4x1o", "0e+1o+2e+3o+4e", "16x0e+16x1o+16x2e"),
+          "mixed": ("64x0e+64x1o+64x2e+32x0o", "0e+1o+2e", "64x1o+64x2e+16x0o")}          # eight slices and one
 
 
 @pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
