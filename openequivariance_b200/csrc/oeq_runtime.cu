@@ -1498,7 +1498,7 @@ int build_uvw_tc(const Problem& p, const TcGeometry& g, Kernel& k) {
 
 // ---- the same with the weights in tensor memory (mirrors the constexpr geometry of uvw_ts_kernels.cuh): at most 64 output
 // channels per irrep, 256 input channels over the paths into one, rows of X in whole 16-byte pieces of four channels.
-constexpr int K_UVW_TS_FWD = 22, TS_ROWS = 16, TS_THREADS = 21 * 32;
+constexpr int K_UVW_TS_FWD = 22, TS_ROWS = 16, TS_STAGES = 4, TS_THREADS = 21 * 32;
 
 bool uvw_ts_geometry(const Problem& p, int& smem) {
     TcGeometry g;
@@ -2705,7 +2705,7 @@ int oeq_tp_launch_info(const oeq_tp* h, int which, int* threads, int* ng, int* p
         if (threads) *threads = TS_THREADS;
         if (ng) *ng = 1;
         if (ps) *ps = 1;
-        if (stages) *stages = 2;
+        if (stages) *stages = TS_STAGES;
         if (smem) *smem = h->fwd_ts.smem;
         if (regs) *regs = h->fwd_ts.regs;
         return OEQ_OK;
