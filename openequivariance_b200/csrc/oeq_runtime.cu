@@ -1518,6 +1518,33 @@ bool uvw_ts_geometry(const Problem& p, int& smem) {
     return smem <= SMEM_LIMIT;
 }
 
+// Whether that kernel is the faster one, by the work of the problem and not of the batch: a row has the same bits in every batch.
+// Time of either, in units of 10 ns per 100 000 rows (fitted to 42 problems, all within 25 %): this kernel's drain costs a tile of 16 rows the same for
+// one slice of 32 input channels as for eight; the other kernel's producers read rows of X with a stride of 2 l + 1 values, slice by
+// slice, and its drain goes with the values of Z.
+// Measured, us for 100 000 rows, shared / tensor memory (at 1 000 rows; estimates tensor / shared):
+//   with 0e+1o+2e: 64x(0e+1o+2e) 413 / 268 (30 / 22; 0.72), 16x 194 / 189 (1.06), 48x(0e+1o+2e) to 64x0e 120 / 66 (0.68)
+//   with 0e+1o: 64x(0e+1o+2e) 227 / 204 (0.84), 64x(0e+1o) 105 / 110 (15.3 / 10.6; 1.07), 16x 52 / 90 (13.3 / 10.2; 1.95)
+//   with 0e: 256x1o to 64x1o 124 / 94 (0.72), 96x 64.5 / 63.5 (0.98), 64x 56.3 / 57.3 (15.3 / 10.2; 1.13); 256x0e to 64x0e 61 / 61 (17.5 /
+//     12.3; 1.16), 128x0e 36 / 49 (15.3 / 10.2; 1.55), 32x0e to 32x0e 19.4 / 37.5 (13.3 / 10.2; 3.8); 64x(0e+1o+2e) 136 / 171 (1.13)
+// Up to 1.1 this kernel loses at most 4 % at 100 000 rows (none below 30 000) and is 15 to 45 % faster below 4 000.
+bool uvw_ts_faster(const Problem& p) {
+    long long tensor = 0, shared = 0;
+    std::vector<bool> used(p.out.size());
+    for (const Instr& t : p.instr) {
+        const long long slices = (p.in1[t.i1].mul + 31) / 32, d1 = p.in1[t.i1].dim, d3 = p.out[t.io].dim, n = (long long)t.cv.size();
+        tensor += slices * (170 + 78 * d3 + 47 * d1 + 30 * n);
+        shared += slices * (112 + 341 * d1 + 44 * n);
+        used[t.io] = true;
+    }
+    for (size_t o = 0; o < p.out.size(); ++o)
+        if (used[o]) {
+            tensor += 2240 + 420 * p.out[o].dim;
+            shared += 9 * p.out[o].dim * p.out[o].mul;
+        }
+    return 10 * tensor <= 11 * shared;
+}
+
 int build_uvw_ts(const Problem& p, Kernel& k) {
     k.is_uvw = true;
     int rc = choose_uvw(p, false, k.uvw);
@@ -2154,7 +2181,7 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if ((rc = build_tp(p, true, b, br))) return rc;
         TcGeometry g;
         int smem = 0, threads = 0;
-        if (uvw_ts_geometry(p, smem)) rc = build_uvw_ts(p, tc);
+        if (uvw_ts_geometry(p, smem) && uvw_ts_faster(p)) rc = build_uvw_ts(p, tc);
         else if (uvw_tc_geometry(p, g)) rc = build_uvw_tc(p, g, tc);
         if (rc) return rc;
         Kernel dw, product, channels;
@@ -2224,7 +2251,7 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
     }
     if (!rc && (!h->has_gemm || gemm_keeps_tiled(h->prob))) rc = build_tp(h->prob, false, h->fwd, h->fwd_row);
     if (!rc) rc = build_tp(h->prob, true, h->bwd, h->bwd_row);
-    if (!rc && uvw_ts_geometry(h->prob, h->ts_smem)) {
+    if (!rc && uvw_ts_geometry(h->prob, h->ts_smem) && uvw_ts_faster(h->prob)) {
         rc = build_uvw_ts(h->prob, h->fwd_ts);
         h->has_ts = rc == OEQ_OK;
     } else if (!rc && uvw_tc_geometry(h->prob, h->tc)) {

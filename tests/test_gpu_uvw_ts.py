@@ -1,5 +1,5 @@
-"""Shared-weight FP32 'uvw' with a batch row per lane (forward with the weights in tensor memory, weight gradient): one row to
-several tiles of 16 or 8 rows per CTA, fewer CTAs than outputs, multiplicities that are no multiple of 32 (padded slices) and
+"""Shared-weight FP32 'uvw' with a batch row per lane (forward with the weights in tensor memory, unless the problem has too few slices
+of 32 input channels for it; weight gradient): one row to several tiles of 16 or 8 rows per CTA, fewer CTAs than outputs, multiplicities that are no multiple of 32 (padded slices) and
 narrower than 64 (padded weight rows), a component count of seven, second inputs too long for registers, arrays off a 16-byte
 boundary, an output without paths."""
 import numpy as np
@@ -16,7 +16,12 @@ SHAPES = {"even": ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
           "padded": ("36x0e+20x1o", "0e+1o+2e", "16x0e+48x1o+32x2e+16x4e"),     # (4e: no paths)
           "seven": ("8x2e+32x3o", "0e+1o", "16x3o+16x2e"),
           "long_y": ("32x0e+4x1o", "0e+1o+2e+3o+4e", "16x0e+16x1o+16x2e"),
+          # the same features in problems whose forward pass has the weights in tensor memory
+          "padded_ts": ("36x1o+20x2e", "0e+1o+2e", "16x0e+48x1o+32x2e+16x5o"),              # (5o: no paths)
+          "seven_ts": ("8x2e+32x3o+32x1o", "0e+1o+2e", "16x3o+16x2e+32x1o"),
+          "long_y_ts": ("32x2e+4x3o", "0e+1o+2e+3o+4e", "16x0e+16x1o+16x2e"),
           "mixed": ("64x0e+64x1o+64x2e+32x0o", "0e+1o+2e", "64x1o+64x2e+16x0o")}          # eight slices and one
+STAGES = {shape: 4 if shape in ("even", "mixed") or shape.endswith("_ts") else 2 for shape in SHAPES}   # four: weights in tensor memory
 
 
 @pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "unaligned"])
@@ -25,6 +30,7 @@ SHAPES = {"even": ("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
 def test_forward(shape, rows, offset):
     p = oeq.FullyConnectedTPProblem(*SHAPES[shape])
     tp = oeq.TensorProduct(p, torch_op=True)
+    assert tp.internal.launch_info(0)["stages"] == STAGES[shape]
     x, y, w, _ = tp_inputs(p, rows, 7)
     w = (w / np.sqrt(max(1, p.weight_numel / len(p.instructions)))).astype(np.float32)
 
@@ -78,27 +84,22 @@ def test_weight_gradient(shape, rows, offset):
         assert torch.equal(tp.backward_helper(*args)[2], dw)
 
 
-@pytest.mark.parametrize("muls", [("32x0e", "32x0e"), ("64x0e+32x1o", "16x0e+48x1o"), ("96x1o", "64x1o")], ids=["one", "two_and_one", "three"])
-def test_fewer_slices_than_producer_sets(muls):
-    """One to three slices of input channels per output, of which producer sets without a slice in a tile read the inputs too:
-    hundreds of tiles per CTA, so that input buffers are filled again and again; every row against the product in FP64."""
-    p = oeq.FullyConnectedTPProblem(muls[0], "0e", muls[1])
-    rows = 1_000_003 if p.irreps_in1.dim < 100 else 300_007
+@pytest.mark.parametrize("few", [32, 64, 96])
+def test_fewer_slices_than_producer_sets(few, monkeypatch):
+    """An output of one to three slices of input channels: producer sets without a slice in a tile read its inputs too.  Hundreds
+    of tiles per CTA, so that input buffers are filled again and again; every row against the FMA kernel."""
+    p = oeq.FullyConnectedTPProblem(f"64x0e+64x1o+64x2e+{few}x0o", "0e+1o+2e", "64x1o+64x2e+16x0o")
+    rows = 150_007
     gen = torch.Generator(device="cuda").manual_seed(3)
-    x, y, w = (torch.randn(*s, device="cuda", generator=gen) for s in ((rows, p.irreps_in1.dim), (rows, 1), (p.weight_numel,)))
+    x, y, w = (torch.randn(*s, device="cuda", generator=gen) for s in ((rows, p.irreps_in1.dim), (rows, p.irreps_in2.dim), (p.weight_numel,)))
     tp = oeq.TensorProduct(p, torch_op=True)
-    z = tp(x, y, torch.from_numpy(to_oeq(p, w.cpu().numpy())).cuda())
+    assert tp.internal.launch_info(0)["stages"] == 4
+    z = tp(x, y, w)
     tp.check_device_status()
-    first = 0
-    for i in p.instructions:            # second input 0e: a matrix product of each irrep, times the coefficient 1 / sqrt(2 l + 1)
-        a, o, d = p.irreps_in1.slices()[i.i_in1], p.irreps_out.slices()[i.i_out], p.irreps_in1[i.i_in1].ir.dim
-        u, _, v = i.path_shape
-        wi = w[first:first + u * v].double().view(u, v) * (i.path_weight / np.sqrt(d))
-        first += u * v
-        for part in range(0, rows, 100_000):
-            s = slice(part, part + 100_000)
-            want = torch.einsum("bui,uw->bwi", x[s, a].double().unflatten(1, (u, d)), wi).flatten(1) * y[s].double()
-            assert ((z[s, o] - want).abs().max() / want.abs().max()).item() < 5e-6       # (as in test_forward)
+    monkeypatch.setenv("OEQ_B200_UVW_TC", "0")
+    want = oeq.TensorProduct(p, torch_op=True)(x, y, w)
+    for o in p.irreps_out.slices():
+        assert ((z[:, o] - want[:, o]).abs().max() / want[:, o].abs().max()).item() < 1e-5          # (5e-6 each, as in test_forward)
 
 
 def test_gradients_of_many_outputs():

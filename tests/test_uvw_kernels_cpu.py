@@ -18,6 +18,10 @@ def stages(*irreps):
     (("64x1o+64x2e", "0e+1o", "64x1o"), TENSOR),
     (("64x1o+66x2e", "0e+1o", "64x1o"), SHARED),            # rows of X in no whole pieces of four channels
     (("64x1o+64x2e", "0e+1o", "80x1o"), SHARED),            # more than 64 output channels
+    (("32x0e", "0e", "32x0e"), SHARED),                     # too few slices of input channels
+    (("64x1o", "0e", "64x1o"), SHARED),
+    (("96x1o", "0e", "64x1o"), TENSOR),
+    (("64x2e", "0e", "64x2e"), TENSOR),
 ])
 def test_kernel_with_the_weights_in_tensor_memory(irreps, kernel):
     assert stages(*irreps) == kernel
