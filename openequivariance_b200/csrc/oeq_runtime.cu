@@ -1618,6 +1618,55 @@ bool uvw_tc_dw_geometry(const Problem& p, int& smem, int& threads) {
     return smem <= SMEM_LIMIT;
 }
 
+// Which of the two weight-gradient kernels a batch takes.  The wider one (uvw_tc_bwd_kernels.cuh) has an MMA tile of 128 rows for a group
+// of two paths (one where they have more than 64 channels), a stage of 32 (row, component) pairs for each, and deals the groups over the
+// CTAs while those suffice; the other one (uvw_ts_dw_kernels.cuh) sums four slices of 32 channels per MMA, eight batch rows at a time.
+//   Few rows: tiles of eight rows times the outputs are few CTAs, each with all slices of its output, against groups that are dealt.
+//     wider / other in us, with the sum over CTAs: 64x(0e+1o+2e) with 0e+1o+2e (22 slices) 20 rows 19.9 / 31.7, 500 23.7 / 37.9, but 1 000
+//     (groups no longer dealt) 64.5 / 40; with 0e+1o (14 slices) 20 rows 19.5 / 25.6, 1 000 25.3 / 31.7, 2 000 50 / 34; 32x(0e+1o+2e)
+//     with 0e+1o+2e (11) 20 rows 17.4 / 23.5; 64x(0e+1o) with 0e+1o (8 slices, two outputs) 200 rows 21.5 / 21.5; but 16x(0e+1o) (4)
+//     17.2 / 13.3, 16x(0e+1o+2e+3o) with 0e (4 slices, four outputs) 23.6 / 19.5
+//   Many rows: a scalar output has one MMA of K = 8 per tile and slices, and the other kernel does its rounds for that; outputs of more
+//     components gain.  100 000 rows, with 0e: 64x0e to 16x0e 58 / 73, 128x0e to 64x0e 69 / 84, 32x0e 60 / 65, 128x1o to 64x1o 99 / 107, but
+//     64x1o 118 / 86, 32x2e 173 / 81, 32x3o 245 / 90; 64x(0e+1o) with 0e+1o 159 / 176, 16x 158 / 151; at 10 000 rows 21.5 / 19.5, 27.6 / 26.7,
+//     21.5 / 19.5, 29.7 / 29.2, ..., 42 / 38.  The sum over the outputs below is the loss at 100 000 rows in us, roughly.
+struct DwChoice {
+    unsigned groups = 0;                    // of paths, in the wider kernel
+    bool few = false, many = false;         // the wider kernel is the faster one at few, at many rows
+    long long wider_ctas(long long batch, int sms) const { return std::max<long long>(1, std::min<long long>(sms, (batch + 31) / 32)); }
+    bool wider(long long batch, int sms) const {
+        return (few && wider_ctas(batch, sms) * groups <= sms) || (many && batch > 100ll * sms);
+    }
+};
+
+DwChoice uvw_dw_choice(const Problem& p) {
+    DwChoice c;
+    int slices_all = 0, outputs = 0, loss = 0;
+    for (size_t o = 0; o < p.out.size(); ++o) {
+        unsigned paths = 0, per = 2;
+        int slices = 0;
+        for (const Instr& t : p.instr)
+            if (t.io == (int)o) {
+                ++paths;
+                slices += (p.in1[t.i1].mul + 31) / 32;
+                if (p.in1[t.i1].mul > 64) per = 1;
+            }
+        if (!paths) continue;
+        const unsigned groups = (paths + per - 1) / per;
+        const int dim = p.out[o].dim;
+        c.groups += groups;
+        slices_all += slices;
+        ++outputs;
+        if (groups > 1) loss -= dim == 1 ? 30 : 60;
+        else if (dim == 1) loss += 12;
+        else if (slices == 4) loss += dim == 3 ? 7 : -5;
+        else loss -= dim == 3 ? 25 : 60;
+    }
+    c.few = c.groups > 1 && slices_all > 3 * outputs;
+    c.many = loss > 0;
+    return c;
+}
+
 // ---- dX and dY of the same class of problems in two steps over a scratch array dT [row][path][u][k]:
 //   dT_p[b,u,k] = sum_w W_p[u,w] dZ[b,w,k]: a 'uvw' forward pass from the output irreps, with the second input the
 //   number 1 and the weights transposed, one output block per path (`product`);
@@ -2097,8 +2146,10 @@ struct oeq_tp {
     Kernel fwd_tc;              // the same with the weights in shared memory, for wider problems
     bool has_tc = false;
     Kernel bwd_dw_tc;           // tensor-core weight gradient of the same class of problems
-    bool has_bwd_tc = false, dw_ts = false;     // dw_ts: from rows formed a batch row per lane
-    int dw_smem = 0, dw_threads = 0;
+    Kernel bwd_dw_ts;           // the same from rows formed a batch row per lane
+    bool has_bwd_tc = false, has_dw_ts = false, has_dw_tc = false;          // either; which
+    int dw_smem = 0, dw_threads = 0, dw_ts_smem = 0;
+    DwChoice dw_choice;
     // dX and dY of the same class of problems: dT = W dZ on the tensor cores, then the channel-wise backward pass
     Problem grad_product, grad_channels;
     Kernel grad_product_k, grad_channels_k;
@@ -2186,7 +2237,10 @@ int oeq_precompile(const oeq_problem_desc* desc, int kinds) {
         if (rc) return rc;
         Kernel dw, product, channels;
         if (uvw_tc_dw_geometry(p, smem, threads)) {
-            if ((rc = uvw_ts_dw_geometry(p, smem) ? build_uvw_ts_dw(p, dw) : build_uvw_tc_bwd(p, K_UVW_TC_DW, dw))) return rc;
+            const DwChoice choice = uvw_dw_choice(p);
+            const bool ts = uvw_ts_dw_geometry(p, smem);
+            Kernel wider;
+            if ((ts && (rc = build_uvw_ts_dw(p, dw))) || ((!ts || choice.few || choice.many) && (rc = build_uvw_tc_bwd(p, K_UVW_TC_DW, wider)))) return rc;
             Problem pp, pc;
             rc = build_uvw_gradients(p, pp, pc, g, product, channels);
             if (rc && rc != OEQ_ERR_UNSUPPORTED) return rc;
@@ -2259,8 +2313,11 @@ int oeq_tp_create(const oeq_problem_desc* desc, oeq_tp** out) {
         h->has_tc = rc == OEQ_OK;
     }
     if (!rc && uvw_tc_dw_geometry(h->prob, h->dw_smem, h->dw_threads)) {
-        h->dw_ts = uvw_ts_dw_geometry(h->prob, h->dw_smem);
-        rc = h->dw_ts ? build_uvw_ts_dw(h->prob, h->bwd_dw_tc) : build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
+        h->dw_choice = uvw_dw_choice(h->prob);
+        h->has_dw_ts = uvw_ts_dw_geometry(h->prob, h->dw_ts_smem);
+        h->has_dw_tc = !h->has_dw_ts || h->dw_choice.few || h->dw_choice.many;
+        if (h->has_dw_ts) rc = build_uvw_ts_dw(h->prob, h->bwd_dw_ts);
+        if (!rc && h->has_dw_tc) rc = build_uvw_tc_bwd(h->prob, K_UVW_TC_DW, h->bwd_dw_tc);
         h->has_bwd_tc = rc == OEQ_OK;
         if (!rc) {
             const int rc2 = build_uvw_gradients(h->prob, h->grad_product, h->grad_channels, h->grad_tc, h->grad_product_k, h->grad_channels_k);
@@ -2286,7 +2343,7 @@ int oeq_tp_destroy(oeq_tp* h) {
     if (h->d_status) cudaFree(h->d_status);
     if (h->d_packed) cudaFree(h->d_packed);
     if (h->d_packed_t) cudaFree(h->d_packed_t);
-    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_row, &h->bwd_row, &h->fwd_ts, &h->fwd_tc, &h->bwd_dw_tc, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
+    for (Kernel* k : {&h->fwd, &h->bwd, &h->fwd_row, &h->bwd_row, &h->fwd_ts, &h->fwd_tc, &h->bwd_dw_tc, &h->bwd_dw_ts, &h->grad_product_k, &h->grad_channels_k, &h->gemm, &h->gemm_dw, &h->dbl})
         if (k->lib) cudaLibraryUnload(k->lib);
     delete h;
     return OEQ_OK;
@@ -2571,19 +2628,20 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
         if (h->has_bwd_tc) {
             // weight gradient on the tensor cores (per-CTA partial sums in the workspace, then the fixed-order
             // reduction); the FMA kernel computes dX and dY only
-            Kernel& k = h->bwd_dw_tc;
+            const bool ts = h->has_dw_ts && !(h->has_dw_tc && h->dw_choice.wider(batch, main.sm_count));
+            Kernel& k = ts ? h->bwd_dw_ts : h->bwd_dw_tc;
             if (!k.loaded) {
                 OEQ_CUDA(cudaLibraryLoadData(&k.lib, k.code.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-                OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, h->dw_ts ? "oeq_uvw_ts_dw_kernel" : "oeq_uvw_tc_dw_kernel"));
-                OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, h->dw_ts ? "oeq_ts_reduce" : "oeq_reduce_partials"));
+                OEQ_CUDA(cudaLibraryGetKernel(&k.fn, k.lib, ts ? "oeq_uvw_ts_dw_kernel" : "oeq_uvw_tc_dw_kernel"));
+                OEQ_CUDA(cudaLibraryGetKernel(&k.reduce_fn, k.lib, ts ? "oeq_ts_reduce" : "oeq_reduce_partials"));
                 int dev = 0;
                 OEQ_CUDA(cudaGetDevice(&dev));
                 OEQ_CUDA(cudaDeviceGetAttribute(&k.sm_count, cudaDevAttrMultiProcessorCount, dev));
-                k.smem = h->dw_smem;
+                k.smem = ts ? h->dw_ts_smem : h->dw_smem;
                 OEQ_CUDA(cudaFuncSetAttribute((const void*)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem));
                 k.loaded = true;
             }
-            if (h->dw_ts) {
+            if (ts) {
                 const long long tiles = (batch + TG_ROWS - 1) / TG_ROWS * (long long)p.out.size();
                 const long long slices = (long long)(workspace_bytes / ((size_t)p.w_numel * p.elem()));
                 if (slices < std::min<long long>(k.sm_count, (batch + 31) / 32))
@@ -2598,20 +2656,14 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
                 void* rargs[] = {&ws, &dW, &rows, &ctas};
                 OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((p.w_numel + 31) / 32), dim3(256), rargs, 0, st));
             } else {
-                long long dw_ctas = std::max<long long>(1, std::min<long long>(k.sm_count, (batch + 31) / 32));
+                long long dw_ctas = h->dw_choice.wider_ctas(batch, k.sm_count);
                 if ((size_t)dw_ctas * p.w_numel * p.elem() > workspace_bytes)
                     return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
                 struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; }
                     tp{X, Y, dZ, workspace, batch, h->d_status};
                 void* targs[] = {&tp};
                 // groups of paths that fill the 128 rows of an MMA (tb_groups in the kernel); few rows: dealt over CTAs
-                unsigned dw_groups = 0;
-                for (size_t o = 0; o < p.out.size(); ++o) {
-                    unsigned paths = 0, per = 2;
-                    for (const Instr& t : p.instr)
-                        if (t.io == (int)o) { ++paths; if (p.in1[t.i1].mul > 64) per = 1; }
-                    dw_groups += (paths + per - 1) / per;
-                }
+                unsigned dw_groups = h->dw_choice.groups;
                 if (dw_ctas * dw_groups > k.sm_count) dw_groups = 1;
                 OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)dw_ctas, dw_groups), dim3((unsigned)h->dw_threads), targs, (size_t)k.smem, st));
                 int n = p.w_numel;

@@ -84,6 +84,21 @@ def test_weight_gradient(shape, rows, offset):
         assert torch.equal(tp.backward_helper(*args)[2], dw)
 
 
+# On both sides of the rows up to which the wider kernel deals its groups of paths (148 SMs; five and six groups), and from which it has the
+# weight gradients of scalar outputs.
+@pytest.mark.parametrize("irreps,rows", [(SHAPES["even"], 768), (SHAPES["even"], 769), (SHAPES["mixed"], 928), (SHAPES["mixed"], 929),
+                                         (("64x0e", "0e", "16x0e"), 14_800), (("64x0e", "0e", "16x0e"), 14_801)])
+def test_weight_gradient_kernels_by_rows(irreps, rows):
+    p = oeq.FullyConnectedTPProblem(*irreps)
+    tp = oeq.TensorProduct(p, torch_op=True)
+    x, y, w, dz = tp_inputs(p, rows, 17)
+    args = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
+    dw = tp.backward_helper(*args)[2]
+    tp.check_device_status()
+    assert rel_err(to_e3nn(p, dw.cpu().numpy()), orc.tp_backward(p, x, y, w, dz)[2]) < 5e-6         # (as in test_weight_gradient)
+    assert torch.equal(tp.backward_helper(*args)[2], dw)
+
+
 @pytest.mark.parametrize("few", [32, 64, 96])
 def test_fewer_slices_than_producer_sets(few, monkeypatch):
     """An output of one to three slices of input channels: producer sets without a slice in a tile read its inputs too.  Hundreds
