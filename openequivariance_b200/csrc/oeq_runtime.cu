@@ -2643,17 +2643,19 @@ int oeq_tp_backward(oeq_tp* h, int64_t batch, const void* X, const void* Y, cons
             }
             if (ts) {
                 const long long tiles = (batch + TG_ROWS - 1) / TG_ROWS * (long long)p.out.size();
-                const long long slices = (long long)(workspace_bytes / ((size_t)p.w_numel * p.elem()));
-                if (slices < std::min<long long>(k.sm_count, (batch + 31) / 32))
+                // (the CTAs, and with them the order of the sums, do not depend on the workspace: an output has no more of them than the
+                // least workspace that a call may come with holds partial gradients; with a CTA per tile, one output, 32x2e with 0e took
+                // 10.5 us up to 800 rows, with half as many 12.4)
+                int most = (int)std::max(ctas, h->dw_choice.wider_ctas(batch, k.sm_count)), all = (int)std::min<long long>(k.sm_count, tiles);
+                if ((size_t)most * p.w_numel * p.elem() > workspace_bytes)
                     return fail(OEQ_ERR_INVALID, "workspace too small for the shared-weight gradient (see oeq_tp_workspace_bytes)");
-                int ctas = (int)std::min<long long>({(long long)k.sm_count, 256, tiles, slices});
-                struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; int in_vec; }
-                    tp{X, Y, dZ, workspace, batch, h->d_status, aligned16(X) && aligned16(Y) && aligned16(dZ)};
+                struct { const void* X; const void* Y; const void* dZ; void* ws; long long batch; int* status; int in_vec, most; }
+                    tp{X, Y, dZ, workspace, batch, h->d_status, aligned16(X) && aligned16(Y) && aligned16(dZ), most};
                 void* targs[] = {&tp};
-                OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)ctas), dim3(TS_THREADS), targs, (size_t)k.smem, st));
+                OEQ_CUDA(cudaLaunchKernel((const void*)k.fn, dim3((unsigned)all), dim3(TS_THREADS), targs, (size_t)k.smem, st));
                 const void* ws = workspace;
                 long long rows = batch;
-                void* rargs[] = {&ws, &dW, &rows, &ctas};
+                void* rargs[] = {&ws, &dW, &rows, &all, &most};
                 OEQ_CUDA(cudaLaunchKernel((const void*)k.reduce_fn, dim3((p.w_numel + 31) / 32), dim3(256), rargs, 0, st));
             } else {
                 long long dw_ctas = h->dw_choice.wider_ctas(batch, k.sm_count);

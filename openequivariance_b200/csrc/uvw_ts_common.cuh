@@ -23,8 +23,9 @@ constexpr int ts_slices(int o) {
 // COST, and an output's tiles in equal runs to its CTAs (fewer CTAs than outputs take a run of every output).  Code for two outputs
 // does not fit the instruction caches: a CTA that goes from one output to the next is 1.4 times slower than the others, and so
 // are two CTAs on neighbouring SMs, which are two of consecutive numbers, that work on different ones; hence even bounds.
+// No output has more than `most` of them.
 template <int O, int (*COST)(int)>
-__device__ __forceinline__ void ts_ctas(int ctas, int& from, int& to) {
+__device__ __forceinline__ void ts_ctas(int ctas, int most, int& from, int& to) {
     int total = 0, outputs = 0;
     sfor<0, N_OUT>([&](auto o_) {
         constexpr int cost = COST(o_);
@@ -49,12 +50,13 @@ __device__ __forceinline__ void ts_ctas(int ctas, int& from, int& to) {
             }
         });
     }
+    to = to - from < most ? to : from + most;
 }
 template <int O, int ROWS, int (*COST)(int)>
-__device__ __forceinline__ void ts_deal(long long batch, int cta, int ctas, int& lo, int& hi) {
+__device__ __forceinline__ void ts_deal(long long batch, int cta, int ctas, int most, int& lo, int& hi) {
     const long long tiles = (batch + ROWS - 1) / ROWS;
     int from, to;
-    ts_ctas<O, COST>(ctas, from, to);
+    ts_ctas<O, COST>(ctas, most, from, to);
     const bool mine = cta >= from && cta < to;
     lo = mine ? (int)(tiles * (cta - from) / (to - from)) : 0;
     hi = mine ? (int)(tiles * (cta - from + 1) / (to - from)) : 0;

@@ -29,10 +29,11 @@ struct UvwTsDwParams {
     const float* X;
     const float* Y;
     const float* dZ;
-    float* ws;                  // [gridDim.x][W_NUMEL] partial weight gradients; a CTA writes those of the outputs it works on
+    float* ws;                  // [most][W_NUMEL] partial weight gradients: CTA n of those of an output writes that output's part of [n]
     long long batch;
     int* status;
     int in_vec;                 // X, Y and dZ start on a 16-byte boundary
+    int most;                   // CTAs of an output at most
 };
 
 constexpr int TG_ROWS = 8;                      // batch rows of a tile: the K of an MMA
@@ -199,7 +200,9 @@ template <int O>
 __device__ __forceinline__ void tg_store(const UvwTsDwParams& p, unsigned tmem_base, int set, int w, int lane) {
     constexpr int MW = OUT_MUL[O];
     if (set >= tg_mtiles(O)) return;
-    float* out = p.ws + (long long)blockIdx.x * W_NUMEL;
+    int from, to;
+    ts_ctas<O, tg_cost>(gridDim.x, p.most, from, to);
+    float* out = p.ws + (long long)((int)blockIdx.x - from) * W_NUMEL;
     const int slice = 4 * set + (w & 3);
 #pragma unroll 1
     for (int w0 = 16 * (w >> 2); w0 < MW; w0 += 32) {
@@ -430,7 +433,7 @@ __device__ void uvw_ts_dw(const UvwTsDwParams& p) {
         constexpr int O = o_;
         if constexpr (ts_slices(O) > 0) {
             int lo, hi;
-            ts_deal<O, TG_ROWS, tg_cost>(p.batch, blockIdx.x, gridDim.x, lo, hi);
+            ts_deal<O, TG_ROWS, tg_cost>(p.batch, blockIdx.x, gridDim.x, p.most, lo, hi);
             if (lo < hi) {
                 const TgBars bars(smem, O);
                 if (warp < TG_PW) {
@@ -459,10 +462,10 @@ __device__ void uvw_ts_dw(const UvwTsDwParams& p) {
 
 extern "C" __global__ void __launch_bounds__(oeq::TG_THREADS, 1) oeq_uvw_ts_dw_kernel(const oeq::UvwTsDwParams p) { oeq::uvw_ts_dw(p); }
 
-// Fixed-order sum of the partial weight gradients of `ctas` CTAs.  A weight's output irrep has the tiles of CTAs [from, to); with fewer
-// tiles than those, tile j is CTA from + ceil((j + 1) n / tiles) - 1's.  Bound by the latency of the loads, eight in flight: with every
+// Fixed-order sum of the partial weight gradients of the CTAs.  A weight's output irrep has n of them; with fewer tiles than those,
+// tile j is CTA ceil((j + 1) n / tiles) - 1's.  Bound by the latency of the loads, eight in flight: with every
 // CTA's run looked up by a thread of every block it took 8.7 us at 1 000 rows, now 7.1, and 5.4 / 3.5 at 20.
-extern "C" __global__ void __launch_bounds__(256) oeq_ts_reduce(const float* __restrict__ ws, float* __restrict__ out, long long batch, int ctas) {
+extern "C" __global__ void __launch_bounds__(256) oeq_ts_reduce(const float* __restrict__ ws, float* __restrict__ out, long long batch, int ctas, int most) {
     using namespace oeqd;
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
@@ -474,14 +477,17 @@ extern "C" __global__ void __launch_bounds__(256) oeq_ts_reduce(const float* __r
     oeq::sfor<0, N_OUT>([&](auto o_) {
         constexpr int O = o_;
         if constexpr (oeq::ts_slices(O) > 0)
-            if (o == O) oeq::ts_ctas<O, oeq::tg_cost>(ctas, from, to);
+            if (o == O) oeq::ts_ctas<O, oeq::tg_cost>(ctas, most, from, to);
     });
     const long long all = (batch + oeq::TG_ROWS - 1) / oeq::TG_ROWS;
     const int n = to - from, tiles = all < n ? (int)all : n;
     float s = 0.f;
-    if (i < W_NUMEL) {
+    if (i < W_NUMEL && tiles == n) {
 #pragma unroll 8
-        for (int j = row; j < tiles; j += 8) s += ws[(long long)(from + (tiles == n ? j : ((j + 1) * n + tiles - 1) / tiles - 1)) * W_NUMEL + i];
+        for (int j = row; j < tiles; j += 8) s += ws[(long long)j * W_NUMEL + i];
+    } else if (i < W_NUMEL) {
+#pragma unroll 8
+        for (int j = row; j < tiles; j += 8) s += ws[(long long)(((j + 1) * n + tiles - 1) / tiles - 1) * W_NUMEL + i];
     }
     part[row][lane] = s;
     __syncthreads();

@@ -371,7 +371,7 @@ __device__ void uvw_ts_forward(const UvwTsParams& p) {
         constexpr int O = o_;
         if constexpr (ts_slices(O) > 0) {
             int lo, hi;
-            ts_deal<O, TS_ROWS, ts_cost>(p.batch, blockIdx.x, gridDim.x, lo, hi);
+            ts_deal<O, TS_ROWS, ts_cost>(p.batch, blockIdx.x, gridDim.x, gridDim.x, lo, hi);
             if (lo < hi) {
                 const TsBars bars(smem, O);
                 // (the output before is complete: its shared and tensor memory are free)

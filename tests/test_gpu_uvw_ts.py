@@ -99,6 +99,36 @@ def test_weight_gradient_kernels_by_rows(irreps, rows):
     assert torch.equal(tp.backward_helper(*args)[2], dw)
 
 
+@pytest.mark.parametrize("rows", [20, 100, 1000])
+@pytest.mark.parametrize("irreps", [SHAPES["even"], SHAPES["seven"], ("64x0e", "0e", "64x0e")], ids=["even", "seven", "one"])
+def test_weight_gradient_in_the_least_workspace(irreps, rows):
+    """The order of the sums does not depend on how many partial weight gradients the workspace holds."""
+    p = oeq.FullyConnectedTPProblem(*irreps)
+    tp = oeq.TensorProduct(p)
+    x, y, w, dz = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in tp_inputs(p, rows, 19))
+    grads = [torch.empty_like(t) for t in (x, y, w)]
+    stream, stated = torch.cuda.current_stream().cuda_stream, tp.internal.workspace_bytes(rows)
+    ws = torch.empty(stated, dtype=torch.uint8, device="cuda")
+
+    def gradient(size):
+        tp.internal.backward(rows, *(t.data_ptr() for t in (x, y, w, dz, *grads, ws)), size, stream)
+        return grads[2].clone()
+
+    want, part = gradient(stated), p.weight_numel * 4
+    accepted = []
+    for n in range(1, stated // part):
+        try:
+            got = gradient(n * part)
+        except RuntimeError as e:
+            assert "workspace too small" in str(e) and not accepted
+            continue
+        assert torch.equal(got, want)
+        accepted.append(n)
+        if len(accepted) == 3:
+            break
+    assert accepted and accepted[0] <= (rows + 3) // 4
+
+
 @pytest.mark.parametrize("few", [32, 64, 96])
 def test_fewer_slices_than_producer_sets(few, monkeypatch):
     """An output of one to three slices of input channels: producer sets without a slice in a tile read its inputs too.  Hundreds
