@@ -42,21 +42,26 @@ constexpr int TG_ROOM = 222 * 1024;              // shared memory for operands a
 constexpr int TG_PW = TG_SETS * TG_SET, TG_BW = 4, TG_THREADS = (TG_PW + TG_BW + 1) * 32;
 // Runs of tiles that the MMAs sum in one accumulator: an MMA adds to it less exactly than a rounded sum, and the error grows with the
 // length of a chain.  After a run the accumulators are added to sums, in tensor memory too, while the MMAs go on in others.  The
-// boundaries are those of the row ranges that the CTAs of uvw_tc_bwd_kernels.cuh have, so that no chain is longer than there and the
-// two kernels round much alike: relative errors at 5 000 / 20 000 / 100 000 rows 6.5e-7 / 2.4e-6 / 1.2e-5, there 7.8e-7 / 2.8e-6 /
-// 1.4e-5, and 4.8e-6 between the two at 100 000.  (Runs of 40 / components tiles, with lo.hi beside hi.lo, cost the same and are
-// 7.8e-7 off at 100 000, but then 1.3e-5 from the other kernel.)
+// boundaries are those of the row ranges that the CTAs of uvw_tc_bwd_kernels.cuh have, so that the two kernels round much alike; ranges of
+// more than TG_CHAIN tiles are cut into equal runs, so that the error does not go on growing.  64x(0e+1o+2e) with 0e+1o+2e, relative
+// errors at 5 000 / 20 000 / 100 000 / 400 000 rows: 6.5e-7 / 2.4e-6 / 6.2e-6 / 8.6e-6, with whole ranges 6.5e-7 / 2.4e-6 / 1.2e-5 / 4.7e-5.
+// (Runs of 40 / components tiles, with lo.hi beside hi.lo, cost the same and are 7.8e-7 off at 100 000 rows, but then 1.3e-5 from
+// the wider kernel.)
+constexpr unsigned TG_CHAIN = 64;
 struct TgSegments {
     int i, next;                                // the next boundary
     static __device__ unsigned tiles(long long batch) { return (unsigned)((batch + TG_ROWS - 1) / TG_ROWS); }
-    static __device__ unsigned parts(long long batch) { return min((tiles(batch) + 3) / 4, gridDim.x); }
+    static __device__ unsigned parts(long long batch) {         // each range in equal runs
+        const unsigned t = tiles(batch), ranges = min((t + 3) / 4, gridDim.x);
+        return ranges * ((t + ranges * TG_CHAIN - 1) / (ranges * TG_CHAIN));
+    }
     __device__ TgSegments(long long batch, int tile_lo) : i((unsigned)tile_lo / (tiles(batch) / parts(batch) + 1)) {
         do advance(batch); while (next <= tile_lo);
     }
     __device__ void advance(long long batch) {  // boundary i of all: tiles * i / parts
         const unsigned t = tiles(batch), p = parts(batch);
         ++i;
-        next = (int)(i * (t / p) + i * (t % p) / p);
+        next = (int)(i * (t / p) + (unsigned)((unsigned long long)i * (t % p) / p));
     }
     __device__ int count(long long batch, int tile_hi) {        // segments of the CTA's run
         int n = 1;

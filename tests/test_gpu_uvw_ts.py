@@ -99,6 +99,24 @@ def test_weight_gradient_kernels_by_rows(irreps, rows):
     assert torch.equal(tp.backward_helper(*args)[2], dw)
 
 
+def test_weight_gradient_of_many_rows():
+    """The chains of additions within an accumulator have a length that does not grow with the batch."""
+    p = oeq.FullyConnectedTPProblem("64x2e", "0e", "64x2e")
+    tp = oeq.TensorProduct(p, torch_op=True)
+    rows, want = 600_000, 0
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x, y, w, dz = (torch.randn(*s, device="cuda", generator=gen)
+                   for s in ((rows, p.irreps_in1.dim), (rows, 1), (p.weight_numel,), (rows, p.irreps_out.dim)))
+    dw = to_e3nn(p, tp.backward_helper(x, y, w, dz)[2].cpu().numpy())
+    tp.check_device_status()
+    for part in range(0, rows, 50_000):
+        s = slice(part, part + 50_000)
+        want = want + torch.einsum("buk,bwk->uw", (x[s].double() * y[s].double()).unflatten(1, (64, 5)), dz[s].double().unflatten(1, (64, 5)))
+    want = want.flatten().cpu().numpy() * p.instructions[0].path_weight / np.sqrt(5)        # (the coefficients of 2e x 0e are 1 / sqrt(5))
+    # 320 additions a chain, each off by at most 2^-23 of the sum so far, against 2 500 in a CTA's share of the rows (9e-5 measured)
+    assert rel_err(dw, want) < 320 * 2 ** -23
+
+
 @pytest.mark.parametrize("rows", [20, 100, 1000])
 @pytest.mark.parametrize("irreps", [SHAPES["even"], SHAPES["seven"], ("64x0e", "0e", "64x0e")], ids=["even", "seven", "one"])
 def test_weight_gradient_in_the_least_workspace(irreps, rows):
