@@ -88,6 +88,7 @@ TC_SHAPES = [
     ("32x1o+96x2e", "1o+2e+3o", "64x0e+16x1o+32x3o", 130),              # l = 3 output: 7 accumulator rows per batch row
     ("8x0e+8x1o", "0e+1o", "128x0e", 50),                                # wide N, very short K
 ]
+TC_STAGES = {TC_SHAPES[0][0]: 4, TC_SHAPES[1][0]: 2, TC_SHAPES[2][0]: 4, TC_SHAPES[3][0]: 2}      # four: weights in tensor memory
 
 
 @pytest.mark.parametrize("in1,in2,out,batch", TC_SHAPES, ids=[s[2] for s in TC_SHAPES])
@@ -97,6 +98,7 @@ def test_tensor_core_forward_matches_oracle_and_fma_path(in1, in2, out, batch, m
     p = oeq.FullyConnectedTPProblem(in1, in2, out)
     tp = oeq.TensorProduct(p, torch_op=True)
     assert tp.internal.launch_info(0)["threads"] == 21 * 32       # tensor-core kernel selected
+    assert tp.internal.launch_info(0)["stages"] == TC_STAGES[in1]
     x, y, w, dz = tp_inputs(p, batch, 21)
     w = (w / np.sqrt(max(1, p.weight_numel / len(p.instructions)))).astype(np.float32)
     xt, yt, wt = (torch.from_numpy(a).cuda() for a in (x, y, to_oeq(p, w)))
@@ -150,6 +152,7 @@ def test_tensor_core_forward_many_tiles_mixed_multiplicities(in1, in2, out, batc
     p = oeq.FullyConnectedTPProblem(in1, in2, out)
     tp = oeq.TensorProduct(p, torch_op=True)
     assert tp.internal.launch_info(0)["threads"] == 21 * 32
+    assert tp.internal.launch_info(0)["stages"] == TC_STAGES[in1]
     x, y, w, _ = tp_inputs(p, batch, 23)
     w = (w / np.sqrt(max(1, p.weight_numel / len(p.instructions)))).astype(np.float32)
     xt, yt, wt = (torch.from_numpy(a).cuda() for a in (x, y, to_oeq(p, w)))

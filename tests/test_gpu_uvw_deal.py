@@ -1,4 +1,5 @@
-"""Shared-weight FP32 'uvw': batches whose chunks of rows are dealt over the CTAs for all output irreps together.  A row's
+"""Shared-weight FP32 'uvw' with the weights in shared memory (W dZ of every problem; the forward pass of some, two operand stages):
+batches whose chunks of rows are dealt over the CTAs for all output irreps together.  A row's
 sums do not depend on the CTA that forms them, so the rows of a dealt batch have the bits of the same rows in batches that
 are too small to be dealt, and the latter are held against the oracle."""
 import numpy as np
@@ -15,15 +16,17 @@ PER_SM = 160        # rows per SM up to which a batch is dealt (more than 32 inp
 
 
 @pytest.mark.parametrize("rows", [1177, 1200, 4001, PER_SM * 148, PER_SM * 148 + 1, 200 * 148])
-@pytest.mark.parametrize("irreps", [("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"),
-                                    ("16x0e+48x1o", "0e+1o", "32x0e+16x1o+48x2e+16x4e")],   # (4e: no paths)
-                         ids=["even", "uneven"])
-def test_dealt_rows(irreps, rows):
+@pytest.mark.parametrize("irreps,stages", [(("64x0e+64x1o+64x2e", "0e+1o+2e", "64x0e+64x1o+64x2e"), 4),
+                                           (("16x0e+48x1o", "0e+1o", "32x0e+16x1o+48x2e+16x4e"), 2),   # (4e: no paths)
+                                           (("64x0e+64x1o", "0e+1o", "96x0e+16x1o+16x4e"), 2)],
+                         ids=["even", "uneven", "wide"])
+def test_dealt_rows(irreps, stages, rows):
     p = oeq.FullyConnectedTPProblem(*irreps)
     x, y, w, dz = tp_inputs(p, rows, 5)
     w = (w / 8).astype(np.float32)
     dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, y, to_oeq(p, w), dz)]
     tp = oeq.TensorProduct(p, torch_op=True)
+    assert tp.internal.launch_info(0)["stages"] == stages
     got = [tp(*dev[:3]), *tp.backward_helper(*dev)[:2]]
     blocks = [(0, 200), (rows // 2, rows // 2 + 300), (rows - 41, rows)]
     for lo, hi in blocks:

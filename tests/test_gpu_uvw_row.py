@@ -81,6 +81,9 @@ def test_staged_rows(irreps, batch, offset, dtype):
     for got, ref in zip((z, dx, dy), want):
         assert rel_err(got.cpu().numpy()[some], ref) < REL_TOL[dtype]
     assert rel_err(to_e3nn(p, dw.cpu().numpy()[some]), want[3]) < REL_TOL[dtype]
+    # (a CTA has two rows' weights in shared memory; two such CTAs have to fit an SM, and those of 'docking' in FP64 do not)
+    staged = [tp.internal.launch_info(which)["smem_bytes"] >= 2 * p.weight_numel * np.dtype(dtype).itemsize for which in (0, 1)]
+    assert staged == [not (irreps is STAGED[2] and dtype is np.float64)] * 2
     again = (tp(x, y, w), *tp.backward_helper(x, y, w, dz))         # every row, not only those compared: the same bits
     for a, b in zip((z, dx, dy, dw), again):
         assert torch.equal(a, b)

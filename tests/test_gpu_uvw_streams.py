@@ -12,11 +12,15 @@ from helpers import tp_inputs, to_oeq
 pytestmark = pytest.mark.gpu
 
 
+# (with 0e: weights packed for the forward pass too, in FP32)
+@pytest.mark.parametrize("in2", ["0e+1o", "0e"])
 @pytest.mark.parametrize("entry", ["op", "python"])
 @pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
-def test_overlapping_calls(dtype, entry):
-    p = oeq.FullyConnectedTPProblem("64x0e+64x1o", "0e+1o", "64x0e+64x1o", irrep_dtype=dtype, weight_dtype=dtype)
+def test_overlapping_calls(dtype, entry, in2):
+    p = oeq.FullyConnectedTPProblem("64x0e+64x1o", in2, "64x0e+64x1o", irrep_dtype=dtype, weight_dtype=dtype)
     tp = oeq.TensorProduct(p, torch_op=True)
+    if dtype is np.float32:
+        assert (tp.internal.forward_workspace_bytes() > 0) == (in2 == "0e")
     forward, backward = (tp.forward, tp.backward_helper) if entry == "op" else (tp._forward_impl, tp._backward_impl)
     inputs = []
     for seed in range(4):
