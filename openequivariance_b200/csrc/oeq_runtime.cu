@@ -1760,7 +1760,7 @@ bool uvw_row_supported(const Problem& p) {
 
 // Rows per SM up to which the row kernel is the faster one (0: always).  It pays a CTA's barriers and phases per row, the
 // tiled kernel shares them among 16 rows; with few weights a row that is what counts once every SM has rows enough.
-// Measured, tiled against row kernel in us (30 000 rows unless stated, second input 0e+1o...):
+// Measured, tiled against row kernel in us (30 000 rows unless stated, second input 0e+1o..., rows that are not staged):
 //   forward: FP32 by the input channels of all paths: 8x(0e+1o) (32) 51 / 84, 12x(0e+1o) (48) 121 / 141, 8 -> 64 channels (32)
 //     74 / 102, but 16x(0e+1o) (64) 225 / 127, 4x(0e..3o) (136) 199 / 174; 2 000 rows 12 / 12 and 14 / 16.  FP64, whose tiled
 //     kernel is slower: 1x(0e+1o) (4) 20 / 45, but 4x(0e+1o) (16) 74 / 66; one tile of output channels keeps one warp of eight
@@ -1768,6 +1768,8 @@ bool uvw_row_supported(const Problem& p) {
 //   backward: by the weights per path: FP32 4x(0e+1o) (16) 53 / 123, 4x(0e..3o) (16) 657 / 1000, 8x(0e+1o+2e) (64) 260 / 299,
 //     but 12x(0e+1o) (144) 215 / 131; FP64 4x(0e..3o) 961 / 3029 (1 000 rows 92 / 123), 8x(0e+1o+2e) (64) 668 / 897 (2 000 rows
 //     57 / 70, 1 000 rows 55 / 41), but without l = 2 8x(0e+1o) (64) 221 / 154; fewer than eight output channels leave most lanes idle: 128x0e -> 4x0e 88 / 113.
+// Staged rows (below) are faster than that, and the lines stand where they stood: 30 000 rows forward FP32 8x(0e+1o) 50 / 35, 12x 118 / 41,
+//   4x 34 / 35, FP64 128x0e with 4x0e -> 4x0e 809 / 97; backward FP32 8x 92 / 72, the latter 346 / 158, but 4x 51 / 73; FP64 4x(0e..3o) 953 / 1061.
 int uvw_row_limit(const Problem& p, bool bwd) {
     long long uv = 0, tiles = 0;
     int dim = 1, width = 0;
@@ -1787,6 +1789,9 @@ int uvw_row_limit(const Problem& p, bool bwd) {
 
 // Staged rows (uvw_row_kernels.cuh): bulk copies want rows of whole 16-byte pieces, and two stages have to leave room for a
 // second CTA on an SM.  Shared memory of a CTA, 0 where a row does not qualify.
+// Loads where a weight is used / staged, us, 2 011 rows: forward 4x(0e+1o) with 0e+1o 6.5 / 6.4, 32x 24 / 10, 16x(0e+1o) with 4x(0e+1o) 70 / 12, FP64 32x 39 / 15;
+// backward 4x 8.4 / 8.4, 32x 18.8 / 16.7, 8x(0e..3o) with 0e..3o 87 / 47, FP64 16x 21 / 13, 32x0e with 4x0e 23 / 21.  30 shapes at 20 to 30 000 rows:
+// none slower by more than a microsecond or 2 % (FP64 32x0e with 4x0e, backward, 30 000 rows 325 / 331).
 constexpr int K_UVW_STAGED_FWD = 14, K_UVW_STAGED_BWD = 15, UVW_STAGED_BYTES = (228 * 1024) / 2 - 1024;
 constexpr int UVW_STAGED_UNITS = 256;      // (the compiler deals them)
 

@@ -15,9 +15,10 @@
 // products there, and rows of X and dZ are read from memory with a stride of 2l+1 values.
 // Every wait is bounded; on expiry the role records a code in *status and goes through the rest of its barriers without
 // work, and the CTA frees its tensor memory.
-// Measured, 64x(0e+1o+2e) with 0e+1o+2e, without the sum over CTAs, uvw_tc_bwd_kernels.cuh / this kernel: 100 000 rows 498 / 372 us,
-// 8 000 69 / 55, 1 000 55 / 30, but 20 rows 13 / 23.  At 30 000 rows issue slots are busy for
-// 53 %, the load and store unit for 41 %, the tensor pipe for 20 %; waits at barriers are the rest.
+// Measured, 64x(0e+1o+2e) with 0e+1o+2e, calls with the sum over CTAs, uvw_tc_bwd_kernels.cuh / this kernel: 100 000 rows 517 / 380 us, 10 000
+// 99 / 73, 1 000 65 / 40, but 500 rows 24 / 38 and 20 rows 20 / 32, which the wider kernel therefore takes, as it does many rows of scalar outputs
+// (uvw_dw_choice in the runtime).  At 30 000 rows issue slots are busy for 53 %, the load and store unit for 41 %, the tensor pipe for
+// 20 %; waits at barriers are the rest.
 #pragma once
 #include "oeq_common.cuh"
 #include "uvw_ts_common.cuh"
