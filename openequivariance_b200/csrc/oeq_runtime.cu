@@ -1523,11 +1523,11 @@ bool uvw_ts_geometry(const Problem& p, int& smem) {
 // one slice of 32 input channels as for eight; the other kernel's producers read rows of X with a stride of 2 l + 1 values, slice by
 // slice, and its drain goes with the values of Z.
 // Measured, us for 100 000 rows, shared / tensor memory (at 1 000 rows; estimates tensor / shared):
-//   with 0e+1o+2e: 64x(0e+1o+2e) 413 / 268 (30 / 22; 0.72), 16x 194 / 189 (1.06), 48x(0e+1o+2e) to 64x0e 120 / 66 (0.68)
-//   with 0e+1o: 64x(0e+1o+2e) 227 / 204 (0.84), 64x(0e+1o) 105 / 110 (15.3 / 10.6; 1.07), 16x 52 / 90 (13.3 / 10.2; 1.95)
+//   with 0e+1o+2e: 64x(0e+1o+2e) 413 / 272 (30 / 23; 0.72), 16x 194 / 183 (1.06), 48x(0e+1o+2e) to 64x0e 120 / 66 (0.68)
+//   with 0e+1o: 64x(0e+1o+2e) 237 / 209 (0.84), 64x(0e+1o) 106 / 109 (15.3 / 10.6; 1.07), 16x 52 / 90 (13.3 / 10.2; 1.95)
 //   with 0e: 256x1o to 64x1o 124 / 94 (0.72), 96x 64.5 / 63.5 (0.98), 64x 56.3 / 57.3 (15.3 / 10.2; 1.13); 256x0e to 64x0e 61 / 61 (17.5 /
 //     12.3; 1.16), 128x0e 36 / 49 (15.3 / 10.2; 1.55), 32x0e to 32x0e 19.4 / 37.5 (13.3 / 10.2; 3.8); 64x(0e+1o+2e) 136 / 171 (1.13)
-// Up to 1.1 this kernel loses at most 4 % at 100 000 rows (none below 30 000) and is 15 to 45 % faster below 4 000.
+// Up to 1.1 this kernel loses at most 3 % at 100 000 rows, none up to 30 000, and is 4 to 47 % faster up to 4 000.
 bool uvw_ts_faster(const Problem& p) {
     long long tensor = 0, shared = 0;
     std::vector<bool> used(p.out.size());

@@ -18,8 +18,8 @@
 // Every wait is bounded; on expiry the role records a code in *status and goes through the rest of its barriers without
 // work, and the CTA frees its tensor memory.
 // Measured against uvw_tc_kernels.cuh (weights in shared memory, which then has no room for rows of X), 64x(0e+1o+2e) with
-// 0e+1o+2e, calls from a cold cache, with the packing of the weights: 100 000 rows 453 -> 267 us, 20 000 120 -> 71, 4 000 46 -> 31,
-// 1 000 34 -> 23, 20 rows 38 -> 24; relative error against 64 bits 1.2e-6 -> 6.2e-7 (hi.lo has accumulators of its own).  Problems of few
+// 0e+1o+2e, calls from a cold cache, with the packing of the weights: 100 000 rows 413 -> 272 us, 10 000 67 -> 46, 4 000 44 -> 31,
+// 1 000 30 -> 23, 20 rows 33 -> 20; relative error against 64 bits 1.2e-6 -> 6.2e-7 (hi.lo has accumulators of its own).  Problems of few
 // slices of input channels are slower here and keep the other kernel (uvw_ts_faster in the runtime).
 // Bound by shared memory: per batch row 140 cycles of T's stores, 140 of the MMAs reading it, 80 of x and y, 72 of the epilogue
 // and 54 of the input copies, and conflicts between them, of 700; the tensor pipe is busy for 37 %, issue slots for 42 %.
