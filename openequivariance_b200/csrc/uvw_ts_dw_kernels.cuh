@@ -106,7 +106,9 @@ struct TgBars {
     }
 };
 
-// Time of a tile.  Measured, 64x(0e+1o+2e) with 0e+1o+2e: 2 150, 2 930 and 3 370 cycles for 6, 8 and 8 slices of 1, 3 and 5 components.
+// Time of a tile.  Measured, 64x(0e+1o+2e) with 0e+1o+2e: 2 150, 2 930 and 3 370 cycles for 6, 8 and 8 slices of 1, 3 and 5 components; with 0e,
+// one output, 1 / 2 / 4 slices: 1 100-1 400 / 1 300 / 1 400-1 550 of one component, 1 300-1 600 / 1 600 / 2 050 of three, 1 500 / 1 800 / 2 250 of five (up to a third
+// less than the estimate, but alike for the outputs of a problem: none of 18 with several outputs is slower than in the wider kernel for it).
 constexpr int tg_cost(int o) { return ts_slices(o) ? 22 * OUT_D[o] + 15 * ts_slices(o) + 103 : 0; }
 
 // matrix descriptor: MN-major, 128-byte rows with 32-byte atoms; blocks of 32 channels `block` bytes apart, four rows 512 bytes
